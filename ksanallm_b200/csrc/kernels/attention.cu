@@ -12,11 +12,13 @@
 // Prefill: 64 rows per CTA (4 warps x 16), K/V tiles of 64 tokens, online
 // softmax in fp32 (exp2), only the NEW query rows are computed: the causal
 // offset is kv_len - q_len, so cached prefixes cost no attention work.
-// Decode: one CTA per (kv head, sequence, split); the 4 warps walk disjoint
-// 16-token slices of each tile, partial (m, l, O) are merged in shared memory
-// and, when the sequence was split, by a small reduce kernel.
+// Decode: all (sequence, kv head, tile) units of a launch lie in one line that is cut into equal ranges, one per
+// resident CTA (paged_decode_stream_kernel); 4 warps walk disjoint 16-token slices of each tile, a fifth keeps the
+// tile ring full by TMA. Caches that TMA cannot read (other block sizes or strides) take paged_decode_kernel: one
+// CTA per (kv head, sequence, split), all threads copying, and a small reduce kernel.
 //
-// FP8 (e4m3) caches are dequantised with a per-layer scale while staging tiles.
+// FP8 (e4m3) caches: the decode kernel multiplies the stored values in f16 (exact) and applies the per-layer scales
+// to scores and outputs; the other kernels dequantise while staging tiles.
 //
 // Head sizes: a kernel is compiled for a padded head size DP (64, 128, 192, 256); the real query/key size D and value
 // size Dv are run-time values up to DP (multiples of 8), padded with zeros in shared memory only (TMA fills the
@@ -34,8 +36,9 @@
 #include "sm100_ptx.cuh"
 #include "pdl.cuh"
 #include "fp8_scale.cuh"
-#include <cuda_fp8.h>
+#include <atomic>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_fp8.h>
 #include <stdint.h>
 
@@ -44,7 +47,7 @@ namespace ksana {
 // K/V staging modes: plain cp.async (any block size), FP8 cache with conversion, or TMA: one elected thread
 // issues a 2-D bulk tensor copy per (cache block, 64-column half) - the per-16-byte address arithmetic of
 // the cp.async path made the decode kernel instruction-bound at a third of HBM bandwidth.
-enum KvMode { kKvCpAsync = 0, kKvFp8 = 1, kKvTma = 2 };
+enum KvMode { kKvCpAsync = 0, kKvFp8 = 1, kKvTma = 2, kKvTmaFp8 = 3 };
 
 typedef __nv_bfloat16 bf16;
 constexpr int kTileTok = 64;     // KV tokens per shared-memory tile
@@ -80,6 +83,10 @@ struct AttnParams {
   float k_scale, v_scale;                // fp8 cache dequant scales
   // decode split workspace
   float* part_o; float* part_ml; int num_splits;
+  // stream decode: tile ring, partial results of cut (sequence, head) items [2 * CTAs][rows][Dv] and [2 * CTAs][rows][2],
+  // arrival counters [B * heads] (zero before and after every launch)
+  int B, stages, stage_bytes, rows, vec_out;
+  float* cut_o; float* cut_ml; unsigned int* counters;
   int* err;                              // device word set when a bounded wait gave up
   // decode, head dim 128: also emit the output as the FP8 operand of the next GEMM (e4m3 values [T][Hq*D] and one
   // power-of-two scale per row and head, [Hq][oscale_ld]), quantised from the bf16-rounded values exactly as the
@@ -269,18 +276,19 @@ __device__ __forceinline__ void warp_pv(float (&o)[D / 8][4], const float (&s)[N
 // Mask + online-softmax update for one warp's 16 x (NT*8) score tile.
 // Rows lane/4 and lane/4+8; limit[i] = last visible kv position of that row (-1 = row inactive), lo[i] = first position
 // inside its window (tokens below `keep` are seen as well).
-template <int D, int NT>
+// PERM: column 2t + e of an 8-token group is token t + 4e (the FP8 form's order).
+template <int D, int NT, bool PERM = false>
 __device__ __forceinline__ void softmax_update(float (&s)[NT][4], float (&o)[D / 8][4], float (&m)[2], float (&l)[2],
                                                const int (&limit)[2], const int (&lo)[2], int keep, const float (&slope)[2],
-                                               int tok0, int lane, float scale_log2) {
+                                               int tok0, int lane, const float (&scale_log2)[2]) {
   float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int i = e >> 1;
-      const int tok = tok0 + j * 8 + (lane & 3) * 2 + (e & 1);
-      float v = s[j][e] * scale_log2;
+      const int tok = tok0 + j * 8 + (PERM ? (lane & 3) + (e & 1) * 4 : (lane & 3) * 2 + (e & 1));
+      float v = s[j][e] * scale_log2[i];
       if (slope[i] != 0.f) v += slope[i] * 1.44269504f * static_cast<float>(tok - limit[i]);
       v = (tok <= limit[i] && (tok >= lo[i] || tok < keep)) ? v : -INFINITY;
       s[j][e] = v;
@@ -300,8 +308,10 @@ __device__ __forceinline__ void softmax_update(float (&s)[NT][4], float (&o)[D /
     m[i] = mnew[i];
     l[i] *= corr[i];
   }
+  if (__any_sync(0xffffffffu, corr[0] != 1.f || corr[1] != 1.f)) {      // most tiles leave every row's maximum as it was
 #pragma unroll
-  for (int n = 0; n < D / 8; ++n) { o[n][0] *= corr[0]; o[n][1] *= corr[0]; o[n][2] *= corr[1]; o[n][3] *= corr[1]; }
+    for (int n = 0; n < D / 8; ++n) { o[n][0] *= corr[0]; o[n][1] *= corr[0]; o[n][2] *= corr[1]; o[n][3] *= corr[1]; }
+  }
 #pragma unroll
   for (int j = 0; j < NT; ++j) {
 #pragma unroll
@@ -429,6 +439,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
 #pragma unroll
   for (int n = 0; n < D / 8; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+  const float sl2[2] = {p.scale_log2, p.scale_log2};
 
   bool ok = true;
   for (int t = 0; t < ntiles; ++t) {
@@ -444,7 +455,7 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
     float sc[8][4];
     warp_qk<D, 8>(sc, qf, ks + buf * kTileTok * D, 0, lane);
     if constexpr (SIG) sigmoid_weights<8>(sc, limit, lo, p.keep, bias, p.bias_len - 1, tok0, lane, p.scale_log2);
-    else softmax_update<D, 8>(sc, o, m, l, limit, lo, p.keep, slope, tok0, lane, p.scale_log2);
+    else softmax_update<D, 8>(sc, o, m, l, limit, lo, p.keep, slope, tok0, lane, sl2);
     warp_pv<D, 8>(o, sc, vs + buf * kTileTok * D, 0, lane);
   }
   if (!ok) {                      // a bounded wait gave up: leave the output untouched, report through the error word
@@ -479,17 +490,15 @@ paged_prefill_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_con
   }
 }
 
-// ------------------------------------------------------------------------------ decode
+// ------------------------------------------------------------------------------ decode, caches that TMA cannot read
 // grid (Hkv x row groups, B, splits). Rows = up to 16 of the G query heads of kv head g, one new token each.
 template <int D, int MODE, bool SIG>
 __global__ void __launch_bounds__(kAttnThreads)
-paged_decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const AttnParams p) {
+paged_decode_kernel(const AttnParams p) {
   constexpr bool FP8 = MODE == kKvFp8;
   constexpr int kKvStages = kv_stages(D);
   extern __shared__ uint8_t smem_attn_raw[];
   uint8_t* smem_attn = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_attn_raw) + 1023) & ~uintptr_t(1023));
-  __shared__ uint64_t full_bar[kKvStages];
-  __shared__ uint32_t abort_word;
   __shared__ float red4[4];
   bf16* qs = reinterpret_cast<bf16*>(smem_attn);            // 16 x D
   bf16* ks = qs + 16 * D;                                   // kKvStages x (64 x D)
@@ -523,19 +532,9 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
   float* bias_s = reinterpret_cast<float*>(ks + decode_ring(D, shared));
   if (SIG && p.bias_smem)
     for (int i = threadIdx.x; i < G * p.bias_len; i += kAttnThreads) bias_s[i] = p.bias[static_cast<size_t>(head0) * p.bias_len + i];
-  if (MODE == kKvTma && threadIdx.x == 0) {
-    for (int i = 0; i < kKvStages; ++i) mbar_init(&full_bar[i], 1);
-    abort_word = 0;
-    mbar_fence_init();
-  }
   __syncthreads();
   auto issue = [&](int t) {
     const int st = (t - t_begin) % kKvStages, tok0 = tile_at(tiles, t) * kTileTok;
-    if (MODE == kKvTma) {
-      if (threadIdx.x == 0 && t < t_end)
-        tma_issue_kv<D>(ks + st * kTileTok * D, vs + st * kTileTok * D, shared, &full_bar[st], &k_map, &v_map, p, table, g, tok0, kv_len);
-      return;
-    }
     if (t < t_end) {
       load_kv_tile<D, FP8>(ks + st * kTileTok * D, p, table, g, 0, tok0, kv_len, p.k_scale);
       if (!shared) load_kv_tile<D, FP8>(vs + st * kTileTok * D, p, table, g, 1, tok0, kv_len, p.v_scale);
@@ -568,29 +567,20 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
   float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
   if (SIG) { m[0] = m[1] = 0.f; }            // nothing is rescaled when partial sums are merged
 
-  bool ok = true;
+  const float sl2[2] = {p.scale_log2, p.scale_log2};
   for (int t = t_begin; t < t_end; ++t) {
     const int buf = (t - t_begin) % kKvStages, tok0 = tile_at(tiles, t) * kTileTok;
-    if (MODE == kKvTma) {
-      if (!mbar_wait(&full_bar[buf], ((t - t_begin) / kKvStages) & 1, &abort_word)) { ok = false; break; }
-      zero_v_tail<D>(vs + buf * kTileTok * D, kv_len - tok0);
-    } else {
-      cp_wait<kKvStages - 2>();
-    }
+    cp_wait<kKvStages - 2>();
     __syncthreads();
     issue(t + kKvStages - 1);
     float sc[2][4];
     warp_qk<D, 2>(sc, qf, ks + buf * kTileTok * D, warp * 16, lane);
     if constexpr (SIG) sigmoid_weights<2>(sc, limit, lo, p.keep, bias, p.bias_len - 1, tok0 + warp * 16, lane, p.scale_log2);
-    else softmax_update<D, 2>(sc, o, m, l, limit, lo, p.keep, slope, tok0 + warp * 16, lane, p.scale_log2);
+    else softmax_update<D, 2>(sc, o, m, l, limit, lo, p.keep, slope, tok0 + warp * 16, lane, sl2);
     warp_pv<D, 2>(o, sc, vs + buf * kTileTok * D, warp * 16, lane);
   }
   cp_wait<0>();
   __syncthreads();                // the merge area aliases the K ring: every warp must be out of the loop
-  if (!ok) {
-    if (threadIdx.x == 0 && p.err) atomicExch(p.err, 4);
-    return;
-  }
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
@@ -637,6 +627,483 @@ paged_decode_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_cons
       p.part_o[base * Dv + d] = acc;
       if (d == 0) { p.part_ml[base * 2] = mm; p.part_ml[base * 2 + 1] = ll; }
     }
+  }
+}
+
+// ------------------------------------------------------------------------------ decode, stream form
+// Bound by HBM (every K/V byte is read once). A grid of one CTA per (head, sequence, split) of equal split counts left
+// the longest sequences of a ragged batch and a nearly empty last wave to a few CTAs; here the units are cut evenly, whatever the
+// lengths, and an item (sequence, kv head row group) that lies in several CTAs' ranges is summed by the CTA that delivers
+// its last piece, so there is no second launch either. A warp of its own issues the TMA boxes (block table entries
+// read by its lanes in parallel), which took the table's latency out of the compute warps' path.
+constexpr int kStreamThreads = 160;      // 4 warps that compute, 1 that loads
+constexpr int kStreamMaxStages = 8;
+constexpr int kStreamMinTiles = 1;       // tiles per CTA below which fewer CTAs take part
+
+__device__ __forceinline__ void stream_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
+
+struct StreamItem { int s, h, t0, t1, n; };     // tiles [t0, t1) of the n tiles of sequence s, row group h
+
+// the item of unit u; `s` only ever moves forward
+__device__ __forceinline__ void stream_item(const int* first, int heads, long long u, long long end, int& s, StreamItem& it) {
+  while (static_cast<long long>(first[s + 1]) * heads <= u) ++s;
+  const int n = first[s + 1] - first[s];
+  const long long r = u - static_cast<long long>(first[s]) * heads;
+  it.s = s; it.n = n;
+  it.h = r < (1LL << 31) ? static_cast<int>(r) / n : static_cast<int>(r / n);
+  it.t0 = static_cast<int>(r - static_cast<long long>(it.h) * n);
+  const long long room = end - u;
+  it.t1 = room < n - it.t0 ? it.t0 + static_cast<int>(room) : n;
+}
+
+__device__ __forceinline__ TileRange decode_tiles(const AttnParams& p, int kv_len) {
+  return visited_tiles(p.window > 0 ? kv_len - p.window : 0, p.keep, (kv_len + kTileTok - 1) / kTileTok, kTileTok);
+}
+
+__device__ __forceinline__ void mma16816_f16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint32_t pack_f16(float a, float b) {
+  const __half2 v = __floats2half2_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+// four e4m3 values as two f16 pairs, exactly
+__device__ __forceinline__ void f16_of_e4m3(uint32_t w, uint32_t& low, uint32_t& high) {
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %2;\n\tcvt.rn.f16x2.e4m3x2 %0, l;\n\tcvt.rn.f16x2.e4m3x2 %1, h;\n\t}"
+      : "=r"(low), "=r"(high) : "r"(w));
+}
+// token of column i of an 8-token group: neighbours lie four rows apart, so that the 16-byte reads of eight lanes (two
+// tokens, four chunks each) fall on different banks of the 128-byte-swizzled tile
+__device__ __forceinline__ int perm8(int i) { return (i >> 1) | ((i & 1) << 2); }
+
+// One warp, FP8 tile (rows of 128 bytes): S(16 x 16 tokens) = Q K^T. The dimensions are taken in an order of their own: lane t of a
+// row holds dimensions 16 (4 h + t) + 4 w .. + 3 of step (h, w), which is what one 16-byte read of a key row gives.
+__device__ __forceinline__ void warp_qk_fp8(float (&s)[2][4], const uint32_t (&qf)[8][4], const uint8_t* ks, int t0, int lane) {
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+    const int r7 = perm8(lane >> 2);
+    const uint8_t* row = ks + (t0 + j * 8 + r7) * 128;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint4 v = *reinterpret_cast<const uint4*>(row + (((h * 4 + (lane & 3)) ^ r7) << 4));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        uint32_t b0, b1;
+        f16_of_e4m3(w[k], b0, b1);
+        mma16816_f16(s[j], qf[h * 4 + k], b0, b1);
+      }
+    }
+  }
+}
+
+// One warp, FP8 tile: O(16 x 128) += P(16 x 16 tokens) V. Pairs of dimensions travel as one 16-bit element through the transposing
+// load; o[2 c] holds the even and o[2 c + 1] the odd dimensions of chunk c: columns 4t, 4t + 2 and 4t + 1, 4t + 3.
+__device__ __forceinline__ void warp_pv_fp8(float (&o)[16][4], const float (&s)[2][4], const uint8_t* vs, int t0, int lane) {
+  const uint32_t a[4] = {pack_f16(s[0][0], s[0][1]), pack_f16(s[0][2], s[0][3]), pack_f16(s[1][0], s[1][1]), pack_f16(s[1][2], s[1][3])};
+  const int r7 = perm8(lane & 7);
+  const uint8_t* row = vs + (t0 + ((lane >> 3) & 1) * 8 + r7) * 128;
+#pragma unroll
+  for (int c2 = 0; c2 < 4; ++c2) {
+    uint32_t b[4];
+    ldsm_x4_t(b, smem_addr(row + (((c2 * 2 + (lane >> 4)) ^ r7) << 4)));
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      uint32_t e0, o0, e1, o1;
+      f16_of_e4m3(__byte_perm(b[2 * c], 0, 0x3120), e0, o0);
+      f16_of_e4m3(__byte_perm(b[2 * c + 1], 0, 0x3120), e1, o1);
+      mma16816_f16(o[(c2 * 2 + c) * 2], a, e0, e1);
+      mma16816_f16(o[(c2 * 2 + c) * 2 + 1], a, o0, o1);
+    }
+  }
+}
+
+// Four consecutive outputs of one head row (a warp per row, lane's columns d .. d + 3 of Dv); `q`: D = 128 as the next GEMM's FP8
+// operand, quantised from the bf16-rounded values exactly as the stand-alone quantiser would.
+template <int D, bool SIG>
+__device__ __forceinline__ void store_head_row4(const AttnParams& p, int s, int head, int d, float4 v) {
+  const bool on = d < p.Dv;
+  if (SIG && p.gate && on) {
+    const int col = head * p.Dv + d;
+    v.x *= gate_of(p, s, col); v.y *= gate_of(p, s, col + 1); v.z *= gate_of(p, s, col + 2); v.w *= gate_of(p, s, col + 3);
+  }
+  const uint2 w = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  if (p.out && on) {
+    bf16* dst = p.out + static_cast<size_t>(s) * p.out_stride + head * p.Dv + d;
+    if (p.vec_out) {
+      *reinterpret_cast<uint2*>(dst) = w;
+    } else {
+      dst[0] = __float2bfloat16(v.x); dst[1] = __float2bfloat16(v.y); dst[2] = __float2bfloat16(v.z); dst[3] = __float2bfloat16(v.w);
+    }
+  }
+  if constexpr (D == 128) {
+    if (p.outq) {                                                     // Dv = 128: every lane of the warp holds four columns
+      const float f[4] = {__uint_as_float(w.x << 16), __uint_as_float(w.x & 0xffff0000u), __uint_as_float(w.y << 16),
+                          __uint_as_float(w.y & 0xffff0000u)};
+      float am = fmaxf(fmaxf(fabsf(f[0]), fabsf(f[1])), fmaxf(fabsf(f[2]), fabsf(f[3])));
+#pragma unroll
+      for (int x = 16; x > 0; x >>= 1) am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, x));
+      const float sc = fp8_group_scale(am), inv = 1.f / sc;
+      uint32_t q = 0;
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        q |= static_cast<uint32_t>(__nv_cvt_float_to_fp8(f[e] * inv, __NV_SATFINITE, __NV_E4M3)) << (8 * e);
+      uint8_t* dst = p.outq + (static_cast<size_t>(s) * p.Hq + head) * 128 + d;
+      if (p.vec_out) {
+        *reinterpret_cast<uint32_t*>(dst) = q;
+      } else {
+        for (int e = 0; e < 4; ++e) dst[e] = static_cast<uint8_t>(q >> (8 * e));
+      }
+      if (d == 0) p.oscale[static_cast<size_t>(head) * p.oscale_ld + s] = sc;
+    }
+  }
+}
+
+template <int D, int MODE, bool SIG>
+__global__ void __launch_bounds__(kStreamThreads, D <= 128 ? 2 : 1)
+paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const AttnParams p) {
+  constexpr bool FP8 = MODE == kKvTmaFp8;
+  static_assert(!FP8 || (D == 128 && !SIG), "FP8 tiles have rows of 128 bytes");
+  constexpr int kTileBytes = kTileTok * D * (FP8 ? 1 : 2);
+  extern __shared__ uint8_t smem_attn_raw[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_attn_raw) + 1023) & ~uintptr_t(1023));
+  __shared__ uint64_t full_bar[kStreamMaxStages], empty_bar[kStreamMaxStages];
+  __shared__ uint32_t abort_word, last_piece;
+  __shared__ float ml_s[4][16][2];
+  const bool shared = p.kc == p.vc;
+  // the merge area is the consumed last stage of an item where that is large enough, else one of its own behind the ring
+  const bool own_merge = FP8 || shared;
+  uint8_t* behind = ring + p.stages * p.stage_bytes;
+  float* merge_own = reinterpret_cast<float*>(behind);
+  float* bias_s = reinterpret_cast<float*>(behind + (own_merge ? 4 * p.rows * D * 4 : 0));
+  int* first = reinterpret_cast<int*>(bias_s + p.bias_smem);            // [B + 1] tiles before each sequence
+
+  pdl_trigger();
+  pdl_wait();
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int GA = p.Hq / p.Hkv, groups = (GA + 15) / 16, heads = p.Hkv * groups;
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < p.stages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 4); }
+    abort_word = 0;
+    mbar_fence_init();
+    first[0] = 0;
+  }
+  // tiles of every sequence (at least one: an empty sequence's rows are written too), prefix sums; every warp computes them for
+  // itself, so that one barrier is all the set-up waits for
+  int before = 0;
+#pragma unroll 4
+  for (int s0 = 0; s0 < p.B; s0 += 32) {
+    const int s = s0 + lane;
+    int x = s < p.B ? max(1, decode_tiles(p, p.kv_lens[s]).count) : 0;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (s < p.B) first[s + 1] = before + x;                              // the same value from every warp
+    before += __shfl_sync(0xffffffffu, x, 31);
+  }
+  __syncthreads();
+  // ranges: equal numbers of tiles, or of whole items where cut items have no place to be summed in
+  const long long U = static_cast<long long>(before) * heads;
+  const long long I = static_cast<long long>(p.B) * heads;
+  const bool cuts = p.counters != nullptr;
+  const long long most = cuts ? (U + kStreamMinTiles - 1) / kStreamMinTiles : I;
+  const long long P = most < gridDim.x ? most : gridDim.x;
+  const long long c = blockIdx.x;
+  if (c >= P) return;
+  const bool narrow = U * P < (1LL << 32);                             // 64-bit divisions cost a tenth of a short launch
+  auto mul_div = [&](long long x, long long y, long long z) -> long long {
+    return narrow ? static_cast<uint32_t>(x * y) / static_cast<uint32_t>(z) : x * y / z;
+  };
+  auto begin_of = [&](long long k) -> long long {
+    if (cuts) return mul_div(k, U, P);
+    const long long i = k * I / P;
+    if (i >= I) return U;
+    const int s = static_cast<int>(i / heads);
+    return static_cast<long long>(first[s]) * heads + (i % heads) * (first[s + 1] - first[s]);
+  };
+  const long long u_begin = begin_of(c), u_end = begin_of(c + 1);
+  int s_at = 0;                                                          // sequence of u_begin
+  for (int lo = 0, hi = p.B - 1; lo <= hi;) {
+    const int mid = (lo + hi) / 2;
+    if (static_cast<long long>(first[mid]) * heads <= u_begin) { s_at = mid; lo = mid + 1; } else hi = mid - 1;
+  }
+
+  if (warp == 4) {
+    // ---- loads: a box of [block tokens x 64 columns] (FP8: x 128) per cache block and panel, spread over the lanes
+    constexpr int PANELS = FP8 ? 1 : D / 64;
+    int stage = 0; uint32_t phase = 0;
+    bool ok = true;
+    const int bt = p.block_tokens;
+    StreamItem it;
+    for (long long u = u_begin; u < u_end && ok; u += it.t1 - it.t0) {
+      stream_item(first, heads, u, u_end, s_at, it);
+      const int kv_len = p.kv_lens[it.s], g = it.h / groups;
+      const int* table = p.block_table + static_cast<size_t>(it.s) * p.table_stride;
+      const TileRange tiles = decode_tiles(p, kv_len);
+      for (int t = it.t0; t < it.t1 && ok; ++t) {
+        const int tok0 = tile_at(tiles, t) * kTileTok;
+        const int nblk = max(0, min(kTileTok / bt, (kv_len - tok0 + bt - 1) / bt));
+        const int per_blk = (shared ? 1 : 2) * PANELS, boxes = nblk * per_blk;
+        int blk = 0;
+        if (lane < boxes) blk = table[tok0 / bt + lane / per_blk];
+        ok = mbar_wait(&empty_bar[stage], phase ^ 1, &abort_word);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        if (lane == 0) mbar_expect_tx(&full_bar[stage], static_cast<uint32_t>(boxes) * bt * 128);
+        __syncwarp();
+        for (int i = lane; i < boxes; i += 32) {
+          if (i >= 32) blk = table[tok0 / bt + i / per_blk];
+          const int j = i % per_blk, which = j / PANELS, h = j % PANELS;
+          uint8_t* dst = ring + stage * p.stage_bytes + which * kTileBytes + h * (kTileTok * 128) + (i / per_blk) * bt * 128;
+          tma_load_3d(dst, which ? &v_map : &k_map, &full_bar[stage], h * 64, g * bt, blk);
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+    }
+  } else {
+    int stage = 0; uint32_t phase = 0;
+    bool ok = true;
+    StreamItem it;
+    for (long long u = u_begin; u < u_end; u += it.t1 - it.t0) {
+      stream_item(first, heads, u, u_end, s_at, it);
+      const int kv_len = p.kv_lens[it.s], s = it.s;
+      const int g = it.h / groups, head0 = g * GA + (it.h % groups) * 16;
+      const int G = min(16, (g + 1) * GA - head0);             // query heads of this item: head0 .. head0 + G
+      const TileRange tiles = decode_tiles(p, kv_len);
+      const int win_lo = p.window > 0 ? kv_len - p.window : 0;
+      if (SIG && p.bias_smem) {
+        stream_bar();                                          // the previous item's rows are no longer read
+        for (int i = threadIdx.x; i < G * p.bias_len; i += 128) bias_s[i] = p.bias[static_cast<size_t>(head0) * p.bias_len + i];
+        stream_bar();
+      }
+      // Q fragments straight from global memory (the loads of the item's first tiles are in flight meanwhile)
+      uint32_t qf[D / 16][4];
+      float sl2[2] = {p.scale_log2, p.scale_log2};
+      int limit[2], lo[2]; float slope[2];
+      const float* bias[2];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int r = (lane >> 2) + i * 8;
+        limit[i] = r < G ? kv_len - 1 : -1;
+        lo[i] = win_lo;
+        slope[i] = (p.alibi && r < G) ? p.alibi[head0 + r] : 0.f;
+        bias[i] = !SIG ? nullptr : (p.bias_smem ? bias_s : p.bias + static_cast<size_t>(head0) * p.bias_len) + (r < G ? r : 0) * p.bias_len;
+        const bf16* src = p.q + static_cast<size_t>(s) * p.q_stride + static_cast<size_t>(head0 + r) * p.D;
+        if constexpr (!FP8) {
+#pragma unroll
+          for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+            for (int x = 0; x < 2; ++x) {
+              const int col = kk * 16 + x * 8 + (lane & 3) * 2;
+              qf[kk][x * 2 + i] = (r < G && col < p.D) ? *reinterpret_cast<const uint32_t*>(src + col) : 0u;
+            }
+        } else {
+          // f16 rows scaled by a power of two to a largest magnitude in [1, 2): exact but for elements 2^14 below it, whose
+          // rounding is smaller than that of the fp32 sums
+          uint32_t w[2][8];
+          float am = 0.f;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int col = (h * 4 + (lane & 3)) * 16;
+            const bool on = r < G && col < p.D;
+            const uint4 a = on ? *reinterpret_cast<const uint4*>(src + col) : make_uint4(0, 0, 0, 0);
+            const uint4 b = on ? *reinterpret_cast<const uint4*>(src + col + 8) : make_uint4(0, 0, 0, 0);
+            w[h][0] = a.x; w[h][1] = a.y; w[h][2] = a.z; w[h][3] = a.w; w[h][4] = b.x; w[h][5] = b.y; w[h][6] = b.z; w[h][7] = b.w;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              am = fmaxf(am, fmaxf(fabsf(__uint_as_float(w[h][k] << 16)), fabsf(__uint_as_float(w[h][k] & 0xffff0000u))));
+          }
+          am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 1));
+          am = fmaxf(am, __shfl_xor_sync(0xffffffffu, am, 2));
+          const uint32_t e = min(max(__float_as_uint(am) >> 23, 1u), 250u);
+          const float up = __uint_as_float((254u - e) << 23);
+          sl2[i] = p.scale_log2 * p.k_scale * __uint_as_float(e << 23);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              qf[h * 4 + k / 2][(k & 1) * 2 + i] =
+                  pack_f16(__uint_as_float(w[h][k] << 16) * up, __uint_as_float(w[h][k] & 0xffff0000u) * up);
+        }
+      }
+      float o[D / 8][4];
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
+      float m[2] = {-INFINITY, -INFINITY}, l[2] = {0.f, 0.f};
+      if (SIG) { m[0] = m[1] = 0.f; }                          // nothing is rescaled when partial sums are merged
+      uint8_t* held = nullptr;                                 // stage of the item's last tile
+      uint64_t* held_bar = nullptr;
+      for (int t = it.t0; t < it.t1; ++t) {
+        if (ok) ok = mbar_wait(&full_bar[stage], phase, &abort_word);
+        uint8_t* kt = ring + stage * p.stage_bytes;
+        uint8_t* vt = shared ? kt : kt + kTileBytes;
+        const int tok0 = tile_at(tiles, t) * kTileTok, w0 = warp * 16;
+        if (ok) {
+          // V rows past the sequence's end (this warp's own): stale shared memory or whatever the cache holds there; their weights
+          // are exactly 0, but 0 x NaN would poison the output. K needs nothing: its scores are masked.
+          const int valid = kv_len - tok0 - w0;
+          if (valid < 16) {
+            for (int i = lane; i < 16 * (FP8 ? 8 : D / 8); i += 32) {
+              const int r = i / (FP8 ? 8 : D / 8), ch = i % (FP8 ? 8 : D / 8);
+              if (r < valid) continue;
+              if constexpr (FP8) *reinterpret_cast<uint4*>(vt + (w0 + r) * 128 + ch * 16) = make_uint4(0, 0, 0, 0);
+              else *reinterpret_cast<uint4*>(tile_ptr<D, kTileTok>(reinterpret_cast<bf16*>(vt), w0 + r, ch)) = make_uint4(0, 0, 0, 0);
+            }
+            fence_async_smem();
+            __syncwarp();
+          }
+          float sc[2][4];
+          if constexpr (FP8) {
+            warp_qk_fp8(sc, qf, kt, w0, lane);
+            softmax_update<D, 2, true>(sc, o, m, l, limit, lo, p.keep, slope, tok0 + w0, lane, sl2);
+            warp_pv_fp8(o, sc, vt, w0, lane);
+          } else {
+            warp_qk<D, 2>(sc, qf, reinterpret_cast<bf16*>(kt), w0, lane);
+            if constexpr (SIG) sigmoid_weights<2>(sc, limit, lo, p.keep, bias, p.bias_len - 1, tok0 + w0, lane, p.scale_log2);
+            else softmax_update<D, 2>(sc, o, m, l, limit, lo, p.keep, slope, tok0 + w0, lane, sl2);
+            warp_pv<D, 2>(o, sc, reinterpret_cast<bf16*>(vt), w0, lane);
+          }
+        }
+        if (t + 1 == it.t1 && !own_merge) {
+          held = kt; held_bar = &empty_bar[stage];             // released after the merge
+        } else {
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&empty_bar[stage]);
+        }
+        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+      }
+      // ---- the warps' sums: [4 warps][rows][D] floats, columns swizzled by row so that neither side conflicts
+      float* merge = own_merge ? merge_own : reinterpret_cast<float*>(held);
+      const int R = p.rows;
+      stream_bar();                                            // every warp is done with the last tile
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 1);
+        l[i] += __shfl_xor_sync(0xffffffffu, l[i], 2);
+        const int r = (lane >> 2) + i * 8;
+        if (r < R) {
+          if ((lane & 3) == 0) { ml_s[warp][r][0] = m[i]; ml_s[warp][r][1] = l[i]; }
+          float* dst = merge + (warp * R + r) * D;
+          const int x = (r & 7) << 3;
+          if constexpr (FP8) {
+#pragma unroll
+            for (int ch = 0; ch < 8; ++ch)
+              *reinterpret_cast<float4*>(dst + ((ch * 16 + (lane & 3) * 4) ^ x)) =
+                  make_float4(o[2 * ch][2 * i] * p.v_scale, o[2 * ch + 1][2 * i] * p.v_scale, o[2 * ch][2 * i + 1] * p.v_scale,
+                              o[2 * ch + 1][2 * i + 1] * p.v_scale);
+          } else {
+#pragma unroll
+            for (int n = 0; n < D / 8; ++n)
+              *reinterpret_cast<float2*>(dst + ((n * 8 + (lane & 3) * 2) ^ x)) = make_float2(o[n][2 * i], o[n][2 * i + 1]);
+          }
+        }
+      }
+      stream_bar();
+      const bool whole = it.t1 - it.t0 == it.n;
+      const long long slot = 2 * c + (u == u_begin ? 0 : 1);
+      for (int r = warp; r < G; r += 4) {
+        float mm = -INFINITY;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) mm = fmaxf(mm, ml_s[w][r][0]);
+        float f[4], ll = 0.f;
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          f[w] = ml_s[w][r][0] == -INFINITY ? 0.f : exp2f(ml_s[w][r][0] - mm);
+          ll += ml_s[w][r][1] * f[w];
+        }
+        if (whole) ll += sink_term(p, head0 + r, mm);
+        const float inv = SIG ? 1.f : ll > 0.f ? 1.f / ll : 0.f;
+#pragma unroll
+        for (int d0 = 0; d0 < D; d0 += 128) {
+          const int d = d0 + lane * 4;
+          float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (d < D) {
+#pragma unroll
+            for (int w = 0; w < 4; ++w) {
+              const float4 v = *reinterpret_cast<const float4*>(merge + (w * R + r) * D + (d ^ ((r & 7) << 3)));
+              acc.x += v.x * f[w]; acc.y += v.y * f[w]; acc.z += v.z * f[w]; acc.w += v.w * f[w];
+            }
+          }
+          if (whole) {
+            store_head_row4<D, SIG>(p, s, head0 + r, d, make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv));
+          } else if (d < p.Dv) {
+            __stcg(reinterpret_cast<float4*>(p.cut_o + (slot * R + r) * p.Dv + d), acc);
+          }
+        }
+        if (!whole && lane == 0) __stcg(reinterpret_cast<float2*>(p.cut_ml + (slot * R + r) * 2), make_float2(mm, ll));
+      }
+      if (!own_merge) {
+        fence_async_smem();                                    // the stage goes back to the TMA ring
+        __syncwarp();
+        if (lane == 0) mbar_arrive(held_bar);
+      }
+      if (whole) continue;
+      // ---- a cut item: whoever delivers the last piece adds them up, in their order along the line
+      const long long a = u - it.t0, b = a + it.n;             // the item's units
+      auto owner = [&](long long x) {
+        long long k = mul_div(x, P, U);
+        while (k + 1 < P && begin_of(k + 1) <= x) ++k;
+        while (k > 0 && begin_of(k) > x) --k;
+        return k;
+      };
+      const long long cf = owner(a);
+      const int pieces = static_cast<int>(owner(b - 1) - cf) + 1;
+      __threadfence();
+      stream_bar();
+      if (threadIdx.x == 0) {
+        unsigned int* cnt = p.counters + static_cast<size_t>(s) * heads + it.h;
+        const bool last = atomicAdd(cnt, 1u) + 1u == static_cast<unsigned int>(pieces);
+        if (last) *cnt = 0;
+        last_piece = last;
+        __threadfence();
+      }
+      stream_bar();
+      if (last_piece) {
+        const long long slot0 = 2 * cf + (begin_of(cf) < a ? 1 : 0);
+        for (int r = warp; r < G; r += 4) {
+          float mm = -INFINITY;
+          for (int k = lane; k < pieces; k += 32) mm = fmaxf(mm, __ldcg(p.cut_ml + ((k ? 2 * (cf + k) : slot0) * R + r) * 2));
+#pragma unroll
+          for (int x = 16; x > 0; x >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, x));
+          float ll = 0.f;
+          float4 acc[(D + 127) / 128];
+#pragma unroll
+          for (int j = 0; j < (D + 127) / 128; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+          for (int k = 0; k < pieces; ++k) {
+            const long long sl = k ? 2 * (cf + k) : slot0;
+            const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.cut_ml + (sl * R + r) * 2));
+            const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - mm);
+            ll += ml.y * f;
+#pragma unroll
+            for (int j = 0; j < (D + 127) / 128; ++j) {
+              const int d = j * 128 + lane * 4;
+              if (d < p.Dv) {
+                const float4 v = __ldcg(reinterpret_cast<const float4*>(p.cut_o + (sl * R + r) * p.Dv + d));
+                acc[j].x += v.x * f; acc[j].y += v.y * f; acc[j].z += v.z * f; acc[j].w += v.w * f;
+              }
+            }
+          }
+          ll += sink_term(p, head0 + r, mm);
+          const float inv = SIG ? 1.f : ll > 0.f ? 1.f / ll : 0.f;
+#pragma unroll
+          for (int j = 0; j < (D + 127) / 128; ++j)
+            store_head_row4<D, SIG>(p, s, head0 + r, j * 128 + lane * 4,
+                                    make_float4(acc[j].x * inv, acc[j].y * inv, acc[j].z * inv, acc[j].w * inv));
+        }
+      }
+    }
+  }
+  __syncthreads();
+  if (abort_word) {                        // a bounded wait gave up: copies in flight land before the CTA's memory is reused
+    if (threadIdx.x == 0 && p.err) atomicExch(p.err, 4);
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   }
 }
 
@@ -699,12 +1166,32 @@ static bool make_kv_map(CUtensorMap* map, const void* panel, long long block_str
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The same panel of e4m3 values: box = one cache block's tokens x 128 columns.
+static bool make_kv_map_fp8(CUtensorMap* map, const void* panel, long long block_stride, int num_blocks, int Hkv, int D, int block_tokens) {
+  AttnEncodeFn enc = attn_encode_fn();
+  if (!enc || (reinterpret_cast<uintptr_t>(panel) & 15)) return false;
+  cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(Hkv) * block_tokens, static_cast<cuuint64_t>(num_blocks)};
+  cuuint64_t strides[2] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(block_stride)};
+  cuuint32_t box[3] = {128, static_cast<cuuint32_t>(block_tokens), 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<void*>(panel), dims, strides, box, estr,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // The maps of both panels, where the TMA path covers the cache (block sizes that divide a tile, 16-byte strides).
 static bool tma_maps(const AttnParams& p, int num_blocks, CUtensorMap* km, CUtensorMap* vm) {
   const int bt = p.block_tokens;
   if (!(bt == 8 || bt == 16 || bt == 32 || bt == 64) || p.block_stride % 8 || num_blocks <= 0) return false;
   return make_kv_map(km, p.kc, p.block_stride, num_blocks, p.Hkv, p.D, bt) &&
          make_kv_map(vm, p.vc, p.block_stride, num_blocks, p.Hkv, p.Dv, bt);
+}
+
+static bool tma_maps_fp8(const AttnParams& p, int num_blocks, CUtensorMap* km, CUtensorMap* vm) {
+  const int bt = p.block_tokens;
+  if (!(bt == 8 || bt == 16 || bt == 32 || bt == 64) || p.block_stride % 16 || p.D % 16 || p.Dv % 16 || num_blocks <= 0) return false;
+  return make_kv_map_fp8(km, p.kc, p.block_stride, num_blocks, p.Hkv, p.D, bt) &&
+         make_kv_map_fp8(vm, p.vc, p.block_stride, num_blocks, p.Hkv, p.Dv, bt);
 }
 
 template <int D, int MODE, bool SIG = false>
@@ -722,8 +1209,51 @@ static int launch_prefill(const AttnParams& p, const CUtensorMap& km, const CUte
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
+// Partial results of the cut items (two per CTA) and the counters of a stream launch.
+struct StreamWork { float* scratch; long long scratch_bytes; unsigned int* counters; long long counters_len; };
+
+// Returns 1 when the launch does not fit (the caller takes the other kernel).
 template <int D, int MODE, bool SIG>
-static int launch_decode(const AttnParams& p, const CUtensorMap& km, const CUtensorMap& vm, int B, cudaStream_t st) {
+static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap& vm, int B, const StreamWork& w, cudaStream_t st) {
+  constexpr bool FP8 = MODE == kKvTmaFp8;
+  constexpr int kLimit = 226 * 1024, kHalf = 112 * 1024;       // one CTA per SM, two CTAs per SM
+  const bool shared = p.kc == p.vc;
+  const int GA = p.Hq / p.Hkv, heads = p.Hkv * ((GA + 15) / 16);
+  p.B = B;
+  p.rows = GA < 16 ? GA : 16;
+  p.vec_out = !(reinterpret_cast<uintptr_t>(p.out) & 7) && p.out_stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(p.outq) & 3);
+  p.stage_bytes = (shared ? 1 : 2) * kTileTok * D * (FP8 ? 1 : 2);
+  const long long extra = 1024 + ((FP8 || shared) ? 4 * p.rows * D * 4 : 0) + (SIG ? p.bias_smem * 4 : 0) + (B + 1) * 4LL;
+  if (extra + 2 * p.stage_bytes > kLimit) return 1;
+  // as many stages as leave room for a second CTA on the SM, three at least where they fit
+  long long stages = (kHalf - extra) / p.stage_bytes;
+  if (stages < 3) stages = (kLimit - extra) / p.stage_bytes < 3 ? 2 : 3;
+  p.stages = static_cast<int>(stages < kStreamMaxStages ? stages : kStreamMaxStages);
+  const int smem = static_cast<int>(extra) + p.stages * p.stage_bytes;
+  static std::atomic<bool> set[64];
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return -3;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (!set[dev].load(std::memory_order_acquire)) {
+    if (cudaFuncSetAttribute(paged_decode_stream_kernel<D, MODE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit) !=
+        cudaSuccess) return -3;
+    set[dev].store(true, std::memory_order_release);
+  }
+  const int per_sm = smem <= kHalf ? 2 : 1;
+  const long long grid = static_cast<long long>(sms) * per_sm;
+  const long long need = 2 * grid * p.rows * (p.Dv + 2) * 4;
+  if (w.scratch && need <= w.scratch_bytes && w.counters && static_cast<long long>(B) * heads <= w.counters_len) {
+    p.cut_o = w.scratch;
+    p.cut_ml = w.scratch + 2 * grid * p.rows * p.Dv;
+    p.counters = w.counters;
+  }
+  return launch_pdl(paged_decode_stream_kernel<D, MODE, SIG>, dim3(static_cast<unsigned>(grid)), dim3(kStreamThreads), smem, st, km, vm,
+                    p) == cudaSuccess ? 0 : -4;
+}
+
+template <int D, int MODE, bool SIG>
+static int launch_decode(const AttnParams& p, int B, cudaStream_t st) {
   constexpr int most = (16 * D + decode_ring(D, false)) * 2 + 1024 + (SIG ? kBiasSmem * 4 : 0);
   const int smem = (16 * D + decode_ring(D, p.kc == p.vc)) * 2 + 1024 + (SIG ? p.bias_smem * 4 : 0);
   static bool set = false;
@@ -733,7 +1263,7 @@ static int launch_decode(const AttnParams& p, const CUtensorMap& km, const CUten
     set = true;
   }
   dim3 grid(p.Hkv * ((p.Hq / p.Hkv + 15) / 16), B, p.num_splits);
-  if (launch_pdl(paged_decode_kernel<D, MODE, SIG>, grid, dim3(kAttnThreads), smem, st, km, vm, p) != cudaSuccess)
+  if (launch_pdl(paged_decode_kernel<D, MODE, SIG>, grid, dim3(kAttnThreads), smem, st, p) != cudaSuccess)
     return -4;
   if (p.num_splits > 1) {
     if (launch_pdl(decode_reduce_kernel<D>, dim3(p.Hq, B), dim3(D < 128 ? 64 : 128), 0, st, p) != cudaSuccess) return -5;
@@ -759,20 +1289,24 @@ static int dispatch_prefill(const AttnParams& p, int cache_fp8, int num_blocks, 
 }
 
 template <int D>
-static int dispatch_decode(const AttnParams& p, int cache_fp8, int num_blocks, int B, cudaStream_t st) {
+static int dispatch_decode(const AttnParams& p, int cache_fp8, int num_blocks, int B, const StreamWork& w, cudaStream_t st) {
   CUtensorMap km{}, vm{};
+  int rc = 1;
   if (p.bias) {
     if (cache_fp8) return -11;
-    if (tma_maps(p, num_blocks, &km, &vm)) return launch_decode<D, kKvTma, true>(p, km, vm, B, st);
-    return launch_decode<D, kKvCpAsync, true>(p, km, vm, B, st);
+    if (tma_maps(p, num_blocks, &km, &vm)) rc = launch_stream<D, kKvTma, true>(p, km, vm, B, w, st);
+    return rc <= 0 ? rc : launch_decode<D, kKvCpAsync, true>(p, B, st);
   }
-  if constexpr (D <= 128) {
-    if (cache_fp8) return launch_decode<D, kKvFp8, false>(p, km, vm, B, st);
-  } else if (cache_fp8) {
-    return -11;
+  if (cache_fp8) {
+    if constexpr (D <= 128) {
+      if (tma_maps_fp8(p, num_blocks, &km, &vm)) rc = launch_stream<128, kKvTmaFp8, false>(p, km, vm, B, w, st);
+      return rc <= 0 ? rc : launch_decode<D, kKvFp8, false>(p, B, st);
+    } else {
+      return -11;
+    }
   }
-  if (tma_maps(p, num_blocks, &km, &vm)) return launch_decode<D, kKvTma, false>(p, km, vm, B, st);
-  return launch_decode<D, kKvCpAsync, false>(p, km, vm, B, st);
+  if (tma_maps(p, num_blocks, &km, &vm)) rc = launch_stream<D, kKvTma, false>(p, km, vm, B, w, st);
+  return rc <= 0 ? rc : launch_decode<D, kKvCpAsync, false>(p, B, st);
 }
 
 // The padded head size that serves (D, Dv), 0 when none does.
@@ -818,20 +1352,24 @@ extern "C" int ksana_paged_prefill(const void* q, long long q_stride, void* out,
   return -11;
 }
 
-// One new token per sequence. workspace: part_o [B*Hq*splits*Dv] fp32, part_ml [B*Hq*splits*2] fp32 (splits > 1).
+// One new token per sequence. scratch, counters (zero before the first launch): place for the pieces of items that the stream form
+// cuts; without enough of it nothing is cut. num_splits and part_o [B*Hq*splits*Dv], part_ml [B*Hq*splits*2] fp32 (splits > 1)
+// serve caches that TMA cannot read.
 extern "C" int ksana_paged_decode(const void* q, long long q_stride, void* out, long long out_stride,
                                   const void* kc, const void* vc, long long block_stride, int block_tokens,
                                   const int* block_table, int table_stride, const int* kv_lens, const float* alibi,
                                   const float* sinks, int B, int Hq, int Hkv, int D, int Dv, int window, int keep, float scale,
                                   int cache_fp8, float k_scale, float v_scale, int num_splits, float* part_o, float* part_ml,
                                   int num_blocks, void* outq, float* oscale, int oscale_ld, const float* bias, int bias_len,
-                                  const void* gate, long long gate_stride, float out_factor, int* err, cudaStream_t st) {
+                                  const void* gate, long long gate_stride, float out_factor, float* scratch, long long scratch_bytes,
+                                  unsigned int* counters, long long counters_len, int* err, cudaStream_t st) {
   if (B <= 0) return 0;
   if (bias ? (bias_len <= 0 || sinks || alibi || outq) : gate != nullptr) return -14;
   if (outq && (D != 128 || Dv != 128 || !oscale)) return -13;
   if (Hkv <= 0 || Hq % Hkv || q_stride % 8 || (reinterpret_cast<uintptr_t>(q) & 15)) return -10;
   if (num_splits < 1) num_splits = 1;
   if (num_splits > 1 && (!part_o || !part_ml)) return -12;
+  const StreamWork w{scratch, scratch_bytes, counters, counters_len};
   AttnParams p{};
   p.q = (const bf16*)q; p.q_stride = q_stride; p.out = (bf16*)out; p.out_stride = out_stride;
   p.kc = kc; p.vc = vc; p.block_stride = block_stride; p.block_tokens = block_tokens; p.D = D; p.Dv = Dv;
@@ -844,10 +1382,10 @@ extern "C" int ksana_paged_decode(const void* q, long long q_stride, void* out, 
   const int table = bias ? (Hq / Hkv < 16 ? Hq / Hkv : 16) * bias_len : 0;
   p.bias_smem = table <= kBiasSmem ? table : 0;
   switch (padded_head(D, Dv)) {
-    case 64: return dispatch_decode<64>(p, cache_fp8, num_blocks, B, st);
-    case 128: return dispatch_decode<128>(p, cache_fp8, num_blocks, B, st);
-    case 192: return dispatch_decode<192>(p, cache_fp8, num_blocks, B, st);
-    case 256: return dispatch_decode<256>(p, cache_fp8, num_blocks, B, st);
+    case 64: return dispatch_decode<64>(p, cache_fp8, num_blocks, B, w, st);
+    case 128: return dispatch_decode<128>(p, cache_fp8, num_blocks, B, w, st);
+    case 192: return dispatch_decode<192>(p, cache_fp8, num_blocks, B, w, st);
+    case 256: return dispatch_decode<256>(p, cache_fp8, num_blocks, B, w, st);
   }
   return -11;
 }

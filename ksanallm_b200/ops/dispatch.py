@@ -564,9 +564,11 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
                              step.kv_lens, nm, step.max_q_len, Hq, Hkv, D, scale, v_cache=v_cache, window=window, keep=keep,
                              sinks=sinks, weights=weights)
     if ns:
-        seen = min(step.max_kv_len, window + keep + 128) if window > 0 else step.max_kv_len
-        # keys that are the values take half of the shared memory
-        n = decode_splits(ns, Hkv * ((Hq // Hkv + 15) // 16), seen, ctas_per_sm=4 if k_cache.data_ptr() == v_cache.data_ptr() else 2)
+        n = 1
+        if not native.decode_streams(block_tokens):
+            seen = min(step.max_kv_len, window + keep + 128) if window > 0 else step.max_kv_len
+            # keys that are the values take half of the shared memory
+            n = decode_splits(ns, Hkv * ((Hq // Hkv + 15) // 16), seen, ctas_per_sm=4 if k_cache.data_ptr() == v_cache.data_ptr() else 2)
         po = pml = None
         if n > 1:
             po = torch.empty(ns * Hq * n * Dv, dtype=torch.float32, device=qkv.device)
@@ -578,7 +580,7 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
 
 
 def decode_splits(batch: int, hkv: int, max_kv_len: int, sms: int = 148, ctas_per_sm: int = 2) -> int:
-    """Split-KV factor of the decode attention kernel. One CTA serves one (sequence, kv head, split) and two CTAs
+    """Split-KV factor of the decode attention kernel for caches that TMA does not read. One CTA serves one (sequence, kv head, split) and two CTAs
     fit an SM (shared memory), so the time is about waves x (64-token tiles per split + a fixed set-up cost of about
     two tiles); the factor minimising that is chosen, with at least two tiles per split."""
     import os
@@ -605,6 +607,8 @@ def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_l
     result; with ``quant_for`` (the FP8 linear that consumes it) a pure decode step returns the QTensor that linear
     wants, quantised inside the attention kernels."""
     T = qkv.shape[0]
+    if qkv.is_cuda and native.decode_streams(block_tokens):
+        num_splits, workspace = 1, None
     if qkv.is_cuda and quant_for is not None and quant_for.fp8 and num_multi == 0 and num_single and D == 128 and out is None:
         po, pml = workspace if workspace is not None else (None, None)
         if num_splits > 1 and po is None:

@@ -99,7 +99,7 @@ _SIGS = {
     "ksana_paged_prefill": [vp, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32,
                             f32, i32, f32, f32, i32, vp, i32, vp, i64, f32, vp, vp],
     "ksana_paged_decode": [vp, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32,
-                           f32, f32, i32, vp, vp, i32, vp, vp, i32, vp, i32, vp, i64, f32, vp, vp],
+                           f32, f32, i32, vp, vp, i32, vp, vp, i32, vp, i32, vp, i64, f32, vp, i64, vp, i64, vp, vp],
     "ksana_mla_attention": [vp, i64, vp, i64, vp, i64, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, i64, f32, i32, i32, vp,
                             vp, vp, vp],
     "ksana_mla_rope_append": [vp, i64, i32, vp, i64, vp, f32, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, i64, i32, vp, vp],
@@ -957,20 +957,40 @@ def paged_prefill(q, q_stride, out, cache_layer, block_stride, block_tokens, blo
     _check(rc, "ksana_paged_prefill")
 
 
+_decode_workspaces = {}
+
+
+def decode_workspace(device):
+    """Per-device place for the pieces of items that the decode kernel cuts (two per CTA: at most 2 x 148 CTAs x 16 rows of 256
+    columns with their sums) and their arrival counters (zeroed once; the kernel leaves them zero). Launches that share it
+    must be ordered on one stream, as for :func:`gemm_workspace`."""
+    key = torch.device(device).index or 0
+    if key not in _decode_workspaces:
+        _decode_workspaces[key] = (torch.empty(4 * 148 * 16 * 258, dtype=torch.float32, device=device),
+                                   torch.zeros(1 << 16, dtype=torch.int32, device=device))
+    return _decode_workspaces[key]
+
+
+def decode_streams(block_tokens: int) -> bool:
+    """Whether the decode kernel balances a batch by itself (caches that TMA reads); others take a number of splits."""
+    return block_tokens in (8, 16, 32, 64)
+
+
 def paged_decode(q, q_stride, out, cache_layer, block_stride, block_tokens, block_table, kv_lens, B, Hq, Hkv, D, scale,
                  alibi=None, k_scale=1.0, v_scale=1.0, num_splits=1, part_o=None, part_ml=None, out_q=None,
                  out_scale=None, v_cache=None, window=0, keep=0, sinks=None, weights=None):
     """``out_q`` / ``out_scale`` (head dim 128): the output also (or, with ``out`` None, only) as the FP8 operand of the
     next GEMM: e4m3 [B, Hq * D] and scales [Hq, ld]. ``v_cache`` / ``window`` / ``keep`` / ``sinks`` / ``weights``: see
-    :func:`paged_prefill`."""
+    :func:`paged_prefill`. ``num_splits``, ``part_o``, ``part_ml``: for caches that :func:`decode_streams` does not name."""
     fp8 = cache_layer.dtype != torch.bfloat16
     kc, vc, Dv = _panels(cache_layer, v_cache, D)
+    scratch, counters = decode_workspace(q.device)
     rc = lib().ksana_paged_decode(_p(q), q_stride, _p(out), out.stride(0) if out is not None else Hq * Dv, kc, vc,
                                   block_stride, block_tokens, _p(block_table), block_table.stride(0), _p(kv_lens), _p(alibi),
                                   _p(sinks), B, Hq, Hkv, D, Dv, window, keep, float(scale), int(fp8), float(k_scale),
                                   float(v_scale), num_splits, _p(part_o), _p(part_ml), int(cache_layer.shape[0]), _p(out_q),
                                   _p(out_scale), out_scale.stride(0) if out_scale is not None else 0, *_sigmoid_args(weights),
-                                  _p(err_flag(q.device)), _st())
+                                  _p(scratch), scratch.numel() * 4, _p(counters), counters.numel(), _p(err_flag(q.device)), _st())
     _check(rc, "ksana_paged_decode")
 
 
