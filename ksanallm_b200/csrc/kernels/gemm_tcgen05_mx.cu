@@ -19,6 +19,10 @@
 // epilogue drains it into registers and hands it back before storing); BN = 128 double-buffers.
 // No cluster launch, no multicast. Every wait is bounded.
 //
+// Grouped (mixture-of-experts) mode: expert-major rows, every 128-row tile multiplies with the matrix of its own expert
+// (stacked along N with their scales). Through the promoted-FP8 kernel of gemm_tcgen05.cu, which moves every 128-deep K block
+// from TMEM to registers, the expert products ran at half this kernel's rate.
+//
 // The reference has no counterpart of the hardware-scaled path: its FP8 GEMMs are cuBLASLt per-tensor
 // (src/ksana_llm/kernels/nvidia/kernel_wrapper.cpp:1014-1048) or DeepGEMM block-wise on Hopper.
 #include "sm100_ptx.cuh"
@@ -60,6 +64,9 @@ struct MxParams {
   const float* w_scale;
   int* err;
   __nv_bfloat16* push[8]; int push_n; int push_rows;
+  // grouped mode: expert of every 128-row tile (< 0: tile unused), rows of each that hold anything (null: all); N and the scale
+  // rows are those of one expert
+  const int* tile_expert; const int* tile_rows;
 };
 
 constexpr int kMxGroupM = 16;
@@ -111,6 +118,12 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  auto unused = [&](int tile) {                  // grouped mode: a tile behind the last expert's rows
+    if (!p.tile_expert) return false;
+    int m_blk, n_blk;
+    mx_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
+    return p.tile_expert[m_blk] < 0;
+  };
   // Set-up overlapped the previous kernel (programmatic dependent launch); what that kernel produced is read only
   // after pdl_wait(), which every role calls first - except that the producer requests the weight tiles (B, never
   // written while the engine runs) of its first K blocks before it waits.
@@ -123,7 +136,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
       int pre = 0;
-      if (static_cast<int>(blockIdx.x) < num_tiles) {
+      if (static_cast<int>(blockIdx.x) < num_tiles && !p.tile_expert) {
         int m_blk, n_blk;
         mx_tile_coords(blockIdx.x, m_tiles, n_tiles, m_blk, n_blk);
         for (; pre < Cfg::kStages && pre < num_kb; ++pre) {
@@ -136,6 +149,12 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         int m_blk, n_blk;
         mx_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
+        int w_row = n_blk * BN;
+        if (p.tile_expert) {
+          const int e = p.tile_expert[m_blk];
+          if (e < 0) continue;
+          w_row += e * p.N;
+        }
         for (int kb = 0; kb < num_kb; ++kb, ++issued) {
           if (issued < pre) {                 // first round of the ring: the weight tile was requested above
             tma_load_2d(smem + stage * Cfg::kStageBytes, &tma_a, &full_bar[stage], kb * 128, m_blk * kMxBM);
@@ -146,7 +165,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           uint8_t* sa = smem + stage * Cfg::kStageBytes;
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
           tma_load_2d(sa, &tma_a, &full_bar[stage], kb * 128, m_blk * kMxBM);
-          tma_load_2d(sa + Cfg::kABytes, &tma_b, &full_bar[stage], kb * 128, n_blk * BN);
+          tma_load_2d(sa + Cfg::kABytes, &tma_b, &full_bar[stage], kb * 128, w_row);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -162,6 +181,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       uint32_t set = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+        if (unused(tile)) continue;
         if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
@@ -216,6 +236,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       int m_blk, n_blk;
       mx_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
       const int m0 = m_blk * kMxBM;
+      const size_t e0 = p.tile_expert ? static_cast<size_t>(p.tile_expert[m_blk]) * n_blocks : 0;
 #pragma unroll
       for (int r4 = 0; r4 < 4; ++r4) {
         const int row = min(m0 + r4 * 32 + lane, p.M - 1);
@@ -231,7 +252,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           const int kb = min(g * 4 + j, num_kb - 1);
-          r.b[c * 4 + j] = __ldg(p.w_scale + static_cast<size_t>(nb) * num_kb + kb);
+          r.b[c * 4 + j] = __ldg(p.w_scale + (e0 + nb) * num_kb + kb);
         }
       }
     };
@@ -263,8 +284,12 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       return true;
     };
     // (tile, group) sequence of this CTA; `ahead` runs two steps in front of `cur`
-    int ct = static_cast<int>(blockIdx.x), cg = 0, at = ct, ag = 0;
-    auto advance = [&](int& t, int& g) { if (++g == num_groups) { g = 0; t += static_cast<int>(gridDim.x); } };
+    auto used = [&](int t) {
+      while (t < num_tiles && unused(t)) t += static_cast<int>(gridDim.x);
+      return t;
+    };
+    int ct = used(static_cast<int>(blockIdx.x)), cg = 0, at = ct, ag = 0;
+    auto advance = [&](int& t, int& g) { if (++g == num_groups) { g = 0; t = used(t + static_cast<int>(gridDim.x)); } };
     Raw r0, r1, r2;
     if (at < num_tiles) { fetch(at, ag, r0); advance(at, ag); }
     if (at < num_tiles) { fetch(at, ag, r1); advance(at, ag); }
@@ -296,7 +321,8 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       mx_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
       const int row = m_blk * kMxBM + q * 32 + lane;
       const int n0 = n_blk * BN + col_off;
-      const bool row_ok = row < p.M;
+      if (p.tile_expert && p.tile_expert[m_blk] < 0) continue;
+      const bool row_ok = row < p.M && (!p.tile_rows || q * 32 + lane < p.tile_rows[m_blk]);
       if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[EC];
@@ -442,4 +468,26 @@ extern "C" int ksana_gemm_mxfp8(const void* Aq, int lda, const float* a_scale, i
   for (int i = 0; i < push_n && i < 8; ++i) p.push[i] = reinterpret_cast<__nv_bfloat16*>(push_ptrs[i]);
   p.push_n = push_n; p.push_rows = push_rows;
   return bn == 256 ? launch_mx<256>(ma, mb, p, max_ctas, st) : launch_mx<128>(ma, mb, p, max_ctas, st);
+}
+
+// Grouped form: A_q [M,K] expert-major rows (M a multiple of 128), W_q the experts' [N,K] matrices stacked to [E * N, K], w_scale
+// [E * ceil(N/128)][K/128]; tile_expert names the expert of every 128-row tile (-1: unused), tile_rows (may be null) its rows that
+// hold anything. The same conditions on scales, K and N.
+extern "C" int ksana_gemm_grouped_mxfp8(const void* Aq, int lda, const float* a_scale, int a_scale_ld, const void* Wq, int ldw,
+                                        const float* w_scale, void* D, int ldd, int M, int N, int K, int E, const int* tile_expert,
+                                        const int* tile_rows, int* err_flag, cudaStream_t st) {
+  if (M <= 0 || N <= 0 || K <= 0 || E <= 0) return 0;
+  if ((M % 128) || (N % 8) || (K % 128) || (lda % 16) || (ldw % 16) || (ldd % 8) || !tile_expert || !a_scale || !w_scale) return -10;
+  if ((reinterpret_cast<uintptr_t>(Aq) | reinterpret_cast<uintptr_t>(Wq) | reinterpret_cast<uintptr_t>(D)) & 15) return -11;
+  const int bn = (M / kMxBM) * ((N + 255) / 256) >= 148 ? 256 : 128;
+  CUtensorMap ma, mb;
+  if (mx_map(&ma, Aq, M, K, lda, kMxBM)) return -12;
+  if (mx_map(&mb, Wq, E * N, K, ldw, bn)) return -13;
+  MxParams p{};
+  p.M = M; p.N = N; p.K = K;
+  p.D = static_cast<__nv_bfloat16*>(D); p.ldd = ldd;
+  p.a_scale = a_scale; p.a_scale_ld = a_scale_ld; p.w_scale = w_scale;
+  p.err = err_flag;
+  p.tile_expert = tile_expert; p.tile_rows = tile_rows;
+  return bn == 256 ? launch_mx<256>(ma, mb, p, 0, st) : launch_mx<128>(ma, mb, p, 0, st);
 }

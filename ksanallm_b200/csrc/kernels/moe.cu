@@ -174,6 +174,33 @@ __global__ void moe_permute_kernel(const bf16* __restrict__ x, const int* __rest
   }
 }
 
+// The same for rows that are FP8 GEMM operands already (values and one scale per 128 columns): a token is quantised once, not once per
+// expert it goes to, and half the bytes move (8192 tokens x 8 of 7168 columns: 682 us for the bf16 permutation and the quantisation
+// of all its rows before).
+__global__ void moe_permute_fp8_kernel(const uint8_t* __restrict__ q, const float* __restrict__ scale, int scale_ld,
+                                       const int* __restrict__ dst_row, uint8_t* __restrict__ perm, float* __restrict__ perm_scale,
+                                       int perm_ld, int K, int H, int cap, int* err) {
+  __shared__ int dst[kMaxTopK];
+  const int t = blockIdx.x;
+  if (threadIdx.x < K) {
+    const int r = dst_row[t * K + threadIdx.x];
+    if (r >= cap) guard_report(err, kGuardDstRow, r);
+    dst[threadIdx.x] = r < cap ? r : -1;
+  }
+  __syncthreads();
+  const uint4* src = reinterpret_cast<const uint4*>(q + static_cast<size_t>(t) * H);
+  for (int i = threadIdx.x; i < (H >> 4); i += blockDim.x) {
+    const uint4 v = src[i];
+    for (int k = 0; k < K; ++k)
+      if (dst[k] >= 0) reinterpret_cast<uint4*>(perm + static_cast<size_t>(dst[k]) * H)[i] = v;
+  }
+  for (int i = threadIdx.x; i < (H >> 7); i += blockDim.x) {
+    const float v = scale[static_cast<size_t>(i) * scale_ld + t];
+    for (int k = 0; k < K; ++k)
+      if (dst[k] >= 0) perm_scale[static_cast<size_t>(i) * perm_ld + dst[k]] = v;
+  }
+}
+
 // out[t] = (accumulate ? out[t] : 0) + sum_k w[t,k] * y[dst_row[t,k]]
 __global__ void moe_combine_kernel(const bf16* __restrict__ y, const int* __restrict__ dst_row,
                                    const float* __restrict__ topk_w, bf16* __restrict__ out, int K, int H,
@@ -237,6 +264,15 @@ extern "C" int ksana_moe_permute(const void* x, const int* dst_row, void* perm, 
   if (T <= 0) return 0;
   if (H % 8) return -10;
   moe_permute_kernel<<<T, 256, 0, st>>>((const bf16*)x, dst_row, (bf16*)perm, K, H, cap, err);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+extern "C" int ksana_moe_permute_fp8(const void* q, const float* scale, int scale_ld, const int* dst_row, void* perm, float* perm_scale,
+                                     int perm_ld, int T, int K, int H, int cap, int* err, cudaStream_t st) {
+  if (T <= 0) return 0;
+  if (H % 128 || K > kMaxTopK || K <= 0) return -10;
+  moe_permute_fp8_kernel<<<T, 256, 0, st>>>((const uint8_t*)q, scale, scale_ld, dst_row, (uint8_t*)perm, perm_scale, perm_ld, K, H, cap,
+                                            err);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 

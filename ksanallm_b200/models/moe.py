@@ -40,6 +40,8 @@ class MoEWeights:
     shared_gate: Optional[torch.Tensor] = None       # [1, H] sigmoid gate of the shared expert (Qwen2-MoE)
     expert_lo: int = 0
     expert_hi: int = 0
+    router_bf16: Optional[torch.Tensor] = None       # the router as the GEMM's operand (GPU)
+    ue8m0: bool = False                     # the experts' block scales are powers of two: the tensor cores can apply them
     # NVFP4 experts: w13 / w2 hold packed e2m1 pairs ([rows, K/2] bytes), *_bs the e4m3 scales per 16 elements
     # ([rows, K/16]) and *_ts one fp32 tensor scale per local expert
     w13_bs: Optional[torch.Tensor] = None
@@ -141,7 +143,9 @@ def load_moe(cfg: ModelConfig, source, prefix: str, tp_rank, tp_size, device, dt
         w2, w2_s = ref.quant_weight_fp8_block(w2)
     else:
         w13, w2 = _dense(w13).to(dtype).contiguous(), _dense(w2).to(dtype).contiguous()
-    mw = MoEWeights(router, rbias, w13, w13_s, w2, w2_s, E, I, H, expert_lo=lo, expert_hi=hi, **nv)
+    mw = MoEWeights(router, rbias, w13, w13_s, w2, w2_s, E, I, H, expert_lo=lo, expert_hi=hi,
+                    router_bf16=router.to(torch.bfloat16) if router.is_cuda else None,
+                    ue8m0=w13_s is not None and ref.is_pow2(w13_s) and ref.is_pow2(w2_s), **nv)
     sI_full = cfg.shared_expert_intermediate_size
     if sI_full:
         sp = prefix + "mlp.shared_expert."
@@ -226,7 +230,7 @@ def route(model, mw: MoEWeights, x: torch.Tensor):
     K, E = cfg.num_experts_per_tok, mw.num_experts
     if x.is_cuda:
         logits = torch.empty(T, E, dtype=torch.float32, device=x.device)
-        native.gemm_bf16(x, mw.router.to(torch.bfloat16) if mw.router.dtype != torch.bfloat16 else mw.router, out_f32=logits)
+        native.gemm_bf16(x, mw.router_bf16 if mw.router_bf16 is not None else mw.router.to(torch.bfloat16), out_f32=logits)
         return native.moe_route(logits, K, cfg.moe_scoring, cfg.norm_topk_prob, cfg.routed_scaling_factor,
                                 mw.router_bias, cfg.n_group, cfg.topk_group)
     ids, w = route_reference(x.float() @ mw.router.float().t(), cfg, mw.router_bias)
@@ -249,8 +253,9 @@ def moe_partial(model, mw: MoEWeights, x: torch.Tensor, into: Optional[torch.Ten
         dst_row, tile_expert, _, _, cap, tile_rows = native.moe_align(ids, E, mw.expert_lo, mw.expert_hi)
         if mw.expert_lo:
             tile_expert = torch.where(tile_expert >= 0, tile_expert - mw.expert_lo, tile_expert)
-        perm = native.moe_permute(x, dst_row, K, cap, zero=mw.nvfp4)
+        xq = None                            # x as an FP8 operand, for the routed and the shared experts
         if mw.nvfp4:
+            perm = native.moe_permute(x, dst_row, K, cap, zero=True)
             # activations go to NVFP4 too: one tensor scale per GEMM input from its own maximum (no host sync);
             # padding rows are zero so that they do not enter the maximum
             a_ts = native.absmax_scale(x, 448.0 * 6.0)
@@ -261,17 +266,20 @@ def moe_partial(model, mw: MoEWeights, x: torch.Tensor, into: Optional[torch.Ten
             aq, abs_, _ = native.quant_nvfp4(a, a_ts2)
             y = native.gemm_grouped_nvfp4(aq, abs_, a_ts2, mw.w2, mw.w2_bs, mw.w2_ts, tile_expert, n_local, H)
         elif mw.w13_scale is not None:
-            pq, ps = native.quant_fp8(perm)
+            xq = ops.quantize(x)
+            pq, ps = native.moe_permute_fp8(xq.q, xq.s, dst_row, K, cap)
             g = native.gemm_grouped(pq, mw.w13, tile_expert, n_local, 2 * mw.inter, a_scale=ps, w_scale=mw.w13_scale,
-                                    tile_rows=tile_rows)
+                                    tile_rows=tile_rows, hw_scale=mw.ue8m0)
             _, aq, as_ = native.act_mul(g, cfg.activation, True, quant=True, want_out=False)
-            y = native.gemm_grouped(aq, mw.w2, tile_expert, n_local, H, a_scale=as_, w_scale=mw.w2_scale, tile_rows=tile_rows)
+            y = native.gemm_grouped(aq, mw.w2, tile_expert, n_local, H, a_scale=as_, w_scale=mw.w2_scale, tile_rows=tile_rows,
+                                    hw_scale=mw.ue8m0)
         else:
+            perm = native.moe_permute(x, dst_row, K, cap)
             y = dense_experts(perm, mw.w13, mw.w2, tile_expert, tile_rows, n_local, mw.inter, cfg.activation)
         out = into if into is not None else torch.empty(T, H, dtype=x.dtype, device=x.device)
         have_shared = shared and mw.shared_gate_up is not None
         if have_shared:
-            sg = ops.linear(x, mw.shared_gate_up)
+            sg = ops.linear(xq if xq is not None and mw.shared_gate_up.fp8 else x, mw.shared_gate_up)
             sa = ops.act_mul(sg, cfg.activation, True, quant_for=mw.shared_down)
             ops.linear(sa, mw.shared_down, out=out)
             if mw.shared_gate is not None:

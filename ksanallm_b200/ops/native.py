@@ -31,6 +31,7 @@ _SIGS = {
     "ksana_gemm_bf16_tall": [vp, i32, vp, i32, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_mxfp8_tall": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, i32, i32, vp,
                               vp],
+    "ksana_gemm_grouped_mxfp8": [vp, i32, vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp, vp, vp],
     "ksana_gemm_mxfp8_pair": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp, i32, i32, vp, vp],
     "ksana_gemm_fp8_block": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_smallm": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, i64, vp, i32,
@@ -39,6 +40,7 @@ _SIGS = {
     "ksana_moe_route": [vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32, i32, vp],
     "ksana_moe_align": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_moe_permute": [vp, vp, vp, i32, i32, i32, i32, vp, vp],
+    "ksana_moe_permute_fp8": [vp, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_moe_combine": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_smallm_push": [i32, vp, i32, vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, vp, i64, vp, i32, vp, i32, vp, vp],
     "ksana_gemm_smallm_push_signal": [i32, vp, i32, vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, vp, i64, vp, i32, vp, i32,
@@ -1161,10 +1163,11 @@ def ban_tokens(logits, offsets, ids, row_idx=None):
 
 
 # --------------------------------------------------------------------------- mixture of experts
-def gemm_grouped(a, w, tile_expert, E, N, out=None, a_scale=None, w_scale=None, bn=0, tile_rows=None):
+def gemm_grouped(a, w, tile_expert, E, N, out=None, a_scale=None, w_scale=None, bn=0, tile_rows=None, hw_scale=False):
     """Expert-major rows of ``a`` [cap, K] (128-row tiles, one expert each) times stacked W [E*N, K]. ``tile_rows``: rows of every
     tile that hold anything; the others need not be stored (worth it where tiles are mostly empty; with full ones, reading the counts
-    only sets the CTAs apart that share operand tiles in L2, up to twice the time)."""
+    only sets the CTAs apart that share operand tiles in L2, up to twice the time). ``hw_scale``: every scale is a power of two, so
+    the tensor cores may apply them."""
     cap, K = a.shape
     if cap > 191 * E:                  # more than 64 rows per expert on average
         tile_rows = None
@@ -1176,6 +1179,11 @@ def gemm_grouped(a, w, tile_expert, E, N, out=None, a_scale=None, w_scale=None, 
     kind = 0 if a_scale is None else 1
     if out is None:
         out = torch.empty(cap, N, dtype=torch.bfloat16, device=a.device)
+    if hw_scale and bn == 0 and N % 8 == 0:
+        rc = lib().ksana_gemm_grouped_mxfp8(_p(a), a.stride(0), _p(a_scale), a_scale.stride(0), _p(w), w.stride(0), _p(w_scale), _p(out),
+                                            out.stride(0), cap, N, K, E, _p(tile_expert), _p(tile_rows), _p(err_flag(a.device)), _st())
+        _check(rc, "ksana_gemm_grouped_mxfp8")
+        return out
     rc = lib().ksana_gemm_grouped(kind, _p(a), a.stride(0), _p(a_scale), a_scale.stride(0) if a_scale is not None else 0,
                                   _p(w), w.stride(0), _p(w_scale), _p(out), out.stride(0), cap, N, K, E,
                                   _p(tile_expert), _p(tile_rows), bn, _p(err_flag(a.device)), _st())
@@ -1223,6 +1231,17 @@ def moe_permute(x, dst_row, K, cap, zero=False):
     _check(lib().ksana_moe_permute(_p(x), _p(dst_row), _p(perm), T, K, units, cap, _p(err_flag(x.device)), _st()),
            "ksana_moe_permute")
     return perm
+
+
+def moe_permute_fp8(q, scale, dst_row, K, cap):
+    """:func:`moe_permute` of rows that :func:`quant_fp8` has quantised: (values [cap, H], scales [H / 128, cap]); padding rows are
+    undefined."""
+    T, H = q.shape
+    perm = torch.empty(cap, H, dtype=q.dtype, device=q.device)
+    ps = torch.empty(H // 128, cap, dtype=torch.float32, device=q.device)
+    _check(lib().ksana_moe_permute_fp8(_p(q), _p(scale), scale.stride(0), _p(dst_row), _p(perm), _p(ps), ps.stride(0), T, K, H, cap,
+                                       _p(err_flag(q.device)), _st()), "ksana_moe_permute_fp8")
+    return perm, ps
 
 
 def moe_combine(y, dst_row, topk_w, out, K, accumulate):
