@@ -1248,7 +1248,7 @@ static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap&
     p.cut_ml = w.scratch + 2 * grid * p.rows * p.Dv;
     p.counters = w.counters;
   }
-  return launch_pdl(paged_decode_stream_kernel<D, MODE, SIG>, dim3(static_cast<unsigned>(grid)), dim3(kStreamThreads), smem, st, km, vm,
+  return launch_early(paged_decode_stream_kernel<D, MODE, SIG>, dim3(static_cast<unsigned>(grid)), dim3(kStreamThreads), smem, st, km, vm,
                     p) == cudaSuccess ? 0 : -4;
 }
 

@@ -722,7 +722,7 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
     float* ds = oscale ? oscale + m0 : nullptr;
     const int* tr = tile_rows ? tile_rows + m0 / 128 : nullptr;
     const dim3 grid(grid_for((total + kActVecs - 1) / kActVecs, 256));
-#define KSANA_ACT(A, G, Q) launch_pdl(act_mul_kernel<A, G, Q>, grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total, div, in_ld, tr)
+#define KSANA_ACT(A, G, Q) launch_early(act_mul_kernel<A, G, Q>, grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total, div, in_ld, tr)
 #define KSANA_ACT_G(A) (gated ? (outq ? KSANA_ACT(A, true, true) : KSANA_ACT(A, true, false)) \
                               : (outq ? KSANA_ACT(A, false, true) : KSANA_ACT(A, false, false)))
     if (act == 0) KSANA_ACT_G(0);
@@ -751,7 +751,7 @@ extern "C" int ksana_quant_fp8(const void* x, void* q, float* scale, int scale_l
   for (int m0 = 0; m0 < M; m0 += most) {
     const int rows = M - m0 < most ? M - m0 : most;
     const uint32_t total = static_cast<uint32_t>(rows) * nvec;
-    launch_pdl(quant_fp8_kernel, dim3(grid_for((total + 3) / 4, 256)), dim3(256), 0, st, (const bf16*)x + static_cast<size_t>(m0) * x_ld,
+    launch_early(quant_fp8_kernel, dim3(grid_for((total + 3) / 4, 256)), dim3(256), 0, st, (const bf16*)x + static_cast<size_t>(m0) * x_ld,
                (uint8_t*)q + static_cast<size_t>(m0) * K, scale + m0, scale_ld, total, div, x_ld);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
@@ -772,7 +772,7 @@ extern "C" int ksana_embedding(const int* ids, const void* table, const int* pos
                                void* out, int T, int H, int vocab_lo, int vocab_hi, float scale, cudaStream_t st) {
   if (T <= 0) return 0;
   if (H % 8) return -10;
-  launch_pdl(embedding_kernel, dim3(T), dim3(256), 0, st, ids, (const bf16*)table, positions, (const bf16*)pos_table, (bf16*)out, H,
+  launch_early(embedding_kernel, dim3(T), dim3(256), 0, st, ids, (const bf16*)table, positions, (const bf16*)pos_table, (bf16*)out, H,
                                       vocab_lo, vocab_hi, scale);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
@@ -800,11 +800,11 @@ extern "C" int ksana_rope_kv_append(void* qkv, const int* positions, int pos_str
       (reinterpret_cast<uintptr_t>(qkv) % 16) == 0 && (reinterpret_cast<uintptr_t>(cache) % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(cos_sin) % 16) == 0) {
     if (cache_fp8)
-      launch_pdl(rope_kv_append_vec_kernel<uint8_t>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (uint8_t*)cache,
+      launch_early(rope_kv_append_vec_kernel<uint8_t>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (uint8_t*)cache,
                                                             block_stride, block_tokens, Hq, Hkv, D, 1.f / k_scale,
                                                             1.f / v_scale, apply_rope);
     else
-      launch_pdl(rope_kv_append_vec_kernel<bf16>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (bf16*)cache,
+      launch_early(rope_kv_append_vec_kernel<bf16>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (bf16*)cache,
                                                          block_stride, block_tokens, Hq, Hkv, D, 1.f, 1.f, apply_rope);
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }

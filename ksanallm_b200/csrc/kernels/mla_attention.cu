@@ -583,7 +583,7 @@ static cudaError_t launch_rope_append(const void* q, long long q_stride, int nop
   p.qfull = static_cast<T*>(qfull); p.cache = static_cast<T*>(cache); p.block_stride = block_stride;
   p.block_tokens = block_tokens; p.G = G; p.rank = rank; p.rank_p = (rank + 7) / 8 * 8; p.rot = rot; p.rot_p = (rot + 7) / 8 * 8;
   p.max_pos = max_pos; p.num_slots = num_slots; p.err = err;
-  return launch_pdl(mla_rope_append_kernel<T>, dim3(T_), dim3(kLatentThreads), 0, st, p);
+  return launch_early(mla_rope_append_kernel<T>, dim3(T_), dim3(kLatentThreads), 0, st, p);
 }
 
 template <int PANELS, bool FLAT, bool WINDOW>

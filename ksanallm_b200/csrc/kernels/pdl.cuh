@@ -12,9 +12,11 @@
 //   * a kernel launched through launch_pdl() that lacks pdl_wait() would race: only kernels that call it are launched
 //     with the attribute;
 //   * both calls are no-ops in a kernel launched without the attribute.
-// Off by default: in whole decode steps (CUDA graphs of 800 kernels) the measured gain of the early launches was
-// within noise, while graphs of one kernel class back to back gained about a microsecond per launch. KSANA_PDL=1 in
-// the environment switches the attribute on.
+// The attribute is on for the kernels launched through launch_early(): those of decode steps, which leave room on the SM for a
+// neighbour (half its shared memory at most), so that a GEMM's first weight tiles are on their way while the norm or the attention before
+// it ends. 8 layers of 4096, one sequence: 1070 -> 976 us per step, 64 sequences: 1575 -> 1544 us. The others take it with
+// KSANA_PDL=1 only: kernels that need a whole SM gained nothing (graphs of 800 kernels, within noise), and the 4-bit stream, whose CTAs
+// fill the register file, made its step slower (1130 -> 1386 us). KSANA_PDL=0 switches it off everywhere.
 #pragma once
 #include <cuda_runtime.h>
 #include <cstdlib>
@@ -33,11 +35,19 @@ inline bool pdl_enabled() {
   return on;
 }
 
+inline bool pdl_early_enabled() {
+  static const bool on = []() {
+    const char* e = std::getenv("KSANA_PDL");
+    return !(e && e[0] == '0');
+  }();
+  return on;
+}
+
 // kernel<<<grid, block, smem, st>>>(args...) in clusters of `cluster` blocks along x, with the programmatic stream-serialisation
-// attribute (when enabled).
+// attribute where `early`.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st,
-                                      Args&&... args) {
+inline cudaError_t launch_cluster(bool early, void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster, size_t smem, cudaStream_t st,
+                                  Args&&... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -45,7 +55,7 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
   cfg.stream = st;
   cudaLaunchAttribute attr[2];
   unsigned n = 0;
-  if (pdl_enabled()) {
+  if (early) {
     attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[n++].val.programmaticStreamSerializationAllowed = 1;
   }
@@ -63,7 +73,12 @@ inline cudaError_t launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                               Args&&... args) {
-  return launch_pdl_cluster(kernel, grid, block, 1, smem, st, std::forward<Args>(args)...);
+  return launch_cluster(pdl_enabled(), kernel, grid, block, 1, smem, st, std::forward<Args>(args)...);
+}
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_early(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args&&... args) {
+  return launch_cluster(pdl_early_enabled(), kernel, grid, block, 1, smem, st, std::forward<Args>(args)...);
 }
 
 }  // namespace ksana

@@ -241,7 +241,7 @@ static int launch_w4_stream(const W4StreamParams& p, int blocks_y, cudaStream_t 
     set[dev].store(true, std::memory_order_release);
   }
   const int tiles = (p.N + 127) / 128;
-  return launch_pdl_cluster(w4_stream_kernel<NT>, dim3(tiles * p.splits, blocks_y), dim3(kW4sThreads), p.splits, smem, st, p) ==
+  return launch_cluster(pdl_enabled(), w4_stream_kernel<NT>, dim3(tiles * p.splits, blocks_y), dim3(kW4sThreads), p.splits, smem, st, p) ==
                  cudaSuccess ? 0 : -4;
 }
 

@@ -36,6 +36,7 @@ _SIGS = {
     "ksana_gemm_fp8_block": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_smallm": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, i64, vp, i32,
                           vp, vp],
+    "ksana_gemm_decode": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_grouped": [i32, vp, i32, vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp, i32, vp, vp],
     "ksana_moe_route": [vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32, i32, vp],
     "ksana_moe_align": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
@@ -281,6 +282,19 @@ def _gemm_smallm(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K, spli
     return dst
 
 
+DECODE_MAX_K_MX = 1 << 17          # (its table of token exponents holds one share's K blocks)
+DECODE_MAX_M = 64                  # rows up to which a decode GEMM is one tile (or share of one) per CTA; beyond: stream-K
+
+
+def _gemm_decode(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K):
+    dst = out if out_f32 is None else out_f32
+    rc = lib().ksana_gemm_decode(kind, _p(x), x.stride(0), _p(xs), xs.stride(0) if xs is not None else 0, _p(w), w.stride(0), _p(ws),
+                                 _p(out) if out_f32 is None else None, _p(out_f32), dst.stride(0), _p(bias), _p(residual),
+                                 residual.stride(0) if residual is not None else 0, M, N, K, _p(err_flag(x.device)), _st())
+    _check(rc, "ksana_gemm_decode")
+    return dst
+
+
 PAIR_MIN_M = 0                     # CTA-pair (cta_group::2) kernel from this many rows; 0 disables it
 
 
@@ -325,6 +339,8 @@ def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_
     if out is None and out_f32 is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     dst = out if out_f32 is None else out_f32
+    if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K % 8 == 0:
+        return _gemm_decode(0, x, None, w, None, out, out_f32, bias, residual, M, N, K)
     if (M <= SMALL_M_BF16 or splits < 0) and M <= 128 and bn == 0 and K % 8 == 0:
         return _gemm_smallm(0, x, None, w, None, out, out_f32, bias, residual, M, N, K, splits)
     if (BF16_TALL_MIN_M > 0 and M >= BF16_TALL_MIN_M and bn == 0 and splits == 0 and N % 8 == 0 and K % 8 == 0
@@ -446,6 +462,9 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
         # M and wherever the tiled kernel would leave most SMs idle; tiled kernel otherwise (256-wide tiles when
         # they fill the SMs).
         t256 = ((M + 127) // 128) * ((N + 255) // 256)
+        # (wide layers at more than 32 rows: the tiled kernel, 86 against 102 us for 64 x 57344 x 8192, 53 against 61 us for 36864 x 7168)
+        if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K <= DECODE_MAX_K_MX and (M <= 32 or N <= 32768):
+            return _gemm_decode(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K)
         skinny = M <= SMALL_M_FP8 or (M <= 128 and _skinny_wins_mx(M, N, K))
         if (skinny or splits != 0) and M <= 128 and bn == 0:
             return _gemm_smallm(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, splits)
