@@ -5,13 +5,15 @@
 // One CTA owns up to 128 packed query rows of one KV head group: row = (token, head inside the group), so the G query
 // heads that share a KV head reuse every staged K/V tile (whole tokens only: 128 / G of them, the rows behind stay idle). Per 128-token KV tile:
 //   S = Q K^T      tcgen05.mma, both operands K-major in shared memory (TMA, 128-byte swizzle), S in TMEM
-//   softmax        4 warps, one thread per row (TMEM lane): no cross-thread reductions; online max with a
-//                  lazy rescale of O (only when a row's maximum grew by more than 2^8)
+//   softmax        8 warps, two threads per row (TMEM lane), 64 columns each, which exchange their maxima through shared
+//                  memory; online max with a lazy rescale of O (only when a row's maximum grew by more than 2^8)
 //   O += P V       tcgen05.mma with P read from TMEM (bf16 pairs written over S's columns by the softmax warps)
 //                  and V as an MN-major shared-memory operand, O accumulating in TMEM
 // Warp roles: warp 0 TMA producer (Q once; K and V tiles through the block table, one box per cache block and
-// 64-column panel), warp 1 MMA issuer + TMEM owner, warps 2..5 softmax + epilogue. Two CTAs share an SM
-// (96 KB of shared memory, 256 TMEM columns each), so one CTA's softmax overlaps the other's MMAs.
+// 64-column panel), warp 1 MMA issuer + TMEM owner, warps 2..9 softmax + epilogue. Two CTAs share an SM
+// (96 KB of shared memory, 256 TMEM columns each), so one CTA's softmax overlaps the other's MMAs. What bounds the kernel is the
+// softmax between the two products: with one thread per row (128 values in registers, part of them spilled) a tile took it
+// longer than both products of two tiles.
 // With sigmoid weights (SIG) a key's weight is sigmoid(score + bias[head][distance]): no maximum, no sum, no rescale; the
 // heads' bias rows are staged in shared memory where they fit. Outputs may be multiplied by the sigmoid of a gate.
 // Every wait is bounded; a timeout sets the error word and leaves the output untouched.
@@ -27,12 +29,14 @@
 namespace ksana {
 
 typedef __nv_bfloat16 bf16;
-constexpr int kFaThreads = 192;
+constexpr int kFaThreads = 320;
+constexpr int kFaSoftmaxThreads = 256;
 constexpr int kFaTile = 128;                 // query rows per CTA and KV tokens per tile
 constexpr int kFaD = 128;                    // padded head size
 constexpr int kFaPanelBytes = kFaTile * 128; // one 64-column panel of a 128-row tile
 constexpr int kFaTileBytes = 2 * kFaPanelBytes;
-constexpr int kFaSmemBytes = 3 * kFaTileBytes + 1024 + 256;
+constexpr int kFaRowBytes = 2 * 128 * 4;     // the rows' maxima, later sums, of the two halves
+constexpr int kFaSmemBytes = 3 * kFaTileBytes + 1024 + 256 + kFaRowBytes;
 constexpr int kFaBiasBytes = 14 * 1024;      // distance biases of a head group that still let two CTAs share an SM
 constexpr uint32_t kFaTmemCols = 256;        // S / P at columns [0,128), O at [128,256)
 constexpr float kFaRescaleLog2 = 8.f;        // O is rescaled only when a row maximum grew by more than this
@@ -89,7 +93,8 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
   uint64_t* o_full = bars + 7;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 8);
   volatile uint32_t* abort_flag = tmem_slot + 1;
-  float* bias_s = reinterpret_cast<float*>(smem + 3 * kFaTileBytes + 256);
+  float* row_s = reinterpret_cast<float*>(smem + 3 * kFaTileBytes + 256);     // [half][row] maxima, at the end sums
+  float* bias_s = row_s + 2 * 128;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int s = blockIdx.z, g = blockIdx.y;
@@ -113,7 +118,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1); mbar_init(k_full, 1); mbar_init(k_empty, 1); mbar_init(v_full, 1); mbar_init(v_empty, 1);
-    mbar_init(s_full, 1); mbar_init(p_full, 4); mbar_init(o_full, 1);
+    mbar_init(s_full, 1); mbar_init(p_full, 8); mbar_init(o_full, 1);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -212,32 +217,42 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     }
     __syncwarp();
   } else {
-    // ------------------------------------------------------------------ softmax + epilogue (one thread per row)
-    const int qd = warp & 3;
+    // ------------------------------------------------------------------ softmax + epilogue (two threads per row)
+    const int qd = warp & 3, half = (warp - 2) >> 2;       // TMEM lanes of the warp; columns [64 half, 64 half + 64) of S and O
+    const int cb = half * 64, rl = qd * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(qd * 32) << 16;
-    const int vr = row0 + qd * 32 + lane;                  // packed row index inside the sequence
-    const bool active = qd * 32 + lane < p.rows && vr < q_len * G;
+    const int vr = row0 + rl;                              // packed row index inside the sequence
+    const bool active = rl < p.rows && vr < q_len * G;
     const int tok = vr / G, head = g * G + vr % G;
     const int limit = active ? past + tok : -1;            // last visible KV position
     const int lo = WIN ? limit - p.window + 1 : 0;            // first position inside the window
     const int keep = WIN ? p.keep : 0;
-    auto sees = [&](int pos) { return pos <= limit && (!WIN || pos >= lo || pos < keep); };
     const float slope2 = (p.alibi && active) ? p.alibi[head] * 1.44269504f : 0.f;
     const float* near = SIG ? bias_s + (vr % G) * p.bias_ld + kFaTile : nullptr;
     const float* tab = SIG ? p.bias + static_cast<size_t>(head) * p.bias_len : nullptr;
     const int bias_last = SIG ? p.bias_len - 1 : 0;
+    // the two warps of these rows
+    auto pair_sync = [&]() {
+      if (qd == 0) asm volatile("bar.sync 1, 64;" ::: "memory");
+      else if (qd == 1) asm volatile("bar.sync 2, 64;" ::: "memory");
+      else if (qd == 2) asm volatile("bar.sync 3, 64;" ::: "memory");
+      else asm volatile("bar.sync 4, 64;" ::: "memory");
+    };
     float m_used = -CUDART_INF_F, l = 0.f;
     bool ok = true;
     for (int j = 0; j < ntiles; ++j) {
       const uint32_t par = j & 1;
-      const int t0 = tile_start(j);
-      if (!mbar_wait(s_full, par, abort_flag)) { ok = false; break; }
+      const int t0 = tile_start(j), c0 = t0 + cb;          // first position of the tile, of this half
+      if (ok) ok = mbar_wait(s_full, par, abort_flag);
       tc_fence_after();
       const bool biased = slope2 != 0.f || p.scale_log2 <= 0.f;
-      const bool need_mask = (t0 + kFaTile - 1 > limit) ||
-                             (WIN && t0 < lo && t0 + kFaTile > keep);
+      const bool need_mask = (c0 + 63 > limit) || (WIN && c0 < lo && c0 + 64 > keep);
       // lazy rescale of O: keep the old reference maximum unless the row's maximum grew by more than 2^8
       auto update_reference = [&](float mx) {
+        // both halves are in registers once the maxima are exchanged: P may be written over S
+        row_s[half * 128 + rl] = mx;
+        pair_sync();
+        mx = fmaxf(mx, row_s[(half ^ 1) * 128 + rl]);
         float m_new = m_used;
         if (mx > m_used + kFaRescaleLog2 || m_used == -CUDART_INF_F) m_new = (mx == -CUDART_INF_F) ? m_used : mx;
         const bool grow = j > 0 && m_new != m_used && m_used != -CUDART_INF_F;
@@ -246,38 +261,38 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
           l *= f;
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
-            uint32_t o[32];
-            tmem_ld32(tmem_o + lane_off + c * 32, o);
+            uint32_t o[16];
+            tmem_ld16(tmem_o + lane_off + cb + c * 16, o);
             tmem_ld_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
-            tmem_st32(tmem_o + lane_off + c * 32, o);
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * f);
+            tmem_st16(tmem_o + lane_off + cb + c * 16, o);
           }
         }
         m_used = m_new;
         return (m_used == -CUDART_INF_F) ? 0.f : m_used;
       };
-      if constexpr (SIG) {
-        uint32_t r[128];
+      uint32_t r[64];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(tmem_s + lane_off + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
-        tmem_ld_wait();
-        const int from = limit - t0;                       // distance of the tile's first key
+      for (int c = 0; c < 2; ++c) tmem_ld32(tmem_s + lane_off + cb + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
+      tmem_ld_wait();
+      if constexpr (SIG) {
+        const int from = limit - c0;                       // distance of the half's first key
         // the row's visible keys as bits
-        uint32_t seen[4] = {~0u, ~0u, ~0u, ~0u};
+        uint32_t seen[2] = {~0u, ~0u};
         const bool masked = __any_sync(0xffffffffu, need_mask);
         if (masked) {
-          const int last = from, first = lo - t0, kept = keep - t0;
+          const int last = from, first = lo - c0, kept = keep - c0;
 #pragma unroll
-          for (int c = 0; c < 4; ++c) {
+          for (int c = 0; c < 2; ++c) {
             auto below = [&](int n) { return n - c * 32 >= 32 ? ~0u : n - c * 32 <= 0 ? 0u : (1u << (n - c * 32)) - 1u; };   // keys before n
             seen[c] = below(last + 1);
             if (WIN) seen[c] &= ~below(first) | below(kept);
           }
         }
-        auto weigh = [&](auto bias_at) {                   // -log2(e) times the bias of the tile's key i
+        auto weigh = [&](auto bias_at) {                   // -log2(e) times the bias of the half's key i
 #pragma unroll
-          for (int i = 0; i < 128; i += 2) {
+          for (int i = 0; i < 64; i += 2) {
             float w2[2];
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
@@ -288,7 +303,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
             r[i >> 1] = *reinterpret_cast<uint32_t*>(&pb);
           }
         };
-        const bool far = from - (kFaTile - 1) >= bias_last;      // every distance of the row has the last bias
+        const bool far = from - 63 >= bias_last;           // every distance of the row has the last bias
         if (__all_sync(0xffffffffu, far || !active)) {
           const float b = tab[bias_last] * -1.44269504f;
           weigh([&](int) { return b; });
@@ -299,84 +314,50 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         } else {
           weigh([&](int i) { return tab[min(max(from - i, 0), bias_last)] * -1.44269504f; });
         }
+        pair_sync();                                       // the other half has read its part of S, which P is written over
+      } else {
+        // hidden keys (window, diagonal) become -inf in registers
+        const bool any_biased = __any_sync(0xffffffffu, biased);
+        if (any_biased) {                                  // ALiBi (or a scale that is not positive): the finished logits
 #pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_st16(tmem_s + lane_off + c * 16, *reinterpret_cast<uint32_t(*)[16]>(&r[c * 16]));
-      } else if (!__any_sync(0xffffffffu, biased)) {
-        // the whole row in registers with a single TMEM round trip; hidden keys (window, diagonal) become -inf there
-        uint32_t r[128];
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_ld32(tmem_s + lane_off + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
-        tmem_ld_wait();
+          for (int i = 0; i < 64; ++i)
+            r[i] = __float_as_uint(__uint_as_float(r[i]) * p.scale_log2 + slope2 * static_cast<float>(c0 + i - limit));
+        }
         if (__any_sync(0xffffffffu, need_mask)) {
-          const int last = limit - t0, first = lo - t0, kept = keep - t0;       // column bounds of this row
+          const int last = limit - c0, first = lo - c0, kept = keep - c0;       // column bounds of this row
 #pragma unroll
-          for (int i = 0; i < 128; ++i)
+          for (int i = 0; i < 64; ++i)
             if (i > last || (WIN && i < first && i >= kept)) r[i] = 0xff800000u;
         }
         float mx4[4] = {-CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F, -CUDART_INF_F};
 #pragma unroll
-        for (int i = 0; i < 128; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i]));
-        const float mref = update_reference(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * p.scale_log2);
+        for (int i = 0; i < 64; ++i) mx4[i & 3] = fmaxf(mx4[i & 3], __uint_as_float(r[i]));
+        const float factor = any_biased ? 1.f : p.scale_log2;
+        const float mref = update_reference(fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * factor);
         float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 128; i += 2) {
-          const float p0 = fast_exp2(fmaf(__uint_as_float(r[i]), p.scale_log2, -mref));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(r[i + 1]), p.scale_log2, -mref));
+        for (int i = 0; i < 64; i += 2) {
+          const float p0 = fast_exp2(fmaf(__uint_as_float(r[i]), factor, -mref));
+          const float p1 = fast_exp2(fmaf(__uint_as_float(r[i + 1]), factor, -mref));
           l4[(i >> 1) & 3] += p0 + p1;
           __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
           r[i >> 1] = *reinterpret_cast<uint32_t*>(&pb);        // in place: slot i/2 has already been consumed
         }
         l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) tmem_st16(tmem_s + lane_off + c * 16, *reinterpret_cast<uint32_t(*)[16]>(&r[c * 16]));
-      } else {
-        // ALiBi (or a scale that is not positive): masked two-pass form
-        float mx = -CUDART_INF_F;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tmem_s + lane_off + c * 32, r);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            const int pos = t0 + c * 32 + i;
-            const float v = __uint_as_float(r[i]) * p.scale_log2 + slope2 * static_cast<float>(pos - limit);
-            mx = fmaxf(mx, sees(pos) ? v : -CUDART_INF_F);
-          }
-        }
-        const float mref = update_reference(mx);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t r[32];
-          tmem_ld32(tmem_s + lane_off + c * 32, r);
-          tmem_ld_wait();
-          uint32_t pk[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 2) {
-            const int pos = t0 + c * 32 + i;
-            const float v0 = __uint_as_float(r[i]) * p.scale_log2 + slope2 * static_cast<float>(pos - limit) - mref;
-            const float v1 = __uint_as_float(r[i + 1]) * p.scale_log2 + slope2 * static_cast<float>(pos + 1 - limit) - mref;
-            const float p0 = sees(pos) ? fast_exp2(v0) : 0.f;
-            const float p1 = sees(pos + 1) ? fast_exp2(v1) : 0.f;
-            l += p0 + p1;
-            __nv_bfloat162 pb = __floats2bfloat162_rn(p0, p1);
-            pk[i >> 1] = *reinterpret_cast<uint32_t*>(&pb);
-          }
-          tmem_st16(tmem_s + lane_off + c * 16, pk);
-        }
       }
+      tmem_st32(tmem_s + lane_off + half * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
       tmem_st_wait();
       if (t0 + kFaTile > kv_len) {
         // last tile of the sequence: V rows past the sequence end hold stale shared memory or whatever the cache
         // has there; their probabilities are 0, but 0 x NaN would poison O. Zero them before the PV MMA reads.
         // (the keys' product is complete here, so a shared tile is free to be changed)
-        if (!p.shared && !mbar_wait(v_full, par, abort_flag)) { ok = false; break; }
+        if (!p.shared && ok) ok = mbar_wait(v_full, par, abort_flag);
         uint8_t* vt = p.shared && !(j & 1) ? k_s : v_s;
         const int first_bad = kv_len - t0;
-        const int nchunks = (kFaTile - first_bad) * 16;       // 16-byte chunks per row: 2 panels x 8
-        for (int i = threadIdx.x - 64; i < nchunks; i += 128) {
-          const int r = first_bad + (i >> 4), ch = i & 15;
-          *reinterpret_cast<uint4*>(vt + (ch >> 3) * kFaPanelBytes + r * 128 + (((ch & 7) ^ (r & 7)) << 4)) =
+        const int nchunks = ok ? (kFaTile - first_bad) * 16 : 0;       // 16-byte chunks per row: 2 panels x 8
+        for (int i = threadIdx.x - 64; i < nchunks; i += kFaSoftmaxThreads) {
+          const int r_ = first_bad + (i >> 4), ch = i & 15;
+          *reinterpret_cast<uint4*>(vt + (ch >> 3) * kFaPanelBytes + r_ * 128 + (((ch & 7) ^ (r_ & 7)) << 4)) =
               make_uint4(0, 0, 0, 0);
         }
         fence_async_smem();
@@ -385,24 +366,29 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
       __syncwarp();
       if (lane == 0) mbar_arrive(p_full);
     }
+    pair_sync();                                           // the last tile's maxima have been read
+    row_s[half * 128 + rl] = l;
+    pair_sync();
     if (ok && mbar_wait(o_full, 0, abort_flag)) {
       tc_fence_after();
-      if (p.sinks && active) l += exp2f(p.sinks[head] * 1.44269504f - m_used);
-      const float inv = SIG ? 1.f : l > 0.f ? 1.f / l : 0.f;
+      float lt = row_s[rl] + row_s[128 + rl];
+      if (p.sinks && active) lt += exp2f(p.sinks[head] * 1.44269504f - m_used);
+      const float inv = SIG ? 1.f : lt > 0.f ? 1.f / lt : 0.f;
       bf16* dst = p.out + static_cast<size_t>(q0 + tok) * p.out_stride + head * p.Dv;
       const bf16* gate = SIG && p.gate ? p.gate + static_cast<size_t>(q0 + tok) * p.gate_stride + head * p.Dv : nullptr;
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        if (c * 32 >= p.Dv) break;
+      for (int c = 0; c < 2; ++c) {
+        const int col = cb + c * 32;
+        if (col >= p.Dv) break;
         uint32_t r[32];
-        tmem_ld32(tmem_o + lane_off + c * 32, r);
+        tmem_ld32(tmem_o + lane_off + col, r);
         tmem_ld_wait();
         if (active) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
-            if (c * 32 + i >= p.Dv) break;
+            if (col + i >= p.Dv) break;
             if (SIG && gate) {
-              const uint4 gv = *reinterpret_cast<const uint4*>(gate + c * 32 + i);
+              const uint4 gv = *reinterpret_cast<const uint4*>(gate + col + i);
               const __nv_bfloat162* g2 = reinterpret_cast<const __nv_bfloat162*>(&gv);
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -416,7 +402,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
 #pragma unroll
             for (int e = 0; e < 4; ++e)
               o2[e] = __floats2bfloat162_rn(__uint_as_float(r[i + 2 * e]) * inv, __uint_as_float(r[i + 2 * e + 1]) * inv);
-            *reinterpret_cast<uint4*>(dst + c * 32 + i) = ov;
+            *reinterpret_cast<uint4*>(dst + col + i) = ov;
           }
         }
       }
