@@ -99,6 +99,10 @@ _SIGS = {
     "ksana_cast_f32": [vp, vp, i64, vp],
     "ksana_paged_prefill_tc": [vp, i64, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32,
                                i32, i32, f32, i32, vp, i32, vp, i64, f32, vp, vp],
+    "ksana_paged_prefill_pair": [vp, i64, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32,
+                                 vp, vp],
+    "ksana_mha_prefill": [vp, i64, vp, vp, i64, i64, vp, vp, vp, i32, i32, i32, vp, f32, vp, vp],
+    "ksana_gather_latents": [vp, i64, i32, i32, vp, i32, vp, vp, vp, i32, i32, i32, vp],
     "ksana_paged_prefill": [vp, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, i32,
                             f32, i32, f32, f32, i32, vp, i32, vp, i64, f32, vp, vp],
     "ksana_paged_decode": [vp, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32,
@@ -931,6 +935,7 @@ def rope_kv_append(qkv, positions, slots, cos_sin, cache_layer, block_stride, bl
 
 
 PREFILL_TC = True                  # prefill attention on tcgen05 where the kernel covers the configuration
+PREFILL_PAIR = True          # its form with two query tiles per CTA
 
 
 def _panels(cache_layer, v_cache, D):
@@ -971,6 +976,14 @@ def paged_prefill(q, q_stride, out, cache_layer, block_stride, block_tokens, blo
     fp8 = cache_layer.dtype != torch.bfloat16
     kc, vc, Dv = _panels(cache_layer, v_cache, D)
     nblocks = int(cache_layer.shape[0])
+    if PREFILL_TC and PREFILL_PAIR and not fp8 and max(D, Dv) <= 128 and window == 0 and weights is None and max_q_len * (Hq // Hkv) > 128:
+        # two query tiles per CTA; -100 = configuration not covered
+        rc = lib().ksana_paged_prefill_pair(_p(q), q_stride, q.shape[0], _p(out), out.stride(0), kc, vc, block_stride, block_tokens,
+                                            _p(block_table), block_table.stride(0), _p(cu_q), _p(kv_lens), _p(alibi), _p(sinks), B,
+                                            max_q_len, Hq, Hkv, D, Dv, float(scale), nblocks, _p(err_flag(q.device)), _st())
+        if rc != -100:
+            _check(rc, "ksana_paged_prefill_pair")
+            return
     if PREFILL_TC and not fp8 and max(D, Dv) <= 128:
         # tcgen05 kernel (head sizes up to 128, bf16 cache, groups of up to 128 heads); -100 = configuration not covered
         rc = lib().ksana_paged_prefill_tc(_p(q), q_stride, q.shape[0], _p(out), out.stride(0), kc, vc, block_stride,
@@ -1088,6 +1101,25 @@ def mla_rope_append(q, nope, kv, norm_w, eps, positions, slots, cos_sin, qfull, 
         _p(q), q.stride(0), nope, _p(kv), kv.stride(0) if kv is not None else 0, _p(norm_w), float(eps), _p(positions), _p(slots),
         _p(cos_sin), _p(qfull), _p(cache), cache.stride(0), block_tokens, T, G, rank, int(cos_sin.shape[1]), int(cos_sin.shape[0]),
         int(cache.shape[0]) * block_tokens, int(q.dtype == torch.float32), _p(err_flag(q.device)), _st()), "ksana_mla_rope_append")
+
+
+def gather_latents(cache, block_tokens, block_table, kv_lens, cu_k, total, max_kv_len):
+    """Cached latent rows of whole sequences one after the other: [total, DK]; sequence s from row cu_k[s] on."""
+    out = torch.empty(total, cache.shape[-1], dtype=cache.dtype, device=cache.device)
+    _check(lib().ksana_gather_latents(_p(cache), cache.stride(0), block_tokens, cache.shape[-1], _p(block_table), block_table.stride(0),
+                                      _p(kv_lens), _p(cu_k), _p(out), kv_lens.numel(), max_kv_len, int(cache.shape[0]), _st()),
+           "ksana_gather_latents")
+    return out
+
+
+def mha_prefill(q, kx, pe, cu_q, cu_k, kv_lens, max_q_len, scale):
+    """Attention of q [T, heads, 192] against expanded latents: kx [tokens, heads, 128 keys | 128 values], pe [tokens, 64] (a column
+    range): the key columns that all heads share. Sequence s owns the rows cu_k[s] .. cu_k[s] + kv_lens[s]. [T, heads, 128]."""
+    T, G, _ = q.shape
+    out = torch.empty(T, G, 128, dtype=q.dtype, device=q.device)
+    _check(lib().ksana_mha_prefill(_p(q), T, _p(kx), _p(pe), pe.stride(0), kx.shape[0], _p(cu_q), _p(cu_k), _p(kv_lens), kv_lens.numel(),
+                                   max_q_len, G, _p(out), float(scale), _p(err_flag(q.device)), _st()), "ksana_mha_prefill")
+    return out
 
 
 def mla_splits(num_seqs: int, max_q_len: int, max_kv: int, sms: int = 148, halves: int = 2) -> int:
