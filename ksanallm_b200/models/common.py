@@ -42,6 +42,8 @@ class StepInput:
     num_multi_tokens: int = 0
     max_q_len: int = 0
     max_kv_len: int = 0                  # host-side upper bound of kv_lens (split heuristics, no device sync)
+    total_kv_len: int = 0                # sum of kv_lens and (query, visible key) pairs of the step, where the host knows them
+    pairs: int = 0
     logits_rows: Optional[torch.Tensor] = None
     mrope_positions: Optional[torch.Tensor] = None      # [3, T]
     refit_positions: Optional[torch.Tensor] = None      # rows to overwrite with plugin embeddings

@@ -37,8 +37,9 @@ class MLAWeights:
     q_b: LinearWeight                    # [Hq*(nope+rope), q_lora_rank or H]
     kv_a: LinearWeight                   # [kv_lora_rank + rope, H]
     kv_a_norm: torch.Tensor
-    w_uk: torch.Tensor                   # [Hq, nope, kv_lora_rank]
+    w_uk: torch.Tensor                   # [Hq, nope, kv_lora_rank] (both views of one tensor [Hq, nope + v_dim, kv_lora_rank])
     w_uv: torch.Tensor                   # [Hq, v_dim, kv_lora_rank]
+    kv_b: Optional[torch.Tensor] = None  # that tensor
     w_uk_t: Optional[torch.Tensor] = None    # [Hq, kv_lora_rank, nope]: W_uk as the K-major operand of the batched GEMM (built on first use)
 
 
@@ -119,12 +120,41 @@ class DeepseekModel(CommonModel):
                 and q.dtype == torch.bfloat16 and self.block_tokens in (8, 16, 32, 64, 128, 256)
                 and self.kv_cache is not None and self.kv_cache.dtype == torch.bfloat16)
 
+    def _expands(self, mw, step, T) -> bool:
+        """Whether a step's latents are better expanded to keys and values of every head than attended as they are. Per (query, key)
+        pair and head the absorbed form takes 2 x 1088 operations at about 330 TFLOP/s, the expanded one 2 x 320 at about 700, which
+        costs 2 x 512 x 256 per cached token and head (and writing the result) but saves the two per-head products of every query
+        row: 50 ns per cached token against 143 ns per row at 128 heads."""
+        if (mw.kv_b is None or step.num_single or not step.pairs or (self.nope, self.rope, self.vdim, self.lora) != (128, 64, 128, 512)
+                or step.total_kv_len * self.Hq * 512 > 4 << 30):
+            return False
+        share = self.Hq / 128
+        absorbed = step.pairs * self.Hq * 2 * 1088 / 330e12 + T * share * 143e-9
+        return step.pairs * self.Hq * 2 * 320 / 700e12 + step.total_kv_len * share * 50e-9 < 0.9 * absorbed
+
+    def _attention_expanded(self, mw, q, kv, step, cache):
+        """Prompts: keys and values of every head from the cached latents (one plain GEMM), attention over 192 / 128 columns."""
+        from ..ops import native
+        T, Hq = q.shape[0], self.Hq
+        args = (step.positions, step.slots, self.cos_sin)
+        unused = torch.empty(T, 1, self.lora + self.rope, dtype=q.dtype, device=q.device)
+        native.mla_rope_append(q, self.nope, kv, mw.kv_a_norm, self.cfg.rms_norm_eps, *args, unused, cache, self.block_tokens, 1, self.lora)
+        native.mla_rope_append(q, self.nope, None, None, 0.0, *args, q, cache, self.block_tokens, Hq, self.nope)     # in place
+        cu_k = torch.nn.functional.pad(torch.cumsum(step.kv_lens, 0, dtype=torch.int32), (1, 0))
+        lat = native.gather_latents(cache, self.block_tokens, step.block_table, step.kv_lens, cu_k, step.total_kv_len, step.max_kv_len)
+        kx = native.gemm_bf16(lat[:, :self.lora], mw.kv_b.view(-1, self.lora))
+        o = native.mha_prefill(q.view(T, Hq, -1), kx.view(-1, Hq, self.nope + self.vdim), lat[:, self.lora:], step.cu_q, cu_k, step.kv_lens,
+                               step.max_q_len, self.scale)
+        return o.view(T, Hq * self.vdim)
+
     def _attention_native(self, li, mw, q, kv, step):
         """Fused latent norm + rotations + cache append, q_nope W_uk as a batched GEMM into the packed query rows,
         the tcgen05 latent-attention kernel (prefill rows and decode rows in one launch), then W_uv."""
         from ..ops import native
         T, Hq = q.shape[0], self.Hq
         cache = self.kv_cache[:, li - self.layer_lo]                # [blocks, bt, 576]
+        if self._expands(mw, step, T):
+            return self._attention_expanded(mw, q, kv, step, cache)
         qfull = torch.empty(T, Hq, self.lora + self.rope, dtype=q.dtype, device=q.device)
         native.mla_rope_append(q, self.nope, kv, mw.kv_a_norm, self.cfg.rms_norm_eps, step.positions, step.slots,
                                self.cos_sin, qfull, cache, self.block_tokens, Hq, self.lora)
@@ -173,8 +203,8 @@ def build_deepseek(cfg: ModelConfig, source, tp_rank, tp_size, comm, device, dty
         kv_a_norm = get(p + "kv_a_layernorm.weight", (lora,), "ones").to(device=device, dtype=dtype)
         kv_b = _dense(_rows(get(p + "kv_b_proj.weight", (Hq_all * (nope + vdim), lora)), tp_rank, tp_size)).to(device)
         kv_b = kv_b.float().view(Hq, nope + vdim, lora)
-        mla = MLAWeights(q_a, q_a_norm, q_b, kv_a, kv_a_norm, kv_b[:, :nope].contiguous().to(dtype),
-                         kv_b[:, nope:].contiguous().to(dtype))
+        kv_b = kv_b.to(dtype)
+        mla = MLAWeights(q_a, q_a_norm, q_b, kv_a, kv_a_norm, kv_b[:, :nope], kv_b[:, nope:], kv_b)
         o_w = _cols(get(p + "o_proj.weight", (H, Hq_all * vdim)), tp_rank, tp_size)
         lp = f"model.layers.{li}."
         lw = LayerWeights(

@@ -303,6 +303,9 @@ class ModelRunner:
             setattr(step, name, take(T if per_row else nseq))
         kv_lens = np.asarray(plan.kv_lens)
         step.max_kv_len = int(kv_lens.max()) if nseq else 0
+        if plan.num_multi:
+            new, all_ = np.diff(np.asarray(plan.cu_q)).astype(np.int64), kv_lens.astype(np.int64)
+            step.total_kv_len, step.pairs = int(all_.sum()), int((new * all_ - new * (new - 1) // 2).sum())
         step.sample_k = self.candidate_k(plan, extra)
         if plan.num_single:
             max_kv = int(kv_lens[plan.num_multi:].max())
