@@ -7,7 +7,10 @@
 // holds 256 elements = four MMAs of K = 64; each MMA consumes four scales per row, i.e. exactly one 32-bit
 // TMEM word of the 512-byte scale chunk (see gemm_tcgen05_mx.cu for the chunk layout). Per K block of 256
 // elements the scale warp reads 16 scale bytes per row and writes one chunk per MMA and 128-row group.
-// Same warp roles, single 256-column accumulator and bounded waits as the FP8 hardware-scaled kernel.
+// Warp 0 TMA producer, warp 1 MMA issuer, warps 2 and 3 scale packers (alternate K blocks), warps 4..11 epilogue; single 256-column
+// accumulator and bounded waits as in the FP8 hardware-scaled kernel. A K block of MMAs takes about 500 clocks, an SM's intake of its
+// 48 KB of operands about 800: one packer that loaded a block's scales when their buffer was free took 2200 (the latency of its
+// loads), so two of them work in turn, each with the loads of its next block in flight.
 //
 // No counterpart in the reference (its low-bit paths are GPTQ/AWQ W4A16 through Marlin/Machete,
 // 3rdparty/LLM_kernels/csrc/kernels/nvidia/mixture_of_experts and .../machete); the operator is specified by
@@ -21,7 +24,7 @@ namespace ksana {
 constexpr int kF4BM = 128;
 constexpr int kF4RowBytes = 128;
 constexpr int kF4SfStages = 4;
-constexpr int kF4Threads = 96 + 256;
+constexpr int kF4Threads = 128 + 256;
 
 template <int BN>
 struct F4Cfg {
@@ -175,62 +178,80 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       }
     }
     __syncwarp();
-  } else if (warp == 2) {
-    // ------------------------------------------------------------- scale packer
-    int sfs = 0; uint32_t sf_phase = 0;
-    bool ok = true;
+  } else if (warp < 4) {
+    // ------------------------------------------------------------ scale packers
     constexpr int kPerMma = 1 + Cfg::kBChunks;
-    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-      int m_blk, n_blk;
-      f4_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
-      size_t w_row0 = 0;
-      if (p.tile_expert) {
-        const int e = p.tile_expert[m_blk];
-        if (e < 0) continue;
-        w_row0 = static_cast<size_t>(e) * p.expert_rows;
+    struct Raw { uint4 a[4]; uint4 b[Cfg::kBChunks][4]; };
+    // this packer's K blocks: every second one of the CTA's (tile, K block) sequence
+    auto next_tile = [&](int t) {
+      for (; t < num_tiles; t += gridDim.x) {
+        int m_blk, n_blk;
+        f4_tile_coords(t, m_tiles, n_tiles, m_blk, n_blk);
+        if (!p.tile_expert || p.tile_expert[m_blk] >= 0) break;
       }
-      for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) { ok = false; break; }
-        uint8_t* buf = sf_smem + sfs * Cfg::kSfStageBytes;
-        // rows of A: 16 scale bytes per row and K block = one 32-bit word per MMA
-        uint4 ra[4];
+      return t;
+    };
+    auto advance = [&](int& t, int& kb, int by) {
+      for (kb += by; kb >= num_kb && t < num_tiles; kb -= num_kb) t = next_tile(t + static_cast<int>(gridDim.x));
+    };
+    auto fetch = [&](int t, int kb, Raw& r) {           // 16 scale bytes per row and K block = one 32-bit word per MMA
+      int m_blk, n_blk;
+      f4_tile_coords(t, m_tiles, n_tiles, m_blk, n_blk);
+      const size_t w_row0 = p.tile_expert ? static_cast<size_t>(p.tile_expert[m_blk]) * p.expert_rows : 0;
+#pragma unroll
+      for (int r4 = 0; r4 < 4; ++r4) {
+        const int row = m_blk * kF4BM + r4 * 32 + lane;
+        r.a[r4] = row < p.M ? *reinterpret_cast<const uint4*>(p.a_bs + static_cast<size_t>(row) * p.a_bs_ld + kb * 16)
+                            : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int c = 0; c < Cfg::kBChunks; ++c)
 #pragma unroll
         for (int r4 = 0; r4 < 4; ++r4) {
-          const int row = m_blk * kF4BM + r4 * 32 + lane;
-          ra[r4] = row < p.M ? *reinterpret_cast<const uint4*>(p.a_bs + static_cast<size_t>(row) * p.a_bs_ld + kb * 16)
-                             : make_uint4(0, 0, 0, 0);
+          const int n = n_blk * BN + c * 128 + r4 * 32 + lane;
+          r.b[c][r4] = n < p.N ? *reinterpret_cast<const uint4*>(p.w_bs + (w_row0 + n) * p.w_bs_ld + kb * 16)
+                               : make_uint4(0, 0, 0, 0);
         }
-        uint4 rb[Cfg::kBChunks][4];
+    };
+    uint32_t seq = warp - 2;                            // place of the block in the sequence
+    auto emit = [&](const Raw& r) -> bool {
+      const int sfs = seq % kF4SfStages;
+      if (!mbar_wait(&sf_empty[sfs], ((seq / kF4SfStages) & 1) ^ 1, abort_flag)) return false;
+      uint8_t* buf = sf_smem + sfs * Cfg::kSfStageBytes;
+      auto word = [](const uint4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
 #pragma unroll
-        for (int c = 0; c < Cfg::kBChunks; ++c) {
+      for (int k = 0; k < 4; ++k) {
+        *reinterpret_cast<uint4*>(buf + (k * kPerMma) * 512 + lane * 16) =
+            make_uint4(word(r.a[0], k), word(r.a[1], k), word(r.a[2], k), word(r.a[3], k));
 #pragma unroll
-          for (int r4 = 0; r4 < 4; ++r4) {
-            const int n = n_blk * BN + c * 128 + r4 * 32 + lane;
-            rb[c][r4] = n < p.N ? *reinterpret_cast<const uint4*>(p.w_bs + (w_row0 + n) * p.w_bs_ld + kb * 16)
-                                : make_uint4(0, 0, 0, 0);
-          }
-        }
-        auto word = [](const uint4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          *reinterpret_cast<uint4*>(buf + (k * kPerMma) * 512 + lane * 16) =
-              make_uint4(word(ra[0], k), word(ra[1], k), word(ra[2], k), word(ra[3], k));
-#pragma unroll
-          for (int c = 0; c < Cfg::kBChunks; ++c)
-            *reinterpret_cast<uint4*>(buf + (k * kPerMma + 1 + c) * 512 + lane * 16) =
-                make_uint4(word(rb[c][0], k), word(rb[c][1], k), word(rb[c][2], k), word(rb[c][3], k));
-        }
-        fence_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&sf_full[sfs]);
-        if (++sfs == kF4SfStages) { sfs = 0; sf_phase ^= 1; }
+        for (int c = 0; c < Cfg::kBChunks; ++c)
+          *reinterpret_cast<uint4*>(buf + (k * kPerMma + 1 + c) * 512 + lane * 16) =
+              make_uint4(word(r.b[c][0], k), word(r.b[c][1], k), word(r.b[c][2], k), word(r.b[c][3], k));
       }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&sf_full[sfs]);
+      seq += 2;
+      return true;
+    };
+    int t = next_tile(blockIdx.x), kb = 0;              // block of the set that is fetched next
+    if (t < num_tiles) advance(t, kb, warp - 2);
+    Raw r0, r1;
+    bool have0 = t < num_tiles, have1;
+    if (have0) { fetch(t, kb, r0); advance(t, kb, 2); }
+    while (have0) {
+      have1 = t < num_tiles;
+      if (have1) { fetch(t, kb, r1); advance(t, kb, 2); }
+      if (!emit(r0) || !have1) break;
+      have0 = t < num_tiles;
+      if (have0) { fetch(t, kb, r0); advance(t, kb, 2); }
+      if (!emit(r1)) break;
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    const int wg = (warp - 3) >> 2;
+    const int wg = (warp - 4) >> 2;
     constexpr int EC = Cfg::kEpiCols;
     const int col_off = wg * EC;
     int acc = 0; uint32_t acc_phase = 0;
