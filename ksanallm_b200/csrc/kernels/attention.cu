@@ -639,21 +639,26 @@ paged_decode_kernel(const AttnParams p) {
 constexpr int kStreamThreads = 160;      // 4 warps that compute, 1 that loads
 constexpr int kStreamMaxStages = 8;
 constexpr int kStreamMinTiles = 1;       // tiles per CTA below which fewer CTAs take part
+// What an item costs beside its tiles (its query rows, the merge of the warps, the piece that is handed over), in tiles: the line that
+// is cut has so many empty units behind every item.
+constexpr int kStreamItemUnits = 2;
 
 __device__ __forceinline__ void stream_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
-struct StreamItem { int s, h, t0, t1, n; };     // tiles [t0, t1) of the n tiles of sequence s, row group h
+struct StreamItem { int s, h, t0, t1, n, units; };     // tiles [t0, t1) of the n tiles of sequence s, row group h; units taken of the line
 
-// the item of unit u; `s` only ever moves forward
+// the item of unit u (t0 = t1: only the empty units behind its tiles); `s` only ever moves forward
 __device__ __forceinline__ void stream_item(const int* first, int heads, long long u, long long end, int& s, StreamItem& it) {
   while (static_cast<long long>(first[s + 1]) * heads <= u) ++s;
   const int n = first[s + 1] - first[s];
   const long long r = u - static_cast<long long>(first[s]) * heads;
-  it.s = s; it.n = n;
+  it.s = s; it.n = n - kStreamItemUnits;
   it.h = r < (1LL << 31) ? static_cast<int>(r) / n : static_cast<int>(r / n);
-  it.t0 = static_cast<int>(r - static_cast<long long>(it.h) * n);
+  const int at = static_cast<int>(r - static_cast<long long>(it.h) * n);
   const long long room = end - u;
-  it.t1 = room < n - it.t0 ? it.t0 + static_cast<int>(room) : n;
+  it.units = room < n - at ? static_cast<int>(room) : n - at;
+  it.t0 = min(at, it.n);
+  it.t1 = min(at + it.units, it.n);
 }
 
 __device__ __forceinline__ TileRange decode_tiles(const AttnParams& p, int kv_len) {
@@ -798,7 +803,7 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
 #pragma unroll 4
   for (int s0 = 0; s0 < p.B; s0 += 32) {
     const int s = s0 + lane;
-    int x = s < p.B ? max(1, decode_tiles(p, p.kv_lens[s]).count) : 0;
+    int x = s < p.B ? max(1, decode_tiles(p, p.kv_lens[s]).count) + kStreamItemUnits : 0;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -841,8 +846,9 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
     bool ok = true;
     const int bt = p.block_tokens;
     StreamItem it;
-    for (long long u = u_begin; u < u_end && ok; u += it.t1 - it.t0) {
+    for (long long u = u_begin; u < u_end && ok; u += it.units) {
       stream_item(first, heads, u, u_end, s_at, it);
+      if (it.t0 == it.t1) continue;
       const int kv_len = p.kv_lens[it.s], g = it.h / groups;
       const int* table = p.block_table + static_cast<size_t>(it.s) * p.table_stride;
       const TileRange tiles = decode_tiles(p, kv_len);
@@ -870,8 +876,9 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
     int stage = 0; uint32_t phase = 0;
     bool ok = true;
     StreamItem it;
-    for (long long u = u_begin; u < u_end; u += it.t1 - it.t0) {
+    for (long long u = u_begin; u < u_end; u += it.units) {
       stream_item(first, heads, u, u_end, s_at, it);
+      if (it.t0 == it.t1) continue;
       const int kv_len = p.kv_lens[it.s], s = it.s;
       const int g = it.h / groups, head0 = g * GA + (it.h % groups) * 16;
       const int G = min(16, (g + 1) * GA - head0);             // query heads of this item: head0 .. head0 + G
