@@ -205,8 +205,8 @@ __global__ void moe_permute_fp8_kernel(const uint8_t* __restrict__ q, const floa
 __global__ void moe_combine_kernel(const bf16* __restrict__ y, const int* __restrict__ dst_row,
                                    const float* __restrict__ topk_w, bf16* __restrict__ out, int K, int H,
                                    int accumulate, int cap, int* err) {
-  const int t = blockIdx.x;
-  for (int i = threadIdx.x; i < (H >> 3); i += blockDim.x) {
+  const int t = blockIdx.x;                     // (blockIdx.y: a share of the columns, where there are few tokens)
+  for (int i = blockIdx.y * blockDim.x + threadIdx.x; i < (H >> 3); i += gridDim.y * blockDim.x) {
     float acc[8];
     if (accumulate) {
       const uint4 v = reinterpret_cast<const uint4*>(out + static_cast<size_t>(t) * H)[i];
@@ -217,15 +217,30 @@ __global__ void moe_combine_kernel(const bf16* __restrict__ y, const int* __rest
 #pragma unroll
       for (int e = 0; e < 8; ++e) acc[e] = 0.f;
     }
-    for (int k = 0; k < K; ++k) {
-      const int r = dst_row[t * K + k];
-      if (r < 0) continue;
-      if (r >= cap) { if (i == 0) guard_report(err, kGuardDstRow, r); continue; }
-      const float w = topk_w[t * K + k];
-      const uint4 v = reinterpret_cast<const uint4*>(y + static_cast<size_t>(r) * H)[i];
-      const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
+    // eight rows' loads in flight at a time, summed in the order of the choices
+    for (int k0 = 0; k0 < K; k0 += 8) {
+      uint4 v[8];
+      float w[8];
+      bool on[8];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { const float2 f = __bfloat1622float2(p[e]); acc[2 * e] += w * f.x; acc[2 * e + 1] += w * f.y; }
+      for (int k = 0; k < 8; ++k) {
+        const int r = k0 + k < K ? dst_row[t * K + k0 + k] : -1;
+        on[k] = r >= 0 && r < cap;
+        if (r >= cap && i == 0) guard_report(err, kGuardDstRow, r);
+        w[k] = on[k] ? topk_w[t * K + k0 + k] : 0.f;
+        if (on[k]) v[k] = reinterpret_cast<const uint4*>(y + static_cast<size_t>(r) * H)[i];
+      }
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        if (!on[k]) continue;
+        const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v[k]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __bfloat1622float2(p[e]);
+          acc[2 * e] += w[k] * f.x;
+          acc[2 * e + 1] += w[k] * f.y;
+        }
+      }
     }
     uint4 o;
     __nv_bfloat162* op = reinterpret_cast<__nv_bfloat162*>(&o);
@@ -280,6 +295,6 @@ extern "C" int ksana_moe_combine(const void* y, const int* dst_row, const float*
                                  int accumulate, int cap, int* err, cudaStream_t st) {
   if (T <= 0) return 0;
   if (H % 8) return -10;
-  moe_combine_kernel<<<T, 256, 0, st>>>((const bf16*)y, dst_row, topk_w, (bf16*)out, K, H, accumulate, cap, err);
+  moe_combine_kernel<<<dim3(T, T < 148 * 4 ? 4 : 1), 256, 0, st>>>((const bf16*)y, dst_row, topk_w, (bf16*)out, K, H, accumulate, cap, err);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -270,7 +270,7 @@ def moe_partial(model, mw: MoEWeights, x: torch.Tensor, into: Optional[torch.Ten
             pq, ps = native.moe_permute_fp8(xq.q, xq.s, dst_row, K, cap)
             g = native.gemm_grouped(pq, mw.w13, tile_expert, n_local, 2 * mw.inter, a_scale=ps, w_scale=mw.w13_scale,
                                     tile_rows=tile_rows, hw_scale=mw.ue8m0)
-            _, aq, as_ = native.act_mul(g, cfg.activation, True, quant=True, want_out=False)
+            _, aq, as_ = native.act_mul(g, cfg.activation, True, quant=True, want_out=False, tile_rows=tile_rows)
             y = native.gemm_grouped(aq, mw.w2, tile_expert, n_local, H, a_scale=as_, w_scale=mw.w2_scale, tile_rows=tile_rows,
                                     hw_scale=mw.ue8m0)
         else:
