@@ -6,7 +6,9 @@
 // Per tile and group S = Q K^T and O += P V as in attention_tc.cu (S and O in TMEM, P read from TMEM); one group's products run while
 // the other's softmax does. A row's columns are split between two threads (8 softmax warps per group), which exchange their maxima
 // through shared memory. The exponentials (32768 of them, 16 a clock) and the products take about 2000 clocks each for a tile of 256 x
-// 128; what remains is the chain S -> softmax -> P V of a group.
+// 128; what remains is the chain S -> softmax -> P V of a group. Against attention_tc.cu (one group per CTA, two CTAs per SM, which
+// loads, multiplies and takes exponentials in turn), per layer: one prompt of 16384 tokens (32/8 heads) 3692 -> 2839 us, 775 TFLOP/s
+// of the pairs below the diagonal; 8 of 2048 (64/8) 1489 -> 1241; 32 turns of 60-250 tokens on 1000-3500 cached ones 831 -> 633.
 // Warp roles: 0 TMA producer (one or two tiles ahead), 1 and 2 MMA issuers of the groups (1 owns the TMEM), 3..10 and 11..18 the groups'
 // softmax and epilogue. (One issuing thread for both groups kept the tensor pipe at a quarter: it builds and issues 32 MMAs a tile.)
 // No multicast. Every wait is bounded.

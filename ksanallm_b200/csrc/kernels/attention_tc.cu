@@ -13,7 +13,8 @@
 // 64-column panel), warp 1 MMA issuer + TMEM owner, warps 2..9 softmax + epilogue. Two CTAs share an SM
 // (96 KB of shared memory, 256 TMEM columns each), so one CTA's softmax overlaps the other's MMAs. What bounds the kernel is the
 // softmax between the two products: with one thread per row (128 values in registers, part of them spilled) a tile took it
-// longer than both products of two tiles.
+// longer than both products of two tiles (window 512, 4 x 2048 tokens, 32/8 heads: 220 us, 206 us with two threads; sigmoid
+// weights 193 and 184; 64 x 8 new tokens on 2000 cached ones 160 and 149).
 // With sigmoid weights (SIG) a key's weight is sigmoid(score + bias[head][distance]): no maximum, no sum, no rescale; the
 // heads' bias rows are staged in shared memory where they fit. Outputs may be multiplied by the sigmoid of a gate.
 // Every wait is bounded; a timeout sets the error word and leaves the output untouched.
