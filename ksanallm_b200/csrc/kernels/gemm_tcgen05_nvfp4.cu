@@ -8,9 +8,10 @@
 // TMEM word of the 512-byte scale chunk (see gemm_tcgen05_mx.cu for the chunk layout). Per K block of 256
 // elements the scale warp reads 16 scale bytes per row and writes one chunk per MMA and 128-row group.
 // Warp 0 TMA producer, warp 1 MMA issuer, warps 2 and 3 scale packers (alternate K blocks), warps 4..11 epilogue; single 256-column
-// accumulator and bounded waits as in the FP8 hardware-scaled kernel. A K block of MMAs takes about 500 clocks, an SM's intake of its
-// 48 KB of operands about 800: one packer that loaded a block's scales when their buffer was free took 2200 (the latency of its
-// loads), so two of them work in turn, each with the loads of its next block in flight.
+// accumulator and bounded waits as in the FP8 hardware-scaled kernel. The scales of a K block travel by TMA with its operands (16 bytes
+// a row); a packer turns them into chunks in place, from shared memory. Packers that read them from global memory (a 16-byte load in a
+// line of its own per row) took 2200 clocks a K block, two in turn with loads ahead 1600: 9753 x 28672 x 4096 in 1094 and 890 us, x 4096 x
+// 14336 in 612 and 496; so 832 and 432, 1500 clocks a block, of which its MMAs take 512: an SM takes in 54 KB from L2 in that time.
 //
 // No counterpart in the reference (its low-bit paths are GPTQ/AWQ W4A16 through Marlin/Machete,
 // 3rdparty/LLM_kernels/csrc/kernels/nvidia/mixture_of_experts and .../machete); the operator is specified by
@@ -23,22 +24,22 @@ namespace ksana {
 
 constexpr int kF4BM = 128;
 constexpr int kF4RowBytes = 128;
-constexpr int kF4SfStages = 4;
 constexpr int kF4Threads = 128 + 256;
 
 template <int BN>
 struct F4Cfg {
   static constexpr int kABytes = kF4BM * kF4RowBytes;
   static constexpr int kBBytes = BN * kF4RowBytes;
-  static constexpr int kStageBytes = kABytes + kBBytes;
+  static constexpr int kSfOff = kABytes + kBBytes;                 // scales of the stage: rows of 16 bytes, then chunks in their place
+  static constexpr int kSfBytes = (kF4BM + BN) * 16;
+  static constexpr int kStageBytes = kSfOff + kSfBytes;
   static constexpr int kStages = BN == 256 ? 4 : 6;
   static constexpr int kAccStages = BN == 256 ? 1 : 2;
   static constexpr int kBChunks = BN / 128;
-  static constexpr int kSfStageBytes = 4 * (1 + kBChunks) * 512;   // per K block: one A chunk + kBChunks B chunks per MMA
   static constexpr int kSfCols = 4 * 4 * (1 + kBChunks);           // TMEM columns of one scale set (4 MMAs)
   static constexpr int kSfBase = kAccStages * BN;             // first scale column
   static constexpr int kTmemCols = 512;
-  static constexpr int kSmemBytes = kStages * kStageBytes + kF4SfStages * kSfStageBytes + 1024 + 512;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 512;
   static constexpr int kEpiCols = BN / 2;
 };
 
@@ -47,8 +48,6 @@ struct F4Params {
   __nv_bfloat16* D; float* out_f32; int ldd;
   const __nv_bfloat16* bias;
   const __nv_bfloat16* residual; int ldr;
-  const uint8_t* a_bs; int a_bs_ld;        // e4m3 block scales [M][K/16], row stride in bytes
-  const uint8_t* w_bs; int w_bs_ld;        // [N][K/16]
   const float* a_ts; const float* w_ts;    // per-tensor scales (device scalars)
   int* err;
   __nv_bfloat16* push[8]; int push_n; int push_rows;
@@ -70,17 +69,16 @@ __device__ __forceinline__ void f4_tile_coords(int tile, int m_tiles, int n_tile
 
 template <int BN>
 __global__ void __launch_bounds__(kF4Threads, 1)
-gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const F4Params p) {
+gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                  const __grid_constant__ CUtensorMap tma_sa, const __grid_constant__ CUtensorMap tma_sb, const F4Params p) {
   using Cfg = F4Cfg<BN>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sf_smem = smem + Cfg::kStages * Cfg::kStageBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sf_smem + kF4SfStages * Cfg::kSfStageBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kStages * Cfg::kStageBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = full_bar + Cfg::kStages;
-  uint64_t* sf_full = empty_bar + Cfg::kStages;
-  uint64_t* sf_empty = sf_full + kF4SfStages;
-  uint64_t* tfull_bar = sf_empty + kF4SfStages;
+  uint64_t* sf_full = empty_bar + Cfg::kStages;             // the stage's scales are packed
+  uint64_t* tfull_bar = sf_full + Cfg::kStages;
   uint64_t* tempty_bar = tfull_bar + Cfg::kAccStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + Cfg::kAccStages);
   volatile uint32_t* abort_flag = tmem_slot + 1;
@@ -92,8 +90,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const int num_kb = p.K / 256;            // 256 elements = one 128-byte row per stage
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); }
-    for (int i = 0; i < kF4SfStages; ++i) { mbar_init(&sf_full[i], 1); mbar_init(&sf_empty[i], 1); }
+    for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); mbar_init(&sf_full[i], 1); }
     for (int i = 0; i < Cfg::kAccStages; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], 8); }
     *abort_flag = 0;
     mbar_fence_init();
@@ -126,6 +123,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
           tma_load_2d(sa, &tma_a, &full_bar[stage], kb * 128, m_blk * kF4BM);
           tma_load_2d(sa + Cfg::kABytes, &tma_b, &full_bar[stage], kb * 128, b_row);
+          tma_load_2d(sa + Cfg::kSfOff, &tma_sa, &full_bar[stage], kb * 16, m_blk * kF4BM);
+          tma_load_2d(sa + Cfg::kSfOff + kF4BM * 16, &tma_sb, &full_bar[stage], kb * 16, b_row);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -135,7 +134,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     // -------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
-      int sfs = 0; uint32_t sf_phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       uint32_t set = 0;
       bool ok = true;
@@ -149,15 +147,17 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb && ok; ++kb) {
-          if (!mbar_wait(&sf_full[sfs], sf_phase, abort_flag)) { ok = false; break; }
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait(&sf_full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsf = tmem_base + Cfg::kSfBase + set * Cfg::kSfCols;
-          const uint32_t sf_addr = smem_u32(sf_smem + sfs * Cfg::kSfStageBytes);
-          constexpr int kPerMma = 1 + Cfg::kBChunks;          // chunks per MMA: A, then the B halves
-#pragma unroll
-          for (int c = 0; c < 4 * kPerMma; ++c) tmem_cp_sf(tsf + 4 * c, make_sf_desc(sf_addr + 512 * c));
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
+          constexpr int kPerMma = 1 + Cfg::kBChunks;          // chunks per MMA: A, then the B halves
+          const uint64_t sf_desc = make_sf_desc(sa + Cfg::kSfOff);
+#pragma unroll
+          for (int k = 0; k < 4; ++k)                          // in shared memory chunk k of the A rows, then of each 128 B rows
+#pragma unroll
+            for (int c = 0; c < kPerMma; ++c) tmem_cp_sf(tsf + 4 * (k * kPerMma + c), sf_desc + ((c * 2048 + k * 512) >> 4));
           const uint64_t adesc = make_smem_desc_sw128(sa);
           const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::kABytes);
           constexpr uint32_t idesc = make_idesc_nvf4(kF4BM, BN);
@@ -167,8 +167,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                      tsf + 4 * kPerMma * k + 4);
           tc_commit(&empty_bar[stage]);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
-          tc_commit(&sf_empty[sfs]);
-          if (++sfs == kF4SfStages) { sfs = 0; sf_phase ^= 1; }
           set ^= 1;
         }
         if (ok) {
@@ -180,72 +178,37 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     __syncwarp();
   } else if (warp < 4) {
     // ------------------------------------------------------------ scale packers
-    constexpr int kPerMma = 1 + Cfg::kBChunks;
-    struct Raw { uint4 a[4]; uint4 b[Cfg::kBChunks][4]; };
-    // this packer's K blocks: every second one of the CTA's (tile, K block) sequence
-    auto next_tile = [&](int t) {
-      for (; t < num_tiles; t += gridDim.x) {
+    // K block `seq` of the CTA's (tile, K block) sequence; this packer takes every second one
+    uint32_t seq = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
+      if (p.tile_expert) {
         int m_blk, n_blk;
-        f4_tile_coords(t, m_tiles, n_tiles, m_blk, n_blk);
-        if (!p.tile_expert || p.tile_expert[m_blk] >= 0) break;
+        f4_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
+        if (p.tile_expert[m_blk] < 0) continue;
       }
-      return t;
-    };
-    auto advance = [&](int& t, int& kb, int by) {
-      for (kb += by; kb >= num_kb && t < num_tiles; kb -= num_kb) t = next_tile(t + static_cast<int>(gridDim.x));
-    };
-    auto fetch = [&](int t, int kb, Raw& r) {           // 16 scale bytes per row and K block = one 32-bit word per MMA
-      int m_blk, n_blk;
-      f4_tile_coords(t, m_tiles, n_tiles, m_blk, n_blk);
-      const size_t w_row0 = p.tile_expert ? static_cast<size_t>(p.tile_expert[m_blk]) * p.expert_rows : 0;
+      for (int kb = 0; kb < num_kb; ++kb, ++seq) {
+        if ((seq & 1) != static_cast<uint32_t>(warp - 2)) continue;
+        const int stage = seq % Cfg::kStages;
+        if (!mbar_wait(&full_bar[stage], (seq / Cfg::kStages) & 1, abort_flag)) { ok = false; break; }
+        // 128 rows of 16 bytes (one 32-bit word per MMA) become four chunks of 512 bytes, over them
+        uint4* rows = reinterpret_cast<uint4*>(smem + stage * Cfg::kStageBytes + Cfg::kSfOff);
+        uint4 r[1 + Cfg::kBChunks][4];
 #pragma unroll
-      for (int r4 = 0; r4 < 4; ++r4) {
-        const int row = m_blk * kF4BM + r4 * 32 + lane;
-        r.a[r4] = row < p.M ? *reinterpret_cast<const uint4*>(p.a_bs + static_cast<size_t>(row) * p.a_bs_ld + kb * 16)
-                            : make_uint4(0, 0, 0, 0);
+        for (int c = 0; c < 1 + Cfg::kBChunks; ++c)
+#pragma unroll
+          for (int r4 = 0; r4 < 4; ++r4) r[c][r4] = rows[c * 128 + r4 * 32 + lane];
+        __syncwarp();
+        auto word = [](const uint4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
+#pragma unroll
+        for (int c = 0; c < 1 + Cfg::kBChunks; ++c)
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            rows[c * 128 + k * 32 + lane] = make_uint4(word(r[c][0], k), word(r[c][1], k), word(r[c][2], k), word(r[c][3], k));
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&sf_full[stage]);
       }
-#pragma unroll
-      for (int c = 0; c < Cfg::kBChunks; ++c)
-#pragma unroll
-        for (int r4 = 0; r4 < 4; ++r4) {
-          const int n = n_blk * BN + c * 128 + r4 * 32 + lane;
-          r.b[c][r4] = n < p.N ? *reinterpret_cast<const uint4*>(p.w_bs + (w_row0 + n) * p.w_bs_ld + kb * 16)
-                               : make_uint4(0, 0, 0, 0);
-        }
-    };
-    uint32_t seq = warp - 2;                            // place of the block in the sequence
-    auto emit = [&](const Raw& r) -> bool {
-      const int sfs = seq % kF4SfStages;
-      if (!mbar_wait(&sf_empty[sfs], ((seq / kF4SfStages) & 1) ^ 1, abort_flag)) return false;
-      uint8_t* buf = sf_smem + sfs * Cfg::kSfStageBytes;
-      auto word = [](const uint4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        *reinterpret_cast<uint4*>(buf + (k * kPerMma) * 512 + lane * 16) =
-            make_uint4(word(r.a[0], k), word(r.a[1], k), word(r.a[2], k), word(r.a[3], k));
-#pragma unroll
-        for (int c = 0; c < Cfg::kBChunks; ++c)
-          *reinterpret_cast<uint4*>(buf + (k * kPerMma + 1 + c) * 512 + lane * 16) =
-              make_uint4(word(r.b[c][0], k), word(r.b[c][1], k), word(r.b[c][2], k), word(r.b[c][3], k));
-      }
-      fence_async_smem();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&sf_full[sfs]);
-      seq += 2;
-      return true;
-    };
-    int t = next_tile(blockIdx.x), kb = 0;              // block of the set that is fetched next
-    if (t < num_tiles) advance(t, kb, warp - 2);
-    Raw r0, r1;
-    bool have0 = t < num_tiles, have1;
-    if (have0) { fetch(t, kb, r0); advance(t, kb, 2); }
-    while (have0) {
-      have1 = t < num_tiles;
-      if (have1) { fetch(t, kb, r1); advance(t, kb, 2); }
-      if (!emit(r0) || !have1) break;
-      have0 = t < num_tiles;
-      if (have0) { fetch(t, kb, r0); advance(t, kb, 2); }
-      if (!emit(r1)) break;
     }
   } else {
     // ---------------------------------------------------------------- epilogue
@@ -344,20 +307,20 @@ static F4EncodeFn f4_encode_fn() {
   }
   return fn;
 }
-static int f4_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows) {
+static int f4_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int box_rows, int box_cols = 128) {
   F4EncodeFn enc = f4_encode_fn();
   if (!enc) return -1;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld)};
-  cuuint32_t box[2] = {128, static_cast<cuuint32_t>(box_rows)};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
   return enc(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(base), dims, strides, box, estr,
-             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, box_cols == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS ? 0 : -2;
 }
 
 template <int BN>
-static int launch_f4(const CUtensorMap& ma, const CUtensorMap& mb, const F4Params& p, int max_ctas, cudaStream_t st) {
+static int launch_f4(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& sa, const CUtensorMap& sb, const F4Params& p, int max_ctas, cudaStream_t st) {
   using Cfg = F4Cfg<BN>;
   static bool set = false;
   if (!set) {
@@ -375,7 +338,7 @@ static int launch_f4(const CUtensorMap& ma, const CUtensorMap& mb, const F4Param
   const int tiles = ((p.M + kF4BM - 1) / kF4BM) * ((p.N + BN - 1) / BN);
   int grid = tiles < sms ? tiles : sms;
   if (max_ctas > 0 && grid > max_ctas) grid = max_ctas;
-  gemm_nvfp4_kernel<BN><<<grid, kF4Threads, Cfg::kSmemBytes, st>>>(ma, mb, p);
+  gemm_nvfp4_kernel<BN><<<grid, kF4Threads, Cfg::kSmemBytes, st>>>(ma, mb, sa, sb, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -400,19 +363,18 @@ extern "C" int ksana_gemm_nvfp4(const void* Aq, int lda, const void* a_bs, int a
     const int m_tiles = (M + kF4BM - 1) / kF4BM;
     bn = (m_tiles * ((N + 255) / 256) >= 100) ? 256 : 128;
   }
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, sa, sb;
   if (f4_map(&ma, Aq, M, K / 2, lda, kF4BM)) return -12;
   if (f4_map(&mb, Wq, N, K / 2, ldw, bn)) return -13;
+  if (f4_map(&sa, a_bs, M, K / 16, a_bs_ld, kF4BM, 16) || f4_map(&sb, w_bs, N, K / 16, w_bs_ld, bn, 16)) return -14;
   F4Params p{};
   p.M = M; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.out_f32 = static_cast<float*>(out_f32); p.ldd = ldd;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.residual = static_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
-  p.a_bs = static_cast<const uint8_t*>(a_bs); p.a_bs_ld = a_bs_ld;
-  p.w_bs = static_cast<const uint8_t*>(w_bs); p.w_bs_ld = w_bs_ld;
   p.a_ts = a_ts; p.w_ts = w_ts;
   p.err = err_flag;
-  return bn == 256 ? launch_f4<256>(ma, mb, p, max_ctas, st) : launch_f4<128>(ma, mb, p, max_ctas, st);
+  return bn == 256 ? launch_f4<256>(ma, mb, sa, sb, p, max_ctas, st) : launch_f4<128>(ma, mb, sa, sb, p, max_ctas, st);
 }
 
 // Grouped (mixture-of-experts) form: A_q [cap, K/2] holds expert-major rows in 128-row tiles, tile_expert[cap / 128]
@@ -429,16 +391,15 @@ extern "C" int ksana_gemm_grouped_nvfp4(const void* Aq, int lda, const void* a_b
        reinterpret_cast<uintptr_t>(w_bs)) & 15) return -11;
   // a weight tile must not reach into the next expert's rows
   int bn = (bn_hint == 128 || (N % 256)) ? 128 : 256;
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, sa, sb;
   if (f4_map(&ma, Aq, cap, K / 2, lda, kF4BM)) return -12;
   if (f4_map(&mb, Wq, num_experts * N, K / 2, ldw, bn)) return -13;
+  if (f4_map(&sa, a_bs, cap, K / 16, a_bs_ld, kF4BM, 16) || f4_map(&sb, w_bs, num_experts * N, K / 16, w_bs_ld, bn, 16)) return -14;
   F4Params p{};
   p.M = cap; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.ldd = ldd;
-  p.a_bs = static_cast<const uint8_t*>(a_bs); p.a_bs_ld = a_bs_ld;
-  p.w_bs = static_cast<const uint8_t*>(w_bs); p.w_bs_ld = w_bs_ld;
   p.a_ts = a_ts; p.w_ts = w_ts;
   p.err = err_flag;
   p.tile_expert = tile_expert; p.expert_rows = N;
-  return bn == 256 ? launch_f4<256>(ma, mb, p, 0, st) : launch_f4<128>(ma, mb, p, 0, st);
+  return bn == 256 ? launch_f4<256>(ma, mb, sa, sb, p, 0, st) : launch_f4<128>(ma, mb, sa, sb, p, 0, st);
 }
