@@ -5,13 +5,13 @@
 // Both operands are e2m1 values, two per byte (even element in the low nibble), with one e4m3 scale per 16
 // elements along K ([rows, K/16] bytes) and one fp32 scale per tensor. A 128-byte swizzled shared-memory row
 // holds 256 elements = four MMAs of K = 64; each MMA consumes four scales per row, i.e. exactly one 32-bit
-// TMEM word of the 512-byte scale chunk (see gemm_tcgen05_mx.cu for the chunk layout). Per K block of 256
-// elements the scale warp reads 16 scale bytes per row and writes one chunk per MMA and 128-row group.
-// Warp 0 TMA producer, warp 1 MMA issuer, warps 2 and 3 scale packers (alternate K blocks), warps 4..11 epilogue; single 256-column
-// accumulator and bounded waits as in the FP8 hardware-scaled kernel. The scales of a K block travel by TMA with its operands (16 bytes
-// a row); a packer turns them into chunks in place, from shared memory. Packers that read them from global memory (a 16-byte load in a
-// line of its own per row) took 2200 clocks a K block, two in turn with loads ahead 1600: 9753 x 28672 x 4096 in 1094 and 890 us, x 4096 x
-// 14336 in 612 and 496; so 832 and 432, 1500 clocks a block, of which its MMAs take 512: an SM takes in 54 KB from L2 in that time.
+// TMEM word: the scales of 128 rows are four columns, row r in lane r % 32 of column r / 32, the same in all four quarters.
+// Warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 scales, warps 6..13 epilogue; single 256-column accumulator and bounded waits as in
+// the FP8 hardware-scaled kernel. The scales of a K block travel by TMA with its operands (16 bytes a row); four warps, one per quarter
+// of TMEM, write them there from registers. (tcgen05.cp of 512-byte chunks, twelve a block, took about 80 clocks each between the MMAs of two
+// blocks, 1500 clocks a block with 512 of MMAs; now about 1070. A tile of 256 x 192 with them was slower by its work: 1002 us.) 9753 x
+// 28672 x 4096: 1094 us with scales loaded by a packer warp on demand, 832 by TMA and tcgen05.cp, 695 now (3.3 PFLOP/s); 9753 x 4096 x
+// 14336: 612, 432, 319.
 //
 // No counterpart in the reference (its low-bit paths are GPTQ/AWQ W4A16 through Marlin/Machete,
 // 3rdparty/LLM_kernels/csrc/kernels/nvidia/mixture_of_experts and .../machete); the operator is specified by
@@ -24,23 +24,24 @@ namespace ksana {
 
 constexpr int kF4BM = 128;
 constexpr int kF4RowBytes = 128;
-constexpr int kF4Threads = 128 + 256;
+constexpr int kF4Threads = 192 + 256;
 
 template <int BN>
 struct F4Cfg {
   static constexpr int kABytes = kF4BM * kF4RowBytes;
   static constexpr int kBBytes = BN * kF4RowBytes;
-  static constexpr int kSfOff = kABytes + kBBytes;                 // scales of the stage: rows of 16 bytes, then chunks in their place
+  static constexpr int kSfOff = kABytes + kBBytes;                 // scales of the stage: rows of 16 bytes
   static constexpr int kSfBytes = (kF4BM + BN) * 16;
   static constexpr int kStageBytes = kSfOff + kSfBytes;
   static constexpr int kStages = BN == 256 ? 4 : 6;
   static constexpr int kAccStages = BN == 256 ? 1 : 2;
   static constexpr int kBChunks = BN / 128;
-  static constexpr int kSfCols = 4 * 4 * (1 + kBChunks);           // TMEM columns of one scale set (4 MMAs)
+  static constexpr int kSfCols = 4 * 4 * (1 + kBChunks);           // TMEM columns of one scale set (4 MMAs), a set per stage
   static constexpr int kSfBase = kAccStages * BN;             // first scale column
   static constexpr int kTmemCols = 512;
   static constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 512;
   static constexpr int kEpiCols = BN / 2;
+  static_assert(kSfBase + kStages * kSfCols <= kTmemCols && kStageBytes % 1024 == 0 && kSmemBytes <= 227 * 1024, "tile does not fit");
 };
 
 struct F4Params {
@@ -77,7 +78,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + Cfg::kStages * Cfg::kStageBytes);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = full_bar + Cfg::kStages;
-  uint64_t* sf_full = empty_bar + Cfg::kStages;             // the stage's scales are packed
+  uint64_t* sf_full = empty_bar + Cfg::kStages;             // the stage's scales are in TMEM
   uint64_t* tfull_bar = sf_full + Cfg::kStages;
   uint64_t* tempty_bar = tfull_bar + Cfg::kAccStages;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + Cfg::kAccStages);
@@ -90,7 +91,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   const int num_kb = p.K / 256;            // 256 elements = one 128-byte row per stage
 
   if (threadIdx.x == 0) {
-    for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); mbar_init(&sf_full[i], 1); }
+    for (int i = 0; i < Cfg::kStages; ++i) { mbar_init(&full_bar[i], 1); mbar_init(&empty_bar[i], 1); mbar_init(&sf_full[i], 4); }
     for (int i = 0; i < Cfg::kAccStages; ++i) { mbar_init(&tfull_bar[i], 1); mbar_init(&tempty_bar[i], 8); }
     *abort_flag = 0;
     mbar_fence_init();
@@ -135,7 +136,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     if (lane == 0) {
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
-      uint32_t set = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
         if (p.tile_expert) {
@@ -150,14 +150,9 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
           if (!mbar_wait(&sf_full[stage], phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
-          const uint32_t tsf = tmem_base + Cfg::kSfBase + set * Cfg::kSfCols;
+          const uint32_t tsf = tmem_base + Cfg::kSfBase + stage * Cfg::kSfCols;
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
-          constexpr int kPerMma = 1 + Cfg::kBChunks;          // chunks per MMA: A, then the B halves
-          const uint64_t sf_desc = make_sf_desc(sa + Cfg::kSfOff);
-#pragma unroll
-          for (int k = 0; k < 4; ++k)                          // in shared memory chunk k of the A rows, then of each 128 B rows
-#pragma unroll
-            for (int c = 0; c < kPerMma; ++c) tmem_cp_sf(tsf + 4 * (k * kPerMma + c), sf_desc + ((c * 2048 + k * 512) >> 4));
+          constexpr int kPerMma = 1 + Cfg::kBChunks;          // groups of 128 scale rows: A, then the B halves
           const uint64_t adesc = make_smem_desc_sw128(sa);
           const uint64_t bdesc = make_smem_desc_sw128(sa + Cfg::kABytes);
           constexpr uint32_t idesc = make_idesc_nvf4(kF4BM, BN);
@@ -167,7 +162,6 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
                      tsf + 4 * kPerMma * k + 4);
           tc_commit(&empty_bar[stage]);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
-          set ^= 1;
         }
         if (ok) {
           tc_commit(&tfull_bar[acc]);
@@ -176,10 +170,10 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       }
     }
     __syncwarp();
-  } else if (warp < 4) {
-    // ------------------------------------------------------------ scale packers
-    // K block `seq` of the CTA's (tile, K block) sequence; this packer takes every second one
-    uint32_t seq = 0;
+  } else if (warp < 6) {
+    // ------------------------------------------------------------ scale warps, one per TMEM quarter (the scales are in all four)
+    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    int stage = 0; uint32_t phase = 0;
     bool ok = true;
     for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
       if (p.tile_expert) {
@@ -187,34 +181,39 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         f4_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
         if (p.tile_expert[m_blk] < 0) continue;
       }
-      for (int kb = 0; kb < num_kb; ++kb, ++seq) {
-        if ((seq & 1) != static_cast<uint32_t>(warp - 2)) continue;
-        const int stage = seq % Cfg::kStages;
-        if (!mbar_wait(&full_bar[stage], (seq / Cfg::kStages) & 1, abort_flag)) { ok = false; break; }
-        // 128 rows of 16 bytes (one 32-bit word per MMA) become four chunks of 512 bytes, over them
-        uint4* rows = reinterpret_cast<uint4*>(smem + stage * Cfg::kStageBytes + Cfg::kSfOff);
-        uint4 r[1 + Cfg::kBChunks][4];
+      for (int kb = 0; kb < num_kb; ++kb) {
+        // the stage was loaded after its MMAs had ended, so that its scale columns are free too
+        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+        tc_fence_after();
+        constexpr int kPerMma = 1 + Cfg::kBChunks;
+        const uint4* rows = reinterpret_cast<const uint4*>(smem + stage * Cfg::kStageBytes + Cfg::kSfOff);
+        // 16 bytes a row are one word per MMA; a group of 128 rows takes four columns per MMA: row r in lane r % 32 of column r / 32
+        uint32_t v[Cfg::kSfCols];
 #pragma unroll
-        for (int c = 0; c < 1 + Cfg::kBChunks; ++c)
+        for (int c = 0; c < kPerMma; ++c)
 #pragma unroll
-          for (int r4 = 0; r4 < 4; ++r4) r[c][r4] = rows[c * 128 + r4 * 32 + lane];
-        __syncwarp();
-        auto word = [](const uint4& v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : (k == 2 ? v.z : v.w)); };
-#pragma unroll
-        for (int c = 0; c < 1 + Cfg::kBChunks; ++c)
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            rows[c * 128 + k * 32 + lane] = make_uint4(word(r[c][0], k), word(r[c][1], k), word(r[c][2], k), word(r[c][3], k));
-        fence_async_smem();
+          for (int r4 = 0; r4 < 4; ++r4) {
+            const uint4 x = rows[c * 128 + r4 * 32 + lane];
+            v[4 * c + r4] = x.x;
+            v[4 * (kPerMma + c) + r4] = x.y;
+            v[4 * (2 * kPerMma + c) + r4] = x.z;
+            v[4 * (3 * kPerMma + c) + r4] = x.w;
+          }
+        const uint32_t dst = tmem_base + lane_base + Cfg::kSfBase + stage * Cfg::kSfCols;
+        tmem_st32(dst, *reinterpret_cast<uint32_t(*)[32]>(&v[0]));
+        if constexpr (Cfg::kSfCols > 32) tmem_st16(dst + 32, *reinterpret_cast<uint32_t(*)[16]>(&v[32]));
+        tmem_st_wait();
+        tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(&sf_full[stage]);
+        if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
-    const int wg = (warp - 4) >> 2;
+    const int wg = (warp - 6) >> 2;
     constexpr int EC = Cfg::kEpiCols;
     const int col_off = wg * EC;
     int acc = 0; uint32_t acc_phase = 0;
