@@ -9,7 +9,8 @@
 //   * a CTA owns one 128-feature tile, or one of S equal shares of its K range; the S CTAs of a tile are a cluster and add their fp32
 //     sums through distributed shared memory (one cluster barrier instead of the exchange);
 //   * half an SM's shared memory per CTA: two share an SM, so that one streams while the other starts or ends, and under
-//     programmatic dependent launch the weights of this kernel are on their way while the kernel before it finishes.
+//     programmatic dependent launch the weights of this kernel are on their way while the kernel before it finishes (where the
+//     caller says that nothing in flight writes them).
 // Against gemm_smallm.cu (us, in graphs): bf16, 1 row, 6144 x 4096 21 -> 12, 4096 x 4096 18 -> 9, 28672 x 4096 50 -> 37, 4096 x 14336
 // 30 -> 20; e4m3, 64 rows, 8192 x 8192 29 -> 18, 8192 x 28672 61 -> 52. Wide e4m3 layers at more than 32 rows stay with the tiled
 // kernel (57344 x 8192, 64 rows: 86 against 102 us here, where every weight tile is followed by its 8 KB of activations).
@@ -334,7 +335,7 @@ static bool gd_map(CUtensorMap* map, const void* base, int rows, int cols, int l
 }
 
 template <int MP, int KIND>
-static int launch_gemm_decode(const CUtensorMap& mw, const CUtensorMap& mx, const GemmDecodeParams& p, cudaStream_t st) {
+static int launch_gemm_decode(const CUtensorMap& mw, const CUtensorMap& mx, const GemmDecodeParams& p, bool early, cudaStream_t st) {
   using Cfg = GemmDecodeCfg<MP, KIND>;
   const int num_kb = (p.K + Cfg::kElems - 1) / Cfg::kElems;
   const int smem = Cfg::kFixedBytes + (KIND == 2 ? ((num_kb + p.splits - 1) / p.splits) * MP : 0);
@@ -347,8 +348,8 @@ static int launch_gemm_decode(const CUtensorMap& mw, const CUtensorMap& mx, cons
     if (cudaFuncSetAttribute(gemm_decode_kernel<MP, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024) != cudaSuccess) return -3;
     set[dev].store(true, std::memory_order_release);
   }
-  return launch_cluster(pdl_early_enabled(), gemm_decode_kernel<MP, KIND>, dim3(((p.N + 127) / 128) * p.splits), dim3(Cfg::kThreads), p.splits, smem, st,
-                            mw, mx, p) == cudaSuccess ? 0 : -4;
+  return launch_cluster(early && pdl_early_enabled(), gemm_decode_kernel<MP, KIND>, dim3(((p.N + 127) / 128) * p.splits),
+                        dim3(Cfg::kThreads), p.splits, smem, st, mw, mx, p) == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace ksana
@@ -356,10 +357,12 @@ static int launch_gemm_decode(const CUtensorMap& mw, const CUtensorMap& mx, cons
 using namespace ksana;
 
 // kind 0: X [M,K], W [N,K] bf16, K a multiple of 8. kind 2: e4m3 with power-of-two scales, K a multiple of 128. Output bf16 (D) or fp32
-// (out_f32); residual may alias D. -20: more than 64 rows; -22: K too long for one launch (kind 2).
+// (out_f32); residual may alias D. fixed_w: no work in flight writes W. The first weight tiles are requested before the kernel ahead has
+// been waited for, so only then may this one be launched early; W made by an earlier kernel of the stream takes an ordinary launch.
+// -20: more than 64 rows; -22: K too long for one launch (kind 2).
 extern "C" int ksana_gemm_decode(int kind, const void* X, int ldx, const float* a_scale, int a_scale_ld, const void* W, int ldw,
                                  const float* w_scale, void* D, void* out_f32, int ldd, const void* bias, const void* residual, int ldr,
-                                 int M, int N, int K, int* err_flag, cudaStream_t st) {
+                                 int M, int N, int K, int fixed_w, int* err_flag, cudaStream_t st) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 64) return -20;
   if (kind != 0 && kind != 2) return -10;
@@ -382,9 +385,10 @@ extern "C" int ksana_gemm_decode(int kind, const void* X, int ldx, const float* 
   // 100 / 129; bf16, 16 rows, 6144 x 4096 21 / 14 / 12 / 16, 4096 x 14336 67 / 37 / 23 / 22, 28672 x 4096 38 / 44 / 49 / 58.
   p.splits = 1;
   while (p.splits < 8 && tiles * p.splits < 148 && num_kb >= p.splits * 8) p.splits *= 2;
+  const bool early = fixed_w != 0;
   if (kind == 0)
-    return MP == 16 ? launch_gemm_decode<16, 0>(mw, mx, p, st) : MP == 32 ? launch_gemm_decode<32, 0>(mw, mx, p, st)
-                                                                          : launch_gemm_decode<64, 0>(mw, mx, p, st);
-  return MP == 16 ? launch_gemm_decode<16, 2>(mw, mx, p, st) : MP == 32 ? launch_gemm_decode<32, 2>(mw, mx, p, st)
-                                                                        : launch_gemm_decode<64, 2>(mw, mx, p, st);
+    return MP == 16 ? launch_gemm_decode<16, 0>(mw, mx, p, early, st) : MP == 32 ? launch_gemm_decode<32, 0>(mw, mx, p, early, st)
+                                                                                 : launch_gemm_decode<64, 0>(mw, mx, p, early, st);
+  return MP == 16 ? launch_gemm_decode<16, 2>(mw, mx, p, early, st) : MP == 32 ? launch_gemm_decode<32, 2>(mw, mx, p, early, st)
+                                                                               : launch_gemm_decode<64, 2>(mw, mx, p, early, st);
 }

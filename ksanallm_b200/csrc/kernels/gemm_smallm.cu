@@ -882,7 +882,7 @@ static int make_map_packed4(CUtensorMap* map, const void* base, int rows, int k)
 }
 
 template <int MP, int KIND>
-static int launch_smallm(const CUtensorMap& mw, const CUtensorMap& mx, const SmallMParams& p, int ctas,
+static int launch_smallm(const CUtensorMap& mw, const CUtensorMap& mx, const SmallMParams& p, int ctas, bool early,
                          cudaStream_t st) {
   using Cfg = SmallMCfg<MP, KIND>;
   // the opt-in to large dynamic shared memory is a per-device attribute of the function
@@ -895,8 +895,8 @@ static int launch_smallm(const CUtensorMap& mw, const CUtensorMap& mx, const Sma
                              Cfg::kSmemBytes) != cudaSuccess) return -3;
     set[dev].store(true, std::memory_order_release);
   }
-  return launch_pdl(gemm_smallm_kernel<MP, KIND>, dim3(ctas), dim3(Cfg::kThreads), Cfg::kSmemBytes, st, mw, mx, p) ==
-                 cudaSuccess ? 0 : -4;
+  return launch_cluster(early && pdl_enabled(), gemm_smallm_kernel<MP, KIND>, dim3(ctas), dim3(Cfg::kThreads), 1, Cfg::kSmemBytes, st, mw,
+                        mx, p) == cudaSuccess ? 0 : -4;
 }
 
 // How many persistent CTAs share the n_tiles x num_kb (tile, K block) units. Measured on 64-row FP8 problems (graphs
@@ -982,13 +982,14 @@ extern "C" void ksana_smallm_set_profile(void* buf) { g_smallm_prof = static_cas
 // counters: n_tiles words, zero before the first launch (the kernel leaves them zero).
 // kind 0: X, W bf16. kind 1: e4m3 with fp32 scales. kind 2: e4m3 with power-of-two scales, applied by the tensor
 // cores. ctas_hint > 0 fixes the number of persistent CTAs
-// (1 = no K splitting at all when there is a single tile per CTA...). Returns 0 on success; -20 when M > 128.
+// (1 = no K splitting at all when there is a single tile per CTA...). fixed_w: no work in flight writes W, so that its first tiles may be
+// requested before the kernel ahead has been waited for. Returns 0 on success; -20 when M > 128.
 static int smallm_impl(int kind, const void* X, int ldx, const float* a_scale, int a_scale_ld, const void* W,
                        int ldw, const float* w_scale, void* D, void* out_f32, int ldd, const void* bias,
                        const void* residual, int ldr, int M, int N, int K, int ctas_hint, void* scratch,
                        long long scratch_bytes, void* counters, int counters_len, int* err_flag,
                        cudaStream_t st, const unsigned long long* push_ptrs, int push_n, const void* w4_scale = nullptr,
-                       const void* w4_zs = nullptr, int w4_group = 0, const PushSignal* sig = nullptr) {
+                       const void* w4_zs = nullptr, int w4_group = 0, const PushSignal* sig = nullptr, bool fixed_w = true) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   if (M > 128) return -20;
   if (kind < 0 || kind > 3) return -10;
@@ -1062,9 +1063,9 @@ static int smallm_impl(int kind, const void* X, int ldx, const float* a_scale, i
   }
   const int ctas = static_cast<int>(P);
 #define KSANA_SM_DISPATCH(MPV)                                                                        \
-  case MPV: return kind == 0 ? launch_smallm<MPV, 0>(mw, mx, p, ctas, st)                            \
-                 : (kind == 1 ? launch_smallm<MPV, 1>(mw, mx, p, ctas, st)                            \
-                 : (kind == 2 ? launch_smallm<MPV, 2>(mw, mx, p, ctas, st) : launch_smallm<MPV, 3>(mw, mx, p, ctas, st)));
+  case MPV: return kind == 0 ? launch_smallm<MPV, 0>(mw, mx, p, ctas, fixed_w, st)                   \
+                 : (kind == 1 ? launch_smallm<MPV, 1>(mw, mx, p, ctas, fixed_w, st)                   \
+                 : (kind == 2 ? launch_smallm<MPV, 2>(mw, mx, p, ctas, fixed_w, st) : launch_smallm<MPV, 3>(mw, mx, p, ctas, fixed_w, st)));
   switch (MP) {
     KSANA_SM_DISPATCH(16)
     KSANA_SM_DISPATCH(32)
@@ -1095,10 +1096,11 @@ extern "C" int ksana_smallm_estimate(int kind, int M, int N, int K, int* ctas_ou
 extern "C" int ksana_gemm_smallm(int kind, const void* X, int ldx, const float* a_scale, int a_scale_ld, const void* W,
                                  int ldw, const float* w_scale, void* D, void* out_f32, int ldd, const void* bias,
                                  const void* residual, int ldr, int M, int N, int K, int ctas_hint, void* scratch,
-                                 long long scratch_bytes, void* counters, int counters_len, int* err_flag,
+                                 long long scratch_bytes, void* counters, int counters_len, int fixed_w, int* err_flag,
                                  cudaStream_t st) {
   return smallm_impl(kind, X, ldx, a_scale, a_scale_ld, W, ldw, w_scale, D, out_f32, ldd, bias, residual, ldr, M, N, K,
-                     ctas_hint, scratch, scratch_bytes, counters, counters_len, err_flag, st, nullptr, 0);
+                     ctas_hint, scratch, scratch_bytes, counters, counters_len, err_flag, st, nullptr, 0, nullptr, nullptr, 0, nullptr,
+                     fixed_w != 0);
 }
 
 // Weight-only 4-bit weights (kind 3): W = packed levels [N, K/2], fp16 scale and zero*scale [N, K/group], group a multiple

@@ -8,7 +8,9 @@
 //
 // Rules used in this library:
 //   * pdl_trigger() as early as possible; pdl_wait() before the first global-memory access that is not a read of
-//     weights / constants (those are never written while the engine runs);
+//     weights / constants that no work in flight writes. The caller vouches for a GEMM's weight operand (`fixed_w`): loaded weights
+//     are never written while the engine runs; a matrix that a step makes (4-bit weights expanded into scratch) is not one of them, and
+//     its GEMM takes an ordinary launch;
 //   * a kernel launched through launch_pdl() that lacks pdl_wait() would race: only kernels that call it are launched
 //     with the attribute;
 //   * both calls are no-ops in a kernel launched without the attribute.

@@ -142,7 +142,7 @@ class DeepseekModel(CommonModel):
         native.mla_rope_append(q, self.nope, None, None, 0.0, *args, q, cache, self.block_tokens, Hq, self.nope)     # in place
         cu_k = torch.nn.functional.pad(torch.cumsum(step.kv_lens, 0, dtype=torch.int32), (1, 0))
         lat = native.gather_latents(cache, self.block_tokens, step.block_table, step.kv_lens, cu_k, step.total_kv_len, step.max_kv_len)
-        kx = native.gemm_bf16(lat[:, :self.lora], mw.kv_b.view(-1, self.lora))
+        kx = native.gemm_bf16(lat[:, :self.lora], mw.kv_b.view(-1, self.lora), fixed_w=True)
         o = native.mha_prefill(q.view(T, Hq, -1), kx.view(-1, Hq, self.nope + self.vdim), lat[:, self.lora:], step.cu_q, cu_k, step.kv_lens,
                                step.max_q_len, self.scale)
         return o.view(T, Hq * self.vdim)

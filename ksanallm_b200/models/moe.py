@@ -230,7 +230,10 @@ def route(model, mw: MoEWeights, x: torch.Tensor):
     K, E = cfg.num_experts_per_tok, mw.num_experts
     if x.is_cuda:
         logits = torch.empty(T, E, dtype=torch.float32, device=x.device)
-        native.gemm_bf16(x, mw.router_bf16 if mw.router_bf16 is not None else mw.router.to(torch.bfloat16), out_f32=logits)
+        if mw.router_bf16 is not None:
+            native.gemm_bf16(x, mw.router_bf16, out_f32=logits, fixed_w=True)
+        else:
+            native.gemm_bf16(x, mw.router.to(torch.bfloat16), out_f32=logits)
         return native.moe_route(logits, K, cfg.moe_scoring, cfg.norm_topk_prob, cfg.routed_scaling_factor,
                                 mw.router_bias, cfg.n_group, cfg.topk_group)
     ids, w = route_reference(x.float() @ mw.router.float().t(), cfg, mw.router_bias)

@@ -122,7 +122,8 @@ def quantize(x: torch.Tensor) -> QTensor:
 
 
 def linear(x, W: LinearWeight, residual=None, out=None, out_f32: bool = False):
-    """y = x W^T (+bias) (+residual). ``x`` may be a QTensor when W is FP8. ``out`` may alias ``residual``."""
+    """y = x W^T (+bias) (+residual). ``x`` may be a QTensor when W is FP8. ``out`` may alias ``residual``. ``W`` holds loaded weights:
+    no work that is still in flight writes them."""
     if W.w4a16:
         if isinstance(x, QTensor):
             raise TypeError("4-bit weight-only layers take bf16 activations")
@@ -159,14 +160,15 @@ def linear(x, W: LinearWeight, residual=None, out=None, out_f32: bool = False):
                 x = quantize(x)
             if out_f32:
                 o = torch.empty(x.q.shape[0], W.out_features, dtype=torch.float32, device=x.q.device)
-                return native.gemm_fp8(x.q, x.s, W.wq, W.ws, bias=W.bias, residual=residual, out_f32=o, hw_scale=W.ue8m0)
-            return native.gemm_fp8(x.q, x.s, W.wq, W.ws, out=out, bias=W.bias, residual=residual, hw_scale=W.ue8m0)
+                return native.gemm_fp8(x.q, x.s, W.wq, W.ws, bias=W.bias, residual=residual, out_f32=o, hw_scale=W.ue8m0,
+                                       fixed_w=True)
+            return native.gemm_fp8(x.q, x.s, W.wq, W.ws, out=out, bias=W.bias, residual=residual, hw_scale=W.ue8m0, fixed_w=True)
         if W.w.dtype == torch.float32:
             return native.gemm_f32(x, W.w, out=out, bias=W.bias, residual=residual)
         if out_f32:
             o = torch.empty(x.shape[0], W.out_features, dtype=torch.float32, device=x.device)
-            return native.gemm_bf16(x, W.w, bias=W.bias, residual=residual, out_f32=o)
-        return native.gemm_bf16(x, W.w, out=out, bias=W.bias, residual=residual)
+            return native.gemm_bf16(x, W.w, bias=W.bias, residual=residual, out_f32=o, fixed_w=True)
+        return native.gemm_bf16(x, W.w, out=out, bias=W.bias, residual=residual, fixed_w=True)
     # CPU statement
     if W.fp8:
         xq = x if isinstance(x, QTensor) else QTensor(*ref.quant_fp8(x))

@@ -35,8 +35,8 @@ _SIGS = {
     "ksana_gemm_mxfp8_pair": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp, i32, i32, vp, vp],
     "ksana_gemm_fp8_block": [vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_smallm": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, i64, vp, i32,
-                          vp, vp],
-    "ksana_gemm_decode": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, vp, vp],
+                          i32, vp, vp],
+    "ksana_gemm_decode": [i32, vp, i32, vp, i32, vp, i32, vp, vp, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_grouped": [i32, vp, i32, vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, vp, vp, i32, vp, vp],
     "ksana_moe_route": [vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, f32, i32, i32, i32, i32, vp],
     "ksana_moe_align": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
@@ -274,14 +274,14 @@ def gemm_workspace(device):
     return _workspaces[key]
 
 
-def _gemm_smallm(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K, splits):
+def _gemm_smallm(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K, splits, fixed_w):
     dst = out if out_f32 is None else out_f32
     scratch, counters = gemm_workspace(x.device)
     rc = lib().ksana_gemm_smallm(kind, _p(x), x.stride(0), _p(xs), xs.stride(0) if xs is not None else 0, _p(w),
                                  w.stride(0), _p(ws), _p(out) if out_f32 is None else None, _p(out_f32), dst.stride(0),
                                  _p(bias), _p(residual), residual.stride(0) if residual is not None else 0, M, N, K,
                                  max(splits, 0), _p(scratch), scratch.numel() * 4, _p(counters), counters.numel(),
-                                 _p(err_flag(x.device)), _st())
+                                 int(fixed_w), _p(err_flag(x.device)), _st())
     _check(rc, "ksana_gemm_smallm")
     return dst
 
@@ -290,11 +290,11 @@ DECODE_MAX_K_MX = 1 << 17          # (its table of token exponents holds one sha
 DECODE_MAX_M = 64                  # rows up to which a decode GEMM is one tile (or share of one) per CTA; beyond: stream-K
 
 
-def _gemm_decode(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K):
+def _gemm_decode(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K, fixed_w):
     dst = out if out_f32 is None else out_f32
     rc = lib().ksana_gemm_decode(kind, _p(x), x.stride(0), _p(xs), xs.stride(0) if xs is not None else 0, _p(w), w.stride(0), _p(ws),
                                  _p(out) if out_f32 is None else None, _p(out_f32), dst.stride(0), _p(bias), _p(residual),
-                                 residual.stride(0) if residual is not None else 0, M, N, K, _p(err_flag(x.device)), _st())
+                                 residual.stride(0) if residual is not None else 0, M, N, K, int(fixed_w), _p(err_flag(x.device)), _st())
     _check(rc, "ksana_gemm_decode")
     return dst
 
@@ -335,8 +335,9 @@ def _pair_ok(M, N, K, kind, bn, out_f32, max_ctas):
             and N >= 256 and K % (128 if kind else 8) == 0)
 
 
-def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_ctas=0, splits=0):
-    """out[M,N] = x[M,K] @ w[N,K]^T (+bias)(+residual). bf16 in, bf16 (or fp32) out."""
+def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_ctas=0, splits=0, fixed_w=False):
+    """out[M,N] = x[M,K] @ w[N,K]^T (+bias)(+residual). bf16 in, bf16 (or fp32) out. ``fixed_w``: no work that is still in flight
+    writes ``w`` (loaded weights): the kernel may request it before the work ahead of it has ended."""
     M, K = x.shape
     N = w.shape[0]
     assert x.stride(1) == 1 and w.stride(1) == 1 and w.shape[1] == K
@@ -344,9 +345,9 @@ def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
     dst = out if out_f32 is None else out_f32
     if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K % 8 == 0:
-        return _gemm_decode(0, x, None, w, None, out, out_f32, bias, residual, M, N, K)
+        return _gemm_decode(0, x, None, w, None, out, out_f32, bias, residual, M, N, K, fixed_w)
     if (M <= SMALL_M_BF16 or splits < 0) and M <= 128 and bn == 0 and K % 8 == 0:
-        return _gemm_smallm(0, x, None, w, None, out, out_f32, bias, residual, M, N, K, splits)
+        return _gemm_smallm(0, x, None, w, None, out, out_f32, bias, residual, M, N, K, splits, fixed_w)
     if (BF16_TALL_MIN_M > 0 and M >= BF16_TALL_MIN_M and bn == 0 and splits == 0 and N % 8 == 0 and K % 8 == 0
             and ((M + 255) // 256) * ((N + 255) // 256) >= 148):
         return gemm_bf16_tall(x, w, out, bias, residual, out_f32, max_ctas)
@@ -453,9 +454,10 @@ def _skinny_wins_mx(M, N, K, sms=148):
 
 
 def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, bn=0, max_ctas=0, splits=0,
-             hw_scale=False):
+             hw_scale=False, fixed_w=False):
     """Block-scaled FP8 GEMM. xq [M,K] e4m3, xs [K/128, ld] fp32; wq [N,K] e4m3, ws [ceil(N/128), K/128] fp32.
-    hw_scale: every scale is a power of two, so the tensor cores may apply them (large-M path)."""
+    hw_scale: every scale is a power of two, so the tensor cores may apply them (large-M path). ``fixed_w``: as for
+    :func:`gemm_bf16`."""
     M, K = xq.shape
     N = wq.shape[0]
     if out is None and out_f32 is None:
@@ -468,10 +470,10 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
         t256 = ((M + 127) // 128) * ((N + 255) // 256)
         # (wide layers at more than 32 rows: the tiled kernel, 86 against 102 us for 64 x 57344 x 8192, 53 against 61 us for 36864 x 7168)
         if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K <= DECODE_MAX_K_MX and (M <= 32 or N <= 32768):
-            return _gemm_decode(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K)
+            return _gemm_decode(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, fixed_w)
         skinny = M <= SMALL_M_FP8 or (M <= 128 and _skinny_wins_mx(M, N, K))
         if (skinny or splits != 0) and M <= 128 and bn == 0:
-            return _gemm_smallm(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, splits)
+            return _gemm_smallm(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, splits, fixed_w)
         if MX_TALL_MIN_M > 0 and M >= MX_TALL_MIN_M and bn == 0 and _tall_wins(M, N, K, max_ctas):
             return gemm_mxfp8_tall(xq, xs, wq, ws, out, bias, residual, out_f32, max_ctas)
         if MX_PAIR_MIN_M > 0 and M >= MX_PAIR_MIN_M and bn == 0 and max_ctas == 0 and t256 >= 148:
@@ -481,7 +483,7 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
                               max_ctas)
     skinny = M <= SMALL_M_FP8 or (M <= 64 and K >= 16384 and N <= 16384)
     if (skinny or splits < 0) and M <= 128 and bn == 0:
-        return _gemm_smallm(1, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, splits)
+        return _gemm_smallm(1, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, splits, fixed_w)
     if bn == 0 and M <= 128:
         bn = 128 if N >= 10240 else 64     # decode-sized rows on the tiled kernel: measured best tile widths
     rc = lib().ksana_gemm_fp8_block(_p(xq), xq.stride(0), _p(xs), xs.stride(0), _p(wq), wq.stride(0), _p(ws),
@@ -614,7 +616,7 @@ def linear_w4(x, q4, scale, zs, out=None, bias=None, residual=None):
         _w4_scratch[key] = buf
     w = buf[: N * K].view(N, K)
     _check(lib().ksana_w4_dequant(_p(q4), _p(scale), _p(zs), _p(w), K, N, K, g, _st()), "ksana_w4_dequant")
-    return gemm_bf16(x, w, out=out, bias=bias, residual=residual)
+    return gemm_bf16(x, w, out=out, bias=bias, residual=residual, fixed_w=False)      # written by the launch before
 
 
 def quant_fp8(x, q=None, s=None):
