@@ -71,8 +71,12 @@ __device__ __forceinline__ uint2 pack8_e4m3(const float (&f)[8], float inv_scale
   }
   return make_uint2(w[0], w[1]);
 }
-// 1 / scale for a power of two, exactly
-__device__ __forceinline__ float pow2_inverse(float s) { return __uint_as_float(0x7F000000u - __float_as_uint(s)); }
+// 1 / scale for a scale of fp8_group_scale, exactly: a power of two up to 2^120, or infinite (a group that holds an infinity), whose
+// inverse is 0: finite values become 0 and infinite ones NaN
+__device__ __forceinline__ float pow2_inverse(float s) {
+  const uint32_t b = __float_as_uint(s);
+  return __uint_as_float(b < 0x7F000000u ? 0x7F000000u - b : 0u);
+}
 // largest magnitude of eight bf16 values over the 16 lanes that share one 128-element group, on packed pairs
 __device__ __forceinline__ float group16_absmax(const uint4& v) {
   const __nv_bfloat162* p = reinterpret_cast<const __nv_bfloat162*>(&v);
