@@ -640,10 +640,13 @@ paged_decode_kernel(const AttnParams p) {
 // through registers before.
 constexpr int kStreamThreads = 160;      // 4 warps that compute, 1 that loads
 constexpr int kStreamMaxStages = 8;
-constexpr int kStreamMinTiles = 1;       // tiles per CTA below which fewer CTAs take part
 // What an item costs beside its tiles (its query rows, the merge of the warps, the piece that is handed over), in tiles: the line that
 // is cut has so many empty units behind every item.
 constexpr int kStreamItemUnits = 2;
+// What a piece of a cut item costs beyond that, in tiles (its sums out and in again, a fence, the arrival); and what the even cut costs,
+// whose CTAs have a second, shorter piece before or behind the first and some more to compute.
+constexpr int kStreamPieceUnits = 3;
+constexpr int kStreamCutUnits = 10;
 
 __device__ __forceinline__ void stream_bar() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
@@ -771,7 +774,7 @@ __device__ __forceinline__ void store_head_row4(const AttnParams& p, int s, int 
 }
 
 template <int D, int MODE, bool SIG>
-__global__ void __launch_bounds__(kStreamThreads, D <= 128 ? 2 : 1)
+__global__ void __launch_bounds__(kStreamThreads, D <= 64 ? 3 : D <= 128 ? 2 : 1)
 paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, const AttnParams p) {
   constexpr bool FP8 = MODE == kKvTmaFp8;
   static_assert(!FP8 || (D == 128 && !SIG), "FP8 tiles have rows of 128 bytes");
@@ -781,6 +784,8 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   __shared__ uint64_t full_bar[kStreamMaxStages], empty_bar[kStreamMaxStages];
   __shared__ uint32_t abort_word, last_piece;
   __shared__ float ml_s[4][16][2];
+  __shared__ long long line_s[2];                 // units and CTAs of an even cut: read where a cut item is summed, not held in registers
+  __shared__ int piece_s[2];                      // this CTA's piece of its item and the tiles of a piece (0: the even cut)
   const bool shared = p.kc == p.vc;
   // the merge area is the consumed last stage of an item where that is large enough, else one of its own behind the ring
   const bool own_merge = FP8 || shared;
@@ -801,11 +806,12 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
   }
   // tiles of every sequence (at least one: an empty sequence's rows are written too), prefix sums; every warp computes them for
   // itself, so that one barrier is all the set-up waits for
-  int before = 0;
+  int before = 0, longest = 0;
 #pragma unroll 4
   for (int s0 = 0; s0 < p.B; s0 += 32) {
     const int s = s0 + lane;
     int x = s < p.B ? max(1, decode_tiles(p, p.kv_lens[s]).count) + kStreamItemUnits : 0;
+    longest = max(longest, x);
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const int y = __shfl_up_sync(0xffffffffu, x, o);
@@ -814,31 +820,66 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
     if (s < p.B) first[s + 1] = before + x;                              // the same value from every warp
     before += __shfl_sync(0xffffffffu, x, 31);
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
   __syncthreads();
-  // ranges: equal numbers of tiles, or of whole items where cut items have no place to be summed in
+  // How the line is shared out: cut evenly, or by items. By items, a CTA takes a run of whole ones, or where there are CTAs enough one of
+  // the `m` pieces of `per` tiles of one. The model counts units on the longest path. Even cut / by items (us): 1 sequence of 517 tokens
+  // 10.1 / 9.3, 25 of 194 (40/8 heads) 16.8 / 10.8, 34 of 51-103 (20/4 heads of 192) 18.2 / 9.1, 18 of 3079 50.3 / 44.5, 9 of 9558 66.5 /
+  // 62; ragged or uneven: 64 of 100-3000 47.5 / 100, 41 of 600 (20/4 heads of 192) 30.8 / 36.1, 128 of 100-400 38.0 / 43.7.
   const long long U = static_cast<long long>(before) * heads;
-  const long long I = static_cast<long long>(p.B) * heads;
-  const bool cuts = p.counters != nullptr;
-  const long long most = cuts ? (U + kStreamMinTiles - 1) / kStreamMinTiles : I;
-  const long long P = most < gridDim.x ? most : gridDim.x;
+  const long long I = static_cast<long long>(p.B) * heads, grid = gridDim.x;
+  const long long p_cut = U < grid ? U : grid;
+  const bool can_cut = p.counters != nullptr, few = I <= grid;
+  const int most = longest - kStreamItemUnits;
+  int per = most, m = 1;
+  if (few && can_cut) {
+    const int share = static_cast<uint32_t>(grid) / static_cast<uint32_t>(I);
+    const int part = max(2, (most + share - 1) / share);
+    if (part + kStreamPieceUnits < most) { per = part; m = (most + per - 1) / per; }
+  }
+  const long long item_units = few ? per + kStreamItemUnits + (m > 1 ? kStreamPieceUnits : 0) : (I + grid - 1) / grid * longest;
+  const bool cuts = can_cut && item_units * p_cut > U + kStreamCutUnits * p_cut;
+  const bool by_piece = !cuts && few;
+  const long long P = cuts ? p_cut : by_piece ? I * m : grid;
   const long long c = blockIdx.x;
   if (c >= P) return;
-  const bool narrow = U * P < (1LL << 32);                             // 64-bit divisions cost a tenth of a short launch
-  auto mul_div = [&](long long x, long long y, long long z) -> long long {
+  const bool narrow = U * grid < (1LL << 32);                          // 64-bit divisions cost a tenth of a short launch
+  auto mul_div = [](long long x, long long y, long long z, bool narrow) -> long long {
     return narrow ? static_cast<uint32_t>(x * y) / static_cast<uint32_t>(z) : x * y / z;
   };
-  auto begin_of = [&](long long k) -> long long {
-    if (cuts) return mul_div(k, U, P);
-    const long long i = k * I / P;
-    if (i >= I) return U;
-    const int s = static_cast<int>(i / heads);
-    return static_cast<long long>(first[s]) * heads + (i % heads) * (first[s + 1] - first[s]);
+  auto item_start = [&](long long i) -> long long {
+    const int s = narrow ? static_cast<int>(static_cast<uint32_t>(i) / static_cast<uint32_t>(heads)) : static_cast<int>(i / heads);
+    return static_cast<long long>(first[s]) * heads + (i - static_cast<long long>(s) * heads) * (first[s + 1] - first[s]);
   };
-  const long long u_begin = begin_of(c), u_end = begin_of(c + 1);
-  int s_at = 0;                                                          // sequence of u_begin
-  for (int lo = 0, hi = p.B - 1; lo <= hi;) {
-    const int mid = (lo + hi) / 2;
-    if (static_cast<long long>(first[mid]) * heads <= u_begin) { s_at = mid; lo = mid + 1; } else hi = mid - 1;
+  auto begin_of = [&](long long k) -> long long {
+    if (cuts) return mul_div(k, U, P, narrow);
+    const long long i = mul_div(k, I, P, narrow);                      // (I <= U)
+    return i >= I ? U : item_start(i);
+  };
+  long long u_begin, u_end;
+  int piece = 0, s_at = 0;                                               // sequence of u_begin
+  if (by_piece) {
+    const int i = static_cast<uint32_t>(c) / static_cast<uint32_t>(m);
+    piece = static_cast<int>(c) - i * m;
+    s_at = static_cast<uint32_t>(i) / static_cast<uint32_t>(heads);
+    const int n = first[s_at + 1] - first[s_at];
+    const int t0 = piece * per, t1 = min(t0 + per, n - kStreamItemUnits);
+    if (t0 >= t1) return;                                              // (an item shorter than the longest)
+    u_begin = item_start(i) + t0;
+    u_end = u_begin + (t1 - t0);
+  } else {
+    u_begin = begin_of(c);
+    u_end = begin_of(c + 1);
+    for (int lo = 0, hi = p.B - 1; lo <= hi;) {
+      const int mid = (lo + hi) / 2;
+      if (static_cast<long long>(first[mid]) * heads <= u_begin) { s_at = mid; lo = mid + 1; } else hi = mid - 1;
+    }
+  }
+
+  if (threadIdx.x == 0) {
+    line_s[0] = U; line_s[1] = P;
+    piece_s[0] = piece; piece_s[1] = by_piece ? per : 0;
   }
 
   if (warp == 4) {
@@ -1054,15 +1095,27 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
       }
       if (whole) continue;
       // ---- a cut item: whoever delivers the last piece adds them up, in their order along the line
-      const long long a = u - it.t0, b = a + it.n;             // the item's units
-      auto owner = [&](long long x) {
-        long long k = mul_div(x, P, U);
-        while (k + 1 < P && begin_of(k + 1) <= x) ++k;
-        while (k > 0 && begin_of(k) > x) --k;
-        return k;
-      };
-      const long long cf = owner(a);
-      const int pieces = static_cast<int>(owner(b - 1) - cf) + 1;
+      const int part = piece_s[1];
+      long long cf, slot0;                                     // CTA and slot of its first piece
+      int pieces;
+      if (part) {
+        cf = c - piece_s[0];
+        slot0 = 2 * cf;
+        pieces = (it.n + part - 1) / part;
+      } else {
+        const long long units = line_s[0], ctas = line_s[1], a = u - it.t0;        // a: the item's first unit
+        const bool small = units * ctas < (1LL << 32);
+        auto begin = [&](long long k) { return mul_div(k, units, ctas, small); };
+        auto owner = [&](long long x) {
+          long long k = mul_div(x, ctas, units, small);
+          while (k + 1 < ctas && begin(k + 1) <= x) ++k;
+          while (k > 0 && begin(k) > x) --k;
+          return k;
+        };
+        cf = owner(a);
+        slot0 = 2 * cf + (begin(cf) < a ? 1 : 0);
+        pieces = static_cast<int>(owner(a + it.n - 1) - cf) + 1;
+      }
       __threadfence();
       stream_bar();
       if (threadIdx.x == 0) {
@@ -1074,28 +1127,38 @@ paged_decode_stream_kernel(const __grid_constant__ CUtensorMap k_map, const __gr
       }
       stream_bar();
       if (last_piece) {
-        const long long slot0 = 2 * cf + (begin_of(cf) < a ? 1 : 0);
         for (int r = warp; r < G; r += 4) {
           float mm = -INFINITY;
           for (int k = lane; k < pieces; k += 32) mm = fmaxf(mm, __ldcg(p.cut_ml + ((k ? 2 * (cf + k) : slot0) * R + r) * 2));
 #pragma unroll
           for (int x = 16; x > 0; x >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, x));
           float ll = 0.f;
-          float4 acc[(D + 127) / 128];
+          constexpr int ND = (D + 127) / 128, NK = ND == 1 ? 8 : 4;      // pieces whose loads are in flight together
+          float4 acc[ND];
 #pragma unroll
-          for (int j = 0; j < (D + 127) / 128; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 4
-          for (int k = 0; k < pieces; ++k) {
-            const long long sl = k ? 2 * (cf + k) : slot0;
-            const float2 ml = __ldcg(reinterpret_cast<const float2*>(p.cut_ml + (sl * R + r) * 2));
-            const float f = ml.x == -INFINITY ? 0.f : exp2f(ml.x - mm);
-            ll += ml.y * f;
+          for (int j = 0; j < ND; ++j) acc[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          for (int k0 = 0; k0 < pieces; k0 += NK) {
+            float2 ml[NK];
+            float4 v[NK][ND];
 #pragma unroll
-            for (int j = 0; j < (D + 127) / 128; ++j) {
-              const int d = j * 128 + lane * 4;
-              if (d < p.Dv) {
-                const float4 v = __ldcg(reinterpret_cast<const float4*>(p.cut_o + (sl * R + r) * p.Dv + d));
-                acc[j].x += v.x * f; acc[j].y += v.y * f; acc[j].z += v.z * f; acc[j].w += v.w * f;
+            for (int k = 0; k < NK; ++k) {
+              const long long sl = k0 + k ? 2 * (cf + k0 + k) : slot0;
+              ml[k] = make_float2(-INFINITY, 0.f);
+              if (k0 + k < pieces) ml[k] = __ldcg(reinterpret_cast<const float2*>(p.cut_ml + (sl * R + r) * 2));
+#pragma unroll
+              for (int j = 0; j < ND; ++j) {
+                const int d = j * 128 + lane * 4;
+                v[k][j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (k0 + k < pieces && d < p.Dv) v[k][j] = __ldcg(reinterpret_cast<const float4*>(p.cut_o + (sl * R + r) * p.Dv + d));
+              }
+            }
+#pragma unroll
+            for (int k = 0; k < NK; ++k) {
+              const float f = ml[k].x == -INFINITY ? 0.f : exp2f(ml[k].x - mm);
+              ll += ml[k].y * f;
+#pragma unroll
+              for (int j = 0; j < ND; ++j) {
+                acc[j].x += v[k][j].x * f; acc[j].y += v[k][j].y * f; acc[j].z += v[k][j].z * f; acc[j].w += v[k][j].w * f;
               }
             }
           }
@@ -1225,7 +1288,7 @@ struct StreamWork { float* scratch; long long scratch_bytes; unsigned int* count
 template <int D, int MODE, bool SIG>
 static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap& vm, int B, const StreamWork& w, cudaStream_t st) {
   constexpr bool FP8 = MODE == kKvTmaFp8;
-  constexpr int kLimit = 226 * 1024, kHalf = 112 * 1024;       // one CTA per SM, two CTAs per SM
+  constexpr int kLimit = 226 * 1024;
   const bool shared = p.kc == p.vc;
   const int GA = p.Hq / p.Hkv, heads = p.Hkv * ((GA + 15) / 16);
   p.B = B;
@@ -1234,22 +1297,25 @@ static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap&
   p.stage_bytes = (shared ? 1 : 2) * kTileTok * D * (FP8 ? 1 : 2);
   const long long extra = 1024 + ((FP8 || shared) ? 4 * p.rows * D * 4 : 0) + (SIG ? p.bias_smem * 4 : 0) + (B + 1) * 4LL;
   if (extra + 2 * p.stage_bytes > kLimit) return 1;
-  // as many stages as leave room for a second CTA on the SM, three at least where they fit
-  long long stages = (kHalf - extra) / p.stage_bytes;
-  if (stages < 3) stages = (kLimit - extra) / p.stage_bytes < 3 ? 2 : 3;
-  p.stages = static_cast<int>(stages < kStreamMaxStages ? stages : kStreamMaxStages);
-  const int smem = static_cast<int>(extra) + p.stages * p.stage_bytes;
   static std::atomic<bool> set[64];
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return -3;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  // Two CTAs per SM, each with as many stages as that leaves room for, three at least where they fit. Three where heads are small and two
+  // CTAs per SM would have several items each: an item's fixed parts are most of its time then (158 sequences of 3-191 tokens, 64/8 heads
+  // of 64: 25.9 -> 20.4 us; but 3 of 2299-4598 14.9 -> 17.3, which are cut into more pieces).
+  const int want = D <= 64 && static_cast<long long>(B) * heads > 2LL * sms ? 3 : 2, share = (want == 3 ? 74 : 112) * 1024;
+  long long stages = (share - extra) / p.stage_bytes;
+  if (stages < 3) stages = (kLimit - extra) / p.stage_bytes < 3 ? 2 : 3;
+  p.stages = static_cast<int>(stages < kStreamMaxStages ? stages : kStreamMaxStages);
+  const int smem = static_cast<int>(extra) + p.stages * p.stage_bytes;
   if (!set[dev].load(std::memory_order_acquire)) {
     if (cudaFuncSetAttribute(paged_decode_stream_kernel<D, MODE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit) !=
         cudaSuccess) return -3;
     set[dev].store(true, std::memory_order_release);
   }
-  const int per_sm = smem <= kHalf ? 2 : 1;
+  const int per_sm = smem <= share ? want : 1;
   const long long grid = static_cast<long long>(sms) * per_sm;
   const long long need = 2 * grid * p.rows * (p.Dv + 2) * 4;
   if (w.scratch && need <= w.scratch_bytes && w.counters && static_cast<long long>(B) * heads <= w.counters_len) {
