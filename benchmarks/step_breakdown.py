@@ -64,7 +64,6 @@ def build_step(torch, model, phase, batch, ctx, q_len, block_tokens):
     sequence, prefill = ``q_len`` new tokens per sequence (context = those tokens). Blocks are laid out
     sequence by sequence."""
     from ksanallm_b200.models.common import StepInput
-    from ksanallm_b200.ops import dispatch as ops
     dev = model.device
     kv = ctx if phase == "decode" else q_len
     bps = (kv + block_tokens - 1) // block_tokens
@@ -92,8 +91,6 @@ def build_step(torch, model, phase, batch, ctx, q_len, block_tokens):
         step.state_slots = torch.arange(batch, dtype=torch.int32, device=dev)
         if model.state is None or model.state.shape[0] < batch:
             model.allocate_state(batch)
-    if phase == "decode":
-        step.decode_splits = ops.decode_splits(batch, model.Hkv, kv)
     return step, batch * bps
 
 

@@ -1228,7 +1228,7 @@ static AttnEncodeFn attn_encode_fn() {
 // 128-byte swizzle. Columns past D arrive as zeros.
 static bool make_kv_map(CUtensorMap* map, const void* panel, long long block_stride, int num_blocks, int Hkv, int D, int block_tokens) {
   AttnEncodeFn enc = attn_encode_fn();
-  if (!enc || (reinterpret_cast<uintptr_t>(panel) & 15)) return false;
+  if (!enc) return false;
   cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(Hkv) * block_tokens, static_cast<cuuint64_t>(num_blocks)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(D) * 2, static_cast<cuuint64_t>(block_stride) * 2};
   cuuint32_t box[3] = {64, static_cast<cuuint32_t>(block_tokens), 1};
@@ -1241,7 +1241,7 @@ static bool make_kv_map(CUtensorMap* map, const void* panel, long long block_str
 // The same panel of e4m3 values: box = one cache block's tokens x 128 columns.
 static bool make_kv_map_fp8(CUtensorMap* map, const void* panel, long long block_stride, int num_blocks, int Hkv, int D, int block_tokens) {
   AttnEncodeFn enc = attn_encode_fn();
-  if (!enc || (reinterpret_cast<uintptr_t>(panel) & 15)) return false;
+  if (!enc) return false;
   cuuint64_t dims[3] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(Hkv) * block_tokens, static_cast<cuuint64_t>(num_blocks)};
   cuuint64_t strides[2] = {static_cast<cuuint64_t>(D), static_cast<cuuint64_t>(block_stride)};
   cuuint32_t box[3] = {128, static_cast<cuuint32_t>(block_tokens), 1};
@@ -1251,17 +1251,24 @@ static bool make_kv_map_fp8(CUtensorMap* map, const void* panel, long long block
              CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-// The maps of both panels, where the TMA path covers the cache (block sizes that divide a tile, 16-byte strides).
+// Whether TMA reads the cache: block sizes that divide a tile, panels and strides on 16-byte boundaries.
+static bool tma_covers(const AttnParams& p, int num_blocks, bool fp8) {
+  const int bt = p.block_tokens, unit = fp8 ? 16 : 8;
+  return (bt == 8 || bt == 16 || bt == 32 || bt == 64) && p.block_stride % unit == 0 && p.D % unit == 0 && p.Dv % unit == 0 &&
+         num_blocks > 0 && !((reinterpret_cast<uintptr_t>(p.kc) | reinterpret_cast<uintptr_t>(p.vc)) & 15);
+}
+
+// The maps of both panels of such a cache.
 static bool tma_maps(const AttnParams& p, int num_blocks, CUtensorMap* km, CUtensorMap* vm) {
   const int bt = p.block_tokens;
-  if (!(bt == 8 || bt == 16 || bt == 32 || bt == 64) || p.block_stride % 8 || num_blocks <= 0) return false;
+  if (!tma_covers(p, num_blocks, false)) return false;
   return make_kv_map(km, p.kc, p.block_stride, num_blocks, p.Hkv, p.D, bt) &&
          make_kv_map(vm, p.vc, p.block_stride, num_blocks, p.Hkv, p.Dv, bt);
 }
 
 static bool tma_maps_fp8(const AttnParams& p, int num_blocks, CUtensorMap* km, CUtensorMap* vm) {
   const int bt = p.block_tokens;
-  if (!(bt == 8 || bt == 16 || bt == 32 || bt == 64) || p.block_stride % 16 || p.D % 16 || p.Dv % 16 || num_blocks <= 0) return false;
+  if (!tma_covers(p, num_blocks, true)) return false;
   return make_kv_map_fp8(km, p.kc, p.block_stride, num_blocks, p.Hkv, p.D, bt) &&
          make_kv_map_fp8(vm, p.vc, p.block_stride, num_blocks, p.Hkv, p.Dv, bt);
 }
@@ -1284,19 +1291,28 @@ static int launch_prefill(const AttnParams& p, const CUtensorMap& km, const CUte
 // Partial results of the cut items (two per CTA) and the counters of a stream launch.
 struct StreamWork { float* scratch; long long scratch_bytes; unsigned int* counters; long long counters_len; };
 
+constexpr int kStreamLimit = 226 * 1024;
+// Shared memory of a stream launch (padded head size d, cache values of `esz` bytes) beside its stages, and of a stage.
+static long long stream_extra(const AttnParams& p, int d, int esz, int B) {
+  const int GA = p.Hq / p.Hkv, rows = GA < 16 ? GA : 16;
+  return 1024 + (esz == 1 || p.kc == p.vc ? 4LL * rows * d * 4 : 0) + p.bias_smem * 4LL + (B + 1) * 4LL;
+}
+static int stream_stage(const AttnParams& p, int d, int esz) { return (p.kc == p.vc ? 1 : 2) * kTileTok * d * esz; }
+static bool stream_fits(const AttnParams& p, int d, int esz, int B) {
+  return stream_extra(p, d, esz, B) + 2 * stream_stage(p, d, esz) <= kStreamLimit;
+}
+
 // Returns 1 when the launch does not fit (the caller takes the other kernel).
 template <int D, int MODE, bool SIG>
 static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap& vm, int B, const StreamWork& w, cudaStream_t st) {
-  constexpr bool FP8 = MODE == kKvTmaFp8;
-  constexpr int kLimit = 226 * 1024;
-  const bool shared = p.kc == p.vc;
+  constexpr int ESZ = MODE == kKvTmaFp8 ? 1 : 2;
+  if (!stream_fits(p, D, ESZ, B)) return 1;
   const int GA = p.Hq / p.Hkv, heads = p.Hkv * ((GA + 15) / 16);
   p.B = B;
   p.rows = GA < 16 ? GA : 16;
   p.vec_out = !(reinterpret_cast<uintptr_t>(p.out) & 7) && p.out_stride % 4 == 0 && !(reinterpret_cast<uintptr_t>(p.outq) & 3);
-  p.stage_bytes = (shared ? 1 : 2) * kTileTok * D * (FP8 ? 1 : 2);
-  const long long extra = 1024 + ((FP8 || shared) ? 4 * p.rows * D * 4 : 0) + (SIG ? p.bias_smem * 4 : 0) + (B + 1) * 4LL;
-  if (extra + 2 * p.stage_bytes > kLimit) return 1;
+  p.stage_bytes = stream_stage(p, D, ESZ);
+  const long long extra = stream_extra(p, D, ESZ, B);
   static std::atomic<bool> set[64];
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
@@ -1307,11 +1323,11 @@ static int launch_stream(AttnParams p, const CUtensorMap& km, const CUtensorMap&
   // of 64: 25.9 -> 20.4 us; but 3 of 2299-4598 14.9 -> 17.3, which are cut into more pieces).
   const int want = D <= 64 && static_cast<long long>(B) * heads > 2LL * sms ? 3 : 2, share = (want == 3 ? 74 : 112) * 1024;
   long long stages = (share - extra) / p.stage_bytes;
-  if (stages < 3) stages = (kLimit - extra) / p.stage_bytes < 3 ? 2 : 3;
+  if (stages < 3) stages = (kStreamLimit - extra) / p.stage_bytes < 3 ? 2 : 3;
   p.stages = static_cast<int>(stages < kStreamMaxStages ? stages : kStreamMaxStages);
   const int smem = static_cast<int>(extra) + p.stages * p.stage_bytes;
   if (!set[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(paged_decode_stream_kernel<D, MODE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLimit) !=
+    if (cudaFuncSetAttribute(paged_decode_stream_kernel<D, MODE, SIG>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamLimit) !=
         cudaSuccess) return -3;
     set[dev].store(true, std::memory_order_release);
   }
@@ -1427,6 +1443,23 @@ extern "C" int ksana_paged_prefill(const void* q, long long q_stride, void* out,
   return -11;
 }
 
+// Rows of distance biases of one head group, where they are staged in shared memory (0: read from global memory).
+static int bias_staged(int Hq, int Hkv, int bias_len) {
+  const int table = (Hq / Hkv < 16 ? Hq / Hkv : 16) * bias_len;
+  return table <= kBiasSmem ? table : 0;
+}
+
+// 1: ksana_paged_decode shares such a batch out by itself (the stream form). 0: it runs the number of splits it is given.
+extern "C" int ksana_decode_streams(const void* kc, const void* vc, long long block_stride, int block_tokens, int B, int Hq, int Hkv, int D,
+                                    int Dv, int cache_fp8, int num_blocks, int bias_len) {
+  const int d = padded_head(D, Dv);
+  if (!d || Hkv <= 0 || Hq < Hkv || Hq % Hkv || (cache_fp8 && d > 128)) return 0;
+  AttnParams p{};
+  p.kc = kc; p.vc = vc; p.block_stride = block_stride; p.block_tokens = block_tokens; p.D = D; p.Dv = Dv; p.Hq = Hq; p.Hkv = Hkv;
+  p.bias_smem = bias_len > 0 ? bias_staged(Hq, Hkv, bias_len) : 0;
+  return tma_covers(p, num_blocks, cache_fp8 != 0) && stream_fits(p, cache_fp8 ? 128 : d, cache_fp8 ? 1 : 2, B);
+}
+
 // One new token per sequence. scratch, counters (zero before the first launch): place for the pieces of items that the stream form
 // cuts; without enough of it nothing is cut. num_splits and part_o [B*Hq*splits*Dv], part_ml [B*Hq*splits*2] fp32 (splits > 1)
 // serve caches that TMA cannot read.
@@ -1454,8 +1487,7 @@ extern "C" int ksana_paged_decode(const void* q, long long q_stride, void* out, 
   p.num_splits = num_splits; p.part_o = part_o; p.part_ml = part_ml; p.err = err;
   p.outq = static_cast<uint8_t*>(outq); p.oscale = oscale; p.oscale_ld = oscale_ld;
   p.bias = bias; p.bias_len = bias_len; p.gate = (const bf16*)gate; p.gate_stride = gate_stride; p.out_factor = out_factor;
-  const int table = bias ? (Hq / Hkv < 16 ? Hq / Hkv : 16) * bias_len : 0;
-  p.bias_smem = table <= kBiasSmem ? table : 0;
+  p.bias_smem = bias ? bias_staged(Hq, Hkv, bias_len) : 0;
   switch (padded_head(D, Dv)) {
     case 64: return dispatch_decode<64>(p, cache_fp8, num_blocks, B, w, st);
     case 128: return dispatch_decode<128>(p, cache_fp8, num_blocks, B, w, st);

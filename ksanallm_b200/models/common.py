@@ -48,7 +48,8 @@ class StepInput:
     mrope_positions: Optional[torch.Tensor] = None      # [3, T]
     refit_positions: Optional[torch.Tensor] = None      # rows to overwrite with plugin embeddings
     refit_embeddings: Optional[torch.Tensor] = None     # [R, hidden] fp32
-    decode_splits: int = 1
+    decode_splits: int = 0               # decode attention over caches that need a number of splits; 0: from max_decode_kv_len
+    max_decode_kv_len: int = 0           # the same bound as max_kv_len over the single-token sequences
     decode_workspace: Optional[tuple] = None
     sample_k: int = 0                    # > 0: tensor-parallel ranks return merged per-shard top-k candidates, not logits
     want_hidden: bool = False            # keep final hidden states / post-norm states for /forward
@@ -248,7 +249,8 @@ class CommonModel:
         return ops.paged_attention(qkv, None, cache_layer, self.block_tokens, step.block_table, step.cu_q, step.kv_lens,
                                    step.num_multi, step.num_single, step.num_multi_tokens, step.max_q_len, self.Hq,
                                    self.Hkv, self.D, self.scale, self.alibi, ks, vs, step.decode_splits,
-                                   step.decode_workspace, quant_for=lw.o_proj)
+                                   step.decode_workspace, quant_for=lw.o_proj,
+                                   max_kv_len=step.max_decode_kv_len or step.max_kv_len)
 
     def row_parallel(self, x, W: LinearWeight, h: torch.Tensor) -> torch.Tensor:
         """h += x W^T, reduced over the tensor-parallel group. Single rank: the add is the GEMM's epilogue."""

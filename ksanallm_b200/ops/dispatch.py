@@ -567,7 +567,7 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
                              sinks=sinks, weights=weights)
     if ns:
         n = 1
-        if not native.decode_streams(block_tokens):
+        if not native.decode_streams(k_cache, v_cache, k_cache.stride(0), block_tokens, ns, Hq, Hkv, D, weights):
             seen = min(step.max_kv_len, window + keep + 128) if window > 0 else step.max_kv_len
             # keys that are the values take half of the shared memory
             n = decode_splits(ns, Hkv * ((Hq // Hkv + 15) // 16), seen, ctas_per_sm=4 if k_cache.data_ptr() == v_cache.data_ptr() else 2)
@@ -582,8 +582,8 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
 
 
 def decode_splits(batch: int, hkv: int, max_kv_len: int, sms: int = 148, ctas_per_sm: int = 2) -> int:
-    """Split-KV factor of the decode attention kernel for caches that TMA does not read. One CTA serves one (sequence, kv head, split) and two CTAs
-    fit an SM (shared memory), so the time is about waves x (64-token tiles per split + a fixed set-up cost of about
+    """Split-KV factor of the decode attention kernel for caches that TMA does not read. One CTA serves one (sequence, kv head, split)
+    and two CTAs fit an SM (shared memory), so the time is about waves x (64-token tiles per split + a fixed set-up cost of about
     two tiles); the factor minimising that is chosen, with at least two tiles per split."""
     import os
     forced = int(os.environ.get("KSANA_DECODE_SPLITS", "0"))
@@ -603,14 +603,18 @@ def decode_splits(batch: int, hkv: int, max_kv_len: int, sms: int = 148, ctas_pe
 
 def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_lens, num_multi, num_single,
                     num_multi_tokens, max_q_len, Hq, Hkv, D, scale, alibi=None, k_scale=1.0, v_scale=1.0,
-                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None):
+                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None, max_kv_len: int = 0):
     """Attention of this step's new tokens (rows of ``qkv``: multi-token sequences first, then one row per
     single-token sequence) against the paged cache, which already holds their K/V. ``out`` None allocates the
     result; with ``quant_for`` (the FP8 linear that consumes it) a pure decode step returns the QTensor that linear
-    wants, quantised inside the attention kernels."""
+    wants, quantised inside the attention kernels. ``num_splits`` and ``workspace`` (the splits' partial results) serve decode rows whose
+    cache the kernel does not share out by itself; 0 splits: chosen from ``max_kv_len``, a bound of the decode rows' context."""
     T = qkv.shape[0]
-    if qkv.is_cuda and native.decode_streams(block_tokens):
-        num_splits, workspace = 1, None
+    if qkv.is_cuda and num_single:
+        if native.decode_streams(cache_layer, None, cache_layer.stride(0), block_tokens, num_single, Hq, Hkv, D):
+            num_splits, workspace = 1, None
+        elif num_splits == 0:
+            num_splits = decode_splits(num_single, Hkv, max_kv_len)
     if qkv.is_cuda and quant_for is not None and quant_for.fp8 and num_multi == 0 and num_single and D == 128 and out is None:
         po, pml = workspace if workspace is not None else (None, None)
         if num_splits > 1 and po is None:

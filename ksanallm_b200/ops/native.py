@@ -107,6 +107,7 @@ _SIGS = {
                             f32, i32, f32, f32, i32, vp, i32, vp, i64, f32, vp, vp],
     "ksana_paged_decode": [vp, i64, vp, i64, vp, vp, i64, i32, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, i32, i32, f32, i32,
                            f32, f32, i32, vp, vp, i32, vp, vp, i32, vp, i32, vp, i64, f32, vp, i64, vp, i64, vp, vp],
+    "ksana_decode_streams": [vp, vp, i64, i32, i32, i32, i32, i32, i32, i32, i32, i32],
     "ksana_mla_attention": [vp, i64, vp, i64, vp, i64, i32, vp, i32, vp, vp, i32, i32, i32, i32, i32, i32, vp, vp, i64, f32, i32, i32, vp,
                             vp, vp, vp],
     "ksana_mla_rope_append": [vp, i64, i32, vp, i64, vp, f32, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, i64, i32, vp, vp],
@@ -1016,9 +1017,12 @@ def decode_workspace(device):
     return _decode_workspaces[key]
 
 
-def decode_streams(block_tokens: int) -> bool:
-    """Whether the decode kernel balances a batch by itself (caches that TMA reads); others take a number of splits."""
-    return block_tokens in (8, 16, 32, 64)
+def decode_streams(cache_layer, v_cache, block_stride, block_tokens, B, Hq, Hkv, D, weights=None) -> bool:
+    """Whether :func:`paged_decode` shares such a batch out over the CTAs by itself (caches that TMA reads); others take a number of
+    splits."""
+    kc, vc, Dv = _panels(cache_layer, v_cache, D)
+    return bool(_load().ksana_decode_streams(kc, vc, block_stride, block_tokens, B, Hq, Hkv, D, Dv, int(cache_layer.dtype != torch.bfloat16),
+                                           int(cache_layer.shape[0]), weights.bias.shape[1] if weights is not None else 0))
 
 
 def paged_decode(q, q_stride, out, cache_layer, block_stride, block_tokens, block_table, kv_lens, B, Hq, Hkv, D, scale,
@@ -1026,7 +1030,7 @@ def paged_decode(q, q_stride, out, cache_layer, block_stride, block_tokens, bloc
                  out_scale=None, v_cache=None, window=0, keep=0, sinks=None, weights=None):
     """``out_q`` / ``out_scale`` (head dim 128): the output also (or, with ``out`` None, only) as the FP8 operand of the
     next GEMM: e4m3 [B, Hq * D] and scales [Hq, ld]. ``v_cache`` / ``window`` / ``keep`` / ``sinks`` / ``weights``: see
-    :func:`paged_prefill`. ``num_splits``, ``part_o``, ``part_ml``: for caches that :func:`decode_streams` does not name."""
+    :func:`paged_prefill`. ``num_splits``, ``part_o``, ``part_ml``: for calls that :func:`decode_streams` says no to."""
     fp8 = cache_layer.dtype != torch.bfloat16
     kc, vc, Dv = _panels(cache_layer, v_cache, D)
     scratch, counters = decode_workspace(q.device)

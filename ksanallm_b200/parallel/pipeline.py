@@ -68,6 +68,7 @@ def micro_step(step: StepInput, cu_host: np.ndarray, a: int, b: int, kv_host: Op
         sub.mrope_positions = step.mrope_positions[:, t0:t1]
     if kv_host is not None and b > a:
         sub.max_kv_len = int(kv_host[a:b].max())
+        sub.max_decode_kv_len = int(kv_host[a + nm:b].max()) if nm < b - a else 0
         if nm == b - a:
             q, kv = q_lens.astype(np.int64), np.asarray(kv_host[a:b], dtype=np.int64)
             sub.total_kv_len, sub.pairs = int(kv.sum()), int((q * (kv - q) + q * (q + 1) // 2).sum())

@@ -308,8 +308,7 @@ class ModelRunner:
             step.total_kv_len, step.pairs = int(all_.sum()), int((new * all_ - new * (new - 1) // 2).sum())
         step.sample_k = self.candidate_k(plan, extra)
         if plan.num_single:
-            max_kv = int(kv_lens[plan.num_multi:].max())
-            step.decode_splits = ops.decode_splits(plan.num_single, self.model.Hkv, max_kv)
+            step.max_decode_kv_len = int(kv_lens[plan.num_multi:].max())
         if extra:
             for k, v in extra.items():
                 setattr(step, k, v)
@@ -363,8 +362,7 @@ class ModelRunner:
         slots.fill_(-1)
         cu_q = torch.arange(bs + 1, dtype=torch.int32, device=self.device)
         step = StepInput(ids, pos, slots, cu_q, kvl, table, 0, bs, bs, 0, 1, logits_rows=None)
-        step.decode_splits = ops.decode_splits(bs, self.model.Hkv, self.graph_max_kv)
-        step.max_kv_len = self.graph_max_kv
+        step.max_kv_len = step.max_decode_kv_len = self.graph_max_kv
         step.sample_k = kx
         for i, (name, _, fill) in enumerate(self.tail_fields):
             setattr(step, name, img[n + i * bs:n + (i + 1) * bs].fill_(fill))
