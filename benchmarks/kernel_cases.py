@@ -141,10 +141,10 @@ def _paged(B, kv_len, Hq, Hkv, D, q_len):
 def case_decode_attn():      # 64 sequences x 2304 cached tokens, 64 q / 8 kv heads: 604 MB of K/V read once
     B, kv, Hq, Hkv, D = 64, 2304, 64, 8, 128
     q, cache, table, cu, kvl, out = _paged(B, kv, Hq, Hkv, D, 1)
-    splits = 1
+    work = native.decode_workspace(DEV)
     for _ in range(2):
         native.paged_decode(q, q.stride(0), out, cache, cache.stride(0), 16, table, kvl, B, Hq, Hkv, D, 1 / math.sqrt(D),
-                            num_splits=splits)
+                            work=work)
 
 
 def case_prefill_attn():     # 4 sequences x 2048 new tokens, 64 q / 8 kv heads

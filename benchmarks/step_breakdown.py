@@ -85,6 +85,9 @@ def build_step(torch, model, phase, batch, ctx, q_len, block_tokens):
     rows = None if phase == "decode" else (cu_q[1:] - 1).to(torch.int32)
     step = StepInput(ids, pos, slots, cu_q, kv_lens, table, logits_rows=rows, **step_kw)
     step.max_kv_len = kv
+    if phase == "decode" and dev.type == "cuda":
+        from ksanallm_b200.ops import native
+        step.decode_workspace = native.decode_workspace(dev)
     if model.needs_prev_ids:
         step.prev_ids = torch.roll(ids, 1)
     if model.needs_state_slots:

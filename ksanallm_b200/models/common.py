@@ -50,7 +50,7 @@ class StepInput:
     refit_embeddings: Optional[torch.Tensor] = None     # [R, hidden] fp32
     decode_splits: int = 0               # decode attention over caches that need a number of splits; 0: from max_decode_kv_len
     max_decode_kv_len: int = 0           # the same bound as max_kv_len over the single-token sequences
-    decode_workspace: Optional[tuple] = None
+    decode_workspace: Optional[tuple] = None    # native.decode_workspace of whoever runs the steps
     sample_k: int = 0                    # > 0: tensor-parallel ranks return merged per-shard top-k candidates, not logits
     want_hidden: bool = False            # keep final hidden states / post-norm states for /forward
     prev_ids: Optional[torch.Tensor] = None   # the token before each row's (-1: none); models with ``needs_prev_ids`` only
@@ -249,8 +249,8 @@ class CommonModel:
         return ops.paged_attention(qkv, None, cache_layer, self.block_tokens, step.block_table, step.cu_q, step.kv_lens,
                                    step.num_multi, step.num_single, step.num_multi_tokens, step.max_q_len, self.Hq,
                                    self.Hkv, self.D, self.scale, self.alibi, ks, vs, step.decode_splits,
-                                   step.decode_workspace, quant_for=lw.o_proj,
-                                   max_kv_len=step.max_decode_kv_len or step.max_kv_len)
+                                   quant_for=lw.o_proj, max_kv_len=step.max_decode_kv_len or step.max_kv_len,
+                                   work=step.decode_workspace)
 
     def row_parallel(self, x, W: LinearWeight, h: torch.Tensor) -> torch.Tensor:
         """h += x W^T, reduced over the tensor-parallel group. Single rank: the add is the GEMM's epilogue."""

@@ -577,7 +577,8 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
             pml = torch.empty(ns * Hq * n * 2, dtype=torch.float32, device=qkv.device)
         native.paged_decode(qkv[tm:], qkv.stride(0), out[tm:], k_cache, k_cache.stride(0), block_tokens, step.block_table[nm:],
                             step.kv_lens[nm:], ns, Hq, Hkv, D, scale, num_splits=n, part_o=po, part_ml=pml, v_cache=v_cache,
-                            window=window, keep=keep, sinks=sinks, weights=weights.rows(tm) if weights is not None else None)
+                            window=window, keep=keep, sinks=sinks, weights=weights.rows(tm) if weights is not None else None,
+                            work=getattr(step, "decode_workspace", None))
     return out
 
 
@@ -603,12 +604,13 @@ def decode_splits(batch: int, hkv: int, max_kv_len: int, sms: int = 148, ctas_pe
 
 def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_lens, num_multi, num_single,
                     num_multi_tokens, max_q_len, Hq, Hkv, D, scale, alibi=None, k_scale=1.0, v_scale=1.0,
-                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None, max_kv_len: int = 0):
+                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None, max_kv_len: int = 0, work=None):
     """Attention of this step's new tokens (rows of ``qkv``: multi-token sequences first, then one row per
     single-token sequence) against the paged cache, which already holds their K/V. ``out`` None allocates the
     result; with ``quant_for`` (the FP8 linear that consumes it) a pure decode step returns the QTensor that linear
     wants, quantised inside the attention kernels. ``num_splits`` and ``workspace`` (the splits' partial results) serve decode rows whose
-    cache the kernel does not share out by itself; 0 splits: chosen from ``max_kv_len``, a bound of the decode rows' context."""
+    cache the kernel does not share out by itself; 0 splits: chosen from ``max_kv_len``, a bound of the decode rows' context. ``work``: see
+    native.paged_decode."""
     T = qkv.shape[0]
     if qkv.is_cuda and num_single:
         if native.decode_streams(cache_layer, None, cache_layer.stride(0), block_tokens, num_single, Hq, Hkv, D):
@@ -624,7 +626,7 @@ def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_l
         osc = torch.empty(Hq, max(4, (T + 3) // 4 * 4), dtype=torch.float32, device=qkv.device)
         native.paged_decode(qkv, qkv.stride(0), None, cache_layer, cache_layer.stride(0), block_tokens, block_table,
                             kv_lens, num_single, Hq, Hkv, D, scale, alibi, k_scale, v_scale, num_splits, po, pml,
-                            out_q=oq, out_scale=osc)
+                            out_q=oq, out_scale=osc, work=work)
         return QTensor(oq, osc)
     if out is None:
         out = torch.empty(T, Hq * D, dtype=qkv.dtype, device=qkv.device)
@@ -639,7 +641,7 @@ def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_l
                 pml = torch.empty(num_single * Hq * num_splits * 2, dtype=torch.float32, device=qkv.device)
             native.paged_decode(qkv[num_multi_tokens:], qkv.stride(0), out[num_multi_tokens:], cache_layer,
                                 cache_layer.stride(0), block_tokens, block_table[num_multi:], kv_lens[num_multi:],
-                                num_single, Hq, Hkv, D, scale, alibi, k_scale, v_scale, num_splits, po, pml)
+                                num_single, Hq, Hkv, D, scale, alibi, k_scale, v_scale, num_splits, po, pml, work=work)
         return out
     q = qkv[:, : Hq * D]
     o = ref.paged_attention(q, cache_layer, block_table, cu_q, kv_lens, Hq, Hkv, D, scale, alibi, k_scale, v_scale)

@@ -7,6 +7,7 @@ back silently to PyTorch ops.
 from __future__ import annotations
 
 import ctypes as C
+import functools
 import math
 from dataclasses import dataclass
 from pathlib import Path
@@ -1003,18 +1004,21 @@ def paged_prefill(q, q_stride, out, cache_layer, block_stride, block_tokens, blo
     _check(rc, "ksana_paged_prefill")
 
 
-_decode_workspaces = {}
+@functools.lru_cache(maxsize=None)
+def _sms(device: torch.device) -> int:
+    return torch.cuda.get_device_properties(device).multi_processor_count
+
+
+DECODE_COUNTERS = 1 << 16
 
 
 def decode_workspace(device):
-    """Per-device place for the pieces of items that the decode kernel cuts (two per CTA: at most 2 x 148 CTAs x 16 rows of 256
-    columns with their sums) and their arrival counters (zeroed once; the kernel leaves them zero). Launches that share it
-    must be ordered on one stream, as for :func:`gemm_workspace`."""
-    key = torch.device(device).index or 0
-    if key not in _decode_workspaces:
-        _decode_workspaces[key] = (torch.empty(4 * 148 * 16 * 258, dtype=torch.float32, device=device),
-                                   torch.zeros(1 << 16, dtype=torch.int32, device=device))
-    return _decode_workspaces[key]
+    """A new place for the pieces of items that the decode kernel cuts (two per CTA, 16 rows of up to 256 columns with their sums) and
+    for their arrival counters, which are zero before the first launch and after every one. It belongs to whoever runs decode
+    steps one after another on one stream (a :class:`~ksanallm_b200.runtime.engine.ModelRunner` has one): launches that share it
+    must not overlap."""
+    return (torch.empty(4 * _sms(torch.device(device)) * 16 * 258, dtype=torch.float32, device=device),
+            torch.zeros(DECODE_COUNTERS, dtype=torch.int32, device=device))
 
 
 def decode_streams(cache_layer, v_cache, block_stride, block_tokens, B, Hq, Hkv, D, weights=None) -> bool:
@@ -1027,13 +1031,18 @@ def decode_streams(cache_layer, v_cache, block_stride, block_tokens, B, Hq, Hkv,
 
 def paged_decode(q, q_stride, out, cache_layer, block_stride, block_tokens, block_table, kv_lens, B, Hq, Hkv, D, scale,
                  alibi=None, k_scale=1.0, v_scale=1.0, num_splits=1, part_o=None, part_ml=None, out_q=None,
-                 out_scale=None, v_cache=None, window=0, keep=0, sinks=None, weights=None):
+                 out_scale=None, v_cache=None, window=0, keep=0, sinks=None, weights=None, work=None):
     """``out_q`` / ``out_scale`` (head dim 128): the output also (or, with ``out`` None, only) as the FP8 operand of the
     next GEMM: e4m3 [B, Hq * D] and scales [Hq, ld]. ``v_cache`` / ``window`` / ``keep`` / ``sinks`` / ``weights``: see
-    :func:`paged_prefill`. ``num_splits``, ``part_o``, ``part_ml``: for calls that :func:`decode_streams` says no to."""
+    :func:`paged_prefill`. ``num_splits``, ``part_o``, ``part_ml``: for calls that :func:`decode_streams` says no to.
+    ``work``: a :func:`decode_workspace` that no other launch in flight uses; None: this call has one of its own."""
     fp8 = cache_layer.dtype != torch.bfloat16
     kc, vc, Dv = _panels(cache_layer, v_cache, D)
-    scratch, counters = decode_workspace(q.device)
+    if work is None:
+        G = Hq // Hkv
+        work = (torch.empty(6 * _sms(q.device) * min(G, 16) * (Dv + 2), dtype=torch.float32, device=q.device),
+                torch.zeros(B * Hkv * ((G + 15) // 16), dtype=torch.int32, device=q.device))
+    scratch, counters = work
     rc = lib().ksana_paged_decode(_p(q), q_stride, _p(out), out.stride(0) if out is not None else Hq * Dv, kc, vc,
                                   block_stride, block_tokens, _p(block_table), block_table.stride(0), _p(kv_lens), _p(alibi),
                                   _p(sinks), B, Hq, Hkv, D, Dv, window, keep, float(scale), int(fp8), float(k_scale),

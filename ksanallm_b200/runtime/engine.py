@@ -112,6 +112,8 @@ class ModelRunner:
         self._ring: list = []
         self._ring_pos = 0
         self._swap_stream = None
+        # this runner's steps follow one another on one stream, eager ones and replayed graphs alike
+        self.decode_workspace = native.decode_workspace(self.device) if self.cuda else None
         self.exchange_candidates = os.environ.get("KSANA_SHARD_SAMPLING", "1") != "0"
         self.pipeline = None             # parallel.pipeline.PipelineRunner when the job has several stages
         # what some models read beside the common step metadata, behind it in the uploads: (field of the plan and of the
@@ -298,7 +300,7 @@ class ModelRunner:
         table = take(nseq * plan.max_blocks).view(nseq, plan.max_blocks)
         rows = take(nsamp)
         step = StepInput(input_ids, positions, slots, cu_q, kv_lens, table, plan.num_multi, plan.num_single, T,
-                         plan.num_multi_tokens, plan.max_q_len, logits_rows=rows)
+                         plan.num_multi_tokens, plan.max_q_len, logits_rows=rows, decode_workspace=self.decode_workspace)
         for name, per_row, _ in self.tail_fields:
             setattr(step, name, take(T if per_row else nseq))
         kv_lens = np.asarray(plan.kv_lens)
@@ -361,7 +363,7 @@ class ModelRunner:
         table = img[4 * bs:n].view(bs, mb)
         slots.fill_(-1)
         cu_q = torch.arange(bs + 1, dtype=torch.int32, device=self.device)
-        step = StepInput(ids, pos, slots, cu_q, kvl, table, 0, bs, bs, 0, 1, logits_rows=None)
+        step = StepInput(ids, pos, slots, cu_q, kvl, table, 0, bs, bs, 0, 1, logits_rows=None, decode_workspace=self.decode_workspace)
         step.max_kv_len = step.max_decode_kv_len = self.graph_max_kv
         step.sample_k = kx
         for i, (name, _, fill) in enumerate(self.tail_fields):
