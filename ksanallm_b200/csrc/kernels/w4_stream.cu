@@ -7,12 +7,12 @@
 // to shared memory for tcgen05.mma, and the hand-offs between its expansion warps and the MMA thread set the pace: 65 us for
 // 16 x 28672 x 4096 (59 MB), 41 us for 16 x 4096 x 14336. This one takes 34 and 22 us (in CUDA graphs, weights from HBM): a fifth
 // of HBM's rate; what is left is the instructions of the expansion and mma.sync's own rate (an eighth of tcgen05's), which is why
-// wide layers at more than 32 rows stay with the other kernel (native.linear_w4). Here a warp owns 16 features and multiplies with mma.sync:
+// wide layers at more than 32 rows stay with the other kernel (ksana_w4_stream_wins). Here a warp owns 16 features and multiplies with mma.sync:
 //   * one 16-byte load per lane and row gives 32 levels; two instructions turn a pair of levels into bf16(128 + level), exactly.
 //     mma.sync takes the pairs as they fall out of the packed word, because the activations are staged in the same order;
 //   * the sums of a group are scaled in fp32: sum(w x) = scale * sum((128 + level) x) - (zs + 128 scale) * sum(x), with the group's sums of
-//     the activations taken when they are staged. No weight is rounded to bf16; what the offset of 128 costs in the fp32 sums is
-//     a thousandth of the result's own rounding;
+//     the activations taken when they are staged. The offset of 128 costs the fp32 sums up to 2^-12 of a group's scale * sum|x| (eight
+//     steps, sums up to 143 of them); no weight is rounded to bf16, which could cost 2^-6. (An infinite activation makes its row NaN.)
 //   * tiles of 128 features are cut along K over the CTAs of a cluster, which add their sums through distributed shared memory.
 #include "pdl.cuh"
 #include <atomic>
@@ -99,18 +99,19 @@ w4_stream_kernel(const W4StreamParams p) {
     // All loads of a panel are in flight together: taken one by one (each waited for before the next), they took longer than the
     // weights of the whole tile.
     constexpr int kSets = NT <= 2 ? 4 : 8;
-    if (p.vec_scales && (cp & 7) == 0) {          // eight groups of a row per load
-      const int octets = (np + 7) / 8;
+    if (p.vec_scales) {                           // eight groups of a row per load, from the octet that holds the panel's first on
+      const int o0 = cp >> 3, octets = ((cp + np - 1) >> 3) - o0 + 1;
       for (int i = threadIdx.x; i < octets * 128; i += kW4sThreads) {
-        const int row = i & 127, o = i >> 7;
-        const size_t at = static_cast<size_t>(min(tile * 128 + row, p.N - 1)) * p.ngroups + cp + o * 8;
+        const int row = i & 127, o = o0 + (i >> 7);
+        const size_t at = static_cast<size_t>(min(tile * 128 + row, p.N - 1)) * p.ngroups + o * 8;
         const uint4 s4 = __ldg(reinterpret_cast<const uint4*>(p.scale + at)), z4 = __ldg(reinterpret_cast<const uint4*>(p.zs + at));
         const uint32_t sw[4] = {s4.x, s4.y, s4.z, s4.w}, zw[4] = {z4.x, z4.y, z4.z, z4.w};
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
           const float sc = __half2float(__ushort_as_half(static_cast<unsigned short>(sw[e >> 1] >> (16 * (e & 1)))));
           const float zz = __half2float(__ushort_as_half(static_cast<unsigned short>(zw[e >> 1] >> (16 * (e & 1)))));
-          if (o * 8 + e < np) sz[(o * 8 + e) * 128 + row] = make_float2(sc, fmaf(128.f, sc, zz));
+          const int q = o * 8 + e - cp;
+          if (q >= 0 && q < np) sz[q * 128 + row] = make_float2(sc, fmaf(128.f, sc, zz));
         }
       }
     } else {
@@ -227,27 +228,112 @@ w4_stream_kernel(const W4StreamParams p) {
   if (p.splits > 1) cluster_sync_all();         // a peer may still read this CTA's sums
 }
 
+// Activations staged at a time when a CTA has `per` chunks: its whole share where that fits, else whole turns of the ring of weights in
+// registers (multiples of kW4sDepth, four at least).
 template <int NT>
-static int launch_w4_stream(const W4StreamParams& p, int blocks_y, cudaStream_t st) {
+static int w4_panel(int per) {
+  int fit = kW4sPanelBytes / (NT * 8 * 256);
+  fit = fit > 16 ? 16 : fit < 4 ? 4 : fit & ~3;
+  return per < fit ? per : fit;
+}
+template <int NT>
+static int w4_smem(int panel) {
   constexpr int MP = NT * 8;
-  const int most = MP * (p.panel_chunks * 256 + 64) + p.panel_chunks * (MP * 4 + 128 * 8), red = MP * kW4sRedPitch * 4;
-  const int smem = most > red ? most : red;
+  const int most = MP * (panel * 256 + 64) + panel * (MP * 4 + 128 * 8), red = MP * kW4sRedPitch * 4;
+  return most > red ? most : red;
+}
+
+constexpr int kW4sSmemLimit = 100 * 1024;
+template <int NT>
+static bool w4_prepare(int dev) {
   static std::atomic<bool> set[64];
-  int dev = 0;
-  cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return -3;
-  if (!set[dev].load(std::memory_order_acquire)) {
-    if (cudaFuncSetAttribute(w4_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 100 * 1024) != cudaSuccess) return -3;
-    set[dev].store(true, std::memory_order_release);
+  if (set[dev].load(std::memory_order_acquire)) return true;
+  if (cudaFuncSetAttribute(w4_stream_kernel<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kW4sSmemLimit) != cudaSuccess) return false;
+  set[dev].store(true, std::memory_order_release);
+  return true;
+}
+
+// Clusters of s CTAs that run at once (they do not fill every group of SMs: 296 CTAs of 64 rows, but 33 clusters of 8).
+template <int NT>
+static int w4_at_once(int dev, int sms, int s) {
+  static std::atomic<int> known[64][9];
+  int n = known[dev][s].load(std::memory_order_relaxed);
+  if (n) return n;
+  if (!w4_prepare<NT>(dev)) return sms / s;
+  cudaLaunchConfig_t cfg{};
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeClusterDimension;
+  attr.val.clusterDim.x = s; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
+  cfg.gridDim = dim3(s); cfg.blockDim = dim3(kW4sThreads);
+  cfg.dynamicSmemBytes = w4_smem<NT>(w4_panel<NT>(16));
+  cfg.attrs = &attr; cfg.numAttrs = 1;
+  if (cudaOccupancyMaxActiveClusters(&n, w4_stream_kernel<NT>, &cfg) != cudaSuccess || n <= 0) {
+    (void)cudaGetLastError();
+    n = sms / s;
   }
-  const int tiles = (p.N + 127) / 128;
-  return launch_cluster(pdl_enabled(), w4_stream_kernel<NT>, dim3(tiles * p.splits, blocks_y), dim3(kW4sThreads), p.splits, smem, st, p) ==
-                 cudaSuccess ? 0 : -4;
+  known[dev][s].store(n, std::memory_order_relaxed);
+  return n;
+}
+
+// Cuts along K, by powers of two (other clusters leave more SMs empty). Up to 16 rows a CTA is short of work in flight more than of SMs:
+// cuts go on while a CTA keeps 2 / 4 / 8 chunks where all CTAs make two per SM / fit at once / do not (us for 1 / 2 / 4 / 8 cuts, 1 row:
+// 1024 x 2048 10.3 / 7.2 / 5.8 / 5.1, 15360 x 5120 28.7 / 24.2 / 21.4 / 23.1, 28672 x 4096 32.1 / 31.8 / 27.8 / 33.3, 21912 x 14208 156 /
+// 115 / 107 / 72). With more rows the multiplications fill an SM: cuts go on while all CTAs fit at once (32 rows: 8192 x 4096 43.9 / 25.7 /
+// 20.0 / 25.6, 27648 x 5120 77 / 57 / 76 / 88; 64 rows: 4096 x 4096 65 / 38 / 21 / 18, 6144 x 4096 65 / 38 / 29 / 32); tiles that do not fit
+// uncut are cut to fill the last wave (32 rows, 57344 x 8192: 239 / 205 / 195 / 219).
+template <int NT>
+static int w4_cuts(int dev, int sms, int tiles, int chunks) {
+  int s = 1;
+  if (NT <= 2) {
+    const int at_once = w4_at_once<NT>(dev, sms, 1);
+    for (; s < 8; s *= 2) {
+      const int t = 2 * s, ctas = tiles * t;
+      if (chunks < (ctas <= 2 * sms ? 2 : ctas <= at_once ? 4 : 8) * t) break;
+    }
+  } else if (tiles > w4_at_once<NT>(dev, sms, 1)) {
+    while (s < 4 && chunks >= 32 * s) s *= 2;
+  } else {
+    while (s < 8 && tiles <= w4_at_once<NT>(dev, sms, 2 * s) && chunks >= 3 * s) s *= 2;
+  }
+  return s;
+}
+
+template <int NT>
+static int launch_w4_stream(W4StreamParams p, int blocks_y, cudaStream_t st) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64 || !w4_prepare<NT>(dev)) return -3;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int tiles = (p.N + 127) / 128, chunks = p.K / 128;
+  p.splits = w4_cuts<NT>(dev, sms, tiles * blocks_y, chunks);
+  p.panel_chunks = w4_panel<NT>((chunks + p.splits - 1) / p.splits);
+  return launch_cluster(pdl_enabled(), w4_stream_kernel<NT>, dim3(tiles * p.splits, blocks_y), dim3(kW4sThreads), p.splits,
+                        w4_smem<NT>(p.panel_chunks), st, p) == cudaSuccess ? 0 : -4;
 }
 
 }  // namespace ksana
 
 using namespace ksana;
+
+// Whether this kernel is the faster one for a shape it takes. One or two rows: the CUDA-core kernel needs no staging, which decides
+// where there are few short rows (1 row here / there, us: 1024 x 2048 5.1 / 4.0, 4864 x 896 5.4 / 3.9; but 512 x 3584 6.0 / 6.2, 2640 x 5120
+// 8.4 / 9.8), and for one row where the scales' rows are no multiple of 4 bytes (8192 x 29568 84 / 71). 33 to 64 rows: a CTA takes 2.05 us a chunk by itself and 3.3 beside
+// another on its SM; the stream-K tensor-core kernel about 14 us and 1.6 per chunk and SM, however they are cut (64 rows, us here / there:
+// 4096 x 4096 18 / 32, 7168 x 5120 35.5 / 40.5, 4096 x 14336 47 / 53, 8192 x 8192 52.5 / 55.6; 5168 x 11136 73 / 56, 12288 x 4096 48 / 46.5,
+// 28672 x 4096 98 / 80).
+extern "C" int ksana_w4_stream_wins(int M, int N, int K, int group) {
+  const int tiles = (N + 127) / 128, chunks = K / 128;
+  int dev = 0, sms = 148;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const long long all = static_cast<long long>(tiles) * chunks;
+  if (M <= 2 && ((K <= 2048 && all <= 2 * sms) || (M == 1 && (K / group) % 2))) return 0;
+  if (M <= 32) return 1;
+  if (M > 64) return 0;
+  const int s = w4_cuts<8>(dev, sms, tiles, chunks), per = (chunks + s - 1) / s, waves = (tiles * s + 2 * sms - 1) / (2 * sms);
+  const float here = 4.f + per * (tiles * s <= sms ? 2.05f : 3.3f) * waves, there = 14.f + 1.6f * static_cast<float>(all) / sms;
+  return here <= there;
+}
 
 // qw [N, K/2] packed levels, scale / zs [N, K/group] fp16; x, out, bias, residual bf16 (out may alias residual). K and group multiples of
 // 128, x rows and qw on 16-byte boundaries; returns -10 otherwise. More than 64 rows take several passes over the weights.
@@ -263,18 +349,6 @@ extern "C" int ksana_w4_stream(const void* x, long long ldx, const void* qw, con
   p.bias = (const bf16*)bias; p.residual = (const bf16*)residual; p.ldr = ldr; p.out = (bf16*)out; p.ldo = ldo;
   p.M = M; p.N = N; p.K = K;
   const int nt = M <= 8 ? 1 : M <= 16 ? 2 : M <= 32 ? 4 : 8;
-  // Cuts along K by powers of two while every CTA keeps four chunks and the CTAs stay within seven per SM: measured at 16 rows (us, for
-  // 1 / 2 / 4 / 8 cuts) N = 4096, K = 4096: 28.7 / 17.1 / 10.5 / 9.9; K = 14336: 92.7 / 48.3 / 28.8 / 22.3; N = 28672, K = 4096:
-  // 38.9 / 38.0 / 34.3 / 39.9.
-  const int tiles = (N + 127) / 128, chunks = K / 128;
-  p.splits = 1;
-  while (p.splits < 8 && static_cast<long long>(tiles) * p.splits * 2 <= 148 * 7 && chunks >= p.splits * 8) p.splits *= 2;
-  // A panel is a CTA's whole share of K where that fits, else whole turns of the weights' ring (four chunks).
-  const int per = (chunks + p.splits - 1) / p.splits;
-  int fit = kW4sPanelBytes / (nt * 8 * 256);
-  fit = fit > 16 ? 16 : fit < 4 ? 4 : fit & ~3;
-
-  p.panel_chunks = per < fit ? per : fit;
   p.vec_scales = p.group_chunks == 1 && p.ngroups % 8 == 0 &&
                  !((reinterpret_cast<uintptr_t>(scale) | reinterpret_cast<uintptr_t>(zs)) & 15);
   const int y = (M + nt * 8 - 1) / (nt * 8);

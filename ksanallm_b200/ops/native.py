@@ -113,6 +113,7 @@ _SIGS = {
                             vp, vp, vp],
     "ksana_mla_rope_append": [vp, i64, i32, vp, i64, vp, f32, vp, vp, vp, vp, vp, i64, i32, i32, i32, i32, i32, i32, i64, i32, vp, vp],
     "ksana_gemm_smallm_w4": [vp, i32, vp, vp, vp, i32, vp, i32, vp, vp, i32, i32, i32, i32, vp, i64, vp, i32, vp, vp],
+    "ksana_w4_stream_wins": [i32, i32, i32, i32],
     "ksana_w4_stream": [vp, i64, vp, vp, vp, vp, vp, i64, vp, i64, i32, i32, i32, i32, vp],
     "ksana_w4_gemv": [vp, i64, vp, vp, vp, vp, vp, i64, vp, i64, i32, i32, i32, i32, vp],
     "ksana_w4_dequant": [vp, vp, vp, vp, i64, i32, i32, i32, vp],
@@ -587,10 +588,9 @@ def linear_w4(x, q4, scale, zs, out=None, bias=None, residual=None):
     g = K // scale.shape[1]
     if out is None:
         out = torch.empty(M, N, dtype=torch.bfloat16, device=x.device)
-    if (W4_TENSOR_CORE and (M <= 32 or (M <= 64 and N <= 8192)) and g % 128 == 0 and K % 128 == 0 and x.stride(0) % 8 == 0
-            and x.data_ptr() % 16 == 0):
-        # weight stream through registers, scales applied per group in fp32. 64 rows: 30 / 19 / 50 us against 35 / 35 / 56 us for
-        # 6144 x 4096, 4096 x 4096 and 4096 x 14336, but 101 against 83 us for 28672 x 4096 (mma.sync is the limit there)
+    if (W4_TENSOR_CORE and M <= 64 and g % 128 == 0 and K % 128 == 0 and x.stride(0) % 8 == 0 and x.data_ptr() % 16 == 0
+            and _load().ksana_w4_stream_wins(M, N, K, g)):
+        # weight stream through registers, scales applied per group in fp32
         _check(lib().ksana_w4_stream(_p(x), x.stride(0), _p(q4), _p(scale), _p(zs), _p(bias), _p(residual),
                                      residual.stride(0) if residual is not None else 0, _p(out), out.stride(0), M, N, K, g, _st()),
                "ksana_w4_stream")
