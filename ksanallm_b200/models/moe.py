@@ -40,7 +40,6 @@ class MoEWeights:
     shared_gate: Optional[torch.Tensor] = None       # [1, H] sigmoid gate of the shared expert (Qwen2-MoE)
     expert_lo: int = 0
     expert_hi: int = 0
-    router_bf16: Optional[torch.Tensor] = None       # the router as the GEMM's operand (GPU)
     ue8m0: bool = False                     # the experts' block scales are powers of two: the tensor cores can apply them
     # NVFP4 experts: w13 / w2 hold packed e2m1 pairs ([rows, K/2] bytes), *_bs the e4m3 scales per 16 elements
     # ([rows, K/16]) and *_ts one fp32 tensor scale per local expert
@@ -143,8 +142,9 @@ def load_moe(cfg: ModelConfig, source, prefix: str, tp_rank, tp_size, device, dt
         w2, w2_s = ref.quant_weight_fp8_block(w2)
     else:
         w13, w2 = _dense(w13).to(dtype).contiguous(), _dense(w2).to(dtype).contiguous()
+    if router.is_cuda:
+        router = router.to(torch.bfloat16)              # the GEMM's operand; the only copy, so that a change to it is seen
     mw = MoEWeights(router, rbias, w13, w13_s, w2, w2_s, E, I, H, expert_lo=lo, expert_hi=hi,
-                    router_bf16=router.to(torch.bfloat16) if router.is_cuda else None,
                     ue8m0=w13_s is not None and ref.is_pow2(w13_s) and ref.is_pow2(w2_s), **nv)
     sI_full = cfg.shared_expert_intermediate_size
     if sI_full:
@@ -230,8 +230,8 @@ def route(model, mw: MoEWeights, x: torch.Tensor):
     K, E = cfg.num_experts_per_tok, mw.num_experts
     if x.is_cuda:
         logits = torch.empty(T, E, dtype=torch.float32, device=x.device)
-        if mw.router_bf16 is not None:
-            native.gemm_bf16(x, mw.router_bf16, out_f32=logits, fixed_w=True)
+        if mw.router.dtype == torch.bfloat16:
+            native.gemm_bf16(x, mw.router, out_f32=logits, fixed_w=True)
         else:
             native.gemm_bf16(x, mw.router.to(torch.bfloat16), out_f32=logits)
         return native.moe_route(logits, K, cfg.moe_scoring, cfg.norm_topk_prob, cfg.routed_scaling_factor,
