@@ -44,6 +44,7 @@ class StepInput:
     max_kv_len: int = 0                  # host-side upper bound of kv_lens (split heuristics, no device sync)
     total_kv_len: int = 0                # sum of kv_lens and (query, visible key) pairs of the step, where the host knows them
     pairs: int = 0
+    multi_pairs: int = 0                 # the pairs of the sequences with several new tokens
     logits_rows: Optional[torch.Tensor] = None
     mrope_positions: Optional[torch.Tensor] = None      # [3, T]
     refit_positions: Optional[torch.Tensor] = None      # rows to overwrite with plugin embeddings
@@ -250,7 +251,7 @@ class CommonModel:
                                    step.num_multi, step.num_single, step.num_multi_tokens, step.max_q_len, self.Hq,
                                    self.Hkv, self.D, self.scale, self.alibi, ks, vs, step.decode_splits,
                                    quant_for=lw.o_proj, max_kv_len=step.max_decode_kv_len or step.max_kv_len,
-                                   work=step.decode_workspace)
+                                   work=step.decode_workspace, multi_pairs=step.multi_pairs)
 
     def row_parallel(self, x, W: LinearWeight, h: torch.Tensor) -> torch.Tensor:
         """h += x W^T, reduced over the tensor-parallel group. Single rank: the add is the GEMM's epilogue."""

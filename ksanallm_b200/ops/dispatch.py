@@ -564,7 +564,7 @@ def panel_attention(qkv, k_cache, v_cache, block_tokens, step, Hq, Hkv, scale, w
     if nm:
         native.paged_prefill(qkv, qkv.stride(0), out, k_cache, k_cache.stride(0), block_tokens, step.block_table, step.cu_q,
                              step.kv_lens, nm, step.max_q_len, Hq, Hkv, D, scale, v_cache=v_cache, window=window, keep=keep,
-                             sinks=sinks, weights=weights)
+                             sinks=sinks, weights=weights, rows=tm, pairs=getattr(step, "multi_pairs", 0))
     if ns:
         n = 1
         if not native.decode_streams(k_cache, v_cache, k_cache.stride(0), block_tokens, ns, Hq, Hkv, D, weights):
@@ -604,13 +604,14 @@ def decode_splits(batch: int, hkv: int, max_kv_len: int, sms: int = 148, ctas_pe
 
 def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_lens, num_multi, num_single,
                     num_multi_tokens, max_q_len, Hq, Hkv, D, scale, alibi=None, k_scale=1.0, v_scale=1.0,
-                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None, max_kv_len: int = 0, work=None):
+                    num_splits=1, workspace=None, quant_for: Optional[LinearWeight] = None, max_kv_len: int = 0, work=None,
+                    multi_pairs: int = 0):
     """Attention of this step's new tokens (rows of ``qkv``: multi-token sequences first, then one row per
     single-token sequence) against the paged cache, which already holds their K/V. ``out`` None allocates the
     result; with ``quant_for`` (the FP8 linear that consumes it) a pure decode step returns the QTensor that linear
     wants, quantised inside the attention kernels. ``num_splits`` and ``workspace`` (the splits' partial results) serve decode rows whose
     cache the kernel does not share out by itself; 0 splits: chosen from ``max_kv_len``, a bound of the decode rows' context. ``work``: see
-    native.paged_decode."""
+    native.paged_decode. ``multi_pairs``: (query, visible key) pairs of the multi-token sequences, 0 where nobody counted them."""
     T = qkv.shape[0]
     if qkv.is_cuda and num_single:
         if native.decode_streams(cache_layer, None, cache_layer.stride(0), block_tokens, num_single, Hq, Hkv, D):
@@ -633,7 +634,8 @@ def paged_attention(qkv, out, cache_layer, block_tokens, block_table, cu_q, kv_l
     if qkv.is_cuda:
         if num_multi:
             native.paged_prefill(qkv, qkv.stride(0), out, cache_layer, cache_layer.stride(0), block_tokens, block_table,
-                                 cu_q, kv_lens, num_multi, max_q_len, Hq, Hkv, D, scale, alibi, k_scale, v_scale)
+                                 cu_q, kv_lens, num_multi, max_q_len, Hq, Hkv, D, scale, alibi, k_scale, v_scale, rows=num_multi_tokens,
+                                 pairs=multi_pairs)
         if num_single:
             po, pml = workspace if workspace is not None else (None, None)
             if num_splits > 1 and po is None:

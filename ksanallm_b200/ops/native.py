@@ -971,16 +971,38 @@ def _sigmoid_args(weights: Optional[SigmoidWeights]):
     return _p(b), b.shape[1], _p(g), g.stride(0) if g is not None else 0, float(weights.factor)
 
 
+def prefill_pair_wins(pairs, rows, B, Hq, Hkv, sms=148) -> bool:
+    """Whether prompts take the attention kernel with two query tiles per CTA, from the (query, visible key) pairs and the rows of a
+    batch. A tile of 128 keys costs it less, a CTA more (about 4 us: 608 threads, two tiles' queries, all of TMEM), and only half as many
+    fit the machine. us with two / one, 32/8 heads of 128: one prompt of 200 tokens 17.1 / 12.7, 512 22.9 / 19.3, 1024 35.4 / 37.5, 5000
+    346 / 416; 64 x 33 41.1 / 35.8; 16 x 33 on 1000 cached tokens 32.9 / 40.6; 64 on 4000 103 / 111. While all CTAs of one tile run at
+    once (two an SM), two pay from about a thousand keys per row, and not at all for groups that leave rows of a tile idle (28/4 heads,
+    64 on 4000: 118.5 / 112.7; 14/2 heads of 64, 300 on 8000: 204 / 183); beyond, from 450 keys (510 with such groups)."""
+    G = Hq // Hkv
+    if G > 128 or B <= 0 or rows <= 0:
+        return False
+    keys, whole = pairs / rows, 128 % G == 0
+    per = 128 // G * G                                           # rows of a tile
+    ctas = Hkv * B * -(-rows * G // (B * per))                   # of one tile each, for sequences of the mean length
+    if ctas < 1.55 * sms:
+        return whole and keys >= 1024
+    return keys >= (448 if whole else 512)
+
+
 def paged_prefill(q, q_stride, out, cache_layer, block_stride, block_tokens, block_table, cu_q, kv_lens, B, max_q_len,
                   Hq, Hkv, D, scale, alibi=None, k_scale=1.0, v_scale=1.0, v_cache=None, window=0, keep=0, sinks=None,
-                  weights=None):
+                  weights=None, rows=0, pairs=0):
     """``v_cache``: V panels of their own (``cache_layer`` then holds the K panels). ``window`` > 0: position i sees j <= i
     with i - j < window or j < keep. ``sinks``: fp32 [Hq] logits in the softmax denominator. ``weights``: see
-    :class:`SigmoidWeights`."""
+    :class:`SigmoidWeights`. ``rows``, ``pairs``: the batch's query rows and (query, visible key) pairs, by which the kernel is chosen
+    (0: all rows of ``q``, the block table full)."""
     fp8 = cache_layer.dtype != torch.bfloat16
     kc, vc, Dv = _panels(cache_layer, v_cache, D)
     nblocks = int(cache_layer.shape[0])
-    if PREFILL_TC and PREFILL_PAIR and not fp8 and max(D, Dv) <= 128 and window == 0 and weights is None and max_q_len * (Hq // Hkv) > 128:
+    rows = rows or q.shape[0]
+    pairs = pairs or rows * max(block_table.shape[1] * block_tokens - max_q_len // 2, 1)
+    if (PREFILL_TC and PREFILL_PAIR and not fp8 and max(D, Dv) <= 128 and window == 0 and weights is None and max_q_len * (Hq // Hkv) > 128
+            and prefill_pair_wins(pairs, rows, B, Hq, Hkv, _sms(q.device))):
         # two query tiles per CTA; -100 = configuration not covered
         rc = lib().ksana_paged_prefill_pair(_p(q), q_stride, q.shape[0], _p(out), out.stride(0), kc, vc, block_stride, block_tokens,
                                             _p(block_table), block_table.stride(0), _p(cu_q), _p(kv_lens), _p(alibi), _p(sinks), B,

@@ -62,15 +62,17 @@ def micro_step(step: StepInput, cu_host: np.ndarray, a: int, b: int, kv_host: Op
                   cu_q=step.cu_q[a:b + 1] - t0, kv_lens=step.kv_lens[a:b], block_table=step.block_table[a:b],
                   num_multi=nm, num_single=(b - a) - nm, num_tokens=t1 - t0, num_multi_tokens=nm_tok,
                   max_q_len=int(q_lens.max()) if len(q_lens) else 0, logits_rows=None, want_hidden=False,
-                  refit_positions=None, refit_embeddings=None, total_kv_len=0, pairs=0)
+                  refit_positions=None, refit_embeddings=None, total_kv_len=0, pairs=0, multi_pairs=0)
     if step.mrope_positions is not None:
         sub.mrope_positions = step.mrope_positions[:, t0:t1]
     if kv_host is not None and b > a:
         sub.max_kv_len = int(kv_host[a:b].max())
         sub.max_decode_kv_len = int(kv_host[a + nm:b].max()) if nm < b - a else 0
+        q, kv = q_lens.astype(np.int64), np.asarray(kv_host[a:b], dtype=np.int64)
+        seen = q * (kv - q) + q * (q + 1) // 2
+        sub.multi_pairs = int(seen[:nm].sum())
         if nm == b - a:
-            q, kv = q_lens.astype(np.int64), np.asarray(kv_host[a:b], dtype=np.int64)
-            sub.total_kv_len, sub.pairs = int(kv.sum()), int((q * (kv - q) + q * (q + 1) // 2).sum())
+            sub.total_kv_len, sub.pairs = int(kv.sum()), int(seen.sum())
     return sub
 
 

@@ -307,7 +307,8 @@ class ModelRunner:
         step.max_kv_len = int(kv_lens.max()) if nseq else 0
         if plan.num_multi:
             new, all_ = np.diff(np.asarray(plan.cu_q)).astype(np.int64), kv_lens.astype(np.int64)
-            step.total_kv_len, step.pairs = int(all_.sum()), int((new * all_ - new * (new - 1) // 2).sum())
+            seen = new * all_ - new * (new - 1) // 2
+            step.total_kv_len, step.pairs, step.multi_pairs = int(all_.sum()), int(seen.sum()), int(seen[:plan.num_multi].sum())
         step.sample_k = self.candidate_k(plan, extra)
         if plan.num_single:
             step.max_decode_kv_len = int(kv_lens[plan.num_multi:].max())
