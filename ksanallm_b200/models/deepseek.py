@@ -132,7 +132,16 @@ class DeepseekModel(CommonModel):
         absorbed = step.pairs * self.Hq * 2 * 1088 / 330e12 + T * share * 143e-9
         return step.pairs * self.Hq * 2 * 320 / 700e12 + step.total_kv_len * share * 50e-9 < 0.9 * absorbed
 
-    def _attention_expanded(self, mw, q, kv, step, cache):
+    def _expansion_room(self, q, step, cache):
+        """Place for the latents of a step's sequences and for their keys and values (up to 4 GB), None where the device has none left:
+        the absorbed form needs none of it."""
+        try:
+            return (torch.empty(step.total_kv_len, cache.shape[-1], dtype=cache.dtype, device=cache.device),
+                    torch.empty(step.total_kv_len, self.Hq * (self.nope + self.vdim), dtype=q.dtype, device=q.device))
+        except torch.cuda.OutOfMemoryError:
+            return None
+
+    def _attention_expanded(self, mw, q, kv, step, cache, room):
         """Prompts: keys and values of every head from the cached latents (one plain GEMM), attention over 192 / 128 columns."""
         from ..ops import native
         T, Hq = q.shape[0], self.Hq
@@ -141,8 +150,9 @@ class DeepseekModel(CommonModel):
         native.mla_rope_append(q, self.nope, kv, mw.kv_a_norm, self.cfg.rms_norm_eps, *args, unused, cache, self.block_tokens, 1, self.lora)
         native.mla_rope_append(q, self.nope, None, None, 0.0, *args, q, cache, self.block_tokens, Hq, self.nope)     # in place
         cu_k = torch.nn.functional.pad(torch.cumsum(step.kv_lens, 0, dtype=torch.int32), (1, 0))
-        lat = native.gather_latents(cache, self.block_tokens, step.block_table, step.kv_lens, cu_k, step.total_kv_len, step.max_kv_len)
-        kx = native.gemm_bf16(lat[:, :self.lora], mw.kv_b.view(-1, self.lora), fixed_w=True)
+        lat = native.gather_latents(cache, self.block_tokens, step.block_table, step.kv_lens, cu_k, step.total_kv_len, step.max_kv_len,
+                                    out=room[0])
+        kx = native.gemm_bf16(lat[:, :self.lora], mw.kv_b.view(-1, self.lora), out=room[1], fixed_w=True)
         o = native.mha_prefill(q.view(T, Hq, -1), kx.view(-1, Hq, self.nope + self.vdim), lat[:, self.lora:], step.cu_q, cu_k, step.kv_lens,
                                step.max_q_len, self.scale)
         return o.view(T, Hq * self.vdim)
@@ -153,8 +163,9 @@ class DeepseekModel(CommonModel):
         from ..ops import native
         T, Hq = q.shape[0], self.Hq
         cache = self.kv_cache[:, li - self.layer_lo]                # [blocks, bt, 576]
-        if self._expands(mw, step, T):
-            return self._attention_expanded(mw, q, kv, step, cache)
+        room = self._expansion_room(q, step, cache) if self._expands(mw, step, T) else None
+        if room is not None:
+            return self._attention_expanded(mw, q, kv, step, cache, room)
         qfull = torch.empty(T, Hq, self.lora + self.rope, dtype=q.dtype, device=q.device)
         native.mla_rope_append(q, self.nope, kv, mw.kv_a_norm, self.cfg.rms_norm_eps, step.positions, step.slots,
                                self.cos_sin, qfull, cache, self.block_tokens, Hq, self.lora)

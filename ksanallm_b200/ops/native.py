@@ -1140,9 +1140,10 @@ def mla_rope_append(q, nope, kv, norm_w, eps, positions, slots, cos_sin, qfull, 
         int(cache.shape[0]) * block_tokens, int(q.dtype == torch.float32), _p(err_flag(q.device)), _st()), "ksana_mla_rope_append")
 
 
-def gather_latents(cache, block_tokens, block_table, kv_lens, cu_k, total, max_kv_len):
+def gather_latents(cache, block_tokens, block_table, kv_lens, cu_k, total, max_kv_len, out=None):
     """Cached latent rows of whole sequences one after the other: [total, DK]; sequence s from row cu_k[s] on."""
-    out = torch.empty(total, cache.shape[-1], dtype=cache.dtype, device=cache.device)
+    if out is None:
+        out = torch.empty(total, cache.shape[-1], dtype=cache.dtype, device=cache.device)
     _check(lib().ksana_gather_latents(_p(cache), cache.stride(0), block_tokens, cache.shape[-1], _p(block_table), block_table.stride(0),
                                       _p(kv_lens), _p(cu_k), _p(out), kv_lens.numel(), max_kv_len, int(cache.shape[0]), _st()),
            "ksana_gather_latents")

@@ -33,12 +33,19 @@ def test_expanded_against_absorbed(monkeypatch):
                      pairs=sum(n * kv - n * (n - 1) // 2 for n, kv in zip(q_lens, kv_lens)))
     got = []
     with torch.inference_mode():
-        for expand in (True, False):
-            monkeypatch.setattr(DeepseekModel, "_expands", lambda self, mw, st, T, e=expand: e)
+        for expand in (True, False, None):
+            monkeypatch.setattr(DeepseekModel, "_expands", lambda self, mw, st, T, e=expand: e is not False)
+            if expand is None:                                               # no room for it: absorbed after all
+                def full(*args, empty=torch.empty, **kw):
+                    if args[0] == sum(kv_lens):
+                        raise torch.cuda.OutOfMemoryError()
+                    return empty(*args, **kw)
+                monkeypatch.setattr(torch, "empty", full)
             model.allocate_kv_cache(sum(nb) + 1, bt)
             model.kv_cache.copy_(torch.randn(model.kv_cache.shape, generator=torch.Generator().manual_seed(5)).to(model.kv_cache))
             got.append((model.forward(step).float(), model.kv_cache.clone()))
             native.check_err_flag(DEV)
+    assert torch.equal(got[1][0], got[2][0]) and torch.equal(got[1][1], got[2][1])
     assert torch.equal(got[0][1][:, 0], got[1][1][:, 0])                     # the first layer appends the same latents
     # two roundings of queries and keys to bf16 in other places
     assert float((got[0][0] - got[1][0]).norm() / got[1][0].norm()) < 2e-2
