@@ -12,8 +12,8 @@
 // Prefill: 64 rows per CTA (4 warps x 16), K/V tiles of 64 tokens, online
 // softmax in fp32 (exp2), only the NEW query rows are computed: the causal
 // offset is kv_len - q_len, so cached prefixes cost no attention work.
-// Decode: all (sequence, kv head, tile) units of a launch lie in one line that is cut into equal ranges, one per
-// resident CTA (paged_decode_stream_kernel); 4 warps walk disjoint 16-token slices of each tile, a fifth keeps the
+// Decode: all (sequence, kv head, tile) units of a launch lie in one line that is shared out over the resident CTAs, in equal
+// ranges or by items, whichever is cheaper (paged_decode_stream_kernel); 4 warps walk disjoint 16-token slices of each tile, a fifth keeps the
 // tile ring full by TMA. Caches that TMA cannot read (other block sizes or strides) take paged_decode_kernel: one
 // CTA per (kv head, sequence, split), all threads copying, and a small reduce kernel.
 //

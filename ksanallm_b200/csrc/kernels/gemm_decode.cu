@@ -8,7 +8,8 @@
 // took about 7 us of every launch, and its 226 KB of shared memory keep any other kernel off the SM. Here:
 //   * a CTA owns one 128-feature tile, or one of S equal shares of its K range; the S CTAs of a tile are a cluster and add their fp32
 //     sums through distributed shared memory (one cluster barrier instead of the exchange);
-//   * half an SM's shared memory per CTA: two share an SM, so that one streams while the other starts or ends, and under
+//   * half an SM's shared memory per CTA (up to 165 KB for e4m3 with K in the tens of thousands, whose token exponents are kept there):
+//     two share an SM, so that one streams while the other starts or ends, and under
 //     programmatic dependent launch the weights of this kernel are on their way while the kernel before it finishes (where the
 //     caller says that nothing in flight writes them).
 // Against gemm_smallm.cu (us, in graphs): bf16, 1 row, 6144 x 4096 21 -> 12, 4096 x 4096 18 -> 9, 28672 x 4096 50 -> 37, 4096 x 14336
@@ -18,6 +19,7 @@
 // Every wait is bounded.
 #include "sm100_ptx.cuh"
 #include "pdl.cuh"
+#include "cluster.cuh"
 #include <atomic>
 #include <cuda_bf16.h>
 
@@ -48,17 +50,6 @@ struct GemmDecodeCfg {
   static constexpr int kFixedBytes = kStages * kStageBytes + kSfBytes + 1024 + 256;      // + exponents [K blocks][MP] (kind 2)
   static_assert(MP * kGdRedPitch * 4 <= kStages * kStageBytes, "the sums lie over the operand ring");
 };
-
-__device__ __forceinline__ float gd_ld_cluster(uint32_t addr, uint32_t rank) {
-  uint32_t remote;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-  return v;
-}
-__device__ __forceinline__ void gd_cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 // feature n of B consecutive tokens from m0 on (those below m1): bias and residual added, rounded once
 template <int B>
@@ -275,7 +266,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   }
   if (S > 1) {
     __syncwarp();
-    gd_cluster_sync();                        // every share's sums are in its CTA's shared memory
+    cluster_sync_all();                        // every share's sums are in its CTA's shared memory
     if (warp >= 2 && warp < 6 && !*abort_flag) {
       const int f = (warp & 3) * 32 + lane, n = tile * 128 + f;
       const int m0 = rank * p.M / S, m1 = (rank + 1) * p.M / S;               // the tokens this CTA finishes
@@ -288,7 +279,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
           for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[k][i] = gd_ld_cluster(base + min(m + i, MP - 1) * (kGdRedPitch * 4), r + k);
+            for (int i = 0; i < 4; ++i) x[k][i] = ld_cluster_f32(base + min(m + i, MP - 1) * (kGdRedPitch * 4), r + k);
 #pragma unroll
           for (int i = 0; i < 4; ++i) v[i] = (v[i] + x[0][i]) + x[1][i];
         }
@@ -296,7 +287,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       }
     }
     __syncwarp();
-    gd_cluster_sync();                        // a peer may still read this CTA's sums
+    cluster_sync_all();                        // a peer may still read this CTA's sums
   }
   tc_fence_before();
   __syncthreads();
@@ -383,8 +374,11 @@ extern "C" int ksana_gemm_decode(int kind, const void* X, int ldx, const float* 
   // fewest shares that give every SM a CTA, four K blocks each at least. Measured (us for 1 / 2 / 4 / 8 shares, cold weights): e4m3, 32
   // rows, N x K = 10240 x 8192 32 / 21 / 27 / 27, 8192 x 8192 31 / 20 / 16 / 21, 4096 x 7168 26 / 17 / 11 / 10, 57344 x 8192 82 / 102 /
   // 100 / 129; bf16, 16 rows, 6144 x 4096 21 / 14 / 12 / 16, 4096 x 14336 67 / 37 / 23 / 22, 28672 x 4096 38 / 44 / 49 / 58.
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   p.splits = 1;
-  while (p.splits < 8 && tiles * p.splits < 148 && num_kb >= p.splits * 8) p.splits *= 2;
+  while (p.splits < 8 && tiles * p.splits < sms && num_kb >= p.splits * 8) p.splits *= 2;
   const bool early = fixed_w != 0;
   if (kind == 0)
     return MP == 16 ? launch_gemm_decode<16, 0>(mw, mx, p, early, st) : MP == 32 ? launch_gemm_decode<32, 0>(mw, mx, p, early, st)

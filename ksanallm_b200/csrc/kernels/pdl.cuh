@@ -14,9 +14,10 @@
 //   * a kernel launched through launch_pdl() that lacks pdl_wait() would race: only kernels that call it are launched
 //     with the attribute;
 //   * both calls are no-ops in a kernel launched without the attribute.
-// The attribute is on for the kernels launched through launch_early(): those of decode steps, which leave room on the SM for a
-// neighbour (half its shared memory at most), so that a GEMM's first weight tiles are on their way while the norm or the attention before
-// it ends. 8 layers of 4096, one sequence: 1070 -> 976 us per step, 64 sequences: 1575 -> 1544 us. The others take it with
+// The attribute is on for the kernels launched through launch_early(): those of decode steps, most of which leave room on the SM for a
+// neighbour, so that a GEMM's first weight tiles are on their way while the norm or the attention before it ends. (Not all do: decode
+// attention with heads of 192 and 256 columns and e4m3 GEMMs with K in the tens of thousands take more than half of the shared memory;
+// what follows them starts as their CTAs end.) 8 layers of 4096, one sequence: 1070 -> 976 us per step, 64 sequences: 1575 -> 1544 us. The others take it with
 // KSANA_PDL=1 only: kernels that need a whole SM gained nothing (graphs of 800 kernels, within noise), and the 4-bit stream, whose CTAs
 // fill the register file, made its step slower (1130 -> 1386 us). KSANA_PDL=0 switches it off everywhere.
 #pragma once

@@ -15,6 +15,7 @@
 //     steps, sums up to 143 of them); no weight is rounded to bf16, which could cost 2^-6. (An infinite activation makes its row NaN.)
 //   * tiles of 128 features are cut along K over the CTAs of a cluster, which add their sums through distributed shared memory.
 #include "pdl.cuh"
+#include "cluster.cuh"
 #include <atomic>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
@@ -50,16 +51,6 @@ __device__ __forceinline__ uint4 ld_stream16(const uint8_t* p) {
 }
 // levels q and q + 4 of a packed word as bf16(128 + level): 0x4300 | level
 __device__ __forceinline__ uint32_t level_pair(uint32_t w, int q) { return ((w >> (4 * q)) & 0x000f000fu) | 0x43004300u; }
-__device__ __forceinline__ float ld_cluster_f32(uint32_t addr, uint32_t rank) {
-  uint32_t remote;
-  float v;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
-  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(remote) : "memory");
-  return v;
-}
-__device__ __forceinline__ void cluster_sync_all() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 
 template <int NT>                               // 8-token column tiles per CTA
 __global__ void __launch_bounds__(kW4sThreads, NT <= 2 ? 4 : NT == 4 ? 3 : 2)
