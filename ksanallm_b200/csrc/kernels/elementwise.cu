@@ -200,11 +200,10 @@ __device__ __forceinline__ float act_fn(float x, int act) {
   return fmaxf(x, 0.f);
 }
 
-// Memory is the bound it nears: gated and quantised, an element reads 4 bytes and writes 1. Two vectors per thread are in flight, and
-// row and column come from a multiplication (the 64-bit division of a flat index was half of the kernel's instructions: 16384 x 28672
-// gated, quantised: 733 us with it, 566 us without, 532 us with maxima on packed pairs: 4.4 TB/s).
-constexpr int kActVecs = 2;
-template <int ACT, bool GATED, bool QUANT>
+// Memory is the bound it nears: gated and quantised, an element reads 4 bytes and writes 1. Row and column come from a multiplication (the
+// 64-bit division of a flat index was half of the kernel's instructions: 16384 x 28672 gated, quantised: 733 us with it, 566 us without,
+// 532 us with maxima on packed pairs: 4.4 TB/s). V vectors of a thread are in flight together; see launch_vectors for how many.
+template <int ACT, bool GATED, bool QUANT, int V>
 __global__ void __launch_bounds__(256)
 act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __restrict__ outq, float* __restrict__ oscale,
                int scale_ld, uint32_t total, FastDiv nvec, int in_ld, const int* __restrict__ tile_rows) {
@@ -212,12 +211,12 @@ act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __r
   pdl_wait();
   const uint32_t step = gridDim.x * blockDim.x;
   // whole warps stay in the loop for the shuffles; nvec is a multiple of 16 with QUANT, so 16 consecutive lanes share (m, group)
-  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; (base & ~31u) < total; base += kActVecs * step) {
-    uint4 g[kActVecs], u[kActVecs];
-    uint32_t m[kActVecs], i[kActVecs];
-    bool on[kActVecs];
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; (base & ~31u) < total; base += V * step) {
+    uint4 g[V], u[V];
+    uint32_t m[V], i[V];
+    bool on[V];
 #pragma unroll
-    for (int k = 0; k < kActVecs; ++k) {
+    for (int k = 0; k < V; ++k) {
       const uint32_t idx = base + k * step;
       on[k] = idx < total;
       m[k] = on[k] ? nvec.div(idx) : 0u;
@@ -230,7 +229,7 @@ act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __r
       }
     }
 #pragma unroll
-    for (int k = 0; k < kActVecs; ++k) {
+    for (int k = 0; k < V; ++k) {
       uint4 packed = make_uint4(0, 0, 0, 0);
       if (on[k]) {
         float gf[8], uf[8], o[8];
@@ -271,12 +270,12 @@ __global__ void act_mul_f32_kernel(const float* __restrict__ in, float* __restri
 
 // x[M,K] bf16 -> e4m3 + one scale per (row, 128 columns); scales stored [K/128][scale_ld]. Index arithmetic and loads in flight as in
 // act_mul_kernel.
+template <int V>
 __global__ void __launch_bounds__(256)
 quant_fp8_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int scale_ld, uint32_t total,
                  FastDiv nvec, int x_ld) {
   pdl_trigger();
   pdl_wait();
-  constexpr int V = 4;
   const uint32_t step = gridDim.x * blockDim.x;
   for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; (base & ~31u) < total; base += V * step) {
     uint4 v[V];
@@ -640,6 +639,15 @@ static inline int grid_for(long long work, int threads, int cap = 148 * 8) {
   if (g < 1) g = 1;
   return static_cast<int>(g > cap ? cap : g);
 }
+// 16-byte vectors per thread of the activation and quantisation kernels: one while all threads are resident at once (300 x 7168 quantised: 2.5
+// us with one, 3.2 with two, 4.0 with four) and for gated inputs, which have two loads in flight anyway (9000 x 14336 gated and quantised
+// 112 / 123 / 114 us); else two (9000 x 14336 quantised 73 / 70 / 81 us, activation without a gate 95.7 / 94 / 97).
+static inline int launch_vectors(long long total, bool gated) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return gated || total <= sms * 2048LL ? 1 : 2;
+}
 static inline int norm_threads(int H) {
   int t = ((H >> 3) + kMaxVec - 1) / kMaxVec;
   t = ((t + 31) / 32) * 32;
@@ -718,14 +726,17 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
     uint8_t* dq = outq ? (uint8_t*)outq + static_cast<size_t>(m0) * I : nullptr;
     float* ds = oscale ? oscale + m0 : nullptr;
     const int* tr = tile_rows ? tile_rows + m0 / 128 : nullptr;
-    const dim3 grid(grid_for((total + kActVecs - 1) / kActVecs, 256));
-#define KSANA_ACT(A, G, Q) launch_early(act_mul_kernel<A, G, Q>, grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total, div, in_ld, tr)
-#define KSANA_ACT_G(A) (gated ? (outq ? KSANA_ACT(A, true, true) : KSANA_ACT(A, true, false)) \
-                              : (outq ? KSANA_ACT(A, false, true) : KSANA_ACT(A, false, false)))
+    const int v = launch_vectors(total, gated);
+    const dim3 grid(grid_for((static_cast<long long>(total) + v - 1) / v, 256));
+#define KSANA_ACT(A, G, Q, V) launch_early(act_mul_kernel<A, G, Q, V>, grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total, div, in_ld, tr)
+#define KSANA_ACT_V(A, Q) (v == 1 ? KSANA_ACT(A, false, Q, 1) : KSANA_ACT(A, false, Q, 2))
+#define KSANA_ACT_G(A) (gated ? (outq ? KSANA_ACT(A, true, true, 1) : KSANA_ACT(A, true, false, 1)) \
+                              : (outq ? KSANA_ACT_V(A, true) : KSANA_ACT_V(A, false)))
     if (act == 0) KSANA_ACT_G(0);
     else if (act == 1) KSANA_ACT_G(1);
     else KSANA_ACT_G(2);
 #undef KSANA_ACT_G
+#undef KSANA_ACT_V
 #undef KSANA_ACT
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
@@ -748,8 +759,10 @@ extern "C" int ksana_quant_fp8(const void* x, void* q, float* scale, int scale_l
   for (int m0 = 0; m0 < M; m0 += most) {
     const int rows = M - m0 < most ? M - m0 : most;
     const uint32_t total = static_cast<uint32_t>(rows) * nvec;
-    launch_early(quant_fp8_kernel, dim3(grid_for((total + 3) / 4, 256)), dim3(256), 0, st, (const bf16*)x + static_cast<size_t>(m0) * x_ld,
-               (uint8_t*)q + static_cast<size_t>(m0) * K, scale + m0, scale_ld, total, div, x_ld);
+    const int v = launch_vectors(total, false);
+    launch_early(v == 1 ? quant_fp8_kernel<1> : quant_fp8_kernel<2>, dim3(grid_for((static_cast<long long>(total) + v - 1) / v, 256)), dim3(256), 0,
+                 st, (const bf16*)x + static_cast<size_t>(m0) * x_ld, (uint8_t*)q + static_cast<size_t>(m0) * K, scale + m0, scale_ld, total, div,
+                 x_ld);
   }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
