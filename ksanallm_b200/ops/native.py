@@ -472,7 +472,11 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
         # they fill the SMs).
         t256 = ((M + 127) // 128) * ((N + 255) // 256)
         # (wide layers at more than 32 rows: the tiled kernel, 86 against 102 us for 64 x 57344 x 8192, 53 against 61 us for 36864 x 7168)
-        if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K <= DECODE_MAX_K_MX and (M <= 32 or N <= 32768):
+        # (small ones at more than 48 rows likewise: adding two shares' sums of 64 tokens takes longer than half of K saves, 7.6 against
+        # 8.5 us for 64 x 1024 x 1024, 8.8 against 9.2 for 64 x 2048 x 1280; with 48 rows 7.6 both, with K of 1536 9.3 and 9.5, of 2048
+        # 10.8 and 7.3)
+        small = M > 48 and K <= 1280 and N <= 4096
+        if M <= DECODE_MAX_M and splits == 0 and bn == 0 and K <= DECODE_MAX_K_MX and (M <= 32 or N <= 32768) and not small:
             return _gemm_decode(2, xq, xs, wq, ws, out, out_f32, bias, residual, M, N, K, fixed_w)
         skinny = M <= SMALL_M_FP8 or (M <= 128 and _skinny_wins_mx(M, N, K))
         if (skinny or splits != 0) and M <= 128 and bn == 0:
