@@ -124,13 +124,22 @@ class DeepseekModel(CommonModel):
         """Whether a step's latents are better expanded to keys and values of every head than attended as they are. Per (query, key)
         pair and head the absorbed form takes 2 x 1088 operations at about 330 TFLOP/s, the expanded one 2 x 320 at about 700, which
         costs 2 x 512 x 256 per cached token and head (and writing the result) but saves the two per-head products of every query
-        row: 50 ns per cached token against 143 ns per row at 128 heads."""
+        row: 50 ns per cached token against 143 ns per row at 128 heads. Neither is faster than one CTA's walk over the longest
+        sequence, 2.1 and 2.4 us per 64 keys, which is all the absorbed form takes while its CTAs (two per 128 rows and heads) run at once;
+        the expansion of 65 to 128 tokens takes 10 us more than its share, by the GEMM for so many rows. us expanded / absorbed: 16 heads, 128
+        tokens 38 / 28, 200 on 3800 cached 185 / 166, 1000 on 11000 498 / 848; 128 heads, 200 on 3800 404 / 502, 64 on 1936 220 / 115."""
+        from ..ops import native
         if (mw.kv_b is None or step.num_single or not step.pairs or (self.nope, self.rope, self.vdim, self.lora) != (128, 64, 128, 512)
                 or step.total_kv_len * self.Hq * 512 > 4 << 30):
             return False
-        share = self.Hq / 128
-        absorbed = step.pairs * self.Hq * 2 * 1088 / 330e12 + T * share * 143e-9
-        return step.pairs * self.Hq * 2 * 320 / 700e12 + step.total_kv_len * share * 50e-9 < 0.9 * absorbed
+        share, tiles = self.Hq / 128, -(-step.max_kv_len // 64)
+        absorbed = tiles * 2.4e-6
+        if -(-T * self.Hq // 128) * 2 > native._sms(self.device):
+            absorbed = max(absorbed, step.pairs * self.Hq * 2 * 1088 / 330e12)
+        expanded = max(tiles * 2.1e-6, step.pairs * self.Hq * 2 * 320 / 700e12) + step.total_kv_len * share * 50e-9
+        if 64 < step.total_kv_len <= 128:
+            expanded += 10e-6
+        return expanded < 0.9 * (absorbed + T * share * 143e-9)
 
     def _expansion_room(self, q, step, cache):
         """Place for the latents of a step's sequences and for their keys and values (up to 4 GB), None where the device has none left:
