@@ -140,6 +140,57 @@ __device__ __forceinline__ void mma_f8(uint32_t d_tmem, uint64_t adesc, uint64_t
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
 }
 
+// The same where a whole warp runs the issuing code and `lead` is set in one of its lanes (elect_one): control flow stays uniform, and
+// so do the descriptors, which the instruction takes from uniform registers. An issuing thread behind a branch spends 80 to 130 clocks on
+// each (measured in the attention of prompts), more than an MMA of 128 x 128 x 16 takes.
+__device__ __forceinline__ void mma_f16_lead(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void mma_f16_ts_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
+                                                uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void tc_commit_lead(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n"
+      ::"r"(smem_u32(bar)), "r"(lead) : "memory");
+}
+// mbar_wait and mbar_arrive of a whole, converged warp: the instruction is one lane's, by a predicate and not by a branch, so that the warp
+// stays converged for what needs that. (32 polling lanes are served one after the other, some 300 clocks even where the phase is over.)
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint32_t lead, volatile uint32_t* abort_flag) {
+  for (uint32_t it = 0; it < kWaitPolls; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred P, e;\n\t"
+        "setp.ne.b32 e, %3, 0;\n\tsetp.ne.b32 P, 0, 0;\n\t"
+        "@e mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.b32 %0, 1, 0, P;\n\t}\n"
+        : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "r"(lead) : "memory");
+    if (__any_sync(0xffffffffu, done)) {
+      __syncwarp();
+      return true;
+    }
+    if ((it & 63u) == 63u && __any_sync(0xffffffffu, *abort_flag != 0)) return false;
+  }
+  *abort_flag = 1;
+  return false;
+}
+__device__ __forceinline__ void mbar_arrive_lead(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}\n" ::"r"(smem_u32(bar)), "r"(lead) : "memory");
+}
+
 // TMEM -> registers: this warp's 32 lanes x 32 consecutive fp32 columns.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
