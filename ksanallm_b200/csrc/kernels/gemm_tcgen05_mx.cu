@@ -17,6 +17,8 @@
 // CTA layout (352 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warp 2 scale packer,
 // warps 3..10 epilogue (two warpgroups split the columns). BN = 256 uses one 256-column accumulator (the
 // epilogue drains it into registers and hands it back before storing); BN = 128 double-buffers.
+// The MMA warp runs its loop as a whole and issues by predicate: an issuing thread behind a branch took some 100 clocks an MMA, as long as
+// the MMA itself (300 x 8192 x 8192 59 -> 41 us, 8000 x 2112 x 7168 125 -> 107, 128 x 8192 x 8192 32 -> 23).
 // No cluster launch, no multicast. Every wait is bounded.
 //
 // Grouped (mixture-of-experts) mode: expert-major rows, every 128-row tile multiplies with the matrix of its own expert
@@ -99,7 +101,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   volatile uint32_t* abort_flag = tmem_slot + 1;
   uint8_t* epi_stage = reinterpret_cast<uint8_t*>(bars) + 512;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m_tiles = (p.M + kMxBM - 1) / kMxBM;
   const int n_tiles = (p.N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
@@ -117,7 +119,8 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
   auto unused = [&](int tile) {                  // grouped mode: a tile behind the last expert's rows
     if (!p.tile_expert) return false;
     int m_blk, n_blk;
@@ -174,30 +177,30 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
     pdl_wait();
-    if (lane == 0) {
+    {
       int stage = 0; uint32_t phase = 0;
       int sfs = 0; uint32_t sf_phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       uint32_t set = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        if (unused(tile)) continue;
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (__any_sync(0xffffffffu, unused(tile))) continue;
+        if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int g = 0; g < num_groups && ok; ++g) {
-          if (!mbar_wait(&sf_full[sfs], sf_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&sf_full[sfs], sf_phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsfa = tmem_base + Cfg::kSfBase + set * Cfg::kSfCols;
           const uint32_t tsfb = tsfa + 4;
           const uint32_t sf_addr = smem_u32(sf_smem + sfs * Cfg::kSfStageBytes);
-          tmem_cp_sf(tsfa, make_sf_desc(sf_addr));
+          tmem_cp_sf_lead(lead, tsfa, make_sf_desc(sf_addr));
 #pragma unroll
-          for (int c = 0; c < Cfg::kBChunks; ++c) tmem_cp_sf(tsfb + 4 * c, make_sf_desc(sf_addr + 512 * (1 + c)));
+          for (int c = 0; c < Cfg::kBChunks; ++c) tmem_cp_sf_lead(lead, tsfb + 4 * c, make_sf_desc(sf_addr + 512 * (1 + c)));
           for (int j = 0; j < 4; ++j) {
             const int kb = g * 4 + j;
             if (kb >= num_kb) break;
-            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
             const uint64_t adesc = make_smem_desc_sw128(sa);
@@ -205,16 +208,16 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
             const uint32_t idesc = make_idesc_mx(kMxBM, BN, static_cast<uint32_t>(j));
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              mma_mxf8(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
-            tc_commit(&empty_bar[stage]);
+              mma_mxf8_lead(lead, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
+            tc_commit_lead(lead, &empty_bar[stage]);
             if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
           }
-          tc_commit(&sf_empty[sfs]);
+          tc_commit_lead(lead, &sf_empty[sfs]);
           if (++sfs == kMxSfStages) { sfs = 0; sf_phase ^= 1; }
           set ^= 1;
         }
         if (ok) {
-          tc_commit(&tfull_bar[acc]);
+          tc_commit_lead(lead, &tfull_bar[acc]);
           if (++acc == Cfg::kAccStages) { acc = 0; acc_phase ^= 1; }
         }
       }

@@ -8,7 +8,8 @@
 // the producer's ring stays full while the MMA thread waits for data) then holds the tensor pipe below 60 %.
 // A 256 x 224 tile needs 60 KB per K block for 1.75 times the MMA work (34 KB per 128 x 256 equivalent). It is
 // the largest tile whose two fp32 accumulators (2 x 224 TMEM columns) leave room for the scale columns. No
-// cluster, no multicast. Every wait is bounded.
+// cluster, no multicast. Every wait is bounded. The MMA warp issues by predicate, as a whole (behind a branch the eight MMAs of a K block
+// took longer to issue than to run: 4000 x 10240 x 8192 270 -> 257 us, 16384 x 8192 x 8192 847 -> 807, 4000 x 8192 x 29568 728 -> 688).
 //
 // CTA layout (352 threads): warp 0 TMA producer, warp 1 MMA issuer + TMEM owner, warp 2 scale packer, warps 3..10
 // epilogue (one warpgroup per accumulator, each drains its 224 columns in two passes of 112).
@@ -82,7 +83,7 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
   volatile uint32_t* abort_flag = tmem_slot + 1;
   uint8_t* epi_stage = reinterpret_cast<uint8_t*>(bars) + 512;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m_tiles = (p.M + kTlBM - 1) / kTlBM;
   const int n_tiles = (p.N + kTlBN - 1) / kTlBN;
   const int num_tiles = m_tiles * n_tiles;
@@ -101,7 +102,8 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -126,28 +128,28 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       int stage = 0; uint32_t phase = 0;
       int sfs = 0; uint32_t sf_phase = 0;
       uint32_t acc_phase = 0;
       uint32_t set = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait(tempty_bar, acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(tempty_bar, acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d0 = tmem_base, d1 = tmem_base + kTlBN;
         for (int g = 0; g < num_groups && ok; ++g) {
-          if (!mbar_wait(&sf_full[sfs], sf_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&sf_full[sfs], sf_phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsfa = tmem_base + kTlSfBase + set * kTlSfCols;
           const uint32_t tsfb = tsfa + 8;
           const uint32_t sf_addr = smem_u32(sf_smem + sfs * kTlSfStageBytes);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) tmem_cp_sf(tsfa + 4 * c, make_sf_desc(sf_addr + 512 * c));
+          for (int c = 0; c < 4; ++c) tmem_cp_sf_lead(lead, tsfa + 4 * c, make_sf_desc(sf_addr + 512 * c));
           for (int j = 0; j < 4; ++j) {
             const int kb = g * 4 + j;
             if (kb >= num_kb) break;
-            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sa = smem_u32(smem + stage * kTlStageBytes);
             const uint64_t adesc0 = make_smem_desc_sw128(sa);
@@ -156,18 +158,18 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
             const uint32_t idesc = make_idesc_mx(128, kTlBN, static_cast<uint32_t>(j));
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-              mma_mxf8(d0, adesc0 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
-              mma_mxf8(d1, adesc1 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa + 4, tsfb);
+              mma_mxf8_lead(lead, d0, adesc0 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
+              mma_mxf8_lead(lead, d1, adesc1 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa + 4, tsfb);
             }
-            tc_commit(&empty_bar[stage]);
+            tc_commit_lead(lead, &empty_bar[stage]);
             if (++stage == kTlStages) { stage = 0; phase ^= 1; }
           }
-          tc_commit(&sf_empty[sfs]);
+          tc_commit_lead(lead, &sf_empty[sfs]);
           if (++sfs == kTlSfStages) { sfs = 0; sf_phase ^= 1; }
           set ^= 1;
         }
         if (ok) {
-          tc_commit(tfull_bar);
+          tc_commit_lead(lead, tfull_bar);
           acc_phase ^= 1;
         }
       }

@@ -9,7 +9,7 @@
 // Warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 scales, warps 6..13 epilogue; single 256-column accumulator and bounded waits as in
 // the FP8 hardware-scaled kernel. The scales of a K block travel by TMA with its operands (16 bytes a row); four warps, one per quarter
 // of TMEM, write them there from registers. (tcgen05.cp of 512-byte chunks, twelve a block, took about 80 clocks each between the MMAs of two
-// blocks, 1500 clocks a block with 512 of MMAs; now about 1070. A tile of 256 x 192 with them was slower by its work: 1002 us.) 9753 x
+// blocks, 1500 clocks a block with 512 of MMAs; now about 1050. A tile of 256 x 192 with them was slower by its work: 1002 us.) 9753 x
 // 28672 x 4096: 1094 us with scales loaded by a packer warp on demand, 832 by TMA and tcgen05.cp, 695 now (3.3 PFLOP/s); 9753 x 4096 x
 // 14336: 612, 432, 319.
 //
@@ -84,7 +84,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + Cfg::kAccStages);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m_tiles = (p.M + kF4BM - 1) / kF4BM;
   const int n_tiles = (p.N + BN - 1) / BN;
   const int num_tiles = m_tiles * n_tiles;
@@ -100,7 +100,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -133,7 +134,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
@@ -141,14 +142,14 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         if (p.tile_expert) {
           int m_blk, n_blk;
           f4_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
-          if (p.tile_expert[m_blk] < 0) continue;
+          if (__any_sync(0xffffffffu, p.tile_expert[m_blk] < 0)) continue;
         }
-        if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         for (int kb = 0; kb < num_kb && ok; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
-          if (!mbar_wait(&sf_full[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&sf_full[stage], phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsf = tmem_base + Cfg::kSfBase + stage * Cfg::kSfCols;
           const uint32_t sa = smem_u32(smem + stage * Cfg::kStageBytes);
@@ -158,13 +159,13 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           constexpr uint32_t idesc = make_idesc_nvf4(kF4BM, BN);
 #pragma unroll
           for (int k = 0; k < 4; ++k)      // 64 elements (32 bytes) per MMA, four e4m3 scales per row and MMA
-            mma_nvf4(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsf + 4 * kPerMma * k,
+            mma_nvf4_lead(lead, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsf + 4 * kPerMma * k,
                      tsf + 4 * kPerMma * k + 4);
-          tc_commit(&empty_bar[stage]);
+          tc_commit_lead(lead, &empty_bar[stage]);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
         if (ok) {
-          tc_commit(&tfull_bar[acc]);
+          tc_commit_lead(lead, &tfull_bar[acc]);
           if (++acc == Cfg::kAccStages) { acc = 0; acc_phase ^= 1; }
         }
       }
@@ -183,7 +184,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       }
       for (int kb = 0; kb < num_kb; ++kb) {
         // the stage was loaded after its MMAs had ended, so that its scale columns are free too
-        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         constexpr int kPerMma = 1 + Cfg::kBChunks;
         const uint4* rows = reinterpret_cast<const uint4*>(smem + stage * Cfg::kStageBytes + Cfg::kSfOff);
@@ -205,7 +206,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&sf_full[stage]);
+        mbar_arrive_lead(lead, &sf_full[stage]);
         if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
@@ -229,7 +230,8 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
         expert = p.tile_expert[m_blk];
         if (expert < 0) continue;
       }
-      if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+      __syncwarp();                             // lanes without a row come from the tile before by another path
+      if (!mbar_wait_warp(&tfull_bar[acc], acc_phase, lead, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[EC];
 #pragma unroll
@@ -237,7 +239,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       tmem_ld_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(&tempty_bar[acc]);     // the accumulator is in registers: the next tile may start
+      mbar_arrive_lead(lead, &tempty_bar[acc]);     // the accumulator is in registers: the next tile may start
       if (++acc == Cfg::kAccStages) { acc = 0; acc_phase ^= 1; }
       if (!row_ok) continue;
       const float alpha = (p.a_ts ? *p.a_ts : 1.f) * (p.w_ts ? p.w_ts[expert] : 1.f);

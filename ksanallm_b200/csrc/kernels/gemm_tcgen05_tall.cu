@@ -62,7 +62,7 @@ gemm_bf16_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int m_tiles = (p.M + kBtBM - 1) / kBtBM;
   const int n_tiles = (p.N + kBtBN - 1) / kBtBN;
   const int num_tiles = m_tiles * n_tiles;
@@ -79,7 +79,8 @@ gemm_bf16_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -104,17 +105,17 @@ gemm_bf16_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc = make_idesc(128, kBtBN, 1, 1);
       int stage = 0; uint32_t phase = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = blockIdx.x; tile < num_tiles && ok; tile += gridDim.x) {
-        if (!mbar_wait(tempty_bar, acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(tempty_bar, acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d0 = tmem_base, d1 = tmem_base + kBtBN;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * kBtStageBytes);
           const uint64_t adesc0 = make_smem_desc_sw128(sa);
@@ -122,14 +123,14 @@ gemm_bf16_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
           const uint64_t bdesc = make_smem_desc_sw128(sa + kBtABytes);
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
-            mma_f16(d0, adesc0 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
-            mma_f16(d1, adesc1 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
+            mma_f16_lead(lead, d0, adesc0 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
+            mma_f16_lead(lead, d1, adesc1 + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0);
           }
-          tc_commit(&empty_bar[stage]);
+          tc_commit_lead(lead, &empty_bar[stage]);
           if (++stage == kBtStages) { stage = 0; phase ^= 1; }
         }
         if (ok) {
-          tc_commit(tfull_bar);
+          tc_commit_lead(lead, tfull_bar);
           acc_phase ^= 1;
         }
       }

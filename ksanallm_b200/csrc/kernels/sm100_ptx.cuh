@@ -102,6 +102,28 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// The same by a whole, converged warp that has `lead` set in one lane (elect_one) and the same coordinates in all: operands in uniform
+// registers. A box that a lane issues behind a branch takes some 100 clocks of its warp, whatever its size: 32 boxes of a tile of 16-token
+// cache blocks took as long as the tile's products.
+__device__ __forceinline__ void tma_load_2d_lead(uint32_t lead, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+      "@e cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}\n"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void tma_load_3d_lead(uint32_t lead, void* smem_dst, const CUtensorMap* m, uint64_t* bar, int x, int y, int z) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %6, 0;\n\t"
+      "@e cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];\n\t}\n"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(smem_u32(bar)), "r"(x), "r"(y), "r"(z), "r"(lead)
+      : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_lead(uint32_t lead, uint64_t* bar, uint32_t bytes) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}\n"
+               ::"r"(smem_u32(bar)), "r"(bytes), "r"(lead) : "memory");
+}
+
 // ------------------------------------------------------------------ tcgen05
 __device__ __forceinline__ void tmem_alloc(uint32_t* smem_dst, uint32_t ncols) {  // whole warp
   asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)),
@@ -151,6 +173,14 @@ __device__ __forceinline__ void mma_f16_lead(uint32_t lead, uint32_t d_tmem, uin
       "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
 }
+__device__ __forceinline__ void mma_f8_lead(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\t"
+      "setp.ne.b32 e, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
+}
 __device__ __forceinline__ void mma_f16_ts_lead(uint32_t lead, uint32_t d_tmem, uint32_t a_tmem, uint64_t bdesc, uint32_t idesc,
                                                 uint32_t accumulate) {
   asm volatile(
@@ -184,6 +214,19 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   }
   *abort_flag = 1;
   return false;
+}
+// Non-blocking probe of a phase by a whole warp.
+__device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity, uint32_t lead) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred P, e;\n\t"
+      "setp.ne.b32 e, %3, 0;\n\tsetp.ne.b32 P, 0, 0;\n\t"
+      "@e mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(done) : "r"(smem_u32(bar)), "r"(parity), "r"(lead) : "memory");
+  const bool any = __any_sync(0xffffffffu, done);
+  __syncwarp();
+  return any;
 }
 __device__ __forceinline__ void mbar_arrive_lead(uint32_t lead, uint64_t* bar) {
   asm volatile(
@@ -299,6 +342,17 @@ __device__ __forceinline__ void mma_mxf8(uint32_t d_tmem, uint64_t adesc, uint64
       "tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb) : "memory");
 }
+__device__ __forceinline__ void tmem_cp_sf_lead(uint32_t lead, uint32_t taddr, uint64_t sdesc) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e tcgen05.cp.cta_group::1.32x128b.warpx4 [%0], %1;\n\t}\n"
+               ::"r"(taddr), "l"(sdesc), "r"(lead) : "memory");
+}
+__device__ __forceinline__ void mma_mxf8_lead(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate, uint32_t tsfa, uint32_t tsfb) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 e, %7, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb), "r"(lead) : "memory");
+}
 // Block-scaled instruction descriptor: e4m3 x e4m3, UE8M0 scales, K-major operands; sf = scale byte of this MMA.
 __host__ __device__ constexpr uint32_t make_idesc_mx(uint32_t m, uint32_t n, uint32_t sf) {
   return (sf << 4) | (1u << 23) | ((n >> 3) << 17) | ((m >> 4) << 24) | (sf << 29);
@@ -310,6 +364,13 @@ __device__ __forceinline__ void mma_nvf4(uint32_t d_tmem, uint64_t adesc, uint64
       "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb) : "memory");
+}
+__device__ __forceinline__ void mma_nvf4_lead(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+                                              uint32_t accumulate, uint32_t tsfa, uint32_t tsfb) {
+  asm volatile(
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 e, %7, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb), "r"(lead) : "memory");
 }
 __host__ __device__ constexpr uint32_t make_idesc_nvf4(uint32_t m, uint32_t n) {
   return (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((m >> 4) << 24);     // e2m1 operands, UE4M3 scales, K-major
