@@ -21,15 +21,17 @@
 // panels row by row into TMEM; the other five panels (latent 256..511 and the rotary part) stay in shared
 // memory next to two 64-token KV stages. Per tile:
 //   S = Q K^T      36 tcgen05.mma (9 panels of 64 columns, K = 16 each, N = 64): 16 with A from TMEM, 20 with A from
-//                  shared memory; B = the staged tile, K-major (TMA, 128-byte swizzle). The 36 MMAs accumulate into
-//                  one tile and are latency-bound as a chain, which is why the tile is 64 tokens wide and not 32
-//                  (measured: same time per tile at either width).
+//                  shared memory; B = the staged tile, K-major (TMA, 128-byte swizzle)
 //   softmax        4 warps, one thread per row (TMEM lane), online maximum with a lazy rescale of O
 //   O += P V       P read from TMEM (bf16 pairs over S's columns), V = MN-major view of the same staged tile
-// The MMA thread issues S of tile j+1 ahead of P V of tile j when it is ready first, so the softmax of one tile
-// overlaps the tensor work of its neighbours. Warp roles: warp 0 TMA producer, warp 1 MMA issuer + TMEM owner,
-// warps 2..5 softmax + epilogue. Split-KV (decode): grid.x carries `nsplit` ranges of KV tiles whose unnormalised
-// partial outputs (fp32 O, running maximum, row sum) are merged by mla_merge_kernel.
+// The MMA warp issues S of tile j+1 ahead of P V of tile j when it is ready first, so the softmax of one tile
+// overlaps the tensor work of its neighbours. Warp roles: warps 0 and 6 TMA producers (keys-only panels, this half's value panels),
+// warp 1 MMA issuer + TMEM owner, warps 2..5 softmax + epilogue. Split-KV (decode): grid.x carries `nsplit` ranges of KV tiles whose
+// unnormalised partial outputs (fp32 O, running maximum, row sum) are merged by mla_merge_kernel.
+// What bounds it: the chain load -> S -> softmax -> P V through two KV stages (no room for a third). Boxes and MMAs issued by a lane behind
+// a branch took 100 clocks each, 5700 a tile of 64 tokens; with converged issuing warps, one producer per kind of panel and keys-only
+// panels handed back when S is complete, about 3000 (the products alone: 2000). us before / after: 64 sequences of 900-1300 tokens, 128
+// heads 75 / 46; 64 of 4096, 16 heads 213 / 110; 32 of 4096, 128 heads 120 / 71; 4 prompts of 100 on 1500 cached tokens 502 / 282.
 // Every wait is bounded; a timeout sets the error word and leaves the output untouched.
 #include "sm100_ptx.cuh"
 #include "guards.cuh"
@@ -40,7 +42,7 @@
 
 namespace ksana {
 
-constexpr int kMlaThreads = 192;
+constexpr int kMlaThreads = 224;
 constexpr int kMlaM = 128;                    // packed query rows per CTA
 constexpr int kMlaTok = 64;                   // KV tokens per tile
 constexpr int kMlaMaxDv = 512, kMlaMaxDk = 576;
@@ -54,7 +56,6 @@ constexpr int kMlaKvBytes = kMlaPanels * kMlaKvPanelBytes;
 constexpr int kMlaStages = 2;                 // KV tiles in flight
 constexpr int kMlaSmemBytes = kMlaQBytes + kMlaStages * kMlaKvBytes + 1024 + 256;
 constexpr uint32_t kMlaTmemCols = 512;        // O half [0,256), S/P buffers at 256 and 320, Q at [384, 512)
-constexpr int kMlaMaxBoxes = kMlaTok / 8;      // TMA boxes per tile with the smallest (8-token) cache blocks
 static_assert(kMlaQTmemPanels * kMlaQPanelBytes <= kMlaStages * kMlaKvBytes, "Q staging must fit in the KV stages");
 constexpr float kMlaRescaleLog2 = 8.f;
 
@@ -102,8 +103,8 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   uint8_t* kv_s = smem + kMlaQBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kMlaQBytes + kMlaStages * kMlaKvBytes);
   uint64_t* q_full = bars;
-  uint64_t* kv_full = bars + 1;      // [kMlaStages]
-  uint64_t* kv_empty = bars + 5;     // [kMlaStages]
+  uint64_t* kv_full = bars + 1;      // [kMlaStages][2]: panels that are keys only, panels that are this half's values too
+  uint64_t* kv_empty = bars + 5;     // [kMlaStages][2]
   uint64_t* s_full = bars + 9;       // [2]
   uint64_t* p_full = bars + 11;      // [2]
   uint64_t* pv_done = bars + 13;
@@ -112,7 +113,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 16);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int s = blockIdx.z, half = blockIdx.y;
   const int G = p.G;
   const int q0 = p.cu_q[s], q_len = p.cu_q[s + 1] - q0;
@@ -139,13 +140,14 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   const int ntiles = max(min(tile_end, tile_lo + per) - tile_lo, 0);
   constexpr int panels = PANELS, q_tmem = PANELS < kMlaQTmemPanels ? PANELS : kMlaQTmemPanels;
   const int cols = min(256, p.dv - half * 256);             // output columns of this half
+  const int v_panels = min(4, panels - 4 * half);           // panels 4 half ..: this half's values (and the keys of some columns)
   const int* table = p.block_table + static_cast<size_t>(s) * p.table_stride;
 
   if (ntiles == 0) {
     // an empty KV range (more splits than tiles): publish "no contribution" for the merge and leave
     // (with a single split this only happens for kv_len == 0, e.g. padding rows of a captured decode graph:
     // their output rows are zeroed)
-    if (warp >= 2) {
+    if (warp >= 2 && warp < 6) {
       const int vr = row0 + (warp & 3) * 32 + lane;
       if (vr < q_len * G) {
         if (p.nsplit > 1) {
@@ -166,7 +168,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
-    for (int i = 0; i < kMlaStages; ++i) { mbar_init(kv_full + i, 1); mbar_init(kv_empty + i, 1); }
+    for (int i = 0; i < 2 * kMlaStages; ++i) { mbar_init(kv_full + i, 1); mbar_init(kv_empty + i, 1); }
     for (int i = 0; i < 2; ++i) { mbar_init(s_full + i, 1); mbar_init(p_full + i, 4); }
     mbar_init(pv_done, 1); mbar_init(o_full, 1); mbar_init(q_moved, 4);
     *abort_flag = 0;
@@ -176,8 +178,49 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();           // one lane of every warp: it polls, arrives and issues for the warp
   const uint32_t tmem_o = tmem_base, tmem_s = tmem_base + 256, tmem_q = tmem_base + 256 + 2 * kMlaTok;
+
+  // KV tiles, by two warps: one brings the panels that are keys only, which are free as soon as the scores of their tile are complete, the
+  // other this half's value panels, free after P V. A box of 16 tokens costs its warp some 60 clocks however the loop is written, as many
+  // as its data take from L2: one warp for all 36 boxes of a tile left the tensor cores waiting.
+  auto load = [&](int part) {
+    const int bt = p.block_tokens, br = p.box_rows, n = part ? v_panels : panels - v_panels;
+    const int boxes = kMlaTok / br;                         // at most 8 (8-token blocks), a lane each
+    // block-table entries of a tile are fetched one tile ahead, so that their global-memory latency is not part
+    // of the chain "buffer freed -> TMA issued"
+    auto fetch = [&](int j) {
+      const int t = (tile_lo + j) * kMlaTok + lane * br;
+      int id = (lane < boxes && t < kv_len) ? __ldg(table + t / bt) : 0;
+      if (id < 0 || id >= p.num_blocks) { guard_report(p.err, kGuardBlockId, id); id = 0; }
+      return id;
+    };
+    int next = fetch(0);
+    bool ok = mbar_wait_warp(q_moved, 0, lead, abort_flag);  // the staging area is free
+    for (int j = 0; j < ntiles; ++j) {
+      const int b = j % kMlaStages, t0 = (tile_lo + j) * kMlaTok;
+      const int nbox = min(boxes, (kv_len - t0 + br - 1) / br), id = next;
+      if (j + 1 < ntiles) next = fetch(j + 1);
+      uint64_t* bar = kv_full + 2 * b + part;
+      ok = ok && mbar_wait_warp(kv_empty + 2 * b + part, ((j / kMlaStages) & 1) ^ 1, lead, abort_flag);
+      if (!ok) break;
+      mbar_expect_tx_lead(lead, bar, static_cast<uint32_t>(nbox) * br * 128 * n);
+#pragma unroll 1
+      for (int bx = 0; bx < nbox; ++bx) {
+        const int blk = __shfl_sync(0xffffffffu, id, bx), t = (t0 + bx * br) % bt;
+        uint8_t* dst = kv_s + b * kMlaKvBytes + bx * br * 128;
+#pragma unroll
+        for (int i = 0; i < 5; ++i) {
+          if (i >= n) break;
+          const int pn = part ? 4 * half + i : half ? (i < 4 ? i : 8) : 4 + i;
+          if (FLAT) tma_load_2d_lead(lead, dst + pn * kMlaKvPanelBytes, &kv_map, bar, pn * 64, blk * p.rows_per_block + t);
+          else tma_load_3d_lead(lead, dst + pn * kMlaKvPanelBytes, &kv_map, bar, pn * 64, t, blk);
+        }
+      }
+    }
+    __syncwarp();
+  };
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -194,70 +237,27 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       }
     }
     __syncwarp();
-    {
-      // KV tiles: the whole warp runs the loop; lane 0 owns the barrier traffic, lanes 0..8 each issue the boxes of
-      // one 64-column panel (36 box copies per tile from a single thread were a microsecond of issue time)
-      const int bt = p.block_tokens, br = p.box_rows;
-      const int boxes = kMlaTok / br;                       // at most kMlaMaxBoxes (8-token blocks)
-      // block-table entries of a tile are fetched one tile ahead, so that their global-memory latency is not part
-      // of the chain "buffer freed -> TMA issued"
-      int blk[kMlaMaxBoxes], blk_next[kMlaMaxBoxes];
-      auto fetch = [&](int j, int (&dst)[kMlaMaxBoxes]) {
-        const int t0 = (tile_lo + j) * kMlaTok;
-#pragma unroll
-        for (int bx = 0; bx < kMlaMaxBoxes; ++bx) {
-          const int t = t0 + bx * br;
-          int id = (bx < boxes && t < kv_len) ? __ldg(table + t / bt) : 0;
-          if (id < 0 || id >= p.num_blocks) { guard_report(p.err, kGuardBlockId, id); id = 0; }
-          dst[bx] = id;
-        }
-      };
-      fetch(0, blk_next);
-      bool ok = mbar_wait(q_moved, 0, abort_flag);           // the staging area is free
-      for (int j = 0; j < ntiles; ++j) {
-        const int b = j % kMlaStages;
-        const int t0 = (tile_lo + j) * kMlaTok;
-        const int nbox = min(boxes, (kv_len - t0 + br - 1) / br);
-#pragma unroll
-        for (int bx = 0; bx < kMlaMaxBoxes; ++bx) blk[bx] = blk_next[bx];
-        if (j + 1 < ntiles) fetch(j + 1, blk_next);
-        ok = ok && mbar_wait(kv_empty + b, ((j / kMlaStages) & 1) ^ 1, abort_flag);
-        if (!__all_sync(0xffffffffu, ok)) break;
-        if (lane == 0) mbar_expect_tx(kv_full + b, static_cast<uint32_t>(nbox) * br * 128 * panels);
-        __syncwarp();
-        if (lane < panels) {
-          uint8_t* dst = kv_s + b * kMlaKvBytes + lane * kMlaKvPanelBytes;
-#pragma unroll
-          for (int bx = 0; bx < kMlaMaxBoxes; ++bx) {
-            if (bx < nbox) {
-              const int t = t0 + bx * br;
-              if (FLAT)
-                tma_load_2d(dst + bx * br * 128, &kv_map, kv_full + b, lane * 64, blk[bx] * p.rows_per_block + t % bt);
-              else
-                tma_load_3d(dst + bx * br * 128, &kv_map, kv_full + b, lane * 64, t % bt, blk[bx]);
-            }
-          }
-        }
-      }
-    }
-    __syncwarp();
+    load(0);
+  } else if (warp == 6) {
+    load(1);
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_qk = make_idesc(128, kMlaTok, 1, 1);
       const uint32_t idesc_pv = make_idesc(128, (cols + 63) / 64 * 64, 1, 1) | (1u << 16);     // B (= V) is MN-major
-      bool ok = mbar_wait(q_full, 0, abort_flag) && mbar_wait(q_moved, 0, abort_flag);
+      bool ok = mbar_wait_warp(q_full, 0, lead, abort_flag) && mbar_wait_warp(q_moved, 0, lead, abort_flag);
       tc_fence_after();
-      const uint32_t qb = smem_u32(q_s);
+      const uint64_t qd = make_smem_desc_sw128(smem_u32(q_s));
       // S of tile j+1 may be issued ahead of P V of tile j (it then overlaps the softmax of tile j), but whichever
       // of the two becomes ready first goes first: issuing P V as soon as P is ready frees the tile's buffer
       // early, which is what gives the next TMA load its lead time. The polls are test_wait (non-blocking): a
       // try_wait on the barrier that is not ready yet suspends the thread and hides the other one becoming ready.
       int s_next = 0, pv_next = 0;         // next tile whose S / P V has not been issued
+      int s_part = 0;                      // of tile s_next: keys-only panels, then the others
       uint32_t idle = 0;
       while (ok && pv_next < ntiles) {
         bool progress = false;
-        if (pv_next < s_next && mbar_test_wait(p_full + (pv_next & 1), (pv_next >> 1) & 1)) {
+        if (pv_next < s_next && mbar_test_warp(p_full + (pv_next & 1), (pv_next >> 1) & 1, lead)) {
           const int j = pv_next, bb = j & 1, st = j % kMlaStages;
           tc_fence_after();
           const uint32_t vb = smem_u32(kv_s + st * kMlaKvBytes) + half * 4 * kMlaKvPanelBytes;
@@ -265,38 +265,53 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
           for (int k = 0; k < kMlaTok / 16; ++k) {
             // 16 tokens per MMA: 8 TMEM columns of P (two bf16 each), 16 rows (2 KB per panel) of the tile
             const uint64_t bdesc = make_smem_desc_mn_sw128(vb + k * 2048, kMlaKvPanelBytes);
-            mma_f16_ts(tmem_o, tmem_s + kMlaTok * bb + 8 * k, bdesc, idesc_pv, (j | k) != 0);
+            mma_f16_ts_lead(lead, tmem_o, tmem_s + kMlaTok * bb + 8 * k, bdesc, idesc_pv, (j | k) != 0);
           }
-          tc_commit(kv_empty + st);
-          tc_commit(pv_done);
-          if (j == ntiles - 1) tc_commit(o_full);
+          tc_commit_lead(lead, kv_empty + 2 * st + 1);
+          tc_commit_lead(lead, pv_done);
+          if (j == ntiles - 1) tc_commit_lead(lead, o_full);
           ++pv_next;
           progress = true;
         } else if (s_next < ntiles && s_next <= pv_next + 1 &&
-                   mbar_test_wait(kv_full + (s_next % kMlaStages), (s_next / kMlaStages) & 1)) {
+                   mbar_test_warp(kv_full + 2 * (s_next % kMlaStages) + s_part, (s_next / kMlaStages) & 1, lead)) {
           // (s_next <= pv_next + 1: the S/P buffer of tile s_next was last read by P V of tile s_next - 2)
-          const int bb = s_next & 1;
+          const int bb = s_next & 1, st = s_next % kMlaStages;
           tc_fence_after();
-          const uint32_t kb = smem_u32(kv_s + (s_next % kMlaStages) * kMlaKvBytes);
-#pragma unroll
-          for (int k = 0; k < 4 * PANELS; ++k) {
-            const int pn = k >> 2;
-            const uint64_t bdesc = make_smem_desc_sw128(kb + pn * kMlaKvPanelBytes) + 2 * (k & 3);
+          const uint32_t kb = smem_u32(kv_s + st * kMlaKvBytes);
+          const uint64_t kd = make_smem_desc_sw128(kb);
+          // four products of a panel of the query and key rows
+          auto panel = [&](int pn, bool first) {
+            const uint64_t bdesc = kd + pn * (kMlaKvPanelBytes >> 4);
             if (pn < kMlaQTmemPanels) {
               // A (16 Q columns = 8 TMEM columns of bf16 pairs) straight from TMEM: no shared-memory read of Q
-              mma_f16_ts(tmem_s + kMlaTok * bb, tmem_q + 8 * k, bdesc, idesc_qk, k != 0);
+#pragma unroll
+              for (int k = 0; k < 4; ++k)
+                mma_f16_ts_lead(lead, tmem_s + kMlaTok * bb, tmem_q + 32 * pn + 8 * k, bdesc + 2 * k, idesc_qk, !(first && k == 0));
             } else {
-              const uint64_t adesc = make_smem_desc_sw128(qb + (pn - kMlaQTmemPanels) * kMlaQPanelBytes) + 2 * (k & 3);
-              mma_f16(tmem_s + kMlaTok * bb, adesc, bdesc, idesc_qk, k != 0);
+              const uint64_t adesc = qd + (pn - kMlaQTmemPanels) * (kMlaQPanelBytes >> 4);
+#pragma unroll
+              for (int k = 0; k < 4; ++k) mma_f16_lead(lead, tmem_s + kMlaTok * bb, adesc + 2 * k, bdesc + 2 * k, idesc_qk, !(first && k == 0));
             }
+          };
+          const int nk = panels - v_panels;
+          if (s_part == 0) {                     // keys-only panels: their place is free when these products have ended
+#pragma unroll 1
+            for (int i = 0; i < nk; ++i) panel(half ? (i < 4 ? i : 8) : 4 + i, i == 0);
+            tc_commit_lead(lead, kv_empty + 2 * st);
+            s_part = 1;
+            idle = 0;
+            continue;
           }
-          tc_commit(s_full + bb);
+#pragma unroll 1
+          for (int i = 0; i < v_panels; ++i) panel(4 * half + i, nk == 0 && i == 0);
+          s_part = 0;
+          tc_commit_lead(lead, s_full + bb);
           ++s_next;
           progress = true;
         }
         if (progress) {
           idle = 0;
-        } else if (++idle >= kWaitPolls || ((idle & 63u) == 63u && *abort_flag)) {
+        } else if (++idle >= kWaitPolls || ((idle & 63u) == 63u && __any_sync(0xffffffffu, *abort_flag != 0))) {
           *abort_flag = 1;
           ok = false;
         }
@@ -313,7 +328,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
     const int limit = active ? past + tok : -1;            // last visible KV position
     const int lowest = WINDOW ? limit - p.window + 1 : 0;              // first visible one
     float m_used = -CUDART_INF_F, l = 0.f;
-    bool ok = mbar_wait(q_full, 0, abort_flag);
+    bool ok = mbar_wait_warp(q_full, 0, lead, abort_flag);
     if (ok) {
       // this thread's Q row, columns [0, 384): staging area (128-byte-swizzled panels) -> registers -> TMEM, in the
       // layout the MMA reads an A operand from TMEM (row = lane, two consecutive bf16 per 32-bit column)
@@ -332,12 +347,12 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(q_moved);
+      mbar_arrive_lead(lead, q_moved);
     }
     for (int j = 0; ok && j < ntiles; ++j) {
       const int b = j & 1;
       const int t0 = (tile_lo + j) * kMlaTok;
-      if (!mbar_wait(s_full + b, (j >> 1) & 1, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_warp(s_full + b, (j >> 1) & 1, lead, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[kMlaTok];
 #pragma unroll
@@ -357,7 +372,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       const bool grow = m_new != m_used && m_used != -CUDART_INF_F;
       if (__any_sync(0xffffffffu, grow)) {
         // P V of the previous tile must have landed in O before O is rescaled (S of this tile was issued ahead of it)
-        if (!mbar_wait(pv_done, (j - 1) & 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(pv_done, (j - 1) & 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const float f = grow ? exp2f(m_used - m_new) : 1.f;
         l *= f;
@@ -399,9 +414,9 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) mbar_arrive(p_full + b);
+      mbar_arrive_lead(lead, p_full + b);
     }
-    if (ok && mbar_wait(o_full, 0, abort_flag)) {
+    if (ok && mbar_wait_warp(o_full, 0, lead, abort_flag)) {
       tc_fence_after();
       if (p.nsplit == 1) {
         const float inv = active ? mla_out_factor(l, m_used, p.sinks, p.gate, p.gate_ld, q0 + tok, head) : 0.f;
@@ -423,6 +438,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
               *reinterpret_cast<uint4*>(dst + c * 32 + i) = ov;
             }
           }
+          __syncwarp();
         }
       } else {
         const size_t prow = (static_cast<size_t>(split) * p.T + q0 + tok) * G + head;
@@ -437,6 +453,7 @@ mla_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_constant__
             for (int i = 0; i < 32; i += 4)
               if (c * 32 + i < cols) *reinterpret_cast<uint4*>(dst + c * 32 + i) = make_uint4(o[i], o[i + 1], o[i + 2], o[i + 3]);
           }
+          __syncwarp();
         }
         if (active && half == 0) {
           p.part_ml[prow * 2] = m_used;
