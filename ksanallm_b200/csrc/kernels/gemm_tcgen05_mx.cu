@@ -18,7 +18,8 @@
 // warps 3..10 epilogue (two warpgroups split the columns). BN = 256 uses one 256-column accumulator (the
 // epilogue drains it into registers and hands it back before storing); BN = 128 double-buffers.
 // The MMA warp runs its loop as a whole and issues by predicate: an issuing thread behind a branch took some 100 clocks an MMA, as long as
-// the MMA itself (300 x 8192 x 8192 59 -> 41 us, 8000 x 2112 x 7168 125 -> 107, 128 x 8192 x 8192 32 -> 23).
+// the MMA itself (300 x 8192 x 8192 59 -> 41 us, 8000 x 2112 x 7168 125 -> 107, 128 x 8192 x 8192 32 -> 23). The epilogue stores whole
+// sectors, 32 bytes a lane (8000 x 24576 x 1536 337 -> 278 us; with 16 bytes a sector reaches the L2 in two halves).
 // No cluster launch, no multicast. Every wait is bounded.
 //
 // Grouped (mixture-of-experts) mode: expert-major rows, every 128-row tile multiplies with the matrix of its own expert
@@ -30,6 +31,7 @@
 #include "sm100_ptx.cuh"
 #include "pdl.cuh"
 #include "push_epilogue.cuh"
+#include "vec8.cuh"
 #include <cuda_bf16.h>
 #include <stdio.h>
 
@@ -66,6 +68,7 @@ struct MxParams {
   const float* w_scale;
   int* err;
   __nv_bfloat16* push[8]; int push_n; int push_rows;
+  int wide;                                  // rows of D start on 32-byte boundaries
   // grouped mode: expert of every 128-row tile (< 0: tile unused), rows of each that hold anything (null: all); N and the scale
   // rows are those of one expert
   const int* tile_expert; const int* tile_rows;
@@ -344,34 +347,44 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       }
       if (!row_ok) continue;
 #pragma unroll
-      for (int c0 = 0; c0 < EC; c0 += 8) {
-        const int col = n0 + c0;
-        if (col >= p.N) continue;
-        float o[8];
+      for (int c0 = 0; c0 < EC; c0 += 16) {
+        uint4 ov[2];
+        const int col0 = n0 + c0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[c0 + i]);
-        if (p.bias) {
-          const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-          const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
+        for (int h8 = 0; h8 < 2; ++h8) {
+          const int col = col0 + h8 * 8;
+          if (col >= p.N) continue;
+          float o[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
-        }
-        if (p.residual) {
-          const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(row) * p.ldr + col);
-          const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+          for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[c0 + h8 * 8 + i]);
+          if (p.bias) {
+            const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+            const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(r2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
-        }
-        if (p.out_f32) {
-          float4* dst = reinterpret_cast<float4*>(p.out_f32 + static_cast<size_t>(row) * p.ldd + col);
-          dst[0] = make_float4(o[0], o[1], o[2], o[3]);
-          dst[1] = make_float4(o[4], o[5], o[6], o[7]);
-        } else {
-          uint4 ov;
-          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
+            for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
+          }
+          if (p.residual) {
+            const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(row) * p.ldr + col);
+            const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(r2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
+          }
+          if (p.out_f32) {
+            float4* dst = reinterpret_cast<float4*>(p.out_f32 + static_cast<size_t>(row) * p.ldd + col);
+            dst[0] = make_float4(o[0], o[1], o[2], o[3]);
+            dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+          }
+          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov[h8]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-          *reinterpret_cast<uint4*>(p.D + static_cast<size_t>(row) * p.ldd + col) = ov;
+        }
+        if (p.out_f32 || col0 >= p.N) continue;
+        __nv_bfloat16* dst = p.D + static_cast<size_t>(row) * p.ldd + col0;
+        if (p.wide && col0 + 16 <= p.N) {
+          st_global_32(dst, ov[0], ov[1]);
+        } else {
+          *reinterpret_cast<uint4*>(dst) = ov[0];
+          if (col0 + 8 < p.N) *reinterpret_cast<uint4*>(dst + 8) = ov[1];
         }
       }
     }
@@ -469,6 +482,7 @@ extern "C" int ksana_gemm_mxfp8(const void* Aq, int lda, const float* a_scale, i
   p.a_scale = a_scale; p.a_scale_ld = a_scale_ld; p.w_scale = w_scale;
   p.err = err_flag;
   for (int i = 0; i < push_n && i < 8; ++i) p.push[i] = reinterpret_cast<__nv_bfloat16*>(push_ptrs[i]);
+  p.wide = push_n == 0 && D && ldd % 16 == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
   p.push_n = push_n; p.push_rows = push_rows;
   return bn == 256 ? launch_mx<256>(ma, mb, p, max_ctas, st) : launch_mx<128>(ma, mb, p, max_ctas, st);
 }
@@ -489,6 +503,7 @@ extern "C" int ksana_gemm_grouped_mxfp8(const void* Aq, int lda, const float* a_
   MxParams p{};
   p.M = M; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.ldd = ldd;
+  p.wide = D && ldd % 16 == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
   p.a_scale = a_scale; p.a_scale_ld = a_scale_ld; p.w_scale = w_scale;
   p.err = err_flag;
   p.tile_expert = tile_expert; p.tile_rows = tile_rows;

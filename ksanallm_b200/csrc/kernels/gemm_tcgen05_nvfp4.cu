@@ -9,14 +9,16 @@
 // Warp 0 TMA producer, warp 1 MMA issuer, warps 2..5 scales, warps 6..13 epilogue; single 256-column accumulator and bounded waits as in
 // the FP8 hardware-scaled kernel. The scales of a K block travel by TMA with its operands (16 bytes a row); four warps, one per quarter
 // of TMEM, write them there from registers. (tcgen05.cp of 512-byte chunks, twelve a block, took about 80 clocks each between the MMAs of two
-// blocks, 1500 clocks a block with 512 of MMAs; now about 1050. A tile of 256 x 192 with them was slower by its work: 1002 us.) 9753 x
-// 28672 x 4096: 1094 us with scales loaded by a packer warp on demand, 832 by TMA and tcgen05.cp, 695 now (3.3 PFLOP/s); 9753 x 4096 x
-// 14336: 612, 432, 319.
+// blocks, 1500 clocks a block with 512 of MMAs; now about 1050;
+// a tile of 256 x 192 with them was slower by its work: 1002 us.) The epilogue stores whole sectors, 32 bytes a lane (with 16 a sector
+// reaches the L2 in two halves). 9753 x 28672 x 4096: 1094 us with scales loaded by a packer warp on demand, 832 by TMA and tcgen05.cp, 695
+// from registers, 627 with the wider stores (3.65 PFLOP/s); 9753 x 4096 x 14336: 612, 432, 319, 282.
 //
 // No counterpart in the reference (its low-bit paths are GPTQ/AWQ W4A16 through Marlin/Machete,
 // 3rdparty/LLM_kernels/csrc/kernels/nvidia/mixture_of_experts and .../machete); the operator is specified by
 // the fp32 statement in ops/reference.py (gemm_nvfp4).
 #include "sm100_ptx.cuh"
+#include "vec8.cuh"
 #include <cuda_bf16.h>
 #include <stdio.h>
 
@@ -52,6 +54,7 @@ struct F4Params {
   const float* a_ts; const float* w_ts;    // per-tensor scales (device scalars)
   int* err;
   __nv_bfloat16* push[8]; int push_n; int push_rows;
+  int wide;                                  // rows of D start on 32-byte boundaries
   // grouped (mixture-of-experts) mode: row tile i multiplies with expert tile_expert[i] (< 0: tile unused); W, w_bs
   // are the experts' matrices stacked along N (expert_rows rows each) and w_ts holds one tensor scale per expert
   const int* tile_expert; int expert_rows;
@@ -244,39 +247,50 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       if (!row_ok) continue;
       const float alpha = (p.a_ts ? *p.a_ts : 1.f) * (p.w_ts ? p.w_ts[expert] : 1.f);
 #pragma unroll
-      for (int c0 = 0; c0 < EC; c0 += 8) {
-        const int col = n0 + c0;
-        if (col >= p.N) continue;
-        float o[8];
+      for (int c0 = 0; c0 < EC; c0 += 16) {
+        uint4 ov[2];
+        const int col0 = n0 + c0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[c0 + i]) * alpha;
-        if (p.bias) {
-          const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
-          const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
+        for (int h8 = 0; h8 < 2; ++h8) {
+          const int col = col0 + h8 * 8;
+          if (col >= p.N) continue;
+          float o[8];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
-        }
-        if (p.residual) {
-          const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(row) * p.ldr + col);
-          const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+          for (int i = 0; i < 8; ++i) o[i] = __uint_as_float(r[c0 + h8 * 8 + i]) * alpha;
+          if (p.bias) {
+            const uint4 bv = *reinterpret_cast<const uint4*>(p.bias + col);
+            const __nv_bfloat162* b2 = reinterpret_cast<const __nv_bfloat162*>(&bv);
 #pragma unroll
-          for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(r2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
-        }
-        if (p.out_f32) {
-          float4* dst = reinterpret_cast<float4*>(p.out_f32 + static_cast<size_t>(row) * p.ldd + col);
-          dst[0] = make_float4(o[0], o[1], o[2], o[3]);
-          dst[1] = make_float4(o[4], o[5], o[6], o[7]);
-        } else {
-          uint4 ov;
-          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
+            for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(b2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
+          }
+          if (p.residual) {
+            const uint4 rv = *reinterpret_cast<const uint4*>(p.residual + static_cast<size_t>(row) * p.ldr + col);
+            const __nv_bfloat162* r2 = reinterpret_cast<const __nv_bfloat162*>(&rv);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(r2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
+          }
+          if (p.out_f32) {
+            float4* dst = reinterpret_cast<float4*>(p.out_f32 + static_cast<size_t>(row) * p.ldd + col);
+            dst[0] = make_float4(o[0], o[1], o[2], o[3]);
+            dst[1] = make_float4(o[4], o[5], o[6], o[7]);
+          }
+          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov[h8]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-          if (p.push_n) {
-            const int owner = min(row / p.push_rows, p.push_n - 1);
-            *reinterpret_cast<uint4*>(p.push[owner] + static_cast<size_t>(row - owner * p.push_rows) * p.ldd + col) = ov;
-          } else {
-            *reinterpret_cast<uint4*>(p.D + static_cast<size_t>(row) * p.ldd + col) = ov;
-          }
+        }
+        if (p.out_f32 || col0 >= p.N) continue;
+        __nv_bfloat16* dst;
+        if (p.push_n) {
+          const int owner = min(row / p.push_rows, p.push_n - 1);
+          dst = p.push[owner] + static_cast<size_t>(row - owner * p.push_rows) * p.ldd + col0;
+        } else {
+          dst = p.D + static_cast<size_t>(row) * p.ldd + col0;
+        }
+        if (p.wide && col0 + 16 <= p.N) {
+          st_global_32(dst, ov[0], ov[1]);
+        } else {
+          *reinterpret_cast<uint4*>(dst) = ov[0];
+          if (col0 + 8 < p.N) *reinterpret_cast<uint4*>(dst + 8) = ov[1];
         }
       }
     }
@@ -371,6 +385,7 @@ extern "C" int ksana_gemm_nvfp4(const void* Aq, int lda, const void* a_bs, int a
   F4Params p{};
   p.M = M; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.out_f32 = static_cast<float*>(out_f32); p.ldd = ldd;
+  p.wide = D && ldd % 16 == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
   p.bias = static_cast<const __nv_bfloat16*>(bias);
   p.residual = static_cast<const __nv_bfloat16*>(residual); p.ldr = ldr;
   p.a_ts = a_ts; p.w_ts = w_ts;
@@ -399,6 +414,7 @@ extern "C" int ksana_gemm_grouped_nvfp4(const void* Aq, int lda, const void* a_b
   F4Params p{};
   p.M = cap; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.ldd = ldd;
+  p.wide = D && ldd % 16 == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
   p.a_ts = a_ts; p.w_ts = w_ts;
   p.err = err_flag;
   p.tile_expert = tile_expert; p.expert_rows = N;

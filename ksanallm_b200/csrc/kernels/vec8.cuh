@@ -36,6 +36,12 @@ template <> __device__ __forceinline__ bf16 from_f<bf16>(float v) { return __flo
 template <> __device__ __forceinline__ float from_f<float>(float v) { return v; }
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.f / (1.f + __expf(-x)); }
 
+// 32 bytes in one store: a whole sector of a row (two 16-byte stores of a lane reach the L2 as two halves of one)
+__device__ __forceinline__ void st_global_32(void* p, const uint4& a, const uint4& b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w) : "memory");
+}
+
 static inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 }  // namespace ksana
