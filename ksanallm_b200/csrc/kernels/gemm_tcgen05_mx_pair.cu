@@ -88,19 +88,22 @@ __device__ __forceinline__ void mp_tmem_dealloc(uint32_t taddr, uint32_t ncols) 
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
 // arrive on the barrier at `bar_cluster_addr` (either CTA of the pair) once the MMAs and copies issued so far are done
-__device__ __forceinline__ void mp_commit(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+__device__ __forceinline__ void mp_commit(uint32_t lead, uint32_t bar_cluster_addr) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %1, 0;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar_cluster_addr), "r"(lead) : "memory");
 }
 // scale chunk (128 rows x 4 bytes, 512 bytes) from each CTA's own shared memory into its own TMEM columns
-__device__ __forceinline__ void mp_tmem_cp_sf(uint32_t taddr, uint64_t sdesc) {
-  asm volatile("tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;" ::"r"(taddr), "l"(sdesc) : "memory");
+__device__ __forceinline__ void mp_tmem_cp_sf(uint32_t lead, uint32_t taddr, uint64_t sdesc) {
+  asm volatile("{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %2, 0;\n\t@e tcgen05.cp.cta_group::2.32x128b.warpx4 [%0], %1;\n\t}\n"
+               ::"r"(taddr), "l"(sdesc), "r"(lead) : "memory");
 }
-__device__ __forceinline__ void mp_mma(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+__device__ __forceinline__ void mp_mma(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
                                        uint32_t tsfa, uint32_t tsfb) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
-      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb) : "memory");
+      "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 e, %7, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@e tcgen05.mma.cta_group::2.kind::mxf8f6f4.block_scale [%0], %1, %2, %3, [%5], [%6], p;\n\t}\n"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb), "r"(lead) : "memory");
 }
 
 __device__ __forceinline__ void mp_tile_coords(int tile, int m_tiles, int n_tiles, int& m_blk, int& n_blk) {
@@ -129,8 +132,8 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(tempty_bar + 1);
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = mp_ctarank();
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t rank = __shfl_sync(0xffffffffu, mp_ctarank(), 0);
   const bool leader = rank == 0;
   const int m_tiles = (p.M + 255) / 256;
   const int n_tiles = (p.N + kMpBN - 1) / kMpBN;
@@ -152,7 +155,8 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
   __syncthreads();
   mp_cluster_sync();           // the peer's barriers are initialised before anything signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
@@ -180,29 +184,29 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     __syncwarp();
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer (leader only)
-    if (leader && lane == 0) {
+    if (leader) {
       int stage = 0; uint32_t phase = 0;
       int sfs = 0; uint32_t sf_phase = 0;
       uint32_t acc_phase = 0;
       uint32_t set = 0;
       bool ok = true;
       for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
-        if (!mbar_wait(tempty_bar, acc_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_warp(tempty_bar, acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base;
         for (int g = 0; g < num_groups && ok; ++g) {
-          if (!mbar_wait(&sf_full[sfs], sf_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&sf_full[sfs], sf_phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsfa = tmem_base + kMpSfBase + set * kMpSfCols;
           const uint32_t tsfb = tsfa + 4;
           const uint32_t sf_addr = smem_u32(sf_smem + sfs * kMpSfStageBytes);
-          mp_tmem_cp_sf(tsfa, make_sf_desc(sf_addr));
-          mp_tmem_cp_sf(tsfb, make_sf_desc(sf_addr + 512));
-          mp_tmem_cp_sf(tsfb + 4, make_sf_desc(sf_addr + 1024));
+          mp_tmem_cp_sf(lead, tsfa, make_sf_desc(sf_addr));
+          mp_tmem_cp_sf(lead, tsfb, make_sf_desc(sf_addr + 512));
+          mp_tmem_cp_sf(lead, tsfb + 4, make_sf_desc(sf_addr + 1024));
           for (int j = 0; j < 4; ++j) {
             const int kb = g * 4 + j;
             if (kb >= num_kb) break;
-            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sa = smem_u32(smem + stage * kMpStageBytes);
             const uint64_t adesc = make_smem_desc_sw128(sa);
@@ -210,20 +214,20 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
             const uint32_t idesc = make_idesc_mx(256, kMpBN, static_cast<uint32_t>(j));
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              mp_mma(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
+              mp_mma(lead, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0, tsfa, tsfb);
             // release this stage in both CTAs
-            mp_commit(mp_map_to_cta(smem_u32(&empty_bar[stage]), 0));
-            mp_commit(mp_map_to_cta(smem_u32(&empty_bar[stage]), 1));
+            mp_commit(lead, mp_map_to_cta(smem_u32(&empty_bar[stage]), 0));
+            mp_commit(lead, mp_map_to_cta(smem_u32(&empty_bar[stage]), 1));
             if (++stage == kMpStages) { stage = 0; phase ^= 1; }
           }
-          mp_commit(mp_map_to_cta(smem_u32(&sf_empty[sfs]), 0));
-          mp_commit(mp_map_to_cta(smem_u32(&sf_empty[sfs]), 1));
+          mp_commit(lead, mp_map_to_cta(smem_u32(&sf_empty[sfs]), 0));
+          mp_commit(lead, mp_map_to_cta(smem_u32(&sf_empty[sfs]), 1));
           if (++sfs == kMpSfStages) { sfs = 0; sf_phase ^= 1; }
           set ^= 1;
         }
         if (ok) {
-          mp_commit(mp_map_to_cta(smem_u32(tfull_bar), 0));
-          mp_commit(mp_map_to_cta(smem_u32(tfull_bar), 1));
+          mp_commit(lead, mp_map_to_cta(smem_u32(tfull_bar), 0));
+          mp_commit(lead, mp_map_to_cta(smem_u32(tfull_bar), 1));
           acc_phase ^= 1;
         }
       }

@@ -3,11 +3,13 @@
 //
 //   D[M,N] = A[M,K] * W[N,K]^T (+bias)(+residual), bf16 x bf16 or block-scaled FP8 (see gemm_tcgen05.cu)
 //
-// Why pairs: the single-CTA kernel fills 48 KB of shared memory per 128x256x(128 B of K) block; at
-// ~64-78 B/clk/SM from L2 that takes longer than the FP8 MMA itself (tensor pipe 35 % busy, measured).
-// In a pair each CTA stages only its own 128 rows of A and HALF of the W tile (128 of the 256 rows):
-// 32 KB per block for the same 128 x 256 output per CTA. The tensor cores of both SMs read both W
-// halves through the pair's shared-memory window.
+// Why pairs: the single-CTA kernel takes 48 KB of operands per 128 x 256 x (128 B of K) block, more than an SM's share of the L2's
+// bandwidth brings in the time of its MMAs. In a pair each CTA stages only its own 128 rows of A and HALF of the W tile (128 of the 256
+// rows): 32 KB per block for the same 128 x 256 output per CTA. The tensor cores of both SMs read both W halves through the pair's
+// shared-memory window. bf16 takes this kernel (native.gemm_bf16) unless 128-row tiles fill their waves much better: us, single CTA /
+// pair, 3103 x 28672 x 4096 597 / 548, 16384 x 28672 x 4096 2990 / 2700, 3103 x 4096 x 14336 318 / 292, 8000 x 32768 x 512 447 / 302,
+// 200 x 4096 x 4096 18.1 / 13.4. What it took: MMAs issued by a converged warp, one commit for both CTAs, stores of whole sectors
+// (8000 x 32768 x 512: 430 with 16-byte stores), tiles of the last wave cut.
 //
 // Protocol (cluster of 2 CTAs, rank 0 = leader):
 //   * each CTA's producer thread loads its A rows and its W half with TMA (cta_group::2 form, no
@@ -19,6 +21,8 @@
 //   * cluster barriers bracket the kernel so that no CTA leaves while its peer may still touch its
 //     shared memory or TMEM. Every wait is bounded.
 #include "sm100_ptx.cuh"
+#include "vec8.cuh"
+#include <atomic>
 #include <cuda_bf16.h>
 #include <stdio.h>
 
@@ -42,6 +46,8 @@ struct PairParams {
   const float* w_scale;
   int* err;
   __nv_bfloat16* push[8]; int push_n; int push_rows;
+  int wide;                                  // rows of D start on 32-byte boundaries
+  int whole, cut;                            // tiles taken whole, column ranges of each further one (1, 2 or 4; bf16)
 };
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {
@@ -61,10 +67,11 @@ __device__ __forceinline__ void remote_arrive(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load of this CTA's tile; completion is signalled on the barrier at cluster address `bar_cluster_addr`
-__device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int x, int y) {
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t lead, void* smem_dst, const CUtensorMap* m, uint32_t bar_cluster_addr, int x, int y) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y)
+      "{\n\t.reg .pred e;\n\tsetp.ne.b32 e, %5, 0;\n\t"
+      "@e cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];\n\t}\n"
+      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(lead)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_dst, uint32_t ncols) {
@@ -76,22 +83,25 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
 }
-// arrive on the barrier at `bar_cluster_addr` (any CTA of the pair) once the MMAs issued so far have completed
-__device__ __forceinline__ void tc_commit_pair(uint32_t bar_cluster_addr) {
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_cluster_addr) : "memory");
+// arrive on the barrier at this place of both CTAs once the MMAs issued so far have completed
+__device__ __forceinline__ void tc_commit_pair(uint32_t lead, uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred e;\n\t.reg .b16 both;\n\tsetp.ne.b32 e, %1, 0;\n\tmov.b16 both, 3;\n\t"
+      "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], both;\n\t}\n"
+      ::"r"(smem_u32(bar)), "r"(lead) : "memory");
 }
-__device__ __forceinline__ void mma_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
+__device__ __forceinline__ void mma_pair(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate,
                                          bool fp8) {
   if (fp8) {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
   } else {
     asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate) : "memory");
+        "{\n\t.reg .pred p, e;\n\tsetp.ne.b32 e, %5, 0;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}\n"
+        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead) : "memory");
   }
 }
 
@@ -105,9 +115,23 @@ __device__ __forceinline__ void pair_tile_coords(int tile, int m_tiles, int n_ti
   n_blk = in_group / gsz;
 }
 
+// A piece of work: a tile, or where the last wave holds few tiles one of `cut` column ranges of one (`whole` tiles come before them).
+// Measured, 74 pairs: 3103 x 6144 x 4096 (312 tiles: 16 in the last wave, cut in four) 136 -> 122 us,
+// 300 x 28672 x 4096 (224: 2) 97 -> 88, 520 x 8192 x 4096 (96: 22, cut in two) 47 -> 40, 400 x 4096 x 14336 (32 in all) 72 -> 56.
+struct PairWork { int m_blk, n0, width; };
+__device__ __forceinline__ PairWork pair_work(int i, int whole, int cut, int m_tiles, int n_tiles) {
+  int m_blk, n_blk, sub = 0;
+  const bool piece = i >= whole;
+  if (piece) { sub = (i - whole) % cut; i = whole + (i - whole) / cut; }
+  pair_tile_coords(i, m_tiles, n_tiles, m_blk, n_blk);
+  const int width = piece ? kPairBN / cut : kPairBN;
+  return {m_blk, n_blk * kPairBN + sub * width, width};
+}
+
 template <int KIND>   // 0 bf16, 1 fp8 block-scaled
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
-gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const PairParams p) {
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
+                 const __grid_constant__ CUtensorMap tma_bs, const PairParams p) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kPairStages * kPairStageBytes);
@@ -119,12 +143,13 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   volatile uint32_t* abort_flag = tmem_slot + 1;
 
   constexpr int kElems = KIND == 0 ? 64 : 128;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = cluster_ctarank();
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+  const uint32_t rank = __shfl_sync(0xffffffffu, cluster_ctarank(), 0);
   const bool leader = rank == 0;
   const int m_tiles = (p.M + 255) / 256;
   const int n_tiles = (p.N + kPairBN - 1) / kPairBN;
-  const int num_tiles = m_tiles * n_tiles;
+  const int whole = KIND == 0 ? p.whole : m_tiles * n_tiles, cut = KIND == 0 ? p.cut : 1;
+  const int num_work = whole + (m_tiles * n_tiles - whole) * cut;
   const int num_kb = (p.K + kElems - 1) / kElems;
   const int pair_id = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
 
@@ -140,27 +165,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   __syncthreads();
   cluster_sync_all();          // the peer's barriers are initialised before anything signals them
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
 
   if (warp == 0) {
     // ---------------------------------------------------------- TMA producer (both CTAs)
-    if (lane == 0) {
-      tma_prefetch_desc(&tma_a);
-      tma_prefetch_desc(&tma_b);
+    {
+      if (lane == 0) { tma_prefetch_desc(&tma_a); tma_prefetch_desc(&tma_b); }
+      __syncwarp();
       int stage = 0; uint32_t phase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
-        int m_blk, n_blk;
-        pair_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
-        const int m0 = m_blk * 256 + static_cast<int>(rank) * 128;
-        const int n0 = n_blk * kPairBN + static_cast<int>(rank) * 128;
+      for (int tile = pair_id; tile < num_work && ok; tile += num_pairs) {
+        const PairWork wk = pair_work(tile, whole, cut, m_tiles, n_tiles);
+        const int m0 = wk.m_blk * 256 + static_cast<int>(rank) * 128, rows = wk.width / 2;
+        const int n0 = wk.n0 + static_cast<int>(rank) * rows;
         for (int kb = 0; kb < num_kb; ++kb) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, lead, abort_flag)) { ok = false; break; }
           uint8_t* sa = smem + stage * kPairStageBytes;
           const uint32_t full_leader = map_to_cta(smem_u32(&full_bar[stage]), 0);
-          if (leader) mbar_expect_tx(&full_bar[stage], 2 * kPairStageBytes);
-          tma_load_2d_pair(sa, &tma_a, full_leader, kb * kElems, m0);
-          tma_load_2d_pair(sa + 128 * kPairRowBytes, &tma_b, full_leader, kb * kElems, n0);
+          if (leader) mbar_expect_tx_lead(lead, &full_bar[stage], 2 * (128 + rows) * kPairRowBytes);
+          tma_load_2d_pair(lead, sa, &tma_a, full_leader, kb * kElems, m0);
+          if (rows == 128) {
+            tma_load_2d_pair(lead, sa + 128 * kPairRowBytes, &tma_b, full_leader, kb * kElems, n0);
+          } else {
+            tma_load_2d_pair(lead, sa + 128 * kPairRowBytes, &tma_bs, full_leader, kb * kElems, n0);
+            if (rows == 64) tma_load_2d_pair(lead, sa + 160 * kPairRowBytes, &tma_bs, full_leader, kb * kElems, n0 + 32);
+          }
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
         }
       }
@@ -168,21 +198,22 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     __syncwarp();
   } else if (warp == 1) {
     // ---------------------------------------------------------- MMA issuer (leader only)
-    if (leader && lane == 0) {
-      constexpr uint32_t idesc = KIND == 0 ? make_idesc(256, kPairBN, 1, 1) : make_idesc(256, kPairBN, 0, 0);
+    if (leader) {
       int stage = 0; uint32_t phase = 0;
       int acc = 0; uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
+      for (int tile = pair_id; tile < num_work && ok; tile += num_pairs) {
+        const int width = pair_work(tile, whole, cut, m_tiles, n_tiles).width;
+        const uint32_t idesc = KIND == 0 ? make_idesc(256, width, 1, 1) : make_idesc(256, width, 0, 0);
         if (KIND == 0) {
-          if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
         }
         for (int kb = 0; kb < num_kb; ++kb) {
           if (KIND == 1) {
-            if (!mbar_wait(&tempty_bar[acc], acc_phase ^ 1, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(&tempty_bar[acc], acc_phase ^ 1, lead, abort_flag)) { ok = false; break; }
           }
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * kPairStageBytes);
           const uint64_t adesc = make_smem_desc_sw128(sa);
@@ -191,21 +222,18 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
           for (int k = 0; k < 4; ++k) {
             const uint32_t accum = KIND == 0 ? ((kb | k) != 0) : (k != 0);
-            mma_pair(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, accum, KIND == 1);
+            mma_pair(lead, d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, accum, KIND == 1);
           }
           // release this stage in both CTAs
-          tc_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 0));
-          tc_commit_pair(map_to_cta(smem_u32(&empty_bar[stage]), 1));
+          tc_commit_pair(lead, &empty_bar[stage]);
           if (++stage == kPairStages) { stage = 0; phase ^= 1; }
           if (KIND == 1) {
-            tc_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 0));
-            tc_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 1));
+            tc_commit_pair(lead, &tfull_bar[acc]);
             if (++acc == kPairAccStages) { acc = 0; acc_phase ^= 1; }
           }
         }
         if (KIND == 0 && ok) {
-          tc_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 0));
-          tc_commit_pair(map_to_cta(smem_u32(&tfull_bar[acc]), 1));
+          tc_commit_pair(lead, &tfull_bar[acc]);
           if (++acc == kPairAccStages) { acc = 0; acc_phase ^= 1; }
         }
       }
@@ -216,15 +244,14 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const int q = warp & 3;
     const uint32_t lane_base = static_cast<uint32_t>(q * 32) << 16;
     const int wg = (warp - 2) >> 2;
-    const int col_off = wg * 128;
     int acc = 0; uint32_t acc_phase = 0;
     bool ok = true;
     const int nkb_scale = (p.K + 127) / 128;
-    for (int tile = pair_id; tile < num_tiles && ok; tile += num_pairs) {
-      int m_blk, n_blk;
-      pair_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
-      const int row = m_blk * 256 + static_cast<int>(rank) * 128 + q * 32 + lane;
-      const int n0 = n_blk * kPairBN + col_off;
+    for (int tile = pair_id; tile < num_work && ok; tile += num_pairs) {
+      const PairWork wk = pair_work(tile, whole, cut, m_tiles, n_tiles);
+      const int cols = wk.width / 2, col_off = wg * cols;      // columns of this warp: 128, 64 or 32
+      const int row = wk.m_blk * 256 + static_cast<int>(rank) * 128 + q * 32 + lane;
+      const int n0 = wk.n0 + col_off;
       const bool row_ok = row < p.M;
       float accv[128];
       if (KIND == 1) {
@@ -233,6 +260,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       }
       auto store_chunk = [&](int c0, const float (&v)[32]) {
         if (!row_ok) return;
+        uint4 ov[4];
 #pragma unroll
         for (int g = 0; g < 4; ++g) {
           const int col = n0 + c0 + g * 8;
@@ -252,16 +280,25 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
 #pragma unroll
             for (int i = 0; i < 4; ++i) { const float2 f = __bfloat1622float2(r2[i]); o[2 * i] += f.x; o[2 * i + 1] += f.y; }
           }
-          uint4 ov;
-          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov);
+          __nv_bfloat162* o2 = reinterpret_cast<__nv_bfloat162*>(&ov[g]);
 #pragma unroll
           for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
-          if (p.push_n) {
-            const int owner = min(row / p.push_rows, p.push_n - 1);
-            *reinterpret_cast<uint4*>(p.push[owner] + static_cast<size_t>(row - owner * p.push_rows) * p.ldd + col) = ov;
-          } else {
-            *reinterpret_cast<uint4*>(p.D + static_cast<size_t>(row) * p.ldd + col) = ov;
-          }
+        }
+        const int col = n0 + c0;
+        __nv_bfloat16* dst;
+        if (p.push_n) {
+          const int owner = min(row / p.push_rows, p.push_n - 1);
+          dst = p.push[owner] + static_cast<size_t>(row - owner * p.push_rows) * p.ldd + col;
+        } else {
+          dst = p.D + static_cast<size_t>(row) * p.ldd + col;
+        }
+        if (p.wide && col + 32 <= p.N) {
+#pragma unroll
+          for (int g = 0; g < 4; g += 2) st_global_32(dst + g * 8, ov[g], ov[g + 1]);
+        } else {
+#pragma unroll
+          for (int g = 0; g < 4; ++g)
+            if (col + g * 8 < p.N) *reinterpret_cast<uint4*>(dst + g * 8) = ov[g];
         }
       };
       const uint32_t tempty_leader_base = map_to_cta(smem_u32(&tempty_bar[0]), 0);
@@ -270,7 +307,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         tc_fence_after();
 #pragma unroll
         for (int c0 = 0; c0 < 128; c0 += 32) {
+          if (c0 >= cols) break;
           uint32_t r[32];
+          __syncwarp();                             // (rows without a place to store skip the chunk before)
           tmem_ld32(tmem_base + lane_base + acc * kPairBN + col_off + c0, r);
           tmem_ld_wait();
           float v[32];
@@ -341,12 +380,12 @@ static PairEncodeFn pair_encode_fn() {
   }
   return fn;
 }
-static int pair_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int esz) {
+static int pair_map(CUtensorMap* map, const void* base, int rows, int cols, int ld, int esz, int box_rows = 128) {
   PairEncodeFn enc = pair_encode_fn();
   if (!enc) return -1;
   cuuint64_t dims[2] = {static_cast<cuuint64_t>(cols), static_cast<cuuint64_t>(rows)};
   cuuint64_t strides[1] = {static_cast<cuuint64_t>(ld) * esz};
-  cuuint32_t box[2] = {static_cast<cuuint32_t>(kPairRowBytes / esz), 128};
+  cuuint32_t box[2] = {static_cast<cuuint32_t>(kPairRowBytes / esz), static_cast<cuuint32_t>(box_rows)};
   cuuint32_t estr[2] = {1, 1};
   return enc(map, esz == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_UINT8, 2,
              const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -355,17 +394,17 @@ static int pair_map(CUtensorMap* map, const void* base, int rows, int cols, int 
 }
 
 template <int KIND>
-static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const PairParams& p, cudaStream_t st) {
-  static bool set = false;
-  if (!set) {
-    if (cudaFuncSetAttribute(gemm_pair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) !=
-        cudaSuccess) return -3;
-    set = true;
-  }
+static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mbs, PairParams p, cudaStream_t st) {
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return -3;
   // Pairs that can be resident at once: GPCs with an odd number of usable SMs leave some SMs without a partner,
   // and a pair that starts only after another one finished would double the kernel's time.
-  static int max_pairs = 0;
+  static std::atomic<int> known[64];
+  int max_pairs = known[dev].load(std::memory_order_acquire);
   if (!max_pairs) {
+    if (cudaFuncSetAttribute(gemm_pair_kernel<KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, kPairSmemBytes) !=
+        cudaSuccess) return -3;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * 74);
     cfg.blockDim = dim3(kPairThreads);
@@ -374,17 +413,19 @@ static int launch_pair(const CUtensorMap& ma, const CUtensorMap& mb, const PairP
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2; attr.val.clusterDim.y = 1; attr.val.clusterDim.z = 1;
     cfg.attrs = &attr; cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel<KIND>, &cfg) != cudaSuccess || n <= 0) {
-      cudaGetLastError();
-      n = 64;
+    if (cudaOccupancyMaxActiveClusters(&max_pairs, gemm_pair_kernel<KIND>, &cfg) != cudaSuccess || max_pairs <= 0) {
+      (void)cudaGetLastError();
+      max_pairs = 64;
     }
-    max_pairs = n;
+    known[dev].store(max_pairs, std::memory_order_release);
   }
   const int tiles = ((p.M + 255) / 256) * ((p.N + kPairBN - 1) / kPairBN);
-  int pairs = max_pairs;
-  if (pairs > tiles) pairs = tiles;
-  gemm_pair_kernel<KIND><<<pairs * 2, kPairThreads, kPairSmemBytes, st>>>(ma, mb, p);
+  // a last wave of few tiles: each in two or four column ranges, as long as all of them run at once
+  const int last = tiles % max_pairs;
+  p.cut = KIND == 0 && last > 0 ? (last * 4 <= max_pairs ? 4 : last * 2 <= max_pairs ? 2 : 1) : 1;
+  p.whole = p.cut > 1 ? tiles - last : tiles;
+  const int work = p.whole + (tiles - p.whole) * p.cut, pairs = work < max_pairs ? work : max_pairs;
+  gemm_pair_kernel<KIND><<<pairs * 2, kPairThreads, kPairSmemBytes, st>>>(ma, mb, mbs, p);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -403,9 +444,9 @@ extern "C" int ksana_gemm_pair(int kind, const void* A, int lda, const float* a_
   if ((N % 8) || (K % (kind == 0 ? 8 : 128)) || (lda % (16 / esz)) || (ldw % (16 / esz)) || (ldd % 8) ||
       (residual && (ldr % 8))) return -10;
   if ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(W)) & 15) return -11;
-  CUtensorMap ma, mb;
+  CUtensorMap ma, mb, mbs;
   if (pair_map(&ma, A, M, K, lda, esz)) return -12;
-  if (pair_map(&mb, W, N, K, ldw, esz)) return -13;
+  if (pair_map(&mb, W, N, K, ldw, esz) || pair_map(&mbs, W, N, K, ldw, esz, 32)) return -13;
   PairParams p{};
   p.M = M; p.N = N; p.K = K;
   p.D = static_cast<__nv_bfloat16*>(D); p.ldd = ldd;
@@ -414,6 +455,7 @@ extern "C" int ksana_gemm_pair(int kind, const void* A, int lda, const float* a_
   p.a_scale = a_scale; p.a_scale_ld = a_scale_ld; p.w_scale = w_scale;
   p.err = err_flag;
   for (int i = 0; i < push_n && i < 8; ++i) p.push[i] = reinterpret_cast<__nv_bfloat16*>(push_ptrs[i]);
+  p.wide = push_n == 0 && ldd % 16 == 0 && (reinterpret_cast<uintptr_t>(D) & 31) == 0;
   p.push_n = push_n; p.push_rows = push_rows;
-  return kind == 0 ? launch_pair<0>(ma, mb, p, st) : launch_pair<1>(ma, mb, p, st);
+  return kind == 0 ? launch_pair<0>(ma, mb, mbs, p, st) : launch_pair<1>(ma, mb, mbs, p, st);
 }

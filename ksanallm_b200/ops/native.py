@@ -302,9 +302,6 @@ def _gemm_decode(kind, x, xs, w, ws, out, out_f32, bias, residual, M, N, K, fixe
     return dst
 
 
-PAIR_MIN_M = 0                     # CTA-pair (cta_group::2) kernel from this many rows; 0 disables it
-
-
 def gemm_pair(kind, x, xs, w, ws, out, bias=None, residual=None, push=None, push_n=0, push_rows=0):
     """CTA-pair tcgen05 GEMM (256 x 256 tiles over two SMs). kind 0: bf16, 1: block-scaled FP8. bf16 output only."""
     M, K = x.shape
@@ -333,9 +330,22 @@ def gemm_bf16_tall(x, w, out=None, bias=None, residual=None, out_f32=None, max_c
     return dst
 
 
-def _pair_ok(M, N, K, kind, bn, out_f32, max_ctas):
-    return (PAIR_MIN_M > 0 and M >= PAIR_MIN_M and bn == 0 and max_ctas == 0 and out_f32 is None and N % 8 == 0
-            and N >= 256 and K % (128 if kind else 8) == 0)
+def _pair_wins(M, N, K, sms=148):
+    """256 x 256 tiles of CTA pairs against 128 x 256 tiles of one CTA, from measured times (in waves of pairs; graphs of a kernel, K =
+    4096): a wave of pairs takes 25 us, a last one of up to a quarter / half of them 10 / 14 (its tiles are cut); a wave of single CTAs 29, a
+    last one of up to half of them 21 (few CTAs find more of the L2's bandwidth each). us, single / pair: 700 x 28672 143 / 127, 200 x 4096
+    18.1 / 13.4, 513 x 4096 28.7 / 25.4; and where single CTAs stay: 300 x 6144 21.0 / 25.2, 1100 x 4096 29.5 / 34.5, 513 x 28672 117 / 121."""
+    if N < 256 or N % 8 or K % 8:
+        return False
+    cols = -(-N // 256)
+    tiles, single = -(-M // 256) * cols, -(-M // 128) * cols
+    if tiles <= 8 and K < 1024:                          # a few microseconds either way: 256 x 896 x 896 6.5 / 6.7
+        return False
+    pairs = sms // 2
+    last = tiles % pairs
+    pair = tiles // pairs + (0.0 if last == 0 else 0.4 if last * 4 <= pairs else 0.57 if last * 2 <= pairs else 1.0)
+    rest = single % sms
+    return pair < 1.18 * (single // sms) + (0.0 if rest == 0 else 0.85 if rest * 2 <= sms else 1.18)
 
 
 def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_ctas=0, splits=0, fixed_w=False):
@@ -354,7 +364,7 @@ def gemm_bf16(x, w, out=None, bias=None, residual=None, out_f32=None, bn=0, max_
     if (BF16_TALL_MIN_M > 0 and M >= BF16_TALL_MIN_M and bn == 0 and splits == 0 and N % 8 == 0 and K % 8 == 0
             and ((M + 255) // 256) * ((N + 255) // 256) >= 148):
         return gemm_bf16_tall(x, w, out, bias, residual, out_f32, max_ctas)
-    if _pair_ok(M, N, K, 0, bn, out_f32, max_ctas):
+    if bn == 0 and max_ctas == 0 and splits == 0 and out_f32 is None and _pair_wins(M, N, K, _sms(x.device)):
         return gemm_pair(0, x, None, w, None, out, bias, residual)
     rc = lib().ksana_gemm_bf16(_p(x), x.stride(0), _p(w), w.stride(0), _p(out) if out_f32 is None else None,
                                _p(out_f32), dst.stride(0), _p(bias), _p(residual),

@@ -63,3 +63,25 @@ def test_tall_bf16(M, N, K):
     native.gemm_bf16_tall(x, w, None, out_f32=of)
     torch.cuda.synchronize()
     assert rel_err(of, ref.gemm(x, w, out_dtype=torch.float32)) < 2e-3
+
+
+@pytest.mark.parametrize("M,N,K,ld", [(300, 600, 200, 0),            # all tiles in four column ranges, the last ones past N
+                                      (130, 256 * 30 + 8, 72, 0),    # two ranges a tile, rows that start off a 32-byte boundary
+                                      (2500, 256 * 8 + 72, 64, 0),   # a whole wave before, one K block
+                                      (700, 1024, 520, 24)])         # rows with a gap
+def test_pair_bf16_cut_tiles(M, N, K, ld):
+    """The last wave's tiles are cut along N: every piece against fp32 (products of bf16 are exact there; the result is rounded once, by
+    2^-9 of itself, and the sums of K terms in another order differ by K 2^-24 of their absolute sum at most)."""
+    torch.manual_seed(M + N)
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    w = torch.randn(N, K, device=DEV, dtype=torch.bfloat16)
+    bias = torch.randn(N, device=DEV, dtype=torch.bfloat16)
+    buf = torch.full((M, N + ld), 7.0, device=DEV, dtype=torch.bfloat16)
+    res = torch.randn(M, N, device=DEV, dtype=torch.bfloat16)
+    out = buf[:, :N]
+    native.gemm_pair(0, x, None, w, None, out, bias, res)
+    native.check_err_flag(DEV)
+    want = x.double() @ w.double().t() + bias.double() + res.double()
+    size = x.double().abs() @ w.double().abs().t() + bias.double().abs() + res.double().abs()
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + (K + 2) * 2.0 ** -23 * size).all())
+    assert bool((buf[:, N:] == 7.0).all())
