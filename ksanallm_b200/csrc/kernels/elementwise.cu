@@ -21,6 +21,8 @@
 #include <stdint.h>
 #include "fp8_scale.cuh"
 #include "fast_div.cuh"
+#include "f32x2.cuh"
+#include "vec8.cuh"
 
 namespace ksana {
 
@@ -95,8 +97,8 @@ __device__ __forceinline__ float group16_absmax(const uint4& v) {
 // mode 0 = RMSNorm, 1 = LayerNorm. One CTA per row; up to kMaxVec vectors per thread.
 constexpr int kMaxVec = 4;
 
-// QUANT: with the fp8 copy. (What a launch does not need is left out of its instance: the plain form of 16384 x 8192 with fp8 copy was
-// paced by its instructions, 166 us; without them and with maxima on packed pairs 159 us, 5.9 TB/s.)
+// QUANT: with the fp8 copy. What a launch does not need is left out of its instance. Layer norms, norms that update a residual and rows that
+// norm_rows_kernel does not take.
 template <int MODE, bool RES, bool QUANT>
 __global__ void norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ residual, const bf16* __restrict__ w,
                             const bf16* __restrict__ beta, bf16* __restrict__ y, uint8_t* __restrict__ yq,
@@ -179,6 +181,118 @@ __global__ void norm_kernel(const bf16* __restrict__ x, bf16* __restrict__ resid
 }
 
 // ----------------------------------------------------------------------------
+// Chunks of 16 elements (32 bytes of bf16) per thread, for launches of many rows: eight lanes share a 128-element group instead of sixteen, so
+// that the group's maximum takes three exchanges per 16 elements instead of eight, and arithmetic runs on packed pairs of floats. After GEMMs
+// that bring the card to its power limit the SM clock is a third lower while memory is not: these kernels are paced by their instructions then.
+struct Chunk16 { uint32_t w[8]; };
+__device__ __forceinline__ Chunk16 ld_chunk(const bf16* p) {
+  Chunk16 c;
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(c.w[0]), "=r"(c.w[1]), "=r"(c.w[2]), "=r"(c.w[3]), "=r"(c.w[4]), "=r"(c.w[5]), "=r"(c.w[6]), "=r"(c.w[7]) : "l"(p) : "memory");
+  return c;
+}
+__device__ __forceinline__ F2 unpack2(uint32_t w) { return f2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+__device__ __forceinline__ uint32_t pack2(F2 p) {
+  float x, y;
+  split(p, x, y);
+  const __nv_bfloat162 b = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&b);
+}
+// largest magnitude of a chunk and those of the lanes that share its 128-element group (eight in a row)
+__device__ __forceinline__ float group8_absmax(const Chunk16& c) {
+  auto b2 = [](uint32_t w) { return *reinterpret_cast<const __nv_bfloat162*>(&w); };
+  __nv_bfloat162 m = __habs2(b2(c.w[0]));
+#pragma unroll
+  for (int k = 1; k < 8; ++k) m = __hmax2(m, __habs2(b2(c.w[k])));
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) {
+    const uint32_t x = __shfl_xor_sync(0xffffffffu, *reinterpret_cast<const uint32_t*>(&m), o);
+    m = __hmax2(m, b2(x));
+  }
+  const float2 f = __bfloat1622float2(m);
+  return fmaxf(f.x, f.y);
+}
+// a chunk times `inv` as 16 e4m3 values
+__device__ __forceinline__ uint4 chunk_e4m3(const Chunk16& c, float inv) {
+  uint32_t o[4];
+  const F2 inv2 = f2(inv);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    float x0, x1, y0, y1;
+    split(unpack2(c.w[2 * k]) * inv2, x0, x1);
+    split(unpack2(c.w[2 * k + 1]) * inv2, y0, y1);
+    const __nv_fp8x2_storage_t lo = __nv_cvt_float2_to_fp8x2(make_float2(x0, x1), __NV_SATFINITE, __NV_E4M3);
+    const __nv_fp8x2_storage_t hi = __nv_cvt_float2_to_fp8x2(make_float2(y0, y1), __NV_SATFINITE, __NV_E4M3);
+    o[k] = static_cast<uint32_t>(lo) | (static_cast<uint32_t>(hi) << 16);
+  }
+  return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// Root-mean-square norm: CTAs stay and take row after row, the next row's loads in flight under the work on this one. One CTA per row
+// (norm_kernel) spent its time waiting and on 21.6 instructions an element. us, there / here: with fp8 copy 16384 x 8192 122 / 74 (5.5 TB/s),
+// 8000 x 7168 60 / 39, 300 x 7168 5.7 / 4.2; 16384 x 4096 56 / 43, 64 x 4096 3.9 / 2.6. V chunks per thread.
+template <bool QUANT, int V>
+__global__ void __launch_bounds__(256, V == 1 ? 4 : V == 2 ? 3 : 2)
+norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, uint8_t* __restrict__ yq,
+                 float* __restrict__ yscale, int scale_ld, int M, int H, float eps) {
+  pdl_trigger();
+  pdl_wait();
+  __shared__ float red[2][8];
+  const int chunks = H >> 4, warps = blockDim.x >> 5;
+  Chunk16 next[V];
+  auto fetch = [&](int row) {
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      if (c < chunks) next[k] = ld_chunk(x + static_cast<size_t>(row) * H + c * 16);
+    }
+  };
+  int row = blockIdx.x, turn = 0;
+  if (row < M) fetch(row);
+  for (; row < M; row += gridDim.x, turn ^= 1) {
+    Chunk16 v[V];
+#pragma unroll
+    for (int k = 0; k < V; ++k) v[k] = next[k];
+    if (row + static_cast<int>(gridDim.x) < M) fetch(row + gridDim.x);
+    F2 s2[2] = {f2(0.f), f2(0.f)};
+#pragma unroll
+    for (int k = 0; k < V; ++k)
+      if (static_cast<int>(threadIdx.x + k * blockDim.x) < chunks) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) { const F2 t = unpack2(v[k].w[e]); s2[e & 1] = fma2(t, t, s2[e & 1]); }
+      }
+    const float s = warp_sum(sum2(s2[0] + s2[1]));
+    if ((threadIdx.x & 31) == 0) red[turn][threadIdx.x >> 5] = s;
+    __syncthreads();                               // (the other set of sums is written only after the next row's)
+    float all = 0.f;
+    for (int i = 0; i < warps; ++i) all += red[turn][i];
+    const F2 rstd = f2(rsqrtf(all / H + eps));
+#pragma unroll
+    for (int k = 0; k < V; ++k) {
+      const int c = threadIdx.x + k * blockDim.x;
+      const bool on = c < chunks;                  // (whole groups of eight lanes where QUANT: H is a multiple of 128)
+      Chunk16 o = {};
+      if (on) {
+        const Chunk16 wc = ld_chunk(w + c * 16);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o.w[e] = pack2(unpack2(v[k].w[e]) * rstd * unpack2(wc.w[e]));
+      }
+      if constexpr (QUANT) {
+        const float scale = fp8_group_scale(group8_absmax(o));
+        if (on) {
+          *reinterpret_cast<uint4*>(yq + static_cast<size_t>(row) * H + c * 16) = chunk_e4m3(o, pow2_inverse(scale));
+          if ((c & 7) == 0) yscale[static_cast<size_t>(c >> 3) * scale_ld + row] = scale;
+        }
+      }
+      if (on && (!QUANT || y)) {
+        st_global_32(y + static_cast<size_t>(row) * H + c * 16, make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]),
+                     make_uint4(o.w[4], o.w[5], o.w[6], o.w[7]));
+      }
+    }
+  }
+}
+
+// ----------------------------------------------------------------------------
 // out[m, i] = act(gate_up[m, i]) * gate_up[m, I + i] ; optional fp8 copy. act: 0 silu 1 gelu(tanh) 2 relu
 // When `gated` is 0 the input is [M, I] and out = act(in). tile_rows (may be null): of every 128 rows only so many hold
 // anything, the others are skipped.
@@ -253,6 +367,52 @@ act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __r
   }
 }
 
+// Gated rows in chunks of 16 elements (see there); arguments as act_mul_kernel, nchunk counts a row's chunks. At full clocks 16384 x 28672
+// quantised 405 -> 379 us (6.2 TB/s), without fp8 16384 x 14336 226 -> 224; quantisation alone of 16384 x 8192 74 -> 67.
+template <int ACT, bool QUANT>
+__global__ void __launch_bounds__(256)
+act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __restrict__ outq, float* __restrict__ oscale, int scale_ld,
+                  uint32_t total, FastDiv nchunk, int in_ld, const int* __restrict__ tile_rows) {
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t step = gridDim.x * blockDim.x, I = nchunk.d * 16;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; (idx & ~31u) < total; idx += step) {
+    bool on = idx < total;                         // whole warps stay in the loop for the exchanges
+    const uint32_t m = on ? nchunk.div(idx) : 0u, i = on ? idx - m * nchunk.d : 0u;
+    if (tile_rows) on = on && static_cast<int>(m & 127) < tile_rows[m >> 7];
+    Chunk16 o = {};
+    if (on) {
+      const bf16* row = in + static_cast<size_t>(m) * in_ld + i * 16;
+      const Chunk16 g = ld_chunk(row), u = ld_chunk(row + I);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        F2 a;
+        if constexpr (ACT == 0) {                  // act_fn on pairs
+          const F2 hx = unpack2(g.w[e]) * f2(0.5f);
+          float x, y;
+          split(hx, x, y);
+          a = fma2(hx, f2(tanh_fast(x), tanh_fast(y)), hx);
+        } else {
+          float x, y;
+          split(unpack2(g.w[e]), x, y);
+          a = f2(act_fn(x, ACT), act_fn(y, ACT));
+        }
+        o.w[e] = pack2(a * unpack2(u.w[e]));
+      }
+    }
+    if constexpr (QUANT) {
+      const float scale = fp8_group_scale(group8_absmax(o));
+      if (on) {
+        *reinterpret_cast<uint4*>(outq + static_cast<size_t>(m) * I + i * 16) = chunk_e4m3(o, pow2_inverse(scale));
+        if ((i & 7) == 0) oscale[static_cast<size_t>(i >> 3) * scale_ld + m] = scale;
+      }
+    }
+    if (on && (!QUANT || out)) {
+      st_global_32(out + static_cast<size_t>(m) * I + i * 16, make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]), make_uint4(o.w[4], o.w[5], o.w[6], o.w[7]));
+    }
+  }
+}
+
 // The same on fp32 rows, with the exponential instead of the approximate tanh.
 __global__ void act_mul_f32_kernel(const float* __restrict__ in, float* __restrict__ out, int M, int I, int in_ld, int act, int gated) {
   pdl_trigger();
@@ -296,6 +456,25 @@ quant_fp8_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __r
         reinterpret_cast<uint2*>(q + static_cast<size_t>(m[k]) * nvec.d * 8)[i[k]] = pack8_e4m3(f, pow2_inverse(sc));
         if ((i[k] & 15) == 0) scale[static_cast<size_t>(i[k] >> 4) * scale_ld + m[k]] = sc;
       }
+    }
+  }
+}
+
+__global__ void __launch_bounds__(256)
+quant_chunks_kernel(const bf16* __restrict__ x, uint8_t* __restrict__ q, float* __restrict__ scale, int scale_ld, uint32_t total,
+                    FastDiv nchunk, int x_ld) {
+  pdl_trigger();
+  pdl_wait();
+  const uint32_t step = gridDim.x * blockDim.x;
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; (idx & ~31u) < total; idx += step) {
+    const bool on = idx < total;
+    const uint32_t m = on ? nchunk.div(idx) : 0u, i = on ? idx - m * nchunk.d : 0u;
+    Chunk16 v = {};
+    if (on) v = ld_chunk(x + static_cast<size_t>(m) * x_ld + i * 16);
+    const float sc = fp8_group_scale(group8_absmax(v));
+    if (on) {
+      *reinterpret_cast<uint4*>(q + static_cast<size_t>(m) * nchunk.d * 16 + i * 16) = chunk_e4m3(v, pow2_inverse(sc));
+      if ((i & 7) == 0) scale[static_cast<size_t>(i >> 3) * scale_ld + m] = sc;
     }
   }
 }
@@ -648,6 +827,13 @@ static inline int launch_vectors(long long total, bool gated) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return gated || total <= sms * 2048LL ? 1 : 2;
 }
+// launches of more 16-byte vectors than threads fit the machine at once
+static inline bool chunks_pay(long long total) {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return total > sms * 2048LL;
+}
 static inline int norm_threads(int H) {
   int t = ((H >> 3) + kMaxVec - 1) / kMaxVec;
   t = ((t + 31) / 32) * 32;
@@ -696,6 +882,22 @@ extern "C" int ksana_norm(const void* x, void* residual, const void* w, const vo
   if (M <= 0) return 0;
   if (H % 8 || H > 8 * kMaxVec * 1024) return -10;
   if (yq && (H % 128)) return -11;
+  // plain root-mean-square norm of aligned rows: the kernel whose CTAs stay (one row has half the barriers and wider loads: 1 x 4096 3.6 -> 2.4 us)
+  if (!layernorm && !residual && !beta && H % 16 == 0 && H <= 16384 &&
+      !((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(yq)) & 31)) {
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int chunks = H / 16, v = chunks <= 256 ? 1 : chunks <= 512 ? 2 : 4;
+    const int threads = ((chunks + v - 1) / v + 31) / 32 * 32, per_sm = (v == 1 ? 4 : v == 2 ? 3 : 2) * (256 / threads > 1 ? 256 / threads : 1);
+    const dim3 grid(M < sms * per_sm ? M : sms * per_sm);
+#define KSANA_NORM_ROWS(Q, V) launch_early(norm_rows_kernel<Q, V>, grid, dim3(threads), 0, st, (const bf16*)x, (const bf16*)w, (bf16*)y, \
+                                           (uint8_t*)yq, yscale, scale_ld, M, H, eps)
+    if (yq) v == 1 ? KSANA_NORM_ROWS(true, 1) : v == 2 ? KSANA_NORM_ROWS(true, 2) : KSANA_NORM_ROWS(true, 4);
+    else v == 1 ? KSANA_NORM_ROWS(false, 1) : v == 2 ? KSANA_NORM_ROWS(false, 2) : KSANA_NORM_ROWS(false, 4);
+#undef KSANA_NORM_ROWS
+    return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  }
   const int threads = norm_threads(H);
 #define KSANA_NORM(MODE, RES, Q) launch_early(norm_kernel<MODE, RES, Q>, dim3(M), dim3(threads), 0, st, (const bf16*)x, (bf16*)residual, \
                                               (const bf16*)w, (const bf16*)beta, (bf16*)y, (uint8_t*)yq, yscale, scale_ld, H, eps)
@@ -726,6 +928,17 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
     uint8_t* dq = outq ? (uint8_t*)outq + static_cast<size_t>(m0) * I : nullptr;
     float* ds = oscale ? oscale + m0 : nullptr;
     const int* tr = tile_rows ? tile_rows + m0 / 128 : nullptr;
+    if (chunks_pay(total) && gated && I % 16 == 0 && in_ld % 16 == 0 &&
+        !((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(dq)) & 31)) {
+      const FastDiv by = make_fast_div(I / 16);
+      const dim3 chunk_grid(grid_for(total / 2, 256));
+#define KSANA_ACT16(A, Q) launch_early(act_chunks_kernel<A, Q>, chunk_grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total / 2, by, in_ld, tr)
+      if (act == 0) dq ? KSANA_ACT16(0, true) : KSANA_ACT16(0, false);
+      else if (act == 1) dq ? KSANA_ACT16(1, true) : KSANA_ACT16(1, false);
+      else dq ? KSANA_ACT16(2, true) : KSANA_ACT16(2, false);
+#undef KSANA_ACT16
+      continue;
+    }
     const int v = launch_vectors(total, gated);
     const dim3 grid(grid_for((static_cast<long long>(total) + v - 1) / v, 256));
 #define KSANA_ACT(A, G, Q, V) launch_early(act_mul_kernel<A, G, Q, V>, grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total, div, in_ld, tr)
@@ -759,6 +972,13 @@ extern "C" int ksana_quant_fp8(const void* x, void* q, float* scale, int scale_l
   for (int m0 = 0; m0 < M; m0 += most) {
     const int rows = M - m0 < most ? M - m0 : most;
     const uint32_t total = static_cast<uint32_t>(rows) * nvec;
+    const bf16* src = (const bf16*)x + static_cast<size_t>(m0) * x_ld;
+    uint8_t* dst = (uint8_t*)q + static_cast<size_t>(m0) * K;
+    if (chunks_pay(total) && x_ld % 16 == 0 && !((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 31)) {
+      launch_early(quant_chunks_kernel, dim3(grid_for(total / 2, 256)), dim3(256), 0, st, src, dst, scale + m0, scale_ld, total / 2,
+                   make_fast_div(K / 16), x_ld);
+      continue;
+    }
     const int v = launch_vectors(total, false);
     launch_early(v == 1 ? quant_fp8_kernel<1> : quant_fp8_kernel<2>, dim3(grid_for((static_cast<long long>(total) + v - 1) / v, 256)), dim3(256), 0,
                  st, (const bf16*)x + static_cast<size_t>(m0) * x_ld, (uint8_t*)q + static_cast<size_t>(m0) * K, scale + m0, scale_ld, total, div,
