@@ -15,6 +15,9 @@
 // Against gemm_smallm.cu (us, in graphs): bf16, 1 row, 6144 x 4096 21 -> 12, 4096 x 4096 18 -> 9, 28672 x 4096 50 -> 37, 4096 x 14336
 // 30 -> 20; e4m3, 64 rows, 8192 x 8192 29 -> 18, 8192 x 28672 61 -> 52. Wide e4m3 layers at more than 32 rows stay with the tiled
 // kernel (57344 x 8192, 64 rows: 86 against 102 us here, where every weight tile is followed by its 8 KB of activations).
+// The producer and the MMA warp run their loops as a whole and issue by predicate (a lane behind a branch takes 100 clocks for a copy or an
+// MMA, which shows where a share is few K blocks long: bf16, 1 row, 4096 x 4096 9.2 -> 8.45, 6144 x 4096 12.4 -> 11.7; e4m3, 64 rows, 10240 x
+// 8192 28.0 -> 26.6).
 // Kinds: 0 bf16; 2 e4m3 with power-of-two scales (1 x 128 activations, 128 x 128 weights) applied by the tensor cores. No multicast.
 // Every wait is bounded.
 #include "sm100_ptx.cuh"
@@ -86,7 +89,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   uint8_t* xs_tab = reinterpret_cast<uint8_t*>(full_bar) + 256;              // kind 2: exponents of the tokens, [K block][MP]
 
   pdl_trigger();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int S = p.splits, rank = static_cast<int>(blockIdx.x) % S, tile = static_cast<int>(blockIdx.x) / S;
   const int num_kb = (p.K + Cfg::kElems - 1) / Cfg::kElems;
   const int kb0 = rank * num_kb / S, kb1 = (rank + 1) * num_kb / S;
@@ -109,70 +112,72 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const uint32_t lead = elect_one();             // one lane of every warp: it polls and issues for the warp
   pdl_wait();
 
   float accv[MP];
   bool ok = true;
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tma_x);
+    {
+      if (lane == 0) tma_prefetch_desc(&tma_x);
+      __syncwarp();
       int stage = 0; uint32_t phase = 0;
       for (int kb = kb0; kb < kb1; ++kb) {
         uint8_t* sw = smem + stage * Cfg::kStageBytes;
         if (kb - kb0 >= Cfg::kStages) {
-          if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) break;
-          mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
-          tma_load_2d(sw, &tma_w, &full_bar[stage], kb * Cfg::kElems, tile * 128);
+          if (!mbar_wait_warp(&empty_bar[stage], phase ^ 1, lead, abort_flag)) break;
+          mbar_expect_tx_lead(lead, &full_bar[stage], Cfg::kStageBytes);
+          tma_load_2d_lead(lead, sw, &tma_w, &full_bar[stage], kb * Cfg::kElems, tile * 128);
         }
-        tma_load_2d(sw + Cfg::kWBytes, &tma_x, &full_bar[stage], kb * Cfg::kElems, 0);
+        tma_load_2d_lead(lead, sw + Cfg::kWBytes, &tma_x, &full_bar[stage], kb * Cfg::kElems, 0);
         if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
       }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       int stage = 0; uint32_t phase = 0;
       if constexpr (KIND == 0) {
         constexpr uint32_t idesc = make_idesc(128, MP, 1, 1);
         for (int kb = kb0; kb < kb1; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes);
           const uint64_t wdesc = make_smem_desc_sw128(sw), xdesc = make_smem_desc_sw128(sw + Cfg::kWBytes);
 #pragma unroll
-          for (int k = 0; k < 4; ++k) mma_f16(tmem_base, wdesc + 2 * k, xdesc + 2 * k, idesc, (kb != kb0) || k != 0);
-          tc_commit(&empty_bar[stage]);
+          for (int k = 0; k < 4; ++k) mma_f16_lead(lead, tmem_base, wdesc + 2 * k, xdesc + 2 * k, idesc, (kb != kb0) || k != 0);
+          tc_commit_lead(lead, &empty_bar[stage]);
           if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
         }
       } else {
         // groups of up to four K blocks share one pair of scale chunks (byte j of a chunk = block g0 + j)
         int sfs = 0; uint32_t sf_phase = 0, set = 0;
         for (int g0 = kb0; g0 < kb1 && ok; g0 += 4) {
-          if (!mbar_wait(&sf_full[sfs], sf_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_warp(&sf_full[sfs], sf_phase, lead, abort_flag)) { ok = false; break; }
           tc_fence_after();
           const uint32_t tsfa = tmem_base + Cfg::kSfBase + set * 8, tsfb = tsfa + 4;
           const uint32_t sf_addr = smem_u32(sf_smem + sfs * 1024);
-          tmem_cp_sf(tsfa, make_sf_desc(sf_addr));
-          tmem_cp_sf(tsfb, make_sf_desc(sf_addr + 512));
+          tmem_cp_sf_lead(lead, tsfa, make_sf_desc(sf_addr));
+          tmem_cp_sf_lead(lead, tsfb, make_sf_desc(sf_addr + 512));
           for (int j = 0; j < 4 && g0 + j < kb1; ++j) {
-            if (!mbar_wait(&full_bar[stage], phase, abort_flag)) { ok = false; break; }
+            if (!mbar_wait_warp(&full_bar[stage], phase, lead, abort_flag)) { ok = false; break; }
             tc_fence_after();
             const uint32_t sw = smem_u32(smem + stage * Cfg::kStageBytes);
             const uint64_t wdesc = make_smem_desc_sw128(sw), xdesc = make_smem_desc_sw128(sw + Cfg::kWBytes);
             const uint32_t idesc = make_idesc_mx(128, MP, static_cast<uint32_t>(j));
 #pragma unroll
             for (int k = 0; k < 4; ++k)
-              mma_mxf8(tmem_base, wdesc + 2 * k, xdesc + 2 * k, idesc, (g0 + j != kb0) || k != 0, tsfa, tsfb);
-            tc_commit(&empty_bar[stage]);
+              mma_mxf8_lead(lead, tmem_base, wdesc + 2 * k, xdesc + 2 * k, idesc, (g0 + j != kb0) || k != 0, tsfa, tsfb);
+            tc_commit_lead(lead, &empty_bar[stage]);
             if (++stage == Cfg::kStages) { stage = 0; phase ^= 1; }
           }
-          tc_commit(&sf_empty[sfs]);
+          tc_commit_lead(lead, &sf_empty[sfs]);
           if (++sfs == kGdSfStages) { sfs = 0; sf_phase ^= 1; }
           set ^= 1;
         }
       }
-      if (ok) tc_commit(done_bar);
+      if (ok) tc_commit_lead(lead, done_bar);
     }
     __syncwarp();
   } else if (warp < 6) {
