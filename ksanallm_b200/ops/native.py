@@ -987,11 +987,11 @@ def _sigmoid_args(weights: Optional[SigmoidWeights]):
 
 def prefill_pair_wins(pairs, rows, B, Hq, Hkv, sms=148) -> bool:
     """Whether prompts take the attention kernel with two query tiles per CTA, from the (query, visible key) pairs and the rows of a
-    batch. A tile of 128 keys costs it less, a CTA more (about 4 us: 608 threads, two tiles' queries, all of TMEM), and only half as many
-    fit the machine. us with two / one, 32/8 heads of 128: one prompt of 200 tokens 17.1 / 12.7, 512 22.9 / 19.3, 1024 35.4 / 37.5, 5000
-    346 / 416; 64 x 33 41.1 / 35.8; 16 x 33 on 1000 cached tokens 32.9 / 40.6; 64 on 4000 103 / 111. While all CTAs of one tile run at
-    once (two an SM), two pay from about a thousand keys per row, and not at all for groups that leave rows of a tile idle (28/4 heads,
-    64 on 4000: 118.5 / 112.7; 14/2 heads of 64, 300 on 8000: 204 / 183); beyond, from 450 keys (510 with such groups)."""
+    batch. A tile of 128 keys costs it half, a CTA more (about 4 us: two tiles' queries, all of TMEM), and only half as many fit the machine.
+    us with one / two, 32/8 heads of 128: one prompt of 200 tokens 12.8 / 13.4, 1024 38 / 24.5, 2000 108 / 62; 64 x 33 31.3 / 31.8, 13 x 300
+    65 / 51, 4 x 700 56 / 38, 40 x 60 on 300 cached tokens 64 / 50, 24 x 150 on 200 82 / 61, 32 x 150 on 2000 394 / 222; 28/4 heads, 24 x 150
+    on 200 64 / 52. Two pay from 160 keys per row on (a fifth less time; below it is a few percent, and none for a few dozen keys). While all
+    CTAs of one tile run at once (two an SM) they pay later, and groups that leave rows of a tile idle keep one."""
     G = Hq // Hkv
     if G > 128 or B <= 0 or rows <= 0:
         return False
@@ -999,8 +999,8 @@ def prefill_pair_wins(pairs, rows, B, Hq, Hkv, sms=148) -> bool:
     per = 128 // G * G                                           # rows of a tile
     ctas = Hkv * B * -(-rows * G // (B * per))                   # of one tile each, for sequences of the mean length
     if ctas < 1.55 * sms:
-        return whole and keys >= 1024
-    return keys >= (448 if whole else 512)
+        return whole and keys >= 288
+    return keys >= 160
 
 
 def paged_prefill(q, q_stride, out, cache_layer, block_stride, block_tokens, block_table, cu_q, kv_lens, B, max_q_len,
