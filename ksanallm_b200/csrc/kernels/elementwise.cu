@@ -604,36 +604,11 @@ __global__ void rope_kv_append_vec_kernel(bf16* __restrict__ qkv, const int* __r
   const int t = blockIdx.x;
   bf16* row = qkv + static_cast<size_t>(t) * (Hq + 2 * Hkv) * D;
   const int half = D >> 1, hv = half >> 3;                   // 16-byte vectors per half head
-  if (apply_rope) {
-    const float* cs = cos_sin + static_cast<size_t>(positions[t]) * D;
-    const int items = (Hq + Hkv) * hv;
-    for (int i = threadIdx.x; i < items; i += blockDim.x) {
-      const int h = i / hv, j0 = (i - h * hv) << 3;
-      bf16* hp = row + static_cast<size_t>(h) * D;
-      float x0[8], x1[8], c[8], sn[8], y0[8], y1[8];
-      unpack8(*reinterpret_cast<const uint4*>(hp + j0), x0);
-      unpack8(*reinterpret_cast<const uint4*>(hp + half + j0), x1);
-      *reinterpret_cast<float4*>(&c[0]) = *reinterpret_cast<const float4*>(cs + j0);
-      *reinterpret_cast<float4*>(&c[4]) = *reinterpret_cast<const float4*>(cs + j0 + 4);
-      *reinterpret_cast<float4*>(&sn[0]) = *reinterpret_cast<const float4*>(cs + half + j0);
-      *reinterpret_cast<float4*>(&sn[4]) = *reinterpret_cast<const float4*>(cs + half + j0 + 4);
-#pragma unroll
-      for (int e = 0; e < 8; ++e) { y0[e] = x0[e] * c[e] - x1[e] * sn[e]; y1[e] = x1[e] * c[e] + x0[e] * sn[e]; }
-      *reinterpret_cast<uint4*>(hp + j0) = pack8(y0);
-      *reinterpret_cast<uint4*>(hp + half + j0) = pack8(y1);
-    }
-    __syncthreads();
-  }
   const int slot = slots[t];
-  if (slot < 0 || cache == nullptr) return;
-  const int blk = slot / block_tokens, off = slot % block_tokens;
+  const bool keep = slot >= 0 && cache != nullptr;
+  const int blk = keep ? slot / block_tokens : 0, off = keep ? slot - blk * block_tokens : 0;
   CacheT* kbase = cache + static_cast<size_t>(blk) * block_stride;
-  const bf16* ksrc = row + static_cast<size_t>(Hq) * D;
-  const int dv = D >> 3, n8 = Hkv * dv;
-  for (int i = threadIdx.x; i < 2 * n8; i += blockDim.x) {
-    const int kv = i / n8, r = i - kv * n8;
-    const int h = r / dv, d = (r - h * dv) << 3;
-    const uint4 v = *reinterpret_cast<const uint4*>(ksrc + (static_cast<size_t>(i) << 3));
+  auto to_cache = [&](int kv, int h, int d, const uint4& v) {
     const size_t dst = ((static_cast<size_t>(kv) * Hkv + h) * block_tokens + off) * D + d;
     if constexpr (sizeof(CacheT) == 1) {
       float f[8];
@@ -641,6 +616,35 @@ __global__ void rope_kv_append_vec_kernel(bf16* __restrict__ qkv, const int* __r
       *reinterpret_cast<uint2*>(kbase + dst) = pack8_e4m3(f, kv ? v_scale_inv : k_scale_inv);
     } else {
       *reinterpret_cast<uint4*>(kbase + dst) = v;
+    }
+  };
+  // queries and keys: two halves of a head at a time, keys on to the cache from registers; then the values, copied
+  const float* cs = apply_rope ? cos_sin + static_cast<size_t>(positions[t]) * D : nullptr;
+  const int first = apply_rope ? 0 : Hq * hv, turned = (Hq + Hkv) * hv, items = turned + Hkv * hv;
+  for (int i = first + threadIdx.x; i < items; i += blockDim.x) {
+    const int h = i / hv, j0 = (i - h * hv) << 3;
+    if (h >= Hq && !keep && (h >= Hq + Hkv || !apply_rope)) continue;
+    bf16* hp = row + static_cast<size_t>(h) * D;
+    uint4 a = *reinterpret_cast<const uint4*>(hp + j0), b = *reinterpret_cast<const uint4*>(hp + half + j0);
+    if (apply_rope && i < turned) {
+      float x0[8], x1[8], c[8], sn[8], y0[8], y1[8];
+      unpack8(a, x0);
+      unpack8(b, x1);
+      *reinterpret_cast<float4*>(&c[0]) = *reinterpret_cast<const float4*>(cs + j0);
+      *reinterpret_cast<float4*>(&c[4]) = *reinterpret_cast<const float4*>(cs + j0 + 4);
+      *reinterpret_cast<float4*>(&sn[0]) = *reinterpret_cast<const float4*>(cs + half + j0);
+      *reinterpret_cast<float4*>(&sn[4]) = *reinterpret_cast<const float4*>(cs + half + j0 + 4);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) { y0[e] = x0[e] * c[e] - x1[e] * sn[e]; y1[e] = x1[e] * c[e] + x0[e] * sn[e]; }
+      a = pack8(y0);
+      b = pack8(y1);
+      *reinterpret_cast<uint4*>(hp + j0) = a;
+      *reinterpret_cast<uint4*>(hp + half + j0) = b;
+    }
+    if (h >= Hq && keep) {
+      const int kv = h >= Hq + Hkv;
+      to_cache(kv, h - Hq - (kv ? Hkv : 0), j0, a);
+      to_cache(kv, h - Hq - (kv ? Hkv : 0), half + j0, b);
     }
   }
 }
@@ -1029,12 +1033,14 @@ extern "C" int ksana_rope_kv_append(void* qkv, const int* positions, int pos_str
   if (neox && rot_dim == D && (D % 16) == 0 && pos_stride == 0 && (block_stride % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(qkv) % 16) == 0 && (reinterpret_cast<uintptr_t>(cache) % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(cos_sin) % 16) == 0) {
+    // as many threads as leave none idle in the last turn: 48 heads of 128 are 384 items, two turns of 192
+    const int items = (Hq + 2 * Hkv) * (D >> 4), turns = (items + 255) / 256, threads = ((items + turns - 1) / turns + 31) / 32 * 32;
     if (cache_fp8)
-      launch_early(rope_kv_append_vec_kernel<uint8_t>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (uint8_t*)cache,
+      launch_early(rope_kv_append_vec_kernel<uint8_t>, dim3(T), dim3(threads), 0, st, (bf16*)qkv, positions, slots, cos_sin, (uint8_t*)cache,
                                                             block_stride, block_tokens, Hq, Hkv, D, 1.f / k_scale,
                                                             1.f / v_scale, apply_rope);
     else
-      launch_early(rope_kv_append_vec_kernel<bf16>, dim3(T), dim3(256), 0, st, (bf16*)qkv, positions, slots, cos_sin, (bf16*)cache,
+      launch_early(rope_kv_append_vec_kernel<bf16>, dim3(T), dim3(threads), 0, st, (bf16*)qkv, positions, slots, cos_sin, (bf16*)cache,
                                                          block_stride, block_tokens, Hq, Hkv, D, 1.f, 1.f, apply_rope);
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }
