@@ -197,6 +197,8 @@ def moe_forward(model, mw: MoEWeights, x: torch.Tensor, h: torch.Tensor) -> torc
     """h += MoE(x) (reduced over the TP group). ``x`` is the normalised hidden state [T, H] (bf16)."""
     if getattr(model, "dp", None) is not None:
         return model.dp.moe(model, mw, x, h)           # attention data parallelism: dispatch / experts / combine
+    if model.tp_size == 1 and x.is_cuda and h.is_contiguous() and h.dtype == x.dtype:
+        return moe_partial(model, mw, x, residual=h)   # the residual is added where the experts' rows are summed
     out = moe_partial(model, mw, x)
     if model.tp_size > 1:
         out = model.comm.all_reduce(out)
@@ -241,12 +243,12 @@ def route(model, mw: MoEWeights, x: torch.Tensor):
 
 
 def moe_partial(model, mw: MoEWeights, x: torch.Tensor, into: Optional[torch.Tensor] = None,
-                shared: bool = True, routing=None) -> torch.Tensor:
+                shared: bool = True, routing=None, residual: Optional[torch.Tensor] = None) -> torch.Tensor:
     """This rank's share of MoE(x): the weighted outputs of the experts (or expert slices) it holds plus its slice
     of the shared expert, before any reduction over ranks. ``into`` ([T, H], e.g. a peer-visible buffer that a
     reduce kernel pulls from) receives the result when given. ``routing`` = (ids [T, K] int32, weights [T, K] fp32)
     decided elsewhere (the row's home rank under expert-parallel all-to-all dispatch; choices of experts this rank
-    does not hold carry id -1) replaces this block's own router."""
+    does not hold carry id -1) replaces this block's own router. ``residual`` [T, H] (GPU): added to the result, before its rounding."""
     cfg = model.cfg
     T, H = x.shape
     K, E = cfg.num_experts_per_tok, mw.num_experts
@@ -288,7 +290,7 @@ def moe_partial(model, mw: MoEWeights, x: torch.Tensor, into: Optional[torch.Ten
             if mw.shared_gate is not None:
                 gate = torch.sigmoid(x.float() @ mw.shared_gate.float().t())
                 out.copy_(out.float() * gate)
-        native.moe_combine(y, dst_row, w, out, K, accumulate=have_shared)
+        native.moe_combine(y, dst_row, w, out, K, accumulate=have_shared, residual=residual)
         return out
     else:
         if routing is not None:

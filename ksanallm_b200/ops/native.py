@@ -43,7 +43,7 @@ _SIGS = {
     "ksana_moe_align": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_moe_permute": [vp, vp, vp, i32, i32, i32, i32, vp, vp],
     "ksana_moe_permute_fp8": [vp, vp, i32, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
-    "ksana_moe_combine": [vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
+    "ksana_moe_combine": [vp, vp, vp, vp, vp, i32, i32, i32, i32, i32, vp, vp],
     "ksana_gemm_smallm_push": [i32, vp, i32, vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, vp, i64, vp, i32, vp, i32, vp, vp],
     "ksana_gemm_smallm_push_signal": [i32, vp, i32, vp, i32, vp, i32, vp, i32, vp, i32, i32, i32, vp, i64, vp, i32, vp, i32,
                                       vp, vp, vp, vp, vp],
@@ -1356,8 +1356,10 @@ def moe_permute_fp8(q, scale, dst_row, K, cap):
     return perm, ps
 
 
-def moe_combine(y, dst_row, topk_w, out, K, accumulate):
+def moe_combine(y, dst_row, topk_w, out, K, accumulate, residual=None):
+    """out = (out +) the weighted sum of every row's choices (+ ``residual``: rows of out's type and layout, e.g. out itself)."""
     T, H = out.shape
-    _check(lib().ksana_moe_combine(_p(y), _p(dst_row), _p(topk_w), _p(out), T, K, H, int(accumulate), int(y.shape[0]),
+    assert residual is None or (residual.shape == out.shape and residual.dtype == out.dtype and residual.is_contiguous())
+    _check(lib().ksana_moe_combine(_p(y), _p(dst_row), _p(topk_w), _p(out), _p(residual), T, K, H, int(accumulate), int(y.shape[0]),
                                    _p(err_flag(out.device)), _st()), "ksana_moe_combine")
     return out

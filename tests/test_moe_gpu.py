@@ -161,3 +161,20 @@ def test_moe_block_with_restricted_choices_matches_cpu_statement():
     assert rel_err(got, want) < 2e-2, rel_err(got, want)
     rows_without = (~keep).all(dim=1).cpu()
     assert float(got[rows_without].abs().max()) == 0.0 if bool(rows_without.any()) else True
+
+
+@pytest.mark.parametrize("T,H,K", [(1, 8, 1), (5, 264, 3), (700, 1032, 9)])
+@pytest.mark.parametrize("accumulate", [False, True])
+def test_combine_with_residual(T, H, K, accumulate):
+    """Rows added where the choices are summed: one rounding of the whole sum (2^-9 of it, fp32 sums before). Left-out choices have no row."""
+    torch.manual_seed(T + H)
+    y = torch.randn(T * K, H, device=DEV, dtype=torch.bfloat16)
+    rows = torch.randperm(T * K, device=DEV).to(torch.int32).view(T, K)
+    rows[:, K // 2] = -1
+    w = torch.rand(T, K, device=DEV)
+    out, res = (torch.randn(T, H, device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    part = torch.where((rows >= 0)[..., None], y[rows.clamp_min(0).long()].double(), 0.0) * w.double()[..., None]
+    want = part.sum(1) + res.double() + (out.double() if accumulate else 0.0)
+    size = part.abs().sum(1) + res.double().abs() + out.double().abs()
+    native.moe_combine(y, rows, w, out, K, accumulate, residual=res)
+    assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + (K + 2) * 2.0 ** -23 * size).all())
