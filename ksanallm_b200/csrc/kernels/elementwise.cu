@@ -771,6 +771,36 @@ __global__ void absmax_kernel(const bf16* __restrict__ x, int rows, int cols, lo
     if (threadIdx.x == 0 && m > 0.f && m == m) atomicMax(acc, __float_as_uint(m));
   }
 }
+// The same in chunks of 16 elements, four in flight a thread, maxima on packed pairs (by: chunks of a row): 9753 x 14336 53 -> 44 us, x 4096 19.8 -> 16.5.
+__global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restrict__ x, uint32_t total, FastDiv by, long long ldx, unsigned int* acc) {
+  __shared__ float red[8];
+  const uint32_t step = gridDim.x * blockDim.x;
+  __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
+  for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += 4 * step) {
+    Chunk16 c[4] = {};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const uint32_t i = base + k * step;
+      if (i < total) {
+        const uint32_t r = by.div(i);
+        c[k] = ld_chunk(x + r * ldx + (i - r * by.d) * 16);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&c[k].w[e])));
+  }
+  const float2 f = __bfloat1622float2(m);
+  const float w = warp_max(fmaxf(f.x, f.y));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float all = red[0];
+    for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) all = fmaxf(all, red[k]);
+    if (all > 0.f) atomicMax(acc, __float_as_uint(all));
+  }
+}
 __global__ void absmax_finish_kernel(unsigned int* acc, float* scale, float inv_divisor, float floor_value) {
   *scale = fmaxf(__uint_as_float(*acc) * inv_divisor, floor_value);
   *acc = 0u;
@@ -848,14 +878,12 @@ static inline int norm_threads(int H) {
 // ----------------------------------------------------------------------------
 // NVFP4 quantisation of GEMM inputs: 16-element blocks along K, e2m1 values (two per byte, even element in the
 // low nibble), one e4m3 scale per block, one fp32 scale per tensor (given): x ~= e2m1 * block_scale * tensor_scale.
+// (row and block by multiplication: the two 64-bit divisions a block took a few percent: 9753 x 14336 73 -> 71.7 us)
 __global__ void quant_nvfp4_kernel(const bf16* __restrict__ x, int ldx, uint8_t* __restrict__ q, int ldq,
-                                   uint8_t* __restrict__ bs, int ldbs, const float* __restrict__ ts, int M, int K) {
-  const int nb = K >> 4;
-  const long long total = static_cast<long long>(M) * nb;
+                                   uint8_t* __restrict__ bs, int ldbs, const float* __restrict__ ts, uint32_t total, FastDiv by) {
   const float inv_ts = 1.f / (ts ? *ts : 1.f);
-  for (long long idx = blockIdx.x * static_cast<long long>(blockDim.x) + threadIdx.x; idx < total;
-       idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-    const int row = static_cast<int>(idx / nb), b = static_cast<int>(idx % nb);
+  for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
+    const uint32_t row = by.div(idx), b = idx - row * by.d;
     const uint4* src = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * ldx + b * 16);
     float f[16];
     unpack8(src[0], *reinterpret_cast<float(*)[8]>(&f[0]));
@@ -996,9 +1024,15 @@ extern "C" int ksana_quant_nvfp4(const void* x, int x_ld, void* q, int q_ld, voi
                                  int K, cudaStream_t st) {
   if (M <= 0) return 0;
   if (K % 16 || x_ld % 8 || q_ld % 8) return -10;
-  const long long total = static_cast<long long>(M) * (K >> 4);
-  quant_nvfp4_kernel<<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x, x_ld, (uint8_t*)q, q_ld, (uint8_t*)bs, bs_ld,
-                                                           ts, M, K);
+  const int nb = K >> 4, most = static_cast<int>((1LL << 30) / nb);       // (flat indices stay below 2^31, a step beyond the end included)
+  if (most < 1) return -10;
+  for (int m0 = 0; m0 < M; m0 += most) {
+    const uint32_t total = static_cast<uint32_t>(M - m0 < most ? M - m0 : most) * nb;
+    quant_nvfp4_kernel<<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x + static_cast<size_t>(m0) * x_ld, x_ld,
+                                                             (uint8_t*)q + static_cast<size_t>(m0) * q_ld, q_ld,
+                                                             (uint8_t*)bs + static_cast<size_t>(m0) * bs_ld, bs_ld, ts, total,
+                                                             make_fast_div(nb));
+  }
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -1096,7 +1130,11 @@ extern "C" int ksana_absmax_scale(const void* x, int rows, int cols, long long l
   if (rows <= 0 || cols <= 0) return 0;
   if ((cols % 8) || (ldx % 8) || divisor <= 0.f || (reinterpret_cast<uintptr_t>(x) & 15)) return -10;
   const long long nvec = static_cast<long long>(rows) * (cols >> 3);
-  absmax_kernel<<<grid_for(nvec, 256), 256, 0, st>>>((const bf16*)x, rows, cols, ldx, (unsigned int*)acc);
+  if (cols % 16 == 0 && ldx % 16 == 0 && !(reinterpret_cast<uintptr_t>(x) & 31) && nvec / 2 < (1LL << 30))
+    absmax_chunks_kernel<<<grid_for(nvec / 2, 256), 256, 0, st>>>((const bf16*)x, static_cast<uint32_t>(nvec / 2), make_fast_div(cols / 16),
+                                                                  ldx, (unsigned int*)acc);
+  else
+    absmax_kernel<<<grid_for(nvec, 256), 256, 0, st>>>((const bf16*)x, rows, cols, ldx, (unsigned int*)acc);
   absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }

@@ -49,3 +49,17 @@ def test_gemm_nvfp4(M, N, K, bn):
     yf = torch.empty(M, N, device=DEV, dtype=torch.float32)
     native.gemm_nvfp4(aq, a_bs, a_ts, wq, w_bs, w_ts, out_f32=yf, bn=bn)
     assert rel_err(yf, ref.gemm_nvfp4(aq, a_bs, a_ts, wq, w_bs, w_ts, out_dtype=torch.float32)) < 2e-3
+
+
+@pytest.mark.parametrize("M,K,ld", [(1, 16, 16), (3, 48, 64), (700, 4096, 4096), (9, 8, 24), (2000, 1040, 1056)])
+def test_absmax_of_rows(M, K, ld):
+    """The largest magnitude wherever it stands, rows with gaps, sizes that are no whole chunks; NaN do not count."""
+    g = torch.Generator(device=DEV).manual_seed(M)
+    buf = torch.full((M, ld), 1e4, device=DEV, dtype=torch.bfloat16)
+    x = buf[:, :K]
+    for at in {(0, 0), (M - 1, K - 1), (M // 2, K // 2)}:
+        x.copy_(torch.empty(M, K, device=DEV, dtype=torch.bfloat16).normal_(generator=g))
+        x[at] = -77.0
+        if M * K > 100:
+            x[M // 3, K // 3] = float("nan")
+        assert float(native.absmax_scale(x, 7.0)) == float(torch.tensor(77.0) * (1.0 / torch.tensor(7.0)))
