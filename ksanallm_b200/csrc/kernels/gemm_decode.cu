@@ -279,12 +279,12 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       const uint32_t base = smem_u32(smem) + f * 4;
       for (int m = m0; m < m1; m += 4) {
         float v[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int r = 0; r < S; r += 2) {      // in rank order; S is even
+        for (int r = 0; r < S; r += 2) {      // in rank order
           float x[2][4];
 #pragma unroll
           for (int k = 0; k < 2; ++k)
 #pragma unroll
-            for (int i = 0; i < 4; ++i) x[k][i] = ld_cluster_f32(base + min(m + i, MP - 1) * (kGdRedPitch * 4), r + k);
+            for (int i = 0; i < 4; ++i) x[k][i] = r + k < S ? ld_cluster_f32(base + min(m + i, MP - 1) * (kGdRedPitch * 4), r + k) : 0.f;
 #pragma unroll
           for (int i = 0; i < 4; ++i) v[i] = (v[i] + x[0][i]) + x[1][i];
         }
@@ -384,6 +384,12 @@ extern "C" int ksana_gemm_decode(int kind, const void* X, int ldx, const float* 
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   p.splits = 1;
   while (p.splits < 8 && tiles * p.splits < sms && num_kb >= p.splits * 8) p.splits *= 2;
+  // Three for two and six for four where all of them run at once with room to spare (a CTA alone on its SM has half the loads in flight; clusters
+  // do not fill every group of SMs, and one that has to wait costs a whole round). us, before / after: e4m3 10240 x 8192, 64 rows 26.9 / 24.1,
+  // 32 rows 21.6 / 20.2; bf16 10240 x 8192, 1 row 31.5 / 28.9, 5120 x 13824, 4 rows 26.8 / 26.2; but 288 CTAs: 6144 x 4096 11.6 / 15.8,
+  // e4m3 12288 x 7168 26.5 / 34.4.
+  const int more = p.splits + p.splits / 2;
+  if ((p.splits == 2 || p.splits == 4) && 20 * tiles * more <= 33 * sms && num_kb >= 8 * more) p.splits = more;
   const bool early = fixed_w != 0;
   if (kind == 0)
     return MP == 16 ? launch_gemm_decode<16, 0>(mw, mx, p, early, st) : MP == 32 ? launch_gemm_decode<32, 0>(mw, mx, p, early, st)

@@ -48,3 +48,21 @@ def test_block_scaled(M, N, K):
     out = res.clone()
     close(native.gemm_fp8(xq, xs, wq, ws, out=out, residual=out, hw_scale=True), want + res.double(), sums)
     native.check_err_flag(DEV)
+
+
+@pytest.mark.parametrize("M", [1, 5, 33, 64])
+@pytest.mark.parametrize("N,K", [(10100, 2056), (5000, 4096)])
+def test_three_and_six_shares(M, N, K):
+    """K ranges cut in three (79 tiles) and six (40): shares of unequal length, fewer tokens than shares."""
+    torch.manual_seed(M + N)
+    x, w = torch.randn(M, K, device=DEV, dtype=torch.bfloat16), torch.randn(N, K, device=DEV, dtype=torch.bfloat16)
+    close(native.gemm_bf16(x, w), x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t())
+    K = K // 128 * 384
+    x = torch.randn(M, K, device=DEV, dtype=torch.bfloat16)
+    xq, xs = native.quant_fp8(x)
+    wq = (torch.randn(N, K, device=DEV) * 64).clamp(-448, 448).to(torch.float8_e4m3fn)
+    ws = 2.0 ** torch.randint(-9, -4, (-(-N // 128), K // 128), device=DEV).float()
+    xd = xq.double() * xs[:, :M].t().repeat_interleave(128, 1).double()
+    wd = wq.double() * ws.repeat_interleave(128, 0)[:N].repeat_interleave(128, 1).double()
+    close(native.gemm_fp8(xq, xs, wq, ws, hw_scale=True), xd @ wd.t(), xd.abs() @ wd.abs().t())
+    native.check_err_flag(DEV)
