@@ -212,6 +212,24 @@ __device__ __forceinline__ float group8_absmax(const Chunk16& c) {
   const float2 f = __bfloat1622float2(m);
   return fmaxf(f.x, f.y);
 }
+// Largest magnitude of what a CTA (up to 8 warps) stored, into *acc (zero or the largest so far, as bits); NaN do not count.
+__device__ __forceinline__ void publish_absmax(__nv_bfloat162 m, unsigned int* acc) {
+  __shared__ float red[8];
+  const float2 f = __bfloat1622float2(m);
+  const float w = warp_max(fmaxf(f.x, f.y));
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    float all = red[0];
+    for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) all = fmaxf(all, red[k]);
+    if (all > 0.f) atomicMax(acc, __float_as_uint(all));
+  }
+}
+__device__ __forceinline__ __nv_bfloat162 chunk_absmax(const Chunk16& c, __nv_bfloat162 m) {
+#pragma unroll
+  for (int e = 0; e < 8; ++e) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&c.w[e])));
+  return m;
+}
 // a chunk times `inv` as 16 e4m3 values
 __device__ __forceinline__ uint4 chunk_e4m3(const Chunk16& c, float inv) {
   uint32_t o[4];
@@ -231,10 +249,11 @@ __device__ __forceinline__ uint4 chunk_e4m3(const Chunk16& c, float inv) {
 // Root-mean-square norm: CTAs stay and take row after row, the next row's loads in flight under the work on this one. One CTA per row
 // (norm_kernel) spent its time waiting and on 21.6 instructions an element. us, there / here: with fp8 copy 16384 x 8192 122 / 74 (5.5 TB/s),
 // 8000 x 7168 60 / 39, 300 x 7168 5.7 / 4.2; 16384 x 4096 56 / 43, 64 x 4096 3.9 / 2.6. V chunks per thread.
-template <bool QUANT, int V>
+// AMAX: *acc takes the largest magnitude of the result (the tensor scale of an NVFP4 operand without a pass of its own).
+template <bool QUANT, int V, bool AMAX>
 __global__ void __launch_bounds__(256, V == 1 ? 4 : V == 2 ? 3 : 2)
 norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, uint8_t* __restrict__ yq,
-                 float* __restrict__ yscale, int scale_ld, int M, int H, float eps) {
+                 float* __restrict__ yscale, int scale_ld, int M, int H, float eps, unsigned int* acc) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[2][8];
@@ -248,6 +267,7 @@ norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* _
     }
   };
   int row = blockIdx.x, turn = 0;
+  __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
   if (row < M) fetch(row);
   for (; row < M; row += gridDim.x, turn ^= 1) {
     Chunk16 v[V];
@@ -277,6 +297,7 @@ norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* _
 #pragma unroll
         for (int e = 0; e < 8; ++e) o.w[e] = pack2(unpack2(v[k].w[e]) * rstd * unpack2(wc.w[e]));
       }
+      if constexpr (AMAX) top = chunk_absmax(o, top);
       if constexpr (QUANT) {
         const float scale = fp8_group_scale(group8_absmax(o));
         if (on) {
@@ -290,6 +311,7 @@ norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* _
       }
     }
   }
+  if constexpr (AMAX) publish_absmax(top, acc);
 }
 
 // ----------------------------------------------------------------------------
@@ -369,13 +391,14 @@ act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __r
 
 // Gated rows in chunks of 16 elements (see there); arguments as act_mul_kernel, nchunk counts a row's chunks. At full clocks 16384 x 28672
 // quantised 405 -> 379 us (6.2 TB/s), without fp8 16384 x 14336 226 -> 224; quantisation alone of 16384 x 8192 74 -> 67.
-template <int ACT, bool QUANT>
+template <int ACT, bool QUANT, bool AMAX>
 __global__ void __launch_bounds__(256)
 act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __restrict__ outq, float* __restrict__ oscale, int scale_ld,
-                  uint32_t total, FastDiv nchunk, int in_ld, const int* __restrict__ tile_rows) {
+                  uint32_t total, FastDiv nchunk, int in_ld, const int* __restrict__ tile_rows, unsigned int* acc) {
   pdl_trigger();
   pdl_wait();
   const uint32_t step = gridDim.x * blockDim.x, I = nchunk.d * 16;
+  __nv_bfloat162 top = __floats2bfloat162_rn(0.f, 0.f);
   for (uint32_t idx = blockIdx.x * blockDim.x + threadIdx.x; (idx & ~31u) < total; idx += step) {
     bool on = idx < total;                         // whole warps stay in the loop for the exchanges
     const uint32_t m = on ? nchunk.div(idx) : 0u, i = on ? idx - m * nchunk.d : 0u;
@@ -400,6 +423,7 @@ act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* 
         o.w[e] = pack2(a * unpack2(u.w[e]));
       }
     }
+    if constexpr (AMAX) top = chunk_absmax(o, top);
     if constexpr (QUANT) {
       const float scale = fp8_group_scale(group8_absmax(o));
       if (on) {
@@ -411,6 +435,7 @@ act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* 
       st_global_32(out + static_cast<size_t>(m) * I + i * 16, make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]), make_uint4(o.w[4], o.w[5], o.w[6], o.w[7]));
     }
   }
+  if constexpr (AMAX) publish_absmax(top, acc);
 }
 
 // The same on fp32 rows, with the exponential instead of the approximate tanh.
@@ -774,7 +799,6 @@ __global__ void absmax_kernel(const bf16* __restrict__ x, int rows, int cols, lo
 }
 // The same in chunks of 16 elements, four in flight a thread, maxima on packed pairs (by: chunks of a row): 9753 x 14336 53 -> 44 us, x 4096 19.8 -> 16.5.
 __global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restrict__ x, uint32_t total, FastDiv by, long long ldx, unsigned int* acc) {
-  __shared__ float red[8];
   const uint32_t step = gridDim.x * blockDim.x;
   __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
   for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += 4 * step) {
@@ -788,19 +812,9 @@ __global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restri
       }
     }
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) m = __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&c[k].w[e])));
+    for (int k = 0; k < 4; ++k) m = chunk_absmax(c[k], m);
   }
-  const float2 f = __bfloat1622float2(m);
-  const float w = warp_max(fmaxf(f.x, f.y));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float all = red[0];
-    for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) all = fmaxf(all, red[k]);
-    if (all > 0.f) atomicMax(acc, __float_as_uint(all));
-  }
+  publish_absmax(m, acc);
 }
 __global__ void absmax_finish_kernel(unsigned int* acc, float* scale, float inv_divisor, float floor_value) {
   *scale = fmaxf(__uint_as_float(*acc) * inv_divisor, floor_value);
@@ -910,8 +924,9 @@ __global__ void quant_nvfp4_kernel(const bf16* __restrict__ x, int ldx, uint8_t*
 
 using namespace ksana;
 
-extern "C" int ksana_norm(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
-                          float* yscale, int scale_ld, int M, int H, float eps, int layernorm, cudaStream_t st) {
+// acc (may be null): also the largest magnitude of y into *acc; -100 where the kernel that does that does not take the call.
+static int norm_impl(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
+                     float* yscale, int scale_ld, int M, int H, float eps, int layernorm, void* acc, cudaStream_t st) {
   if (M <= 0) return 0;
   if (H % 8 || H > 8 * kMaxVec * 1024) return -10;
   if (yq && (H % 128)) return -11;
@@ -924,13 +939,15 @@ extern "C" int ksana_norm(const void* x, void* residual, const void* w, const vo
     const int chunks = H / 16, v = chunks <= 256 ? 1 : chunks <= 512 ? 2 : 4;
     const int threads = ((chunks + v - 1) / v + 31) / 32 * 32, per_sm = (v == 1 ? 4 : v == 2 ? 3 : 2) * (256 / threads > 1 ? 256 / threads : 1);
     const dim3 grid(M < sms * per_sm ? M : sms * per_sm);
-#define KSANA_NORM_ROWS(Q, V) launch_early(norm_rows_kernel<Q, V>, grid, dim3(threads), 0, st, (const bf16*)x, (const bf16*)w, (bf16*)y, \
-                                           (uint8_t*)yq, yscale, scale_ld, M, H, eps)
-    if (yq) v == 1 ? KSANA_NORM_ROWS(true, 1) : v == 2 ? KSANA_NORM_ROWS(true, 2) : KSANA_NORM_ROWS(true, 4);
-    else v == 1 ? KSANA_NORM_ROWS(false, 1) : v == 2 ? KSANA_NORM_ROWS(false, 2) : KSANA_NORM_ROWS(false, 4);
+#define KSANA_NORM_ROWS(Q, V, A) launch_early(norm_rows_kernel<Q, V, A>, grid, dim3(threads), 0, st, (const bf16*)x, (const bf16*)w, (bf16*)y, \
+                                              (uint8_t*)yq, yscale, scale_ld, M, H, eps, static_cast<unsigned int*>(acc))
+    if (acc) v == 1 ? KSANA_NORM_ROWS(false, 1, true) : v == 2 ? KSANA_NORM_ROWS(false, 2, true) : KSANA_NORM_ROWS(false, 4, true);
+    else if (yq) v == 1 ? KSANA_NORM_ROWS(true, 1, false) : v == 2 ? KSANA_NORM_ROWS(true, 2, false) : KSANA_NORM_ROWS(true, 4, false);
+    else v == 1 ? KSANA_NORM_ROWS(false, 1, false) : v == 2 ? KSANA_NORM_ROWS(false, 2, false) : KSANA_NORM_ROWS(false, 4, false);
 #undef KSANA_NORM_ROWS
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }
+  if (acc) return -100;
   const int threads = norm_threads(H);
 #define KSANA_NORM(MODE, RES, Q) launch_early(norm_kernel<MODE, RES, Q>, dim3(M), dim3(threads), 0, st, (const bf16*)x, (bf16*)residual, \
                                               (const bf16*)w, (const bf16*)beta, (bf16*)y, (uint8_t*)yq, yscale, scale_ld, H, eps)
@@ -939,6 +956,43 @@ extern "C" int ksana_norm(const void* x, void* residual, const void* w, const vo
   else residual ? KSANA_NORM_Q(0, true) : KSANA_NORM_Q(0, false);
 #undef KSANA_NORM_Q
 #undef KSANA_NORM
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+extern "C" int ksana_norm(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
+                          float* yscale, int scale_ld, int M, int H, float eps, int layernorm, cudaStream_t st) {
+  return norm_impl(x, residual, w, beta, y, yq, yscale, scale_ld, M, H, eps, layernorm, nullptr, st);
+}
+
+// y = the root-mean-square norm of x times w, and *scale = max(largest |y| / divisor, floor_value); acc: a zero word, zero again afterwards.
+// Read again for that, 9753 x 4096 cost 16.5 us and x 14336 44 us; a 4096-wide NVFP4 layer's prefill of 9753 rows with head 2276 -> 2231 us.
+// -100: not covered (rows off 32-byte boundaries, H no multiple of 16 or above 16384): norm and largest magnitude one after the other do it.
+extern "C" int ksana_norm_absmax(const void* x, const void* w, void* y, int M, int H, float eps, float divisor, float floor_value, void* acc,
+                                 float* scale, cudaStream_t st) {
+  if (M <= 0 || divisor <= 0.f || !acc || !scale) return -10;
+  const int rc = norm_impl(x, nullptr, w, nullptr, y, nullptr, nullptr, 0, M, H, eps, 0, acc, st);
+  if (rc) return rc;
+  absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
+  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+}
+
+// out = act(gate) * up of packed rows and the scale of its largest magnitude, as above. -100: not covered (small launches, no whole chunks).
+extern "C" int ksana_act_mul_absmax(const void* in, void* out, int M, int I, int in_ld, int act, float divisor, float floor_value, void* acc,
+                                    float* scale, cudaStream_t st) {
+  if (M <= 0 || divisor <= 0.f || !acc || !scale) return -10;
+  const long long total = static_cast<long long>(M) * (I >> 3);
+  if (I % 16 || in_ld % 16 || !chunks_pay(total) || total >= (1LL << 31) || ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 31))
+    return -100;
+  const FastDiv by = make_fast_div(I / 16);
+  const dim3 grid(grid_for(total / 2, 256));
+#define KSANA_ACT_AMAX(A) launch_early(act_chunks_kernel<A, false, true>, grid, dim3(256), 0, st, (const bf16*)in, (bf16*)out, \
+                                       static_cast<uint8_t*>(nullptr), static_cast<float*>(nullptr), 0, static_cast<uint32_t>(total / 2), by, in_ld, \
+                                       static_cast<const int*>(nullptr), static_cast<unsigned int*>(acc))
+  if (act == 0) KSANA_ACT_AMAX(0);
+  else if (act == 1) KSANA_ACT_AMAX(1);
+  else KSANA_ACT_AMAX(2);
+#undef KSANA_ACT_AMAX
+  absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
@@ -965,7 +1019,8 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
         !((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(dq)) & 31)) {
       const FastDiv by = make_fast_div(I / 16);
       const dim3 chunk_grid(grid_for(total / 2, 256));
-#define KSANA_ACT16(A, Q) launch_early(act_chunks_kernel<A, Q>, chunk_grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total / 2, by, in_ld, tr)
+#define KSANA_ACT16(A, Q) launch_early(act_chunks_kernel<A, Q, false>, chunk_grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total / 2, by, in_ld, tr, \
+                                          static_cast<unsigned int*>(nullptr))
       if (act == 0) dq ? KSANA_ACT16(0, true) : KSANA_ACT16(0, false);
       else if (act == 1) dq ? KSANA_ACT16(1, true) : KSANA_ACT16(1, false);
       else dq ? KSANA_ACT16(2, true) : KSANA_ACT16(2, false);

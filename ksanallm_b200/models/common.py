@@ -262,7 +262,7 @@ class CommonModel:
     def mlp(self, lw: LayerWeights, x, h: torch.Tensor) -> torch.Tensor:
         cfg = self.cfg
         gu = ops.linear(x, lw.gate_up)
-        a = ops.act_mul(gu, cfg.activation, cfg.gated_mlp, quant_for=lw.down)
+        a = ops.act_mul(gu, cfg.activation, cfg.gated_mlp, quant_for=lw.down, scaled=self.tp_size == 1)
         return self.row_parallel(a, lw.down, h)
 
     def layer_forward(self, li: int, lw: LayerWeights, h: torch.Tensor, step: StepInput) -> torch.Tensor:
@@ -275,7 +275,7 @@ class CommonModel:
             h = ops.norm(h, lw.input_norm, cfg.rms_norm_eps, beta=lw.input_norm_bias, layernorm=ln)
             h = self.mlp(lw, h, h)
             return ops.norm(h, lw.post_norm, cfg.rms_norm_eps, beta=lw.post_norm_bias, layernorm=ln)
-        x = ops.norm(h, lw.input_norm, cfg.rms_norm_eps, beta=lw.input_norm_bias, layernorm=ln, quant_for=lw.qkv)
+        x = ops.norm(h, lw.input_norm, cfg.rms_norm_eps, beta=lw.input_norm_bias, layernorm=ln, quant_for=lw.qkv, scaled=not lw.attn_extra)
         with nvtx.annotate("attention"):
             a = self.attention(li, lw, x, step)
         with nvtx.annotate("o_proj"):
@@ -284,7 +284,7 @@ class CommonModel:
             from .moe import moe_forward
             x = ops.norm(h, lw.post_norm, cfg.rms_norm_eps, beta=lw.post_norm_bias, layernorm=ln)
             return moe_forward(self, lw.moe, x, h)
-        x = ops.norm(h, lw.post_norm, cfg.rms_norm_eps, beta=lw.post_norm_bias, layernorm=ln, quant_for=lw.gate_up)
+        x = ops.norm(h, lw.post_norm, cfg.rms_norm_eps, beta=lw.post_norm_bias, layernorm=ln, quant_for=lw.gate_up, scaled=True)
         with nvtx.annotate("mlp"):
             return self.mlp(lw, x, h)
 

@@ -25,6 +25,20 @@ class QTensor:
         return self.q.shape
 
 
+@dataclass
+class Scaled:
+    """bf16 rows and the tensor scale that an NVFP4 layer quantises them with."""
+    x: torch.Tensor
+    ts: torch.Tensor
+
+    @property
+    def shape(self):
+        return self.x.shape
+
+
+NVFP4_RANGE = 448.0 * 6.0          # largest block scale times largest value
+
+
 class LinearWeight:
     """[N,K] weight of y = x W^T (+bias): dense bf16/fp32, or e4m3 with one fp32 scale per 128x128 block."""
 
@@ -122,8 +136,8 @@ def quantize(x: torch.Tensor) -> QTensor:
 
 
 def linear(x, W: LinearWeight, residual=None, out=None, out_f32: bool = False):
-    """y = x W^T (+bias) (+residual). ``x`` may be a QTensor when W is FP8. ``out`` may alias ``residual``. ``W`` holds loaded weights:
-    no work that is still in flight writes them."""
+    """y = x W^T (+bias) (+residual). ``x`` may be a QTensor when W is FP8, :class:`Scaled` rows when W is NVFP4. ``out`` may alias
+    ``residual``. ``W`` holds loaded weights: no work that is still in flight writes them."""
     if W.w4a16:
         if isinstance(x, QTensor):
             raise TypeError("4-bit weight-only layers take bf16 activations")
@@ -138,10 +152,12 @@ def linear(x, W: LinearWeight, residual=None, out=None, out_f32: bool = False):
         return y
     if W.nvfp4:
         # activations are quantised to NVFP4 too (per-tensor scale from the tensor's own maximum, no host sync)
-        if x.is_cuda and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0:
-            a_ts = native.absmax_scale(x, 448.0 * 6.0)          # one pass over x, scale stays on the device
+        if isinstance(x, Scaled):
+            x, a_ts = x.x, x.ts
+        elif x.is_cuda and x.dtype == torch.bfloat16 and x.shape[1] % 8 == 0 and x.stride(1) == 1 and x.stride(0) % 8 == 0:
+            a_ts = native.absmax_scale(x, NVFP4_RANGE)          # one pass over x, scale stays on the device
         else:
-            a_ts = (x.float().abs().amax() / (448.0 * 6.0)).clamp_min(1e-12).reshape(())
+            a_ts = (x.float().abs().amax() / NVFP4_RANGE).clamp_min(1e-12).reshape(())
         if x.is_cuda:
             aq, a_bs, _ = native.quant_nvfp4(x, a_ts)
             if out_f32:
@@ -181,9 +197,12 @@ def linear(x, W: LinearWeight, residual=None, out=None, out_f32: bool = False):
     return y
 
 
-def norm(x, w, eps, residual=None, beta=None, layernorm=False, quant_for: Optional[LinearWeight] = None):
+def norm(x, w, eps, residual=None, beta=None, layernorm=False, quant_for: Optional[LinearWeight] = None, scaled: bool = False):
     """Returns the normalised activations in the form the consuming linear wants (QTensor for FP8
-    weights on CUDA). ``residual`` (if given) is updated in place with residual + x."""
+    weights on CUDA). ``residual`` (if given) is updated in place with residual + x. ``scaled``: the result goes to :func:`linear` with
+    ``quant_for`` only, so that an NVFP4 layer may get :class:`Scaled` rows."""
+    if scaled and x.is_cuda and x.dtype == torch.bfloat16 and quant_for is not None and quant_for.nvfp4 and residual is None and beta is None and not layernorm:
+        return Scaled(*native.norm_absmax(x, w, eps, NVFP4_RANGE))
     want_q = quant_for is not None and quant_for.fp8 and x.shape[-1] % 128 == 0
     if x.is_cuda:
         if want_q:
@@ -197,7 +216,10 @@ def norm(x, w, eps, residual=None, beta=None, layernorm=False, quant_for: Option
     return QTensor(*ref.quant_fp8(y)) if want_q else y
 
 
-def act_mul(x, kind="silu", gated=True, quant_for: Optional[LinearWeight] = None):
+def act_mul(x, kind="silu", gated=True, quant_for: Optional[LinearWeight] = None, scaled: bool = False):
+    """``scaled``: see :func:`norm`."""
+    if scaled and gated and x.is_cuda and x.dtype == torch.bfloat16 and quant_for is not None and quant_for.nvfp4:
+        return Scaled(*native.act_mul_absmax(x, kind, NVFP4_RANGE))
     inter = x.shape[-1] // 2 if gated else x.shape[-1]
     want_q = quant_for is not None and quant_for.fp8 and inter % 128 == 0
     if x.is_cuda:

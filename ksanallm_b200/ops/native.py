@@ -69,6 +69,8 @@ _SIGS = {
     "ksana_add": [vp, vp, vp, vp, i64, i32, vp],
     "ksana_patch_ids": [vp, vp, vp, vp, i32, i32, i32, vp, vp],
     "ksana_smallm_estimate": [i32, i32, i32, i32, vp],
+    "ksana_norm_absmax": [vp, vp, vp, i32, i32, f32, f32, f32, vp, vp, vp],
+    "ksana_act_mul_absmax": [vp, vp, i32, i32, i32, i32, f32, f32, vp, vp, vp],
     "ksana_absmax_scale": [vp, i32, i32, i64, f32, f32, vp, vp, vp],
     "ksana_rerotate_blocks": [vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i64, vp, vp],
     "ksana_embed_pair": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, f32, i32, vp, vp],
@@ -514,15 +516,19 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
 _absmax_acc = {}
 
 
+def _absmax_words(device):
+    """(the device's word for a largest magnitude, zero between launches; a new scalar for the scale)"""
+    key = (device.type, device.index)
+    if key not in _absmax_acc:
+        _absmax_acc[key] = torch.zeros(1, dtype=torch.int32, device=device)
+    return _absmax_acc[key], torch.empty((), dtype=torch.float32, device=device)
+
+
 def absmax_scale(x, divisor: float, floor: float = 1e-12):
     """max(|x|) / divisor (at least ``floor``) of a bf16 matrix as an fp32 scalar tensor on the device: the tensor
     scale of an NVFP4 activation, without a host round trip or a widened copy of ``x``."""
     rows, cols = x.shape
-    key = (x.device.type, x.device.index)
-    acc = _absmax_acc.get(key)
-    if acc is None:
-        acc = _absmax_acc[key] = torch.zeros(1, dtype=torch.int32, device=x.device)
-    scale = torch.empty((), dtype=torch.float32, device=x.device)
+    acc, scale = _absmax_words(x.device)
     _check(lib().ksana_absmax_scale(_p(x), rows, cols, x.stride(0), float(divisor), float(floor), _p(acc), _p(scale),
                                     _st()), "ksana_absmax_scale")
     return scale
@@ -664,7 +670,36 @@ def norm(x, w, eps, residual=None, beta=None, out=None, layernorm=False, quant=F
     return (out, q, s) if quant else out
 
 
+def norm_absmax(x, w, eps, divisor: float, floor: float = 1e-12):
+    """Root-mean-square norm times w and :func:`absmax_scale` of it, in one pass where the rows allow that: (y, scale)."""
+    M, H = x.shape
+    out = torch.empty(M, H, dtype=torch.bfloat16, device=x.device)
+    if M > 0:
+        acc, scale = _absmax_words(x.device)
+        rc = lib().ksana_norm_absmax(_p(x), _p(w), _p(out), M, H, float(eps), float(divisor), float(floor), _p(acc), _p(scale), _st())
+        if rc != -100:
+            _check(rc, "ksana_norm_absmax")
+            return out, scale
+    norm(x, w, eps, out=out)
+    return out, absmax_scale(out, divisor, floor)
+
+
 _ACTS = {"silu": 0, "swiglu": 0, "gelu": 1, "gelu_new": 1, "gelu_pytorch_tanh": 1, "relu": 2}
+
+
+def act_mul_absmax(x, act, divisor: float, floor: float = 1e-12):
+    """Gated activation and :func:`absmax_scale` of it, in one pass where the rows allow that: (y, scale)."""
+    M, inter = x.shape[0], x.shape[1] // 2
+    out = torch.empty(M, inter, dtype=torch.bfloat16, device=x.device)
+    if M > 0:
+        acc, scale = _absmax_words(x.device)
+        rc = lib().ksana_act_mul_absmax(_p(x), _p(out), M, inter, x.stride(0), _ACTS[act], float(divisor), float(floor), _p(acc), _p(scale),
+                                        _st())
+        if rc != -100:
+            _check(rc, "ksana_act_mul_absmax")
+            return out, scale
+    act_mul(x, act, True, out=out)
+    return out, absmax_scale(out, divisor, floor)
 
 
 def act_mul(x, act="silu", gated=True, out=None, quant=False, q=None, s=None, want_out=True, tile_rows=None):

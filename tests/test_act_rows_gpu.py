@@ -44,3 +44,31 @@ def test_norm_rows(M, H):
         assert torch.equal(out, y)
         for a, b in ((q, s), (q2, s2)):
             assert torch.equal(a.view(torch.uint8).cpu(), rq.view(torch.uint8)) and torch.equal(b[:, :M].cpu(), rs[:, :M])
+
+
+@pytest.mark.parametrize("M,H", [(1, 4096), (7, 16), (700, 8192), (3, 24), (5, 16400)])
+def test_norm_with_largest_magnitude(M, H):
+    """The pass that also takes the result's largest magnitude: bits and scale of one pass after the other; NaN do not count."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.empty(M, H, device="cuda", dtype=torch.bfloat16).normal_(generator=g)
+    w = torch.empty(H, device="cuda", dtype=torch.bfloat16).normal_(generator=g)
+    x[M - 1, H - 1] = 60.0
+    x[0, 0] = float("nan") if M > 1 else 1.0
+    for _ in range(2):
+        y, scale = native.norm_absmax(x, w, 1e-5, 7.0)
+        want = native.norm(x, w, 1e-5)
+        assert torch.equal(y.view(torch.int16), want.view(torch.int16))
+        assert float(scale) == float(native.absmax_scale(want, 7.0)) > 0
+
+
+@pytest.mark.parametrize("M,inter,gap,act", [(1, 4096, 0, "silu"), (300, 14336, 0, "silu"), (2001, 1552, 16, "gelu"), (2000, 1544, 0, "silu")])
+def test_act_with_largest_magnitude(M, inter, gap, act):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    x = torch.empty(M, 2 * inter + gap, device="cuda", dtype=torch.bfloat16).normal_(generator=g)[:, :2 * inter]
+    x[M - 1, inter - 1], x[M - 1, 2 * inter - 1] = 9.0, -50.0
+    x[M // 2, 5] = float("nan")
+    for _ in range(2):
+        y, scale = native.act_mul_absmax(x, act, 7.0)
+        want = native.act_mul(x, act, True)
+        assert torch.equal(y.view(torch.int16), want.view(torch.int16))
+        assert float(scale) == float(native.absmax_scale(want, 7.0)) > 0
