@@ -927,8 +927,8 @@ using namespace ksana;
 // acc (may be null): also the largest magnitude of y into *acc; -100 where the kernel that does that does not take the call.
 static int norm_impl(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
                      float* yscale, int scale_ld, int M, int H, float eps, int layernorm, void* acc, cudaStream_t st) {
-  if (M <= 0) return 0;
-  if (H % 8 || H > 8 * kMaxVec * 1024) return -10;
+  if (M <= 0 || H == 0) return 0;
+  if (H < 0 || H % 8 || H > 8 * kMaxVec * 1024) return -10;
   if (yq && (H % 128)) return -11;
   // plain root-mean-square norm of aligned rows: the kernel whose CTAs stay (one row has half the barriers and wider loads: 1 x 4096 3.6 -> 2.4 us)
   if (!layernorm && !residual && !beta && H % 16 == 0 && H <= 16384 &&
@@ -998,8 +998,8 @@ extern "C" int ksana_act_mul_absmax(const void* in, void* out, int M, int I, int
 
 extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscale, int scale_ld, int M, int I,
                              int in_ld, int act, int gated, const int* tile_rows, cudaStream_t st) {
-  if (M <= 0) return 0;
-  if (I % 8 || in_ld % 8) return -10;
+  if (M <= 0 || I == 0) return 0;
+  if (I < 0 || I % 8 || in_ld % 8) return -10;
   if (outq && (I % 128)) return -11;
   if (act < 0 || act > 2) act = 2;
   // flat indices stay below 2^31: larger inputs go in row ranges (multiples of 128 rows, as tile_rows counts them)
@@ -1052,8 +1052,8 @@ extern "C" int ksana_act_mul_f32(const float* in, float* out, int M, int I, int 
 
 extern "C" int ksana_quant_fp8(const void* x, void* q, float* scale, int scale_ld, int M, int K, int x_ld,
                                cudaStream_t st) {
-  if (M <= 0) return 0;
-  if (K % 128 || x_ld % 8) return -10;
+  if (M <= 0 || K == 0) return 0;
+  if (K < 0 || K % 128 || x_ld % 8) return -10;
   const int nvec = K >> 3;
   const FastDiv div = make_fast_div(nvec);
   const int most = static_cast<int>(((1LL << 31) - 1) / nvec);
@@ -1078,10 +1078,9 @@ extern "C" int ksana_quant_fp8(const void* x, void* q, float* scale, int scale_l
 // x [M, K] bf16 -> q [M, K/2] packed e2m1, bs [M, K/16] e4m3 block scales; ts: device fp32 tensor scale (null = 1).
 extern "C" int ksana_quant_nvfp4(const void* x, int x_ld, void* q, int q_ld, void* bs, int bs_ld, const float* ts, int M,
                                  int K, cudaStream_t st) {
-  if (M <= 0) return 0;
-  if (K % 16 || x_ld % 8 || q_ld % 8) return -10;
+  if (M <= 0 || K == 0) return 0;
+  if (K < 0 || K % 16 || x_ld % 8 || q_ld % 8) return -10;
   const int nb = K >> 4, most = static_cast<int>((1LL << 30) / nb);       // (flat indices stay below 2^31, a step beyond the end included)
-  if (most < 1) return -10;
   for (int m0 = 0; m0 < M; m0 += most) {
     const uint32_t total = static_cast<uint32_t>(M - m0 < most ? M - m0 : most) * nb;
     quant_nvfp4_kernel<<<grid_for(total, 256), 256, 0, st>>>((const bf16*)x + static_cast<size_t>(m0) * x_ld, x_ld,
@@ -1119,7 +1118,7 @@ extern "C" int ksana_rope_kv_append(void* qkv, const int* positions, int pos_str
                                     const float* cos_sin, void* cache, long long block_stride, int block_tokens, int T,
                                     int Hq, int Hkv, int D, int rot_dim, int neox, int mrope_s0, int mrope_s1,
                                     int cache_fp8, float k_scale, float v_scale, int apply_rope, cudaStream_t st) {
-  if (T <= 0) return 0;
+  if (T <= 0 || D == 0 || Hq + 2 * Hkv == 0) return 0;
   if (neox && rot_dim == D && (D % 16) == 0 && pos_stride == 0 && (block_stride % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(qkv) % 16) == 0 && (reinterpret_cast<uintptr_t>(cache) % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(cos_sin) % 16) == 0) {
