@@ -212,18 +212,21 @@ __device__ __forceinline__ float group8_absmax(const Chunk16& c) {
   const float2 f = __bfloat1622float2(m);
   return fmaxf(f.x, f.y);
 }
-// Largest magnitude of what a CTA (up to 8 warps) stored, into *acc (zero or the largest so far, as bits); NaN do not count.
-__device__ __forceinline__ void publish_absmax(__nv_bfloat162 m, unsigned int* acc) {
+// Largest of the threads' magnitudes m (up to 8 warps), at the CTA's place of `parts`; NaN do not count.
+__device__ __forceinline__ void publish_absmax(float m, float* parts) {
   __shared__ float red[8];
-  const float2 f = __bfloat1622float2(m);
-  const float w = warp_max(fmaxf(f.x, f.y));
+  const float w = warp_max(m);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = w;
   __syncthreads();
   if (threadIdx.x == 0) {
     float all = red[0];
     for (int k = 1; k < static_cast<int>(blockDim.x >> 5); ++k) all = fmaxf(all, red[k]);
-    if (all > 0.f) atomicMax(acc, __float_as_uint(all));
+    parts[blockIdx.x] = all;
   }
+}
+__device__ __forceinline__ float larger(__nv_bfloat162 m) {
+  const float2 f = __bfloat1622float2(m);
+  return fmaxf(f.x, f.y);
 }
 __device__ __forceinline__ __nv_bfloat162 chunk_absmax(const Chunk16& c, __nv_bfloat162 m) {
 #pragma unroll
@@ -249,11 +252,11 @@ __device__ __forceinline__ uint4 chunk_e4m3(const Chunk16& c, float inv) {
 // Root-mean-square norm: CTAs stay and take row after row, the next row's loads in flight under the work on this one. One CTA per row
 // (norm_kernel) spent its time waiting and on 21.6 instructions an element. us, there / here: with fp8 copy 16384 x 8192 122 / 74 (5.5 TB/s),
 // 8000 x 7168 60 / 39, 300 x 7168 5.7 / 4.2; 16384 x 4096 56 / 43, 64 x 4096 3.9 / 2.6. V chunks per thread.
-// AMAX: *acc takes the largest magnitude of the result (the tensor scale of an NVFP4 operand without a pass of its own).
+// AMAX: parts[CTA] takes the largest magnitude of its results (the tensor scale of an NVFP4 operand without a pass of its own).
 template <bool QUANT, int V, bool AMAX>
 __global__ void __launch_bounds__(256, V == 1 ? 4 : V == 2 ? 3 : 2)
 norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* __restrict__ y, uint8_t* __restrict__ yq,
-                 float* __restrict__ yscale, int scale_ld, int M, int H, float eps, unsigned int* acc) {
+                 float* __restrict__ yscale, int scale_ld, int M, int H, float eps, float* parts) {
   pdl_trigger();
   pdl_wait();
   __shared__ float red[2][8];
@@ -311,7 +314,7 @@ norm_rows_kernel(const bf16* __restrict__ x, const bf16* __restrict__ w, bf16* _
       }
     }
   }
-  if constexpr (AMAX) publish_absmax(top, acc);
+  if constexpr (AMAX) publish_absmax(larger(top), parts);
 }
 
 // ----------------------------------------------------------------------------
@@ -394,7 +397,7 @@ act_mul_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __r
 template <int ACT, bool QUANT, bool AMAX>
 __global__ void __launch_bounds__(256)
 act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* __restrict__ outq, float* __restrict__ oscale, int scale_ld,
-                  uint32_t total, FastDiv nchunk, int in_ld, const int* __restrict__ tile_rows, unsigned int* acc) {
+                  uint32_t total, FastDiv nchunk, int in_ld, const int* __restrict__ tile_rows, float* parts) {
   pdl_trigger();
   pdl_wait();
   const uint32_t step = gridDim.x * blockDim.x, I = nchunk.d * 16;
@@ -435,7 +438,7 @@ act_chunks_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, uint8_t* 
       st_global_32(out + static_cast<size_t>(m) * I + i * 16, make_uint4(o.w[0], o.w[1], o.w[2], o.w[3]), make_uint4(o.w[4], o.w[5], o.w[6], o.w[7]));
     }
   }
-  if constexpr (AMAX) publish_absmax(top, acc);
+  if constexpr (AMAX) publish_absmax(larger(top), parts);
 }
 
 // The same on fp32 rows, with the exponential instead of the approximate tanh.
@@ -766,11 +769,9 @@ __global__ void rerotate_blocks_kernel(T* __restrict__ cache, const int* __restr
 }
 
 // Largest magnitude of a bf16 matrix as a quantisation scale on the device: scale = max(|x|) / divisor (at least
-// `floor`), without a host round trip and without a widened copy of x. `acc` is a zeroed 32-bit word; magnitudes are
-// non-negative, so their bit patterns order like integers and atomicMax works on them. The finishing kernel writes the
-// scale and leaves `acc` at zero for the next call.
-__global__ void absmax_kernel(const bf16* __restrict__ x, int rows, int cols, long long ldx, unsigned int* acc) {
-  __shared__ float red[32];
+// `floor`), without a host round trip and without a widened copy of x. Every CTA leaves its own maximum in `parts`, which the
+// finishing kernel reads: scratch of one call, so that calls on several streams have nothing in common.
+__global__ void __launch_bounds__(256) absmax_kernel(const bf16* __restrict__ x, int rows, int cols, long long ldx, float* parts) {
   const int vec_per_row = cols >> 3;
   const long long nvec = static_cast<long long>(rows) * vec_per_row;
   float m = 0.f;
@@ -786,19 +787,10 @@ __global__ void absmax_kernel(const bf16* __restrict__ x, int rows, int cols, lo
       m = fmaxf(m, fmaxf(fabsf(f.x), fabsf(f.y)));
     }
   }
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
-  __syncthreads();
-  if (threadIdx.x < 32) {
-    m = threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-    if (threadIdx.x == 0 && m > 0.f && m == m) atomicMax(acc, __float_as_uint(m));
-  }
+  publish_absmax(m, parts);
 }
 // The same in chunks of 16 elements, four in flight a thread, maxima on packed pairs (by: chunks of a row): 9753 x 14336 53 -> 44 us, x 4096 19.8 -> 16.5.
-__global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restrict__ x, uint32_t total, FastDiv by, long long ldx, unsigned int* acc) {
+__global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restrict__ x, uint32_t total, FastDiv by, long long ldx, float* parts) {
   const uint32_t step = gridDim.x * blockDim.x;
   __nv_bfloat162 m = __floats2bfloat162_rn(0.f, 0.f);
   for (uint32_t base = blockIdx.x * blockDim.x + threadIdx.x; base < total; base += 4 * step) {
@@ -814,11 +806,20 @@ __global__ void __launch_bounds__(256) absmax_chunks_kernel(const bf16* __restri
 #pragma unroll
     for (int k = 0; k < 4; ++k) m = chunk_absmax(c[k], m);
   }
-  publish_absmax(m, acc);
+  publish_absmax(larger(m), parts);
 }
-__global__ void absmax_finish_kernel(unsigned int* acc, float* scale, float inv_divisor, float floor_value) {
-  *scale = fmaxf(__uint_as_float(*acc) * inv_divisor, floor_value);
-  *acc = 0u;
+// One CTA: n maxima to the scale. (One thread that read one word took as long as the 1184 values of a full launch do here, about 2 us.)
+__global__ void absmax_finish_kernel(const float* __restrict__ parts, int n, float* scale, float inv_divisor, float floor_value) {
+  __shared__ float red[32];
+  float m = 0.f;
+  for (int i = threadIdx.x; i < n; i += blockDim.x) m = fmaxf(m, parts[i]);
+  m = warp_max(m);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = m;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    m = warp_max(threadIdx.x < (blockDim.x >> 5) ? red[threadIdx.x] : 0.f);
+    if (threadIdx.x == 0) *scale = fmaxf(m * inv_divisor, floor_value);
+  }
 }
 
 // ids[rows[i]] = prev_tokens[src[i]]: a pipelined step takes the input ids of its decode rows straight from the
@@ -924,9 +925,10 @@ __global__ void quant_nvfp4_kernel(const bf16* __restrict__ x, int ldx, uint8_t*
 
 using namespace ksana;
 
-// acc (may be null): also the largest magnitude of y into *acc; -100 where the kernel that does that does not take the call.
+// parts (may be null, nparts places): also the largest magnitude of y by CTA, nparts becoming their number; -100 where the kernel that does
+// that does not take the call.
 static int norm_impl(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
-                     float* yscale, int scale_ld, int M, int H, float eps, int layernorm, void* acc, cudaStream_t st) {
+                     float* yscale, int scale_ld, int M, int H, float eps, int layernorm, float* parts, int* nparts, cudaStream_t st) {
   if (M <= 0 || H == 0) return 0;
   if (H < 0 || H % 8 || H > 8 * kMaxVec * 1024) return -10;
   if (yq && (H % 128)) return -11;
@@ -938,16 +940,18 @@ static int norm_impl(const void* x, void* residual, const void* w, const void* b
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     const int chunks = H / 16, v = chunks <= 256 ? 1 : chunks <= 512 ? 2 : 4;
     const int threads = ((chunks + v - 1) / v + 31) / 32 * 32, per_sm = (v == 1 ? 4 : v == 2 ? 3 : 2) * (256 / threads > 1 ? 256 / threads : 1);
-    const dim3 grid(M < sms * per_sm ? M : sms * per_sm);
+    int ctas = M < sms * per_sm ? M : sms * per_sm;
+    if (parts) *nparts = ctas = ctas < *nparts ? ctas : *nparts;
+    const dim3 grid(ctas);
 #define KSANA_NORM_ROWS(Q, V, A) launch_early(norm_rows_kernel<Q, V, A>, grid, dim3(threads), 0, st, (const bf16*)x, (const bf16*)w, (bf16*)y, \
-                                              (uint8_t*)yq, yscale, scale_ld, M, H, eps, static_cast<unsigned int*>(acc))
-    if (acc) v == 1 ? KSANA_NORM_ROWS(false, 1, true) : v == 2 ? KSANA_NORM_ROWS(false, 2, true) : KSANA_NORM_ROWS(false, 4, true);
+                                              (uint8_t*)yq, yscale, scale_ld, M, H, eps, parts)
+    if (parts) v == 1 ? KSANA_NORM_ROWS(false, 1, true) : v == 2 ? KSANA_NORM_ROWS(false, 2, true) : KSANA_NORM_ROWS(false, 4, true);
     else if (yq) v == 1 ? KSANA_NORM_ROWS(true, 1, false) : v == 2 ? KSANA_NORM_ROWS(true, 2, false) : KSANA_NORM_ROWS(true, 4, false);
     else v == 1 ? KSANA_NORM_ROWS(false, 1, false) : v == 2 ? KSANA_NORM_ROWS(false, 2, false) : KSANA_NORM_ROWS(false, 4, false);
 #undef KSANA_NORM_ROWS
     return cudaGetLastError() == cudaSuccess ? 0 : -4;
   }
-  if (acc) return -100;
+  if (parts) return -100;
   const int threads = norm_threads(H);
 #define KSANA_NORM(MODE, RES, Q) launch_early(norm_kernel<MODE, RES, Q>, dim3(M), dim3(threads), 0, st, (const bf16*)x, (bf16*)residual, \
                                               (const bf16*)w, (const bf16*)beta, (bf16*)y, (uint8_t*)yq, yscale, scale_ld, H, eps)
@@ -961,39 +965,43 @@ static int norm_impl(const void* x, void* residual, const void* w, const void* b
 
 extern "C" int ksana_norm(const void* x, void* residual, const void* w, const void* beta, void* y, void* yq,
                           float* yscale, int scale_ld, int M, int H, float eps, int layernorm, cudaStream_t st) {
-  return norm_impl(x, residual, w, beta, y, yq, yscale, scale_ld, M, H, eps, layernorm, nullptr, st);
+  return norm_impl(x, residual, w, beta, y, yq, yscale, scale_ld, M, H, eps, layernorm, nullptr, nullptr, st);
 }
 
-// y = the root-mean-square norm of x times w, and *scale = max(largest |y| / divisor, floor_value); acc: a zero word, zero again afterwards.
-// Read again for that, 9753 x 4096 cost 16.5 us and x 14336 44 us; a 4096-wide NVFP4 layer's prefill of 9753 rows with head 2276 -> 2231 us.
-// -100: not covered (rows off 32-byte boundaries, H no multiple of 16 or above 16384): norm and largest magnitude one after the other do it.
-extern "C" int ksana_norm_absmax(const void* x, const void* w, void* y, int M, int H, float eps, float divisor, float floor_value, void* acc,
-                                 float* scale, cudaStream_t st) {
-  if (M <= 0 || divisor <= 0.f || !acc || !scale) return -10;
-  const int rc = norm_impl(x, nullptr, w, nullptr, y, nullptr, nullptr, 0, M, H, eps, 0, acc, st);
-  if (rc) return rc;
-  absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
+static int finish_absmax(const float* parts, int n, float* scale, float divisor, float floor_value, cudaStream_t st) {
+  absmax_finish_kernel<<<1, n > 512 ? 1024 : (n + 31) / 32 * 32, 0, st>>>(parts, n, scale, 1.f / divisor, floor_value);
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
+// y = the root-mean-square norm of x times w, and *scale = max(largest |y| / divisor, floor_value); parts: scratch of this call, nparts > 0
+// places. Read again for that, 9753 x 4096 cost 16.5 us and x 14336 44 us; a 4096-wide NVFP4 layer's prefill of 9753 rows with head 2276 ->
+// 2231 us. -100: not covered (rows off 32-byte boundaries, H no multiple of 16 or above 16384): norm and largest magnitude one after the
+// other do it.
+extern "C" int ksana_norm_absmax(const void* x, const void* w, void* y, int M, int H, float eps, float divisor, float floor_value, float* parts,
+                                 int nparts, float* scale, cudaStream_t st) {
+  if (M <= 0 || divisor <= 0.f || !parts || nparts <= 0 || !scale) return -10;
+  if (H <= 0) return -100;
+  const int rc = norm_impl(x, nullptr, w, nullptr, y, nullptr, nullptr, 0, M, H, eps, 0, parts, &nparts, st);
+  return rc ? rc : finish_absmax(parts, nparts, scale, divisor, floor_value, st);
+}
+
 // out = act(gate) * up of packed rows and the scale of its largest magnitude, as above. -100: not covered (small launches, no whole chunks).
-extern "C" int ksana_act_mul_absmax(const void* in, void* out, int M, int I, int in_ld, int act, float divisor, float floor_value, void* acc,
-                                    float* scale, cudaStream_t st) {
-  if (M <= 0 || divisor <= 0.f || !acc || !scale) return -10;
+extern "C" int ksana_act_mul_absmax(const void* in, void* out, int M, int I, int in_ld, int act, float divisor, float floor_value, float* parts,
+                                    int nparts, float* scale, cudaStream_t st) {
+  if (M <= 0 || divisor <= 0.f || !parts || nparts <= 0 || !scale) return -10;
   const long long total = static_cast<long long>(M) * (I >> 3);
   if (I % 16 || in_ld % 16 || !chunks_pay(total) || total >= (1LL << 31) || ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 31))
     return -100;
   const FastDiv by = make_fast_div(I / 16);
-  const dim3 grid(grid_for(total / 2, 256));
+  const dim3 grid(grid_for(total / 2, 256, nparts < 148 * 8 ? nparts : 148 * 8));
 #define KSANA_ACT_AMAX(A) launch_early(act_chunks_kernel<A, false, true>, grid, dim3(256), 0, st, (const bf16*)in, (bf16*)out, \
                                        static_cast<uint8_t*>(nullptr), static_cast<float*>(nullptr), 0, static_cast<uint32_t>(total / 2), by, in_ld, \
-                                       static_cast<const int*>(nullptr), static_cast<unsigned int*>(acc))
+                                       static_cast<const int*>(nullptr), parts)
   if (act == 0) KSANA_ACT_AMAX(0);
   else if (act == 1) KSANA_ACT_AMAX(1);
   else KSANA_ACT_AMAX(2);
 #undef KSANA_ACT_AMAX
-  absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  return finish_absmax(parts, grid.x, scale, divisor, floor_value, st);
 }
 
 extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscale, int scale_ld, int M, int I,
@@ -1020,7 +1028,7 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
       const FastDiv by = make_fast_div(I / 16);
       const dim3 chunk_grid(grid_for(total / 2, 256));
 #define KSANA_ACT16(A, Q) launch_early(act_chunks_kernel<A, Q, false>, chunk_grid, dim3(256), 0, st, src, dst, dq, ds, scale_ld, total / 2, by, in_ld, tr, \
-                                          static_cast<unsigned int*>(nullptr))
+                                          static_cast<float*>(nullptr))
       if (act == 0) dq ? KSANA_ACT16(0, true) : KSANA_ACT16(0, false);
       else if (act == 1) dq ? KSANA_ACT16(1, true) : KSANA_ACT16(1, false);
       else dq ? KSANA_ACT16(2, true) : KSANA_ACT16(2, false);
@@ -1178,20 +1186,23 @@ extern "C" int ksana_rerotate_blocks(void* cache, const int* triples, int n, con
   return cudaGetLastError() == cudaSuccess ? 0 : -4;
 }
 
-// scale[0] = max(max |x| / divisor, floor) for x [rows, cols] bf16 (row stride ldx, cols a multiple of 8); acc: one
-// zeroed 32-bit word of device scratch that the call leaves zeroed.
+// scale[0] = max(max |x| / divisor, floor) for x [rows, cols] bf16 (row stride ldx, cols a multiple of 8); parts:
+// scratch of this call, nparts > 0 places.
 extern "C" int ksana_absmax_scale(const void* x, int rows, int cols, long long ldx, float divisor, float floor_value,
-                                  void* acc, float* scale, cudaStream_t st) {
+                                  float* parts, int nparts, float* scale, cudaStream_t st) {
   if (rows <= 0 || cols <= 0) return 0;
-  if ((cols % 8) || (ldx % 8) || divisor <= 0.f || (reinterpret_cast<uintptr_t>(x) & 15)) return -10;
+  if ((cols % 8) || (ldx % 8) || divisor <= 0.f || !parts || nparts <= 0 || (reinterpret_cast<uintptr_t>(x) & 15)) return -10;
   const long long nvec = static_cast<long long>(rows) * (cols >> 3);
-  if (cols % 16 == 0 && ldx % 16 == 0 && !(reinterpret_cast<uintptr_t>(x) & 31) && nvec / 2 < (1LL << 30))
-    absmax_chunks_kernel<<<grid_for(nvec / 2, 256), 256, 0, st>>>((const bf16*)x, static_cast<uint32_t>(nvec / 2), make_fast_div(cols / 16),
-                                                                  ldx, (unsigned int*)acc);
-  else
-    absmax_kernel<<<grid_for(nvec, 256), 256, 0, st>>>((const bf16*)x, rows, cols, ldx, (unsigned int*)acc);
-  absmax_finish_kernel<<<1, 1, 0, st>>>((unsigned int*)acc, scale, 1.f / divisor, floor_value);
-  return cudaGetLastError() == cudaSuccess ? 0 : -4;
+  const int cap = nparts < 148 * 8 ? nparts : 148 * 8;
+  int ctas;
+  if (cols % 16 == 0 && ldx % 16 == 0 && !(reinterpret_cast<uintptr_t>(x) & 31) && nvec / 2 < (1LL << 30)) {
+    ctas = grid_for(nvec / 2, 256, cap);
+    absmax_chunks_kernel<<<ctas, 256, 0, st>>>((const bf16*)x, static_cast<uint32_t>(nvec / 2), make_fast_div(cols / 16), ldx, parts);
+  } else {
+    ctas = grid_for(nvec, 256, cap);
+    absmax_kernel<<<ctas, 256, 0, st>>>((const bf16*)x, rows, cols, ldx, parts);
+  }
+  return finish_absmax(parts, ctas, scale, divisor, floor_value, st);
 }
 
 extern "C" int ksana_patch_ids(int* ids, const int* rows, const int* src, const int* prev_tokens, int n, int n_ids,

@@ -69,9 +69,9 @@ _SIGS = {
     "ksana_add": [vp, vp, vp, vp, i64, i32, vp],
     "ksana_patch_ids": [vp, vp, vp, vp, i32, i32, i32, vp, vp],
     "ksana_smallm_estimate": [i32, i32, i32, i32, vp],
-    "ksana_norm_absmax": [vp, vp, vp, i32, i32, f32, f32, f32, vp, vp, vp],
-    "ksana_act_mul_absmax": [vp, vp, i32, i32, i32, i32, f32, f32, vp, vp, vp],
-    "ksana_absmax_scale": [vp, i32, i32, i64, f32, f32, vp, vp, vp],
+    "ksana_norm_absmax": [vp, vp, vp, i32, i32, f32, f32, f32, vp, i32, vp, vp],
+    "ksana_act_mul_absmax": [vp, vp, i32, i32, i32, i32, f32, f32, vp, i32, vp, vp],
+    "ksana_absmax_scale": [vp, i32, i32, i64, f32, f32, vp, i32, vp, vp],
     "ksana_rerotate_blocks": [vp, vp, i32, vp, i32, i32, i32, i32, i32, i32, i32, i32, i32, i64, vp, vp],
     "ksana_embed_pair": [vp, vp, vp, vp, vp, vp, i32, i32, i32, i32, i64, i64, i64, f32, i32, vp, vp],
     "ksana_residual_norm": [vp, i32, vp, i32, vp, i32, vp, vp, vp, vp, vp, vp, vp, i32, i32, i32, f32, i32, i32, f32, i32, vp, vp, f32,
@@ -513,23 +513,17 @@ def gemm_fp8(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=None, b
     return dst
 
 
-_absmax_acc = {}
-
-
-def _absmax_words(device):
-    """(the device's word for a largest magnitude, zero between launches; a new scalar for the scale)"""
-    key = (device.type, device.index)
-    if key not in _absmax_acc:
-        _absmax_acc[key] = torch.zeros(1, dtype=torch.int32, device=device)
-    return _absmax_acc[key], torch.empty((), dtype=torch.float32, device=device)
+def _absmax_room(device):
+    """(places for the CTAs' largest magnitudes, a new scalar for the scale), of one call: other streams and threads have their own"""
+    return torch.empty(32 * _sms(device), dtype=torch.float32, device=device), torch.empty((), dtype=torch.float32, device=device)
 
 
 def absmax_scale(x, divisor: float, floor: float = 1e-12):
     """max(|x|) / divisor (at least ``floor``) of a bf16 matrix as an fp32 scalar tensor on the device: the tensor
     scale of an NVFP4 activation, without a host round trip or a widened copy of ``x``."""
     rows, cols = x.shape
-    acc, scale = _absmax_words(x.device)
-    _check(lib().ksana_absmax_scale(_p(x), rows, cols, x.stride(0), float(divisor), float(floor), _p(acc), _p(scale),
+    parts, scale = _absmax_room(x.device)
+    _check(lib().ksana_absmax_scale(_p(x), rows, cols, x.stride(0), float(divisor), float(floor), _p(parts), parts.numel(), _p(scale),
                                     _st()), "ksana_absmax_scale")
     return scale
 
@@ -675,8 +669,9 @@ def norm_absmax(x, w, eps, divisor: float, floor: float = 1e-12):
     M, H = x.shape
     out = torch.empty(M, H, dtype=torch.bfloat16, device=x.device)
     if M > 0:
-        acc, scale = _absmax_words(x.device)
-        rc = lib().ksana_norm_absmax(_p(x), _p(w), _p(out), M, H, float(eps), float(divisor), float(floor), _p(acc), _p(scale), _st())
+        parts, scale = _absmax_room(x.device)
+        rc = lib().ksana_norm_absmax(_p(x), _p(w), _p(out), M, H, float(eps), float(divisor), float(floor), _p(parts), parts.numel(),
+                                     _p(scale), _st())
         if rc != -100:
             _check(rc, "ksana_norm_absmax")
             return out, scale
@@ -692,9 +687,9 @@ def act_mul_absmax(x, act, divisor: float, floor: float = 1e-12):
     M, inter = x.shape[0], x.shape[1] // 2
     out = torch.empty(M, inter, dtype=torch.bfloat16, device=x.device)
     if M > 0:
-        acc, scale = _absmax_words(x.device)
-        rc = lib().ksana_act_mul_absmax(_p(x), _p(out), M, inter, x.stride(0), _ACTS[act], float(divisor), float(floor), _p(acc), _p(scale),
-                                        _st())
+        parts, scale = _absmax_room(x.device)
+        rc = lib().ksana_act_mul_absmax(_p(x), _p(out), M, inter, x.stride(0), _ACTS[act], float(divisor), float(floor), _p(parts),
+                                        parts.numel(), _p(scale), _st())
         if rc != -100:
             _check(rc, "ksana_act_mul_absmax")
             return out, scale
