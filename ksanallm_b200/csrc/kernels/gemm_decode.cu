@@ -193,7 +193,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       }
       mbar_arrive(xs_ready);
     }
-    ok = mbar_wait(done_bar, 0, abort_flag);
+    ok = mbar_wait_all(done_bar, 0, abort_flag);
     if (ok) {
       tc_fence_after();
       const uint32_t at = tmem_base + (static_cast<uint32_t>(q * 32) << 16);
@@ -239,7 +239,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
       int wbase = -1000000, sfs = 0; uint32_t sf_phase = 0;
       wbase = kb0;
       wexp = kb0 + lane < kb1 ? ue8m0_of(ws[kb0 + lane]) : 127u;
-      ok = mbar_wait(xs_ready, 0, abort_flag);
+      ok = mbar_wait_all(xs_ready, 0, abort_flag);
       for (int g0 = kb0; g0 < kb1 && ok; g0 += 4) {
         if (g0 + 4 > wbase + 32) {
           wbase = g0;
@@ -258,7 +258,7 @@ gemm_decode_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             word |= static_cast<uint32_t>(tok < MP && g0 + j < kb1 ? xs_tab[(g0 + j - kb0) * MP + tok] : 127) << (8 * j);
           w[r4] = word;
         }
-        if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_all(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) { ok = false; break; }
         uint8_t* buf = sf_smem + sfs * 1024;
         *reinterpret_cast<uint4*>(buf + lane * 16) = make_uint4(w0, w0, w0, w0);
         *reinterpret_cast<uint4*>(buf + 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);

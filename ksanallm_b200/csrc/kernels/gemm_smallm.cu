@@ -591,7 +591,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
             }
             w[r4] = word;
           }
-          { const long long pt_ = prof_clock(); if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) { ok = false; break; } KSANA_PROF_ADD(4, pt_); }
+          { const long long pt_ = prof_clock(); if (!mbar_wait_all(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) { ok = false; break; } KSANA_PROF_ADD(4, pt_); }
           uint8_t* buf = sf_smem + sfs * 1024;
           *reinterpret_cast<uint4*>(buf + lane * 16) = make_uint4(w0, w0, w0, w0);
           *reinterpret_cast<uint4*>(buf + 512 + lane * 16) = make_uint4(w[0], w[1], w[2], w[3]);
@@ -651,7 +651,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
       for (int i = 0; i < MP; ++i) accv[i] = 0.f;
       if (KIND != 1) {
-        { const long long pt_ = prof_clock(); if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; } KSANA_PROF_ADD(5, pt_); }
+        { const long long pt_ = prof_clock(); if (!mbar_wait_all(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; } KSANA_PROF_ADD(5, pt_); }
         tc_fence_after();
         if constexpr (MP >= 32) {
 #pragma unroll
@@ -694,7 +694,7 @@ gemm_smallm_kernel(const __grid_constant__ CUtensorMap tma_w, const __grid_const
 #pragma unroll
           for (int j = 0; j < NS; ++j) s_cur[j] = s_next[j];
           if (kb + 1 < sg.kb1) fetch(kb + 1, s_next);
-          if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_all(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
           if constexpr (MP >= 32) {
 #pragma unroll

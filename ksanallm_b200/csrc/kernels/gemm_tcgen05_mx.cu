@@ -265,7 +265,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     // rows past M, column blocks past N and K blocks past the end repeat the last valid scale: what they scale
     // is zero-filled by TMA or never stored
     auto emit = [&](const Raw& r) -> bool {
-      if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
+      if (!mbar_wait_all(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
       uint8_t* buf = sf_smem + sfs * Cfg::kSfStageBytes;
       uint32_t w[4];
 #pragma unroll
@@ -329,7 +329,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
       const int n0 = n_blk * BN + col_off;
       if (p.tile_expert && p.tile_expert[m_blk] < 0) continue;
       const bool row_ok = row < p.M && (!p.tile_rows || q * 32 + lane < p.tile_rows[m_blk]);
-      if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_all(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[EC];
 #pragma unroll

@@ -271,7 +271,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     // rows past M, column blocks past N and K blocks past the end repeat the last valid scale: what they scale
     // is zero-filled by TMA or never stored
     auto emit = [&](const Raw& r) -> bool {
-      if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
+      if (!mbar_wait_all(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
       uint8_t* buf = sf_smem + sfs * kMpSfStageBytes;
       uint32_t w[4];
 #pragma unroll
@@ -330,7 +330,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
       const int row = m_blk * 256 + static_cast<int>(rank) * 128 + q * 32 + lane;
       const int n0 = n_blk * kMpBN + col_off;
       const bool row_ok = row < p.M;
-      if (!mbar_wait(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_all(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       uint32_t r[EC];
 #pragma unroll

@@ -216,7 +216,7 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     // rows past M, column blocks past N and K blocks past the end repeat the last valid scale: what they scale
     // is zero-filled by TMA or never stored
     auto emit = [&](const Raw& r) -> bool {
-      if (!mbar_wait(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
+      if (!mbar_wait_all(&sf_empty[sfs], sf_phase ^ 1, abort_flag)) return false;
       uint8_t* buf = sf_smem + sfs * kTlSfStageBytes;
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
@@ -286,7 +286,7 @@ gemm_mxfp8_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
       tl_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
       const int row = m_blk * kTlBM + h * 128 + q * 32 + lane;
       const bool row_ok = row < p.M;
-      if (!mbar_wait(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_all(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       acc_phase ^= 1;
       if (plain) {

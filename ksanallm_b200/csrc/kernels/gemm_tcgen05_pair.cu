@@ -303,13 +303,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
       };
       const uint32_t tempty_leader_base = map_to_cta(smem_u32(&tempty_bar[0]), 0);
       if (KIND == 0) {
-        if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+        if (!mbar_wait_all(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
         tc_fence_after();
 #pragma unroll
         for (int c0 = 0; c0 < 128; c0 += 32) {
           if (c0 >= cols) break;
           uint32_t r[32];
-          __syncwarp();                             // (rows without a place to store skip the chunk before)
           tmem_ld32(tmem_base + lane_base + acc * kPairBN + col_off + c0, r);
           tmem_ld_wait();
           float v[32];
@@ -325,7 +324,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
         const float* ws = p.w_scale + static_cast<size_t>(min(n0 / 128, (p.N + 127) / 128 - 1)) * nkb_scale;
         for (int kb = 0; kb < num_kb; ++kb) {
           const float s = (row_ok ? p.a_scale[static_cast<size_t>(kb) * p.a_scale_ld + row] : 0.f) * ws[kb];
-          if (!mbar_wait(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
+          if (!mbar_wait_all(&tfull_bar[acc], acc_phase, abort_flag)) { ok = false; break; }
           tc_fence_after();
 #pragma unroll
           for (int c0 = 0; c0 < 128; c0 += 32) {

@@ -148,7 +148,7 @@ gemm_bf16_tall_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       bt_tile_coords(tile, m_tiles, n_tiles, m_blk, n_blk);
       const int row = m_blk * kBtBM + h * 128 + q * 32 + lane;
       const bool row_ok = row < p.M;
-      if (!mbar_wait(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
+      if (!mbar_wait_all(tfull_bar, acc_phase, abort_flag)) { ok = false; break; }
       tc_fence_after();
       acc_phase ^= 1;
 #pragma unroll 1

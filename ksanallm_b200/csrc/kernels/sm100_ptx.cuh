@@ -215,6 +215,11 @@ __device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, u
   *abort_flag = 1;
   return false;
 }
+// mbar_wait by every lane of a warp, with one answer for all: where some lanes gave up and others did not, the latter would go on to an
+// instruction that waits for the whole warp.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
+}
 // Non-blocking probe of a phase by a whole warp.
 __device__ __forceinline__ bool mbar_test_warp(uint64_t* bar, uint32_t parity, uint32_t lead) {
   uint32_t done;
@@ -234,8 +239,10 @@ __device__ __forceinline__ void mbar_arrive_lead(uint32_t lead, uint64_t* bar) {
       "@e mbarrier.arrive.shared::cta.b64 _, [%0];\n\t}\n" ::"r"(smem_u32(bar)), "r"(lead) : "memory");
 }
 
-// TMEM -> registers: this warp's 32 lanes x 32 consecutive fp32 columns.
+// TMEM -> registers: this warp's 32 lanes x 32 consecutive fp32 columns. Every access converges its warp first (.sync.aligned wants all lanes
+// at one instruction): lanes without a row to store come from another path than their neighbours, and the compiler need not join them.
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
@@ -247,6 +254,7 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
       : "r"(taddr) : "memory");
 }
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
@@ -278,6 +286,7 @@ __host__ __device__ constexpr uint32_t make_idesc(uint32_t m, uint32_t n, uint32
 
 // Registers -> TMEM: this warp's 32 lanes x N consecutive 32-bit columns.
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "
@@ -289,6 +298,7 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32
       : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16]) {
+  __syncwarp();
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
       "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};"
