@@ -1018,16 +1018,26 @@ def _sigmoid_args(weights: Optional[SigmoidWeights]):
 def prefill_pair_wins(pairs, rows, B, Hq, Hkv, sms=148) -> bool:
     """Whether prompts take the attention kernel with two query tiles per CTA, from the (query, visible key) pairs and the rows of a
     batch. A tile of 128 keys costs it half, a CTA more (about 4 us: two tiles' queries, all of TMEM), and only half as many fit the machine.
-    us with one / two, 32/8 heads of 128: one prompt of 200 tokens 12.8 / 13.4, 1024 38 / 24.5, 2000 108 / 62; 64 x 33 31.3 / 31.8, 13 x 300
-    65 / 51, 4 x 700 56 / 38, 40 x 60 on 300 cached tokens 64 / 50, 24 x 150 on 200 82 / 61, 32 x 150 on 2000 394 / 222; 28/4 heads, 24 x 150
-    on 200 64 / 52. Two pay from 160 keys per row on (a fifth less time; below it is a few percent, and none for a few dozen keys). While all
-    CTAs of one tile run at once (two an SM) they pay later, and groups that leave rows of a tile idle keep one."""
+    us with one / two, 32/8 heads of 128: 13 prompts of 330 tokens 64 / 55, 13 x 500 106 / 80, 1 x 1000 37.6 / 24.9, 16 x 33 on 200 cached
+    tokens 17.2 / 11.8, 32 x 150 on 200 88 / 75; 28/4 heads, 13 x 400 73 / 62. The line lies at 160 keys per row, and at 288 while all CTAs of
+    one tile run at once (two an SM); there groups that leave rows of a tile idle keep one. Two are the faster form below these lines
+    already (13 x 300 57 / 46, 1 x 512 19.1 / 16.1; 28/4 heads, 1 x 1000 37.7 / 25.2), down to about 75 keys.
+    One stays where its CTAs run at once and those of two need a second round, which costs more than the tiles save until rows see some
+    2000 keys (28/4 heads of 64, 8 x 150 on 100 14.8 / 18.5, on 800 35.6 / 41.5; 40/40, 2 x 300 on 300 30.1 / 33.8; 16/16, 6 x 300 on 800
+    45.0 / 46.8, on 2000 86 / 80), or where a whole prompt's last CTAs are short (40/40, 1 x 850 35.7 / 33.2); a few CTAs more, and it
+    stays for short rows only (64/8, 2 x 300 on 100 24.6 / 27.7, on 300 36.7 / 31.4); so it does with idle rows and two rounds against
+    three (14/2, 32 x 150 on 100 26.9 / 28.1, on 300 39.7 / 38.5)."""
     G = Hq // Hkv
     if G > 128 or B <= 0 or rows <= 0:
         return False
     keys, whole = pairs / rows, 128 % G == 0
     per = 128 // G * G                                           # rows of a tile
-    ctas = Hkv * B * -(-rows * G // (B * per))                   # of one tile each, for sequences of the mean length
+    tiles = -(-rows * G // (B * per))                            # of a sequence of the mean length
+    ctas, two = Hkv * B * tiles, Hkv * B * -(-tiles // 2)
+    if two > sms and ctas <= 2.06 * sms and keys < (256 if ctas > 2 * sms else 2000 if keys * B > 0.7 * rows else 320):
+        return False
+    if two > 2 * sms and ctas <= 4 * sms and keys < 256 and not whole:
+        return False
     if ctas < 1.55 * sms:
         return whole and keys >= 288
     return keys >= 160
