@@ -333,19 +333,29 @@ def gemm_bf16_tall(x, w, out=None, bias=None, residual=None, out_f32=None, max_c
 
 
 def _pair_wins(M, N, K, sms=148):
-    """256 x 256 tiles of CTA pairs against 128 x 256 tiles of one CTA, from measured times (in waves of pairs; graphs of a kernel, K =
-    4096): a wave of pairs takes 25 us, a last one of up to a quarter / half of them 10 / 14 (its tiles are cut); a wave of single CTAs 29, a
-    last one of up to half of them 21 (few CTAs find more of the L2's bandwidth each). us, single / pair: 700 x 28672 143 / 127, 200 x 4096
-    18.1 / 13.4, 513 x 4096 28.7 / 25.4; and where single CTAs stay: 300 x 6144 21.0 / 25.2, 1100 x 4096 29.5 / 34.5, 513 x 28672 117 / 121."""
+    """256 x 256 tiles of CTA pairs against 128-row tiles of one CTA, from measured times (in waves of pairs; graphs of a kernel, K =
+    4096): a wave of pairs takes 25 us, a last one of up to a quarter / half of them 10 / 14 (its tiles are cut); a wave of single CTAs with
+    256 columns 29, a last one of up to half of them 21 (few CTAs find more of the L2's bandwidth each). Where narrower tiles of one CTA fill
+    one wave (the kernel picks them by 400 + columns), that takes less: 128 columns 23 us; and with 32 or 64 columns and a short K what a
+    pair costs beside its products, about a microsecond, is not made up for. us, single / pair: 700 x 28672 143 / 127, 200 x 4096 18.1 /
+    13.4, 513 x 4096 28.7 / 25.4; and where single CTAs stay: 300 x 6144 21.0 / 25.2, 1100 x 4096 29.5 / 34.5, 513 x 28672 117 / 121, 2048 x
+    1152 22.3 / 26.0 (K = 14336: 61 / 76); K = 512: 384 x 1152 5.7 / 6.5, 1024 x 1152 6.5 / 7.1, but 384 x 4096 (128 columns) 8.4 / 7.4. Of
+    1080 shapes (136 to 5000 rows, 256 to 28672 columns, K of 128 to 14336) two take the slower kernel by 4 and 7 percent."""
     if N < 256 or N % 8 or K % 8:
         return False
-    cols = -(-N // 256)
-    tiles, single = -(-M // 256) * cols, -(-M // 128) * cols
+    cols, rows = -(-N // 256), -(-M // 128)
+    tiles, single = -(-M // 256) * cols, rows * cols
     if tiles <= 8 and K < 1024:                          # a few microseconds either way: 256 x 896 x 896 6.5 / 6.7
         return False
     pairs = sms // 2
     last = tiles % pairs
     pair = tiles // pairs + (0.0 if last == 0 else 0.4 if last * 4 <= pairs else 0.57 if last * 2 <= pairs else 1.0)
+    ctas, bn = {n: rows * -(-N // n) for n in (256, 128, 64, 32)}, 256
+    for n in (128, 64, 32):                              # as the kernel does
+        if -(-ctas[n] // sms) * (400 + n) < -(-ctas[bn] // sms) * (400 + bn):
+            bn = n
+    if bn < 256 and ctas[bn] <= sms and ((bn <= 64 and K <= 512) or pair >= 1.18 * (400 + bn) / 656):
+        return False
     rest = single % sms
     return pair < 1.18 * (single // sms) + (0.0 if rest == 0 else 0.85 if rest * 2 <= sms else 1.18)
 
