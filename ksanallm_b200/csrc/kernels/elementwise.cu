@@ -21,6 +21,7 @@
 #include <stdint.h>
 #include "fp8_scale.cuh"
 #include "fast_div.cuh"
+#define KSANA_F32X2_FLUSH          // as this file's arithmetic on single floats: a row's bits do not depend on the kernel that a launch takes
 #include "f32x2.cuh"
 #include "vec8.cuh"
 
