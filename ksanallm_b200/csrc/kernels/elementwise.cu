@@ -878,12 +878,12 @@ static inline int launch_vectors(long long total, bool gated) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   return gated || total <= sms * 2048LL ? 1 : 2;
 }
-// launches of more 16-byte vectors than threads fit the machine at once
-static inline bool chunks_pay(long long total) {
+// launches of more 16-byte vectors than threads fit the machine at once (or than `per_sm` for every SM)
+static inline bool chunks_pay(long long total, int per_sm = 2048) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return total > sms * 2048LL;
+  return total > static_cast<long long>(sms) * per_sm;
 }
 static inline int norm_threads(int H) {
   int t = ((H >> 3) + kMaxVec - 1) / kMaxVec;
@@ -1024,7 +1024,10 @@ extern "C" int ksana_act_mul(const void* in, void* out, void* outq, float* oscal
     uint8_t* dq = outq ? (uint8_t*)outq + static_cast<size_t>(m0) * I : nullptr;
     float* ds = oscale ? oscale + m0 : nullptr;
     const int* tr = tile_rows ? tile_rows + m0 / 128 : nullptr;
-    if (chunks_pay(total) && gated && I % 16 == 0 && in_ld % 16 == 0 &&
+    // Half as many threads with twice the work each gain where there are enough of them. us, vectors / chunks, on 148 SMs: not quantised
+    // 307200 vectors 2.4 / 2.8 (gelu 2.9 / 3.6), 409600 2.9 / 3.0 (3.7 / 3.9), 465920 3.1 / 3.0 (4.0 / 3.9), 537600 3.5 / 3.0; quantised
+    // 307200 3.2 / 3.2 (gelu 3.75 / 4.2), 332800 3.5 / 3.3 (4.1 / 4.3), 358400 3.8 / 3.3 (4.5 / 4.4).
+    if (chunks_pay(total, !dq ? 3200 : act == 1 ? 2368 : 2048) && gated && I % 16 == 0 && in_ld % 16 == 0 &&
         !((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(dq)) & 31)) {
       const FastDiv by = make_fast_div(I / 16);
       const dim3 chunk_grid(grid_for(total / 2, 256));
