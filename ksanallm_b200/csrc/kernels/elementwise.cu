@@ -1134,8 +1134,14 @@ extern "C" int ksana_rope_kv_append(void* qkv, const int* positions, int pos_str
   if (neox && rot_dim == D && (D % 16) == 0 && pos_stride == 0 && (block_stride % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(qkv) % 16) == 0 && (reinterpret_cast<uintptr_t>(cache) % 16) == 0 &&
       (reinterpret_cast<uintptr_t>(cos_sin) % 16) == 0) {
-    // as many threads as leave none idle in the last turn: 48 heads of 128 are 384 items, two turns of 192
-    const int items = (Hq + 2 * Hkv) * (D >> 4), turns = (items + 255) / 256, threads = ((items + turns - 1) / turns + 31) / 32 * 32;
+    // as many threads as leave none idle in the last turn: 48 heads of 128 are 384 items, two turns of 192. Few rows spare themselves a turn
+    // that would hold a quarter of the threads: 36 heads, 64 rows 2.5 us in two turns of 160, 2.2 in one of 288 (1000 rows 4.7 / 4.6, but
+    // 4000 11.3 / 12.8)
+    int dev = 0, sms = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    const int items = (Hq + 2 * Hkv) * (D >> 4), full = (items + (T <= 8 * sms ? 191 : 255)) / 256, turns = full > 1 ? full : 1;
+    const int threads = ((items + turns - 1) / turns + 31) / 32 * 32;
     if (cache_fp8)
       launch_early(rope_kv_append_vec_kernel<uint8_t>, dim3(T), dim3(threads), 0, st, (bf16*)qkv, positions, slots, cos_sin, (uint8_t*)cache,
                                                             block_stride, block_tokens, Hq, Hkv, D, 1.f / k_scale,
