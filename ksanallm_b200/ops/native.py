@@ -339,8 +339,9 @@ def _pair_wins(M, N, K, sms=148):
     one wave (the kernel picks them by 400 + columns), that takes less: 128 columns 23 us; and with 32 or 64 columns and a short K what a
     pair costs beside its products, about a microsecond, is not made up for. us, single / pair: 700 x 28672 143 / 127, 200 x 4096 18.1 /
     13.4, 513 x 4096 28.7 / 25.4; and where single CTAs stay: 300 x 6144 21.0 / 25.2, 1100 x 4096 29.5 / 34.5, 513 x 28672 117 / 121, 2048 x
-    1152 22.3 / 26.0 (K = 14336: 61 / 76); K = 512: 384 x 1152 5.7 / 6.5, 1024 x 1152 6.5 / 7.1, but 384 x 4096 (128 columns) 8.4 / 7.4. Of
-    1080 shapes (136 to 5000 rows, 256 to 28672 columns, K of 128 to 14336) two take the slower kernel by 4 and 7 percent."""
+    1152 22.3 / 26.0 (K = 14336: 61 / 76); K = 512: 384 x 1152 5.7 / 6.5, 1024 x 1152 6.5 / 7.1, but 384 x 4096 (128 columns) 8.4 / 7.4; K no
+    multiple of 16: 597 x 824 x 1336 9.1 / 10.6, 341 x 328 x 3704 17.3 / 19.2, 314 x 2712 x 664 8.3 / 9.9. Of 1080 shapes (136
+    to 5000 rows, 256 to 28672 columns, K of 128 to 14336) two take the slower kernel by 4 and 7 percent."""
     if N < 256 or N % 8 or K % 8:
         return False
     cols, rows = -(-N // 256), -(-M // 128)
@@ -354,7 +355,9 @@ def _pair_wins(M, N, K, sms=148):
     for n in (128, 64, 32):                              # as the kernel does
         if -(-ctas[n] // sms) * (400 + n) < -(-ctas[bn] // sms) * (400 + bn):
             bn = n
-    if bn < 256 and ctas[bn] <= sms and ((bn <= 64 and K <= 512) or pair >= 1.18 * (400 + bn) / 656):
+    halves = K % 16 != 0                                 # rows that start inside a sector
+    if bn < 256 and ctas[bn] <= sms and ((bn <= 64 and K <= (1024 if halves else 512)) or (bn == 32 and halves)
+                                         or pair >= 1.18 * (400 + bn) / 656):
         return False
     rest = single % sms
     return pair < 1.18 * (single // sms) + (0.0 if rest == 0 else 0.85 if rest * 2 <= sms else 1.18)
