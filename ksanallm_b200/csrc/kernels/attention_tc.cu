@@ -244,7 +244,9 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     for (int j = 0; j < ntiles; ++j) {
       const uint32_t par = j & 1;
       const int t0 = tile_start(j), c0 = t0 + cb;          // first position of the tile, of this half
-      if (ok) ok = mbar_wait_all(s_full, par, abort_flag);
+      // by every lane for itself: what follows does not depend on the answer, and a vote of the warp costs 0.2 us a tile (8 prompts of 100
+      // tokens, 32/8 heads, 13.5 us with it, 12.7 without)
+      if (ok) ok = mbar_wait(s_full, par, abort_flag);
       tc_fence_after();
       const bool biased = slope2 != 0.f || p.scale_log2 <= 0.f;
       const bool need_mask = (c0 + 63 > limit) || (WIN && c0 < lo && c0 + 64 > keep);
@@ -352,7 +354,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
         // last tile of the sequence: V rows past the sequence end hold stale shared memory or whatever the cache
         // has there; their probabilities are 0, but 0 x NaN would poison O. Zero them before the PV MMA reads.
         // (the keys' product is complete here, so a shared tile is free to be changed)
-        if (!p.shared && ok) ok = mbar_wait_all(v_full, par, abort_flag);
+        if (!p.shared && ok) ok = mbar_wait(v_full, par, abort_flag);
         uint8_t* vt = p.shared && !(j & 1) ? k_s : v_s;
         const int first_bad = kv_len - t0;
         const int nchunks = ok ? (kFaTile - first_bad) * 16 : 0;       // 16-byte chunks per row: 2 panels x 8
@@ -370,7 +372,7 @@ prefill_tc_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_consta
     pair_sync();                                           // the last tile's maxima have been read
     row_s[half * 128 + rl] = l;
     pair_sync();
-    if (ok && mbar_wait_all(o_full, 0, abort_flag)) {
+    if (__all_sync(0xffffffffu, ok && mbar_wait(o_full, 0, abort_flag))) {
       tc_fence_after();
       float lt = row_s[rl] + row_s[128 + rl];
       if (p.sinks && active) lt += exp2f(p.sinks[head] * 1.44269504f - m_used);
