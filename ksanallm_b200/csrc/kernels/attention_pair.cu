@@ -33,7 +33,7 @@ constexpr float kPaRescaleLog2 = 8.f;           // O is rescaled only when a row
 template <int KP>
 struct PairCfg {                                // KP: 64-column panels of queries and keys
   // Keys per tile: what a tile costs beside its keys (two TMEM round trips, the exchange of the maxima, the hand-offs to and from the
-  // MMA thread) counts half as much with 128; three panels leave room for tiles of 64 only.
+  // MMA warp) counts half as much with 128; three panels leave room for tiles of 64 only.
   static constexpr int kTok = KP == 3 ? 64 : 128;
   static constexpr int kStages = KP == 3 ? 3 : 2;             // of keys and of values
   static constexpr int kBufs = KP == 3 ? 2 : 1;               // tiles of S per group: tiles of 64 keys leave room for a second one
@@ -341,8 +341,7 @@ prefill_pair_kernel(const __grid_constant__ CUtensorMap q_map, const __grid_cons
         pair_sync();                                       // ... and both halves of S are in registers: P may be written over it
         mx = fmaxf(mx, other[buf * 512]);
         if (!__any_sync(0xffffffffu, mx > m_used + kPaRescaleLog2)) {
-          clear_values();
-          hand_over(0);
+          hand_over(0);                                      // (no key past kv_len: such a tile is masked)
           if constexpr (PARTS > 1) {
             weights(1, mref);
             hand_over(1);

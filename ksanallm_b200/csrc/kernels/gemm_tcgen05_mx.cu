@@ -232,7 +232,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
     // The scale values of the next two groups are already on their way (plain loads whose results are not
     // touched until their turn) while the warp waits for the buffer of the current group: under the load of
     // the operand stream a group's loads take longer than its four K blocks of MMAs, so fetching on demand
-    // starves the MMA thread. Three register sets rotate by name, not by index, so that no load result is
+    // starves the MMA warp. Three register sets rotate by name, not by index, so that no load result is
     // moved (a move would wait for it).
     int sfs = 0; uint32_t sf_phase = 0;
     const int n_blocks = (p.N + 127) / 128;

@@ -15,7 +15,7 @@
 //   * each CTA's scale warp packs the exponent bytes of its own 128 rows and of all 256 columns into the chunk
 //     layout of gemm_tcgen05_mx.cu in its OWN shared memory and arrives on the leader's "scales full" barrier;
 //     the leader's tcgen05.cp.cta_group::2 then copies each CTA's chunks into that CTA's TMEM;
-//   * the leader's MMA thread issues the pair MMAs; commits release the stage and the scale buffer in both CTAs
+//   * the leader's MMA warp issues the pair MMAs; commits release the stage and the scale buffer in both CTAs
 //     and publish the accumulator to both CTAs' epilogue warps;
 //   * epilogue warps of both CTAs drain their own 128 TMEM lanes into registers and arrive on the leader's
 //     "accumulator empty" barrier (remote arrive), then store;
@@ -238,7 +238,7 @@ gemm_mxfp8_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_c
     // The scale values of the next two groups are already on their way (plain loads whose results are not
     // touched until their turn) while the warp waits for the buffer of the current group: under the load of
     // the operand stream a group's loads take longer than its four K blocks of MMAs, so fetching on demand
-    // starves the MMA thread. Three register sets rotate by name, not by index, so that no load result is
+    // starves the MMA warp. Three register sets rotate by name, not by index, so that no load result is
     // moved (a move would wait for it).
     int sfs = 0; uint32_t sf_phase = 0;
     const int n_blocks = (p.N + 127) / 128;

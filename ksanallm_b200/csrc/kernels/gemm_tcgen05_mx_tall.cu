@@ -5,7 +5,7 @@
 // Operands and restrictions are those of gemm_tcgen05_mx.cu (e4m3 values, power-of-two scales: one per activation
 // row and 128 K-elements stored [K/128][ld], one per 128 x 128 weight block). That kernel's 128 x 256 tile needs
 // 48 KB of operands per 128-deep K block, and what an SM can take in per clock from L2 (about 60 bytes, measured:
-// the producer's ring stays full while the MMA thread waits for data) then holds the tensor pipe below 60 %.
+// the producer's ring stays full while the MMA warp waits for data) then holds the tensor pipe below 60 %.
 // A 256 x 224 tile needs 60 KB per K block for 1.75 times the MMA work (34 KB per 128 x 256 equivalent). It is
 // the largest tile whose two fp32 accumulators (2 x 224 TMEM columns) leave room for the scale columns. No
 // cluster, no multicast. Every wait is bounded. The MMA warp issues by predicate, as a whole (behind a branch the eight MMAs of a K block

@@ -53,7 +53,6 @@ struct F4Params {
   const __nv_bfloat16* residual; int ldr;
   const float* a_ts; const float* w_ts;    // per-tensor scales (device scalars)
   int* err;
-  __nv_bfloat16* push[8]; int push_n; int push_rows;
   int wide;                                  // rows of D start on 32-byte boundaries
   // grouped (mixture-of-experts) mode: row tile i multiplies with expert tile_expert[i] (< 0: tile unused); W, w_bs
   // are the experts' matrices stacked along N (expert_rows rows each) and w_ts holds one tensor scale per expert
@@ -279,13 +278,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_consta
           for (int i = 0; i < 4; ++i) o2[i] = __floats2bfloat162_rn(o[2 * i], o[2 * i + 1]);
         }
         if (p.out_f32 || col0 >= p.N) continue;
-        __nv_bfloat16* dst;
-        if (p.push_n) {
-          const int owner = min(row / p.push_rows, p.push_n - 1);
-          dst = p.push[owner] + static_cast<size_t>(row - owner * p.push_rows) * p.ldd + col0;
-        } else {
-          dst = p.D + static_cast<size_t>(row) * p.ldd + col0;
-        }
+        __nv_bfloat16* dst = p.D + static_cast<size_t>(row) * p.ldd + col0;
         if (p.wide && col0 + 16 <= p.N) {
           st_global_32(dst, ov[0], ov[1]);
         } else {

@@ -14,8 +14,8 @@
 // Protocol (cluster of 2 CTAs, rank 0 = leader):
 //   * each CTA's producer thread loads its A rows and its W half with TMA (cta_group::2 form, no
 //     multicast); both CTAs' loads complete on the LEADER's "full" barrier (expect-tx = bytes of both);
-//   * the leader's MMA thread issues the pair MMA; a commit per CTA releases the stage ("empty") in
-//     each CTA and publishes accumulator stages ("tmem full") to each CTA's epilogue warps;
+//   * the leader's MMA warp issues the pair MMA; one commit, which arrives in both CTAs, releases the stage ("empty") in
+//     each and publishes accumulator stages ("tmem full") to each CTA's epilogue warps;
 //   * epilogue warps of both CTAs read their own 128 TMEM lanes; FP8: promote each 128-deep K block
 //     with the fp32 scale product; they arrive on the leader's "tmem empty" barrier (remote arrive);
 //   * cluster barriers bracket the kernel so that no CTA leaves while its peer may still touch its
