@@ -127,7 +127,9 @@ class DeepseekModel(CommonModel):
         row: 50 ns per cached token against 143 ns per row at 128 heads. Neither is faster than one CTA's walk over the longest
         sequence, 2.1 and 2.4 us per 64 keys, which is all the absorbed form takes while its CTAs (two per 128 rows and heads) run at once;
         the expansion of 65 to 128 tokens takes 10 us more than its share, by the GEMM for so many rows. us expanded / absorbed: 16 heads, 128
-        tokens 38 / 28, 200 on 3800 cached 185 / 166, 1000 on 11000 498 / 848; 128 heads, 200 on 3800 404 / 502, 64 on 1936 220 / 115."""
+        tokens 38 / 28, 200 on 3800 cached 185 / 166, 1000 on 11000 498 / 848; 128 heads, 200 on 3800 404 / 502, 64 on 1936 220 / 115.
+        These rates and times, and with them the line, are those of both forms when one lane issued their MMAs; the absorbed kernel takes
+        0.5 to 0.8 of its time since then, the expanded attention 0.7, the expansion's GEMM 0.7."""
         from ..ops import native
         if (mw.kv_b is None or step.num_single or not step.pairs or (self.nope, self.rope, self.vdim, self.lora) != (128, 64, 128, 512)
                 or step.total_kv_len * self.Hq * 512 > 4 << 30):

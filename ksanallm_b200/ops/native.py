@@ -411,9 +411,12 @@ MX_TALL_MIN_M = 512                # 256 x 224-tile hardware-scaled kernel from 
 
 
 def _tall_wins(M, N, K, max_ctas=0, sms=148):
-    """256 x 224 tiles against 128 x 256 tiles for one problem, from measured behaviour: the tall tile does 1.75
-    times the MMA work at about 1.18 times the rate but cannot overlap its accumulator drain (about three K
-    blocks of time per tile), so it needs a long K and a tile count that fills its last wave."""
+    """256 x 224 tiles against 128 x 256 tiles for one problem: the tall tile does 1.75 times the MMA work at about 1.18 times the rate, and
+    its accumulators are drained (about three K blocks of time per tile where something is added to the result) before the next tile's
+    products, so that a long K and a tile count that fills its last wave favour it. The constants are those of both kernels when one lane
+    issued their MMAs. As they are now, the tall tile is the faster one on the other side of this line as well: us, tall / 128-row, 768 x 7168
+    x 16384 85 / 106, 512 x 10240 x 8192 49 / 59, 4000 x 28672 x 2048 219 / 245, 2000 x 24576 x 1536 70 / 80; and once not where the line
+    has it: 3000 x 4096 x 14336 195 / 182."""
     if K < 4096:
         return False
     ctas = min(sms, max_ctas) if max_ctas > 0 else sms
@@ -461,11 +464,13 @@ def gemm_mxfp8_pair(xq, xs, wq, ws, out=None, bias=None, residual=None, out_f32=
 
 
 def _skinny_wins_mx(M, N, K, sms=148):
-    """Rows 33..128 with tensor-core-applied scales: skinny stream-K kernel or tiled kernel, from their measured
+    """Rows 33..128 with tensor-core-applied scales: skinny stream-K kernel or tiled kernel, from their
     behaviour in CUDA graphs of decode steps (microseconds). Tiled: about 6.5 + 0.37 per 128-deep K block and wave of
     128 x 128 tiles (0.69 with 128 x 256 tiles); one CTA walks the whole K range of its tile, so few tiles leave
     SMs idle. Skinny: the (tile, K block) units are spread evenly over the SMs at about 0.62 per K block and CTA for 64
-    rows (0.9 for 128), plus a higher fixed cost and the cross-CTA reduction of cut tiles."""
+    rows (0.9 for 128), plus a higher fixed cost and the cross-CTA reduction of cut tiles. The tiled kernel's figures date from when one
+    lane issued its MMAs; it is faster now (128 x 8192 x 8192 32 -> 23), and the line gives the skinny one too much: 65 to 128 rows of 1536
+    and 2112 x 7168 take 25 to 30 us there and 19 on the tiled kernel."""
     kb = K // 128
     t128 = (N + 127) // 128
     t256 = (N + 255) // 256
